@@ -50,6 +50,48 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m_tiles, int num_n
     tn = in_group / rows_in_group;
 }
 
+// Rows sorted by expert (sparse mixtures): what the GEMM kernel's SEG variants and the kernels that sort the rows agree on.
+enum { kSegOff = 0, kSegPlain = 1, kSegGlu = 2, kSegRelu2 = 3 };
+constexpr int kSegMaxExperts = 128;
+constexpr int kSegSmemBytes = 2 * (kSegMaxExperts + 1) * 4;
+constexpr int kSegAlign = 32;   // an expert's rows start at a multiple: the 32 rows of an epilogue warp's store
+
+struct SegArgs {
+    const int* counts;                // [E] rows per expert
+    float limit, alpha, up_shift;     // of the gated activation
+    __device__ __forceinline__ float glu(float g, float u) const {
+        g = fminf(g, limit);
+        u = fminf(fmaxf(u, -limit), limit);
+        return g / (1.f + expf(-alpha * g)) * (u + up_shift);
+    }
+};
+
+// One warp: first row and (for num_n_tiles > 0) first tile of every expert; entry E holds the totals.
+__device__ __forceinline__ void segment_starts(const int* counts, int E, int num_n_tiles, int* row, int* tile) {
+    const int lane = threadIdx.x & 31;
+    int rows = 0, tiles = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+        const int n = e0 + lane < E ? counts[e0 + lane] : 0;
+        const int r = (n + kSegAlign - 1) / kSegAlign * kSegAlign, t = (n + kTileM - 1) / kTileM * num_n_tiles;
+        int rs = r, ts = t;           // inclusive sums over the lanes
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int a = __shfl_up_sync(0xffffffffu, rs, o), b = __shfl_up_sync(0xffffffffu, ts, o);
+            if (lane >= o) rs += a, ts += b;
+        }
+        if (e0 + lane < E) {
+            row[e0 + lane] = rows + rs - r;
+            if (tile != nullptr) tile[e0 + lane] = tiles + ts - t;
+        }
+        rows += __shfl_sync(0xffffffffu, rs, 31);
+        tiles += __shfl_sync(0xffffffffu, ts, 31);
+    }
+    if (lane == 0) {
+        row[E] = rows;
+        if (tile != nullptr) tile[E] = tiles;
+    }
+}
+
 // 2-D tensor map: `inner` contiguous elements, `outer` rows with pitch `pitch_elems`;
 // box = {box_inner, box_outer}; SWIZZLE_128B (box_inner * elem_bytes must be 128 B).  elem_bytes 2 = bf16, 4 = fp32.
 int make_tmap_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t pitch_elems,

@@ -14,6 +14,7 @@
 //   expert index >= E means an identity expert: its output is the token's input itself
 // Expert weights are stored [E, in, out] (the layout of the grouped expert layers), gate | up fused on the out dim.
 #include "common.cuh"
+#include "gemm_tcgen05.cuh"
 
 namespace {
 
@@ -42,45 +43,52 @@ __device__ __forceinline__ float glu_act(float g, float u, float limit, float al
 }
 
 // ---- router ---------------------------------------------------------------------------------------------------------
-constexpr int RT_WARPS = 4, RT_GROUP = 8;
+constexpr int RT_WARPS = 4;
 
-template <typename T>
-__global__ void __launch_bounds__(RT_WARPS * 32)
-moe_router_kernel(const T* __restrict__ h, const float* __restrict__ wr, const float* __restrict__ corr,
-                  const float* __restrict__ wsg, int* __restrict__ idx, float* __restrict__ wts,
-                  float* __restrict__ sgate, long long N, int W, int R, int top, float out_scale,
-                  const float* __restrict__ zbias, int mode) {
-    extern __shared__ float smem[];
+// 8 consecutive values of a row
+__device__ __forceinline__ void ld8(const float* p, float* f) {
+    *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(p);
+    *reinterpret_cast<float4*>(f + 4) = *reinterpret_cast<const float4*>(p + 4);
+}
+__device__ __forceinline__ void ld8(const bf16* p, float* f) { unpack8(*reinterpret_cast<const bf16x8*>(p), f); }
+
+// acc[t][i] += <h row t, wr row i> over the columns of this lane.  V = 8: 16- / 32-byte loads (W a multiple of 8, aligned
+// rows); V = 1: any W.  Rows past nt / nr repeat the last one (their sums are not used).
+template <typename T, int V, int TOK, int G>
+__device__ __forceinline__ void router_dots(const T* h, const float* wr, int W, int nt, int nr, float (&acc)[TOK][G]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int t = 0; t < TOK; ++t)
+#pragma unroll
+        for (int i = 0; i < G; ++i) acc[t][i] = 0.f;
+#pragma unroll (TOK == 1 ? 2 : 1)
+    for (int c = lane * V; c < W; c += 32 * V) {
+        float hv[TOK][V];
+#pragma unroll
+        for (int t = 0; t < TOK; ++t) {
+            const T* p = h + (long long)min(t, nt - 1) * W + c;
+            if constexpr (V == 8) ld8(p, hv[t]);
+            else hv[t][0] = ldf(p);
+        }
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+            const float* p = wr + (long long)min(i, nr - 1) * W + c;
+            float wv[V];
+            if constexpr (V == 8) ld8(p, wv);
+            else wv[0] = *p;
+#pragma unroll
+            for (int t = 0; t < TOK; ++t)
+#pragma unroll
+                for (int j = 0; j < V; ++j) acc[t][i] = fmaf(hv[t][j], wv[j], acc[t][i]);
+        }
+    }
+}
+
+// One warp: scores and choice of token n from its logits ps [R]; cs [R]: scratch (choice scores).
+__device__ __forceinline__ void router_select(float* ps, float* cs, const float* corr, int* idx, float* wts, long long n, int R,
+                                              int top, float out_scale, int mode) {
     const bool renorm = mode == 1;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float* ps = smem + (long long)warp * 2 * R;     // probabilities
-    float* cs = ps + R;                             // choice scores
-    const long long n = (long long)blockIdx.x * RT_WARPS + warp;
-    if (n >= N) return;
-    const T* hr = h + n * W;
-    for (int r0 = 0; r0 < R; r0 += RT_GROUP) {
-        float acc[RT_GROUP];
-#pragma unroll
-        for (int i = 0; i < RT_GROUP; ++i) acc[i] = 0.f;
-        for (int c = lane; c < W; c += 32) {
-            const float hv = ldf(hr + c);
-#pragma unroll
-            for (int i = 0; i < RT_GROUP; ++i)
-                if (r0 + i < R) acc[i] = fmaf(hv, wr[(long long)(r0 + i) * W + c], acc[i]);
-        }
-#pragma unroll
-        for (int i = 0; i < RT_GROUP; ++i) {
-            const float z = warp_sum(acc[i]);
-            if (lane == 0 && r0 + i < R) ps[r0 + i] = z + (zbias != nullptr ? zbias[r0 + i] : 0.f);
-        }
-    }
-    if (wsg != nullptr && sgate != nullptr) {
-        float a = 0.f;
-        for (int c = lane; c < W; c += 32) a = fmaf(ldf(hr + c), wsg[c], a);
-        a = warp_sum(a);
-        if (lane == 0) sgate[n] = 1.f / (1.f + expf(-a));
-    }
-    __syncwarp();
+    const int lane = threadIdx.x & 31;
     if (renorm) {                // the choice is made on the logits themselves
         for (int r = lane; r < R; r += 32) cs[r] = ps[r];
     } else if (mode == 2) {      // independent sigmoid scores
@@ -148,6 +156,55 @@ moe_router_kernel(const T* __restrict__ h, const float* __restrict__ wr, const f
         }
         const float inv = out_scale / sum;
         for (int k = 0; k < top; ++k) wts[n * top + k] *= inv;
+    }
+}
+
+// A CTA of RT_WARPS warps.  TOK == 1: one token, the warps share its experts (few tokens: the latency of one token counts).
+// TOK > 1: every warp takes TOK tokens and all experts, so a row of wr that is loaded serves TOK tokens (many tokens: the
+// fp32 rows of wr come from L1 / L2 and are the larger operand). 
+template <typename T, int V, int TOK>
+__global__ void __launch_bounds__(RT_WARPS * 32)
+moe_router_kernel(const T* __restrict__ h, const float* __restrict__ wr, const float* __restrict__ corr,
+                  const float* __restrict__ wsg, int* __restrict__ idx, float* __restrict__ wts,
+                  float* __restrict__ sgate, long long N, int W, int R, int top, float out_scale,
+                  const float* __restrict__ zbias, int mode) {
+    extern __shared__ float smem[];
+    constexpr int G = TOK == 1 ? 4 : 8;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long n0 = TOK == 1 ? blockIdx.x : ((long long)blockIdx.x * RT_WARPS + warp) * TOK;
+    if (n0 >= N) return;                            // TOK == 1: never; else whole warps, which share nothing
+    const int nt = (int)min((long long)TOK, N - n0);
+    float* ps = smem + (TOK == 1 ? 0 : warp * (TOK + 1) * R);       // logits [TOK][R], then scratch [R]
+    const T* hr = h + n0 * W;
+    for (int r0 = TOK == 1 ? warp * G : 0; r0 < R; r0 += TOK == 1 ? RT_WARPS * G : G) {
+        float acc[TOK][G];
+        router_dots<T, V, TOK, G>(hr, wr + (long long)r0 * W, W, nt, R - r0, acc);
+#pragma unroll
+        for (int t = 0; t < TOK; ++t)
+#pragma unroll
+            for (int i = 0; i < G; ++i) {
+                const float z = warp_sum(acc[t][i]);
+                if (lane == 0 && r0 + i < R) ps[t * R + r0 + i] = z + (zbias != nullptr ? zbias[r0 + i] : 0.f);
+            }
+    }
+    if (wsg != nullptr && sgate != nullptr && (TOK > 1 || warp == RT_WARPS - 1)) {
+        float acc[TOK][1];
+        router_dots<T, V, TOK, 1>(hr, wsg, W, nt, 1, acc);
+#pragma unroll
+        for (int t = 0; t < TOK; ++t) {
+            const float z = warp_sum(acc[t][0]);
+            if (lane == 0 && t < nt) sgate[n0 + t] = 1.f / (1.f + expf(-z));
+        }
+    }
+    if constexpr (TOK == 1) {
+        __syncthreads();
+        if (warp == 0) router_select(ps, ps + R, corr, idx, wts, n0, R, top, out_scale, mode);
+    } else {
+        __syncwarp();
+        for (int t = 0; t < nt; ++t) {
+            router_select(ps + t * R, ps + TOK * R, corr, idx, wts, n0 + t, R, top, out_scale, mode);
+            __syncwarp();
+        }
     }
 }
 
@@ -401,22 +458,104 @@ __global__ void glu_bias_vec_kernel(const bf16* __restrict__ src, long long ld, 
     }
 }
 
-template <typename T>
+// Bound by memory.  V = 8: a thread takes 8 consecutive columns (16-byte loads of bf16 rows, W a multiple of 8, aligned
+// rows); V = 1: any W.  8190 tokens x 2048, top 2 (134 MB): 61 us with one column per thread, 24 us (5.6 TB/s).
+template <typename T, int V>
 __global__ void moe_gather_combine_kernel(const T* __restrict__ ys, const int* __restrict__ slot,
                                           const int* __restrict__ idx, const float* __restrict__ wts,
                                           const T* __restrict__ h, const T* __restrict__ shared_out,
                                           const float* __restrict__ sgate, float* __restrict__ y, int top, int W, int E) {
     const long long t = blockIdx.x;
-    for (int c = threadIdx.x; c < W; c += blockDim.x) {
-        float a = 0.f;
+    for (int c = threadIdx.x * V; c < W; c += blockDim.x * V) {
+        float a[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) a[i] = 0.f;
+        auto add = [&](const T* row, float wgt) {
+            float v[V];
+            if constexpr (V == 8) ld8(row + c, v);
+            else v[0] = ldf(row + c);
+#pragma unroll
+            for (int i = 0; i < V; ++i) a[i] = fmaf(wgt, v[i], a[i]);
+        };
         for (int j = 0; j < top; ++j) {
             const int e = idx[t * top + j];
-            const float wgt = wts[t * top + j];
-            const float v = (e < 0 || e >= E) ? ldf(h + t * W + c) : ldf(ys + (long long)slot[t * top + j] * W + c);
-            a = fmaf(wgt, v, a);
+            add((e < 0 || e >= E) ? h + t * W : ys + (long long)slot[t * top + j] * W, wts[t * top + j]);
         }
-        if (shared_out != nullptr) a = fmaf(sgate != nullptr ? sgate[t] : 1.f, ldf(shared_out + t * W + c), a);
-        y[t * W + c] = a;
+        if (shared_out != nullptr) add(shared_out + t * W, sgate != nullptr ? sgate[t] : 1.f);
+        if constexpr (V == 8) {
+            float4* dst = reinterpret_cast<float4*>(y + t * W + c);
+            dst[0] = make_float4(a[0], a[1], a[2], a[3]);
+            dst[1] = make_float4(a[4], a[5], a[6], a[7]);
+        } else {
+            y[t * W + c] = a[0];
+        }
+    }
+}
+
+// ---- rows sorted by expert, without a host read ---------------------------------------------------------------------------
+// count: how many pairs chose every expert, and every pair's place among its expert's pairs (in no particular order: a row's
+// result does not depend on its place).  gather: expert e's rows start where segment_starts (gemm_tcgen05.cuh) says, which the
+// grouped product works out the same way; a warp copies one pair's input row there (8190 tokens x 2048, top 2: 24 us for
+// 134 MB; a host-side argsort, bincount and index before: 50 us of GPU time and two waits for the device).
+constexpr int CNT_THREADS = 256, CNT_PAIRS = 2048;      // pairs per block
+
+__global__ void __launch_bounds__(CNT_THREADS)
+moe_count_kernel(const int* __restrict__ idx, int* __restrict__ counts, int* __restrict__ place, long long P, int E) {
+    extern __shared__ int hist[];                       // [E] pairs of this block, then [E] the block's first place
+    int* first = hist + E;
+    for (int e = threadIdx.x; e < E; e += CNT_THREADS) hist[e] = 0;
+    __syncthreads();
+    const long long p0 = (long long)blockIdx.x * CNT_PAIRS;
+    int mine[CNT_PAIRS / CNT_THREADS];
+#pragma unroll
+    for (int i = 0; i < CNT_PAIRS / CNT_THREADS; ++i) {
+        const long long p = p0 + i * CNT_THREADS + threadIdx.x;
+        const int e = p < P ? idx[p] : -1;
+        mine[i] = e >= 0 && e < E ? atomicAdd(hist + e, 1) : 0;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += CNT_THREADS) first[e] = hist[e] > 0 ? atomicAdd(counts + e, hist[e]) : 0;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < CNT_PAIRS / CNT_THREADS; ++i) {
+        const long long p = p0 + i * CNT_THREADS + threadIdx.x;
+        const int e = p < P ? idx[p] : -1;
+        if (e >= 0 && e < E) place[p] = first[e] + mine[i];
+    }
+}
+
+constexpr int GA_WARPS = 8;
+
+// slot [P] (in: place, out: row of the pair); x [rows, W] <- h[p / top] (times in_scale[p], rounded)
+__global__ void __launch_bounds__(GA_WARPS * 32)
+moe_gather_rows_kernel(const bf16* __restrict__ h, const int* __restrict__ idx, const int* __restrict__ counts,
+                       int* __restrict__ slot, const float* __restrict__ in_scale, bf16* __restrict__ x, long long P, int top,
+                       int W8, int E) {
+    __shared__ int row0[nxd_gemm::kSegMaxExperts + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp == 0) nxd_gemm::segment_starts(counts, E, 0, row0, nullptr);
+    __syncthreads();
+    const long long p = (long long)blockIdx.x * GA_WARPS + warp;
+    if (p >= P) return;
+    const int e = idx[p];
+    if (e < 0 || e >= E) return;                        // identity expert: the combination reads h itself
+    const int row = row0[e] + slot[p];
+    __syncwarp();                                       // every lane has read the place
+    if (lane == 0) slot[p] = row;
+    const bf16x8* src = reinterpret_cast<const bf16x8*>(h) + p / top * W8;
+    bf16x8* dst = reinterpret_cast<bf16x8*>(x) + (long long)row * W8;
+    if (in_scale == nullptr) {
+#pragma unroll 4
+        for (int c = lane; c < W8; c += 32) dst[c] = src[c];
+    } else {
+        const float s = in_scale[p];
+        for (int c = lane; c < W8; c += 32) {
+            float v[8];
+            unpack8(src[c], v);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] *= s;
+            dst[c] = pack8(v);
+        }
     }
 }
 
@@ -430,17 +569,44 @@ NXD_API int nxd_moe_router(int dtype, const void* h, const float* wr, const floa
                            const float* zbias, int mode, void* stream) {
     if (N == 0) return 0;
     NXD_REQUIRE(top >= 1 && top <= R, "router: top %d of %d", top, R);
-    const size_t smem = (size_t)RT_WARPS * 2 * R * sizeof(float);
-    NXD_REQUIRE(smem <= 48 * 1024, "router: %d outputs", R);
-    const unsigned blocks = (unsigned)((N + RT_WARPS - 1) / RT_WARPS);
-    if (dtype == 0)
-        moe_router_kernel<bf16><<<blocks, RT_WARPS * 32, smem, (cudaStream_t)stream>>>((const bf16*)h, wr, corr, wsg, idx,
-                                                                                      wts, sgate, N, W, R, top, out_scale,
-                                                                                      zbias, mode);
-    else
-        moe_router_kernel<float><<<blocks, RT_WARPS * 32, smem, (cudaStream_t)stream>>>((const float*)h, wr, corr, wsg,
-                                                                                       idx, wts, sgate, N, W, R, top,
-                                                                                       out_scale, zbias, mode);
+    NXD_REQUIRE((size_t)8 * R * sizeof(float) <= 48 * 1024, "router: %d outputs", R);
+    // one token per CTA while the tokens are too few to fill the chip with a warp per 4 tokens (or the logits of 16 tokens
+    // do not fit shared memory)
+    const bool single = N < 16ll * nxd_num_sms() || (size_t)RT_WARPS * 5 * R * sizeof(float) > 48 * 1024;
+    const size_t smem = (size_t)(single ? 2 : RT_WARPS * 5) * R * sizeof(float);
+    const bool vec = W % 8 == 0 && ((uintptr_t)h % 16) == 0 && ((uintptr_t)wr % 16) == 0 && ((uintptr_t)wsg % 16) == 0;
+    const unsigned blocks = (unsigned)(single ? N : (N + RT_WARPS * 4 - 1) / (RT_WARPS * 4));
+#define NXD_RT(T, V, TOK)                                                                                               \
+    moe_router_kernel<T, V, TOK><<<blocks, RT_WARPS * 32, smem, (cudaStream_t)stream>>>(                                \
+        (const T*)h, wr, corr, wsg, idx, wts, sgate, N, W, R, top, out_scale, zbias, mode)
+#define NXD_RT_V(T, V)                                                                                                  \
+    do {                                                                                                                \
+        if (single) NXD_RT(T, V, 1); else NXD_RT(T, V, 4);                                                              \
+    } while (0)
+    if (dtype == 0) {
+        if (vec) NXD_RT_V(bf16, 8); else NXD_RT_V(bf16, 1);
+    } else {
+        if (vec) NXD_RT_V(float, 8); else NXD_RT_V(float, 1);
+    }
+#undef NXD_RT_V
+#undef NXD_RT
+    NXD_LAUNCH_CHECK();
+    return 0;
+}
+
+// Rows of the pairs sorted by expert.  counts [E] int32: ZEROED by the caller, out: pairs of every expert; slot [P] int32 out:
+// the pair's row in x (not written for identity experts); x [rows, W] bf16 with rows >= P + 32 E, W a multiple of 8.
+NXD_API int nxd_moe_sort_rows(const void* h, const int* idx, int* counts, int* slot, const float* in_scale, void* x, long long P,
+                              int top, int W, int E, void* stream) {
+    if (P == 0) return 0;
+    NXD_REQUIRE(E > 0 && E <= nxd_gemm::kSegMaxExperts && W % 8 == 0, "sort rows: %d experts, width %d", E, W);
+    NXD_REQUIRE(((uintptr_t)h % 16) == 0 && ((uintptr_t)x % 16) == 0, "sort rows: rows must be 16-byte aligned");
+    cudaStream_t st = (cudaStream_t)stream;
+    moe_count_kernel<<<(unsigned)((P + CNT_PAIRS - 1) / CNT_PAIRS), CNT_THREADS, 2 * E * sizeof(int), st>>>(idx, counts, slot,
+                                                                                                           P, E);
+    NXD_LAUNCH_CHECK();
+    moe_gather_rows_kernel<<<(unsigned)((P + GA_WARPS - 1) / GA_WARPS), GA_WARPS * 32, 0, st>>>(
+        (const bf16*)h, idx, counts, slot, in_scale, (bf16*)x, P, top, W / 8, E);
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -552,12 +718,17 @@ NXD_API int nxd_moe_gather_combine(int dtype, const void* ys, const int* slot, c
                                    int top, int W, int E, void* stream) {
     if (N == 0) return 0;
     NXD_REQUIRE(N < (1ll << 31), "combine: %lld tokens", N);
-    if (dtype == 0)
-        moe_gather_combine_kernel<bf16><<<(unsigned)N, 128, 0, (cudaStream_t)stream>>>(
-            (const bf16*)ys, slot, idx, wts, (const bf16*)h, (const bf16*)shared_out, sgate, y, top, W, E);
-    else
-        moe_gather_combine_kernel<float><<<(unsigned)N, 128, 0, (cudaStream_t)stream>>>(
-            (const float*)ys, slot, idx, wts, (const float*)h, (const float*)shared_out, sgate, y, top, W, E);
+    auto al = [](const void* p) { return ((uintptr_t)p % 16) == 0; };
+    const bool vec = W % 8 == 0 && al(ys) && al(h) && al(shared_out) && al(y);
+#define NXD_GC(T, V)                                                                                     \
+    moe_gather_combine_kernel<T, V><<<(unsigned)N, 128, 0, (cudaStream_t)stream>>>(                      \
+        (const T*)ys, slot, idx, wts, (const T*)h, (const T*)shared_out, sgate, y, top, W, E)
+    if (dtype == 0) {
+        if (vec) NXD_GC(bf16, 8); else NXD_GC(bf16, 1);
+    } else {
+        if (vec) NXD_GC(float, 8); else NXD_GC(float, 1);
+    }
+#undef NXD_GC
     NXD_LAUNCH_CHECK();
     return 0;
 }

@@ -47,7 +47,7 @@ GROUPS = {
 # everything a bf16 serving step of the window / sparse-MoE families touches: their own kernels, the GEMM kernels behind
 # the linear layers, and the tcgen05 flash attention that the windowed prefill is an instantiation of
 GROUPS["window_moe_serving"] = GROUPS["window_moe"] + [
-    "gemm_tcgen05.cu", "gemm_smallm.cu", "fused_gemm_ar.cu", "tma_host.cu", "flash_attn_tc.cu", "attn_tc_host.cu"]
+    "moe_forward.cu", "gemm_tcgen05.cu", "gemm_smallm.cu", "fused_gemm_ar.cu", "tma_host.cu", "flash_attn_tc.cu", "attn_tc_host.cu"]
 
 # the hybrid families (chunked / latent attention, recurrent matrix memory, dense feed-forward): the attention-over-cache
 # kernels, the norm kernels, their own two sources and the GEMM kernels behind the linear layers
@@ -58,13 +58,13 @@ GROUPS["hybrid_serving"] = ["window_attention.cu", "post_norm.cu", "latent_atten
 # the delta-rule hybrids (gated delta rule, differential window attention, dense and sparse gated feed-forward on a
 # gated parallel residual): the attention-over-cache, norm, sparse-MoE and recurrent-output kernels, the recurrence's
 # own source and the GEMM kernels behind the linear layers
-GROUPS["delta_serving"] = ["window_attention.cu", "post_norm.cu", "moe_sparse.cu", "mlstm.cu", "delta_rule.cu",
+GROUPS["delta_serving"] = ["window_attention.cu", "post_norm.cu", "moe_sparse.cu", "moe_forward.cu", "mlstm.cu", "delta_rule.cu",
                            "runtime.cu", "gemm_tcgen05.cu", "gemm_smallm.cu", "fused_gemm_ar.cu", "tma_host.cu"]
 
 # the retention hybrids (softmax attention with sinks next to fixed-decay linear attention, several residual streams,
 # dense and sparse gated feed-forward): attention over the cache, sparse MoE, the head norm / gate of recurrent outputs,
 # their own two sources, the GEMM kernels behind the linear layers and the tcgen05 flash attention of sink-free prompts
-GROUPS["retention_serving"] = ["window_attention.cu", "moe_sparse.cu", "mlstm.cu", "retention.cu", "hyper_connection.cu",
+GROUPS["retention_serving"] = ["window_attention.cu", "moe_sparse.cu", "moe_forward.cu", "mlstm.cu", "retention.cu", "hyper_connection.cu",
                                "runtime.cu", "gemm_tcgen05.cu", "gemm_smallm.cu", "fused_gemm_ar.cu", "tma_host.cu",
                                "flash_attn_tc.cu", "attn_tc_host.cu"]
 
@@ -79,7 +79,7 @@ GROUPS["scored_serving"] = ["window_attention.cu", "latent_attention.cu", "strea
 # the state-space family (selective scan and state-space heads behind short convolutions, capped attention next to the latter,
 # clamped gated and sparse feed-forward on a pre-norm fp32 stream): attention over the cache, the stream's norms, sparse MoE
 # and its activation, the mixers' own source, the GEMM kernels behind the linear layers and the tcgen05 flash attention
-GROUPS["state_space_serving"] = ["window_attention.cu", "state_space.cu", "stream_norm.cu", "moe_sparse.cu", "mlstm.cu",
+GROUPS["state_space_serving"] = ["window_attention.cu", "state_space.cu", "stream_norm.cu", "moe_sparse.cu", "moe_forward.cu", "mlstm.cu",
                                  "runtime.cu", "gemm_tcgen05.cu", "gemm_smallm.cu", "fused_gemm_ar.cu", "tma_host.cu",
                                  "flash_attn_tc.cu", "attn_tc_host.cu"]
 

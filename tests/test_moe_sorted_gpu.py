@@ -1,0 +1,78 @@
+"""The sparse mixture on rows that are sorted by expert on the device, and the router, against float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _reference(h, idx, wts, w_in, w_down, limit, alpha, shift, scale_input):
+    h, w_in, w_down = h.double(), w_in.double(), w_down.double()
+    E, y = w_in.shape[0], torch.zeros_like(h)
+    for j in range(idx.shape[1]):
+        for e in range(E):
+            rows = (idx[:, j] == e).nonzero()[:, 0]
+            w = wts[rows, j].double().unsqueeze(1)
+            # an input weight is applied in fp32 and the scaled row is rounded to bf16
+            x = (h[rows].float() * w.float()).bfloat16().double() if scale_input else h[rows]
+            z = x @ w_in[e]
+            if limit is None:
+                a = z.clamp(min=0).square()
+            else:
+                g, u = z.chunk(2, dim=-1)
+                g, u = g.clamp(max=limit), u.clamp(-limit, limit)
+                a = g * torch.sigmoid(alpha * g) * (u + shift)
+            y[rows] += (a @ w_down[e]) * (1.0 if scale_input else w)
+        rows = (idx[:, j] >= E).nonzero()[:, 0]
+        y[rows] += wts[rows, j].double().unsqueeze(1) * h[rows]
+    return y
+
+
+# tokens around the 32-row alignment, the 128- / 256-row tiles and empty experts; widths around the 64-column staging and the
+# 128 / 256-column tiles; the most experts
+@pytest.mark.parametrize("N,E,top,W,F", [(1, 3, 2, 8, 8), (31, 1, 1, 72, 40), (33, 5, 2, 136, 72), (257, 4, 4, 264, 200),
+                                         (1000, 7, 3, 64, 136), (700, 128, 2, 128, 64), (3000, 2, 1, 1024, 512)])
+@pytest.mark.parametrize("form", ["glu", "input", "relu2"])
+def test_sorted_experts_match_float64(N, E, top, W, F, form):
+    from neuronx_distributed_llama3_2_b200.ops import moe_sparse as ms
+
+    g = torch.Generator(device="cuda").manual_seed(N + E)
+
+    def normal(*s):
+        return torch.randn(*s, generator=g, device="cuda")
+
+    h = normal(N, W).bfloat16()
+    w_in = (normal(E, W, F if form == "relu2" else 2 * F) * W ** -0.5).bfloat16()
+    w_down = (normal(E, F, W) * F ** -0.5).bfloat16()
+    # expert 0 is never chosen when there is another one; index E is an identity expert
+    idx = torch.randint(min(1, E - 1), E + 1, (N, top), generator=g, device="cuda").to(torch.int32)
+    wts = torch.rand(N, top, generator=g, device="cuda") + 0.1
+    scale_input = form == "input"
+    limit = None if form == "relu2" else 1.5
+    assert ms.sorted_forward_applies(h, w_in, w_down)
+    shared, gate = normal(N, W).bfloat16(), torch.rand(N, generator=g, device="cuda")
+    ones = torch.where(idx < E, torch.ones_like(wts), wts)
+    out = ms.sorted_forward(h, idx, ones if scale_input else wts, w_in, w_down, limit is not None, limit or 0.0, 1.7, 1.0,
+                            wts if scale_input else None, shared, gate)
+    ref = _reference(h, idx, wts, w_in, w_down, limit, 1.7, 1.0, scale_input)
+    ref += shared.double() * gate.double().unsqueeze(1)
+    # the activation and the expert's output are rounded to bf16 once each: 2^-9 of the value each, and fp32 sums
+    assert (out.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
+
+
+@pytest.mark.parametrize("N,W,R", [(5, 72, 3), (5, 50, 37), (2400, 64, 37), (2401, 50, 9), (2369, 200, 700)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_router_forms_match_float64(N, W, R, dtype):
+    from neuronx_distributed_llama3_2_b200.ops import moe_sparse as ms
+
+    g = torch.Generator(device="cuda").manual_seed(N)
+    h = torch.randn(N, W, generator=g, device="cuda").to(dtype)
+    w = torch.randn(R, W, generator=g, device="cuda") * W ** -0.5
+    gate = torch.randn(1, W, generator=g, device="cuda") * W ** -0.5
+    idx, wts, sg = ms.route(h, w, None, 2, 1.5, gate)
+    z = h.double() @ w.double().t()
+    p = torch.softmax(z, dim=-1)
+    top = torch.topk(p, 2, dim=-1)
+    # fp32 sums of W terms: a choice may differ only between scores that are closer than their rounding
+    assert (p.gather(1, idx.long()) - top.values).abs().max() <= 1e-5
+    assert (wts.double() - 1.5 * p.gather(1, idx.long())).abs().max() <= 1e-5
+    assert (sg.double() - torch.sigmoid(h.double() @ gate.double()[0])).abs().max() <= 1e-5
