@@ -365,6 +365,15 @@ int nxd_flash_attn_fwd_tc_scored(const void* q, const void* k, const void* v, vo
                                  const float* slopes, const float* sinks, float softcap, const float* log_r1,
                                  const float* log_r2, const float* sigmoid_bias, const void* gate, long long gate_ld,
                                  int gate_cols, float gate_mul, void* stream);
+/* the same for a portion of tokens over the KV cache (contiguous or pages of a multiple of 64 rows) */
+int nxd_attn_prefill_cache_tc(const void* q, const void* cache_k, const void* cache_v, long long k_line, long long k_head,
+                              long long k_row, long long v_line, long long v_head, long long v_row, long long lines,
+                              int cache_rows, const int* block_table, int page_size, int table_cols, void* out,
+                              const int* q_start, const int* n_new, const int* seq_ids, const float* slopes,
+                              const float* sinks, int B, int Tn, int H, int G, int D, float scale, int window, int keep_first,
+                              float softcap, const float* log_r1, const float* log_r2, const float* sigmoid_bias,
+                              const void* gate, long long gate_ld, int gate_cols, float gate_mul, long long out_ld,
+                              void* stream);
 /* differential attention: maps [N, 2 * H, Dv] (first H heads = map 1, last H = map 2) -> out [N, H * Dv] =
  * rms_head(a1 - lambda * a2) * (1 - diff), lambda = exp(<lq1, lk1>) - exp(<lq2, lk2>) + diff (vectors fp32 [D]) */
 int nxd_diff_attn_combine(int dtype, const void* maps, void* out, const float* lq1, const float* lk1, const float* lq2,

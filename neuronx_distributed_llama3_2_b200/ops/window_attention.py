@@ -257,6 +257,40 @@ def _out_rows(out: Optional[torch.Tensor], q: torch.Tensor, rows: int, H: int, D
     return out, out.stride(0)
 
 
+# tokens x cache rows from which the tcgen05 kernel over the cache serves a portion.  Measured against the mma.sync kernel at 16
+# and 32 heads of 64 / 128, 1 to 3 rows, portions of 16 .. 1024 after 1 .. 3000 tokens: below, both are bound by the call itself
+# (25 to 31 us); above, 31 .. 71 us against 32 .. 203 us without score changes and 61 .. 209 against 105 .. 815 us with them.
+TC_CACHE_MIN_WORK = 150_000
+
+
+def _tc_cache(L):
+    """``nxd_attn_prefill_cache_tc`` of library ``L`` with its argument types declared (numbers go over as they are)."""
+    fn = L.nxd_attn_prefill_cache_tc
+    if not fn.argtypes:
+        p, i, l, f = _c.c_void_p, _c.c_int, _c.c_longlong, _c.c_float
+        fn.argtypes = [p] * 3 + [l] * 7 + [i, p, i, i] + [p] * 6 + [i] * 5 + [f, i, i] + [f, p, p, p, p, l, i, f, l, p]
+    return fn
+
+
+def _tc_cache_applies(q, cache_k, cache_v, out, G: int, bt, page_size: int, gate, gate_elements) -> bool:
+    """Whether the tcgen05 kernel over the cache takes these operands: bf16, equal key and value sizes of 64 or 128, one
+    value head per key head, TMA-compatible strides and bases, pages of whole 64-row tiles."""
+    B, T, H, D = q.shape
+    kb, vb = cache_k.shape, cache_v.shape
+    if (D not in (64, 128) or kb != vb or H % G or B >= 65536 or not T or q.dtype != torch.bfloat16
+            or cache_k.dtype != q.dtype or cache_v.dtype != q.dtype):
+        return False
+    k0, k1, k2, _ = cache_k.stride()
+    v0, v1, v2, _ = cache_v.stride()
+    if min(k0, k1, k2, v0, v1, v2) <= 0 or (k0 | k1 | k2 | v0 | v1 | v2 | out.stride(0)) % 8:
+        return False
+    if (cache_k.data_ptr() | cache_v.data_ptr() | q.data_ptr() | out.data_ptr()) % 16:
+        return False
+    if bt is not None and (page_size != kb[2] or page_size % 64):
+        return False
+    return not gate_elements or (gate.data_ptr() % 16 == 0 and gate.stride(-2) % 8 == 0)
+
+
 def window_attention_prefill(q: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Tensor, q_start: torch.Tensor,
                              scale: float, window: Optional[int] = None, keep_first: int = 0,
                              slopes: Optional[torch.Tensor] = None, n_new: Optional[torch.Tensor] = None,
@@ -270,8 +304,8 @@ def window_attention_prefill(q: torch.Tensor, cache_k: torch.Tensor, cache_v: to
     """``gate [B, T, H]``: output gate pre-activations (may be a column range of a projection output); ``gate_elements``:
     ``[B, T, H * Dv]``.  ``out [B * T, H * Dv]``: a buffer (or a column range of one) for the result.
 
-    ``impl``: ``auto`` | ``generic`` (fp32-math tile kernel, any sizes) | ``mma`` (bf16 tensor-core kernel, an error
-    where it does not apply) -- for tests and measurements.
+    ``impl``: ``auto`` | ``generic`` (fp32-math tile kernel, any sizes) | ``mma`` (bf16 mma.sync kernel, an error
+    where it does not apply) | ``tc`` (tcgen05 kernel, likewise) -- for tests and measurements.
 
     ``q [B, T, H, D]``: new tokens of every row at positions ``q_start[b] + t`` (their keys / values already in the
     cache) -> ``[B, T, H, Dv]``.  Rows ``t >= n_new[b]`` are padding and come out as zeros."""
@@ -284,8 +318,25 @@ def window_attention_prefill(q: torch.Tensor, cache_k: torch.Tensor, cache_v: to
         qs, nn_, sid = _i32(q_start), _i32(n_new), _i32(seq_ids)
         cargs, bt = _cache_args(cache_k, cache_v, block_table, page_size, rows=True)
         sk = sinks.float().contiguous() if sinks is not None else None
-        L = _lib.lib(GROUP)
         margs, _keep = _mod_args(softcap, log_bias, sigmoid_bias, gate, q, Dv if gate_elements else 0, gate_mul, out_ld)
+        if impl == "tc" or (impl == "auto" and not chunk and not value_heads and T * (
+                cache_k.shape[2] * (bt.shape[1] if bt is not None else 1)) >= TC_CACHE_MIN_WORK):
+            tc = _tc_cache_applies(q, cache_k, cache_v, out, G, bt, page_size, gate, gate_elements)
+            assert tc and not chunk and not value_heads or impl == "auto"
+            if tc:
+                L = _lib.lib("window_moe_serving")
+                r1, r2, pb = _keep
+                k0, k1, k2, _ = cache_k.stride()
+                v0, v1, v2, _ = cache_v.stride()
+                ptrs = [t.data_ptr() if t is not None else None for t in (bt, out, qs, nn_, sid, slopes, sk, r1, r2, pb, gate)]
+                rc = _tc_cache(L)(
+                    q.data_ptr(), cache_k.data_ptr(), cache_v.data_ptr(), k0, k1, k2, v0, v1, v2, cache_k.shape[0],
+                    cache_k.shape[2], ptrs[0], page_size if bt is not None else 0, bt.shape[1] if bt is not None else 0,
+                    *ptrs[1:7], B, T, H, G, D, scale, w, keep_first, float(softcap) if softcap else 0.0, *ptrs[7:],
+                    gate.stride(-2) if gate is not None else 0, Dv if gate_elements else 0, gate_mul, out_ld, _lib.stream_ptr())
+                _lib.check(rc, "nxd_attn_prefill_cache_tc", L)
+                return out.view(B, T, H, Dv) if out_ld == 0 else out
+        L = _lib.lib(GROUP)
         rc = L.nxd_scored_attn_prefill(_c.c_int(_code(q.dtype)), _lib.ptr(q), _lib.ptr(cache_k), _lib.ptr(cache_v),
                                        *cargs, _lib.ptr(out), _lib.ptr(qs), _lib.ptr(nn_), _lib.ptr(sid),
                                        _lib.ptr(slopes), _lib.ptr(sk), _c.c_int(B), _c.c_int(T), _c.c_int(H), _c.c_int(G),

@@ -1,0 +1,63 @@
+"""Attention of a portion of tokens over the KV cache on the tcgen05 kernel, against the fp32 restatement."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+FORMS = ["plain", "window", "kept", "sinks", "capped", "sigmoid", "gated", "columns"]
+
+
+@pytest.mark.parametrize("D", [64, 128])
+# portions around the 128-row query tile, starts around the 64-row key tile, padded and empty rows
+@pytest.mark.parametrize("T,starts,n_new", [(64, [0, 1, 63], None), (65, [64, 700, 129], [65, 1, 0]), (200, [5, 0, 333], [129, 200, 64]),
+                                            (300, [128, 20, 961], None)])
+@pytest.mark.parametrize("page", [0, 64, 128])
+@pytest.mark.parametrize("form", FORMS)
+def test_portion_over_the_cache_matches_the_restatement(D, T, starts, n_new, page, form):
+    from neuronx_distributed_llama3_2_b200.ops import window_attention as wa
+
+    B, H, G, lines = len(starts), 4, 2, 5
+    g = torch.Generator(device="cuda").manual_seed(T + D + page)
+
+    def normal(*s):
+        return torch.randn(*s, generator=g, device="cuda")
+
+    S = 1408                                            # rows of a line, a multiple of the pages
+    line = torch.tensor([3, 0, 2], dtype=torch.int32, device="cuda")
+    k, v = (normal(lines, G, S, D).bfloat16() for _ in range(2))
+    ends = [s + (T if n_new is None else n) for s, n in zip(starts, n_new or starts)]
+    for b, e in enumerate(ends):                        # what lies behind a sequence's end is never looked at
+        k[line[b], :, e:] = float("nan")
+        v[line[b], :, e:] = float("nan")
+    q = normal(B, T, H, D).bfloat16()
+    kw = {"window": {}, "plain": {}, "kept": {"keep_first": 70}, "sinks": {"sinks": normal(H)},
+          "capped": {"softcap": 3.0, "log_bias": (normal(H).abs(), normal(H).abs())},
+          "sigmoid": {"sigmoid_bias": normal(H), "softcap": 20.0}, "gated": {"gate": normal(B, T, H).bfloat16()},
+          "columns": {"gate": normal(B, T, H * D).bfloat16(), "gate_elements": True, "gate_mul": 2.0}}[form]
+    window = None if form in ("plain", "sinks") else 100
+    slopes = wa.distance_slopes(H, device="cuda") if form in ("window", "kept", "gated") else None
+    new = None if n_new is None else torch.tensor(n_new, dtype=torch.int32, device="cuda")
+    start = torch.tensor(starts, dtype=torch.int32, device="cuda")
+    ck, cv, paged = k, v, {}
+    if page:
+        table = torch.randperm(lines * S // page, generator=g, device="cuda").reshape(lines, -1)
+        ck, cv = torch.empty(lines * S // page, G, page, D, dtype=k.dtype, device="cuda"), None
+        cv = torch.empty_like(ck)
+        for dst, src in ((ck, k), (cv, v)):
+            dst[table.reshape(-1)] = src.reshape(lines, G, -1, page, D).transpose(1, 2).reshape(-1, G, page, D)
+        paged = {"block_table": table.to(torch.int32), "page_size": page}
+    wide = torch.full((B * T, H * D + 64), 7.0, dtype=q.dtype, device="cuda")
+    out = wa.window_attention_prefill(q, ck, cv, start, D ** -0.5, window, slopes=slopes, n_new=new, seq_ids=line, impl="tc",
+                                      out=wide[:, 32:32 + H * D], **kw, **paged).reshape(B, T, H, D)
+    assert (wide[:, :32] == 7).all() and (wide[:, -32:] == 7).all()
+    gate = kw.pop("gate", None)
+    keep = kw.pop("keep_first", 0)
+    for b in range(B):
+        n, e = ends[b] - starts[b], ends[b]
+        assert not out[b, n:].any()                     # padding rows come out as zeros
+        if n == 0:
+            continue
+        ref = wa.window_attention_ref(q[b, :n], k[line[b], :, :e], v[line[b], :, :e], torch.arange(starts[b], e, device="cuda"),
+                                      D ** -0.5, window, keep, slopes, gate=None if gate is None else gate[b, :n], **kw)
+        # the weights and the result are rounded to bf16: 2^-9 of each weight and of the value
+        assert (out[b, :n].float() - ref).norm() <= 2.0 ** -7 * ref.norm()
