@@ -92,6 +92,128 @@ __global__ void delta_prep_kernel(const T* __restrict__ proj, long long ld, int 
     for (int i = lane; i < dim; i += 32) dst[i] *= r;            // every lane rescales what it wrote itself
 }
 
+// The same for 4 taps and sizes of 32 V channels (D = 32 V, Dv a multiple): a lane owns V neighbouring channels of one query,
+// key or value piece and walks a strip of tokens with the last three inputs in registers, so every projection value is
+// read once (the general kernel reads it once per tap, 2 bytes at a time).  Bound by memory: 4 x 2048 tokens, 4 + 4 heads of
+// 128 and 4 of 256 (100 MB with the fp32 results): 44 us, 177 us with the general kernel.
+constexpr int PREP_STRIP = 16, PREP_AHEAD = 4;
+
+template <int V>
+__device__ __forceinline__ void ld_v(const float* p, float* f) {
+    if constexpr (V == 2) {
+        const float2 a = *reinterpret_cast<const float2*>(p);
+        f[0] = a.x, f[1] = a.y;
+    } else {
+#pragma unroll
+        for (int i = 0; i < V; i += 4) *reinterpret_cast<float4*>(f + i) = *reinterpret_cast<const float4*>(p + i);
+    }
+}
+template <int V>
+__device__ __forceinline__ void ld_v(const bf16* p, float* f) {
+    uint32_t w[V / 2];
+    if constexpr (V == 2) w[0] = *reinterpret_cast<const uint32_t*>(p);
+    if constexpr (V == 4) *reinterpret_cast<uint2*>(w) = *reinterpret_cast<const uint2*>(p);
+    if constexpr (V == 8) *reinterpret_cast<uint4*>(w) = *reinterpret_cast<const uint4*>(p);
+#pragma unroll
+    for (int i = 0; i < V / 2; ++i) {
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const bf162*>(w + i));
+        f[2 * i] = a.x, f[2 * i + 1] = a.y;
+    }
+}
+template <int V>
+__device__ __forceinline__ void st_v(float* p, const float* f) {
+    if constexpr (V == 2) *reinterpret_cast<float2*>(p) = make_float2(f[0], f[1]);
+    else
+#pragma unroll
+        for (int i = 0; i < V; i += 4) *reinterpret_cast<float4*>(p + i) = make_float4(f[i], f[i + 1], f[i + 2], f[i + 3]);
+}
+
+template <typename T, int V>
+__global__ void __launch_bounds__(256)
+delta_prep_strip_kernel(const T* __restrict__ proj, long long ld, int off_q, int off_k, int off_v,
+                        const float* __restrict__ conv_w, const float* __restrict__ conv_state, float* __restrict__ qn,
+                        float* __restrict__ kn, float* __restrict__ vn, const int* __restrict__ q_start,
+                        const int* __restrict__ n_new, const int* __restrict__ seq_ids, int units, int Tn, int H, int G, int Dv,
+                        float qscale, float unit_eps) {
+    constexpr int D = 32 * V, TAPS = 4, K = TAPS - 1;
+    const int lane = threadIdx.x & 31, u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (u >= units) return;
+    const int b = blockIdx.z, s0 = blockIdx.y * PREP_STRIP;
+    const int n = n_new != nullptr ? min(n_new[b], Tn) : Tn;
+    const int s_end = min(n, s0 + PREP_STRIP);
+    if (s0 >= s_end) return;
+    const int C = 2 * G * D + H * Dv;
+    const int c = u * D + lane * V;                              // channel in q | k | v order
+    long long col;
+    float* dst;                                                  // of the batch row's first token
+    long long pitch;
+    if (u < G) {
+        col = off_q + c, dst = qn + (long long)b * Tn * G * D + c, pitch = (long long)G * D;
+    } else if (u < 2 * G) {
+        col = off_k + c - G * D, dst = kn + (long long)b * Tn * G * D + c - G * D, pitch = (long long)G * D;
+    } else {
+        col = off_v + c - 2 * G * D, dst = vn + (long long)b * Tn * H * Dv + c - 2 * G * D, pitch = (long long)H * Dv;
+    }
+    const int line = seq_ids != nullptr ? seq_ids[b] : b, p0 = q_start[b];
+    const float* st = conv_state + (long long)line * K * C;
+    const T* src = proj + (long long)b * Tn * ld + col;
+    float w[V * TAPS], x[TAPS + PREP_AHEAD - 1][V];              // x[i]: inputs of step s - K + i
+#pragma unroll
+    for (int i = 0; i < V * TAPS; i += 4)
+        *reinterpret_cast<float4*>(w + i) = *reinterpret_cast<const float4*>(conv_w + (long long)c * TAPS + i);
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+        const int s = s0 - K + i;
+        if (s >= 0) {
+            ld_v<V>(src + s * ld, x[i]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < V; ++e) x[i][e] = p0 + s < 0 ? 0.f : st[(long long)(K + s) * C + c + e];
+        }
+    }
+    const float mul = u < G ? qscale : 1.f;
+    for (int s = s0; s < s_end; s += PREP_AHEAD) {
+#pragma unroll
+        for (int a = 0; a < PREP_AHEAD; ++a)
+            ld_v<V>(src + min(s + a, s_end - 1) * ld, x[K + a]);
+#pragma unroll
+        for (int a = 0; a < PREP_AHEAD; ++a) {
+            if (s + a >= s_end) break;
+            float v[V], ss = 0.f;
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+                float acc = 0.f;
+#pragma unroll
+                for (int j = 0; j < TAPS; ++j) acc = fmaf(w[e * TAPS + j], x[a + j][e], acc);
+                v[e] = silu_f(acc);
+                ss = fmaf(v[e], v[e], ss);
+            }
+            if (u < 2 * G) {
+                const float r = mul / sqrtf(warp_sum(ss) + unit_eps);
+#pragma unroll
+                for (int e = 0; e < V; ++e) v[e] *= r;
+            }
+            st_v<V>(dst + (s + a) * pitch, v);
+        }
+#pragma unroll
+        for (int i = 0; i < K; ++i)
+#pragma unroll
+            for (int e = 0; e < V; ++e) x[i][e] = x[PREP_AHEAD + i][e];
+    }
+}
+
+template <typename T, int V>
+int launch_prep_strip(const void* proj, long long ld, int off_q, int off_k, int off_v, const float* conv_w,
+                      const float* conv_state, float* qn, float* kn, float* vn, const int* q_start, const int* n_new,
+                      const int* seq_ids, int B, int Tn, int H, int G, int Dv, float qscale, float unit_eps, cudaStream_t st) {
+    const int units = 2 * G + H * (Dv / (32 * V));
+    dim3 grid((units + 7) / 8, (Tn + PREP_STRIP - 1) / PREP_STRIP, B);
+    delta_prep_strip_kernel<T, V><<<grid, 256, 0, st>>>((const T*)proj, ld, off_q, off_k, off_v, conv_w, conv_state, qn, kn, vn,
+                                                        q_start, n_new, seq_ids, units, Tn, H, G, Dv, qscale, unit_eps);
+    NXD_LAUNCH_CHECK();
+    return 0;
+}
+
 template <typename T>
 __global__ void delta_conv_state_kernel(const T* __restrict__ proj, long long ld, int off_q, int off_k, int off_v,
                                         float* __restrict__ conv_state, const int* __restrict__ q_start,
@@ -344,6 +466,403 @@ int launch_scan(const float* qn, const float* kn, const float* vn, const float* 
     return 0;
 }
 
+// ---- chunk-wise form (one decay per head) --------------------------------------------------------------------------------
+// For a chunk of CH tokens with start state S, Gamma_t the product of the chunk's decays up to t and L[t][s] their product
+// over (s, t], the errors u of all tokens solve one triangular system:
+//
+//   A[t][s] = beta_t L[t][s] (k_t . k_s), s < t;    (I + A) U = diag(beta) (V - diag(Gamma) K S)
+//   O = diag(Gamma) Q S + P U,  P[t][s] = L[t][s] (q_t . k_s), s <= t;    S <- Gamma_CH S + (diag(L[CH-1][.]) K)^T U
+//
+// (the WY form of Householder products; Yang, Wang, Zhang, Shen, Kim, "Parallelizing Linear Transformers with the Delta Rule
+// over Sequence Length").  Decay ratios are products, never quotients or exponentials of sums, so a decay of any size is
+// exact to rounding and underflows to the right limit.  Two kernels, all fp32:
+//   delta_chunk_system  per (chunk, head, row), in parallel: (I + A)^-1 diag(beta), P, Gamma and L[CH-1][.] to scratch
+//   delta_chunk_scan    per (32 value columns, head, row), sequential over chunks with the state slice in shared memory:
+//                       four products per chunk, register-tiled, on packed pairs of fp32 multiply-adds (pairs run along the
+//                       contraction, so both operands are read as 16-byte pieces and nothing is shuffled)
+// Bound by the fp32 pipes of the second kernel: a token costs 3 D + CH multiply-adds per value column, like token by token, but
+// 64 tokens are independent, where delta_scan waits for two dot products and a shuffle tree per token.  Its own limit is the
+// shared memory that feeds them (0.4 floats read per multiply-add).  4 x 2048 tokens, 4 heads of 128 x 256: 69 + 348 us against
+// 779 us token by token.
+constexpr int CH = 64, CP = CH + 4, CW_THREADS = 256, CW_COLS = 32;
+
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t pack2(float x, float y) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float lo2(uint64_t v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi2(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ ulonglong2 ld_pairs(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
+
+// acc[i][j] += <a row i, b row j> over 4 values
+template <int R, int C>
+__device__ __forceinline__ void dot_step(uint64_t (&acc)[R][C], const ulonglong2 (&a)[R], const ulonglong2 (&b)[C]) {
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < C; ++j) acc[i][j] = fma2(a[i].y, b[j].y, fma2(a[i].x, b[j].x, acc[i][j]));
+}
+
+template <int R, int C>
+__device__ __forceinline__ void add_pairs(uint64_t (&acc)[R][C], const uint64_t (&part)[R][C]) {
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < C; ++j) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc[i][j]) : "l"(part[i][j]));
+}
+
+// scratch per (row, head, chunk): M [CH][CH] = (I + A)^-1 diag(beta), P [CH][CH], Gamma [CH], L[CH-1][.] [CH]
+constexpr int CHUNK_FLOATS = 2 * CH * CH + 2 * CH;
+
+template <int D>
+__global__ void __launch_bounds__(CW_THREADS, 2)
+delta_chunk_system_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ gate,
+                          long long ld_a, int a_off, const float* __restrict__ beta, long long ld_b, int b_off,
+                          float* __restrict__ scratch, const int* __restrict__ n_new, int Tn, int H, int G) {
+    extern __shared__ __align__(16) float smem[];
+    float* Ks = smem;                    // [CH][CP] 64 key channels at a time
+    float* Qs = Ks + CH * CP;            // [CH][CP]
+    float* As = Qs + CH * CP;            // [CH][CP] A
+    float* Ls = As + CH * CP;            // [CH][CP] L
+    float* Ts = Ks;                      // [CH][CP] columns of (I + A)^-1, once the products are done
+    __shared__ float gs[CH], bs[CH];
+    const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, kvh = h / (H / G), tid = threadIdx.x;
+    const int lane = tid & 31, warp = tid >> 5;
+    const int n = n_new != nullptr ? min(n_new[b], Tn) : Tn;
+    const int nt = min(CH, n - c * CH);  // real tokens; the others change nothing (k = q = 0, beta = 0, g = 1)
+    if (nt <= 0) return;                 // the scan does not look at this chunk
+    const long long row0 = (long long)b * Tn + c * CH;
+    if (tid < CH) {
+        gs[tid] = tid < nt ? gate[(row0 + tid) * ld_a + a_off + h] : 1.f;
+        bs[tid] = tid < nt ? beta[(row0 + tid) * ld_b + b_off + h] : 0.f;
+    }
+    // rows of a thread: r and CH/2 + r of K and of Q; columns cg + 8 j, of which the upper half of the rows needs j < 4
+    const int r = warp * 4 + (lane >> 3), cg = lane & 7;
+    float lower[4][4] = {}, right[2][4] = {};                    // all four rows, j < 4; rows CH/2 + r, j >= 4
+    for (int d0 = 0; d0 < D; d0 += 64) {
+        __syncthreads();
+        for (int i = tid; i < CH * 16; i += CW_THREADS) {
+            const int t = i >> 4, d = (i & 15) * 4;
+            const long long src = ((row0 + t) * G + kvh) * D + d0 + d;
+            float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), qv = kv;
+            if (t < nt) kv = *reinterpret_cast<const float4*>(kn + src), qv = *reinterpret_cast<const float4*>(qn + src);
+            *reinterpret_cast<float4*>(Ks + t * CP + d) = kv;
+            *reinterpret_cast<float4*>(Qs + t * CP + d) = qv;
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int d1 = 0; d1 < 64; d1 += 16) {                    // sums of 16, as in the scan
+            uint64_t p[4][4] = {}, q[2][4] = {};
+#pragma unroll
+            for (int d = d1; d < d1 + 16; d += 4) {
+                const ulonglong2 a[4] = {ld_pairs(Ks + r * CP + d), ld_pairs(Qs + r * CP + d), ld_pairs(Ks + (r + CH / 2) * CP + d),
+                                         ld_pairs(Qs + (r + CH / 2) * CP + d)};
+                ulonglong2 kb[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) kb[j] = ld_pairs(Ks + (cg + 8 * j) * CP + d);
+                dot_step(p, a, kb);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) kb[j] = ld_pairs(Ks + (cg + 8 * j + 32) * CP + d);
+                const ulonglong2 a2[2] = {a[2], a[3]};
+                dot_step(q, a2, kb);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) lower[i][j] += lo2(p[i][j]) + hi2(p[i][j]);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) right[i][j] += lo2(q[i][j]) + hi2(q[i][j]);
+            }
+        }
+    }
+    if (tid < CH) {                      // column s of L: running products of the decays behind s
+        float l = 1.f;
+        for (int t = 0; t < CH; ++t) {
+            if (t > tid) l *= gs[t];
+            Ls[t * CP + tid] = t >= tid ? l : 0.f;
+        }
+    }
+    __syncthreads();
+    float* out = scratch + (((long long)b * H + h) * gridDim.x + c) * CHUNK_FLOATS;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int t = r + half * (CH / 2);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int s = cg + 8 * j;
+            const float l = Ls[t * CP + s], kk = j < 4 ? lower[2 * half][j & 3] : right[0][j & 3];
+            const float qk = j < 4 ? lower[2 * half + 1][j & 3] : right[1][j & 3];
+            As[t * CP + s] = s < t ? bs[t] * l * kk : 0.f;
+            out[CH * CH + t * CH + s] = s <= t ? l * qk : 0.f;
+        }
+    }
+    if (tid < CH) {
+        out[2 * CH * CH + tid] = Ls[tid * CP] * gs[0];
+        out[2 * CH * CH + CH + tid] = Ls[(CH - 1) * CP + tid];
+    }
+    __syncthreads();
+    // columns of X = (I + A)^-1 by forward substitution, four lanes a column; Ts[col][t]
+    const int col = tid >> 2, part = tid & 3;
+    float* x = Ts + col * CP;
+    for (int t = part; t < CH; t += 4) x[t] = t == col ? 1.f : 0.f;
+    __syncwarp();
+    for (int t = 1; t < CH; ++t) {       // the lanes of a warp hold 8 neighbouring columns: rows above them stay zero
+        if (t <= (col & ~7)) continue;
+        float d = 0.f;
+#pragma unroll 4
+        for (int s = (col & ~7) + part; s < t; s += 4) d = fmaf(As[t * CP + s], x[s], d);
+        d += __shfl_xor_sync(0xffffffffu, d, 1);
+        d += __shfl_xor_sync(0xffffffffu, d, 2);
+        if (part == 0 && t > col) x[t] = -d;
+        __syncwarp();
+    }
+    __syncthreads();
+    for (int i = tid; i < CH * CH; i += CW_THREADS) {
+        const int t = i / CH, s = i % CH;
+        out[i] = s <= t ? Ts[s * CP + t] * bs[s] : 0.f;
+    }
+}
+
+// grid (Dv / 32, H, B).  Rows of a thread in the 64-row products: 4 w + rg and 60 - 4 w + rg (w the warp, rg = lane / 8), so
+// that the triangular products cost every warp the same; columns cg + 8 i (cg = lane % 8).
+template <int D>
+__global__ void __launch_bounds__(CW_THREADS, D == 64 ? 2 : 1)
+delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vn,
+                        const float* __restrict__ scratch, float* __restrict__ S, float* __restrict__ out,
+                        const int* __restrict__ q_start, const int* __restrict__ n_new, const int* __restrict__ seq_ids, int Tn,
+                        int NC, int H, int G, int Dv) {
+    extern __shared__ __align__(16) float smem[];
+    constexpr int DP = D + 4, DT = D / 32, KB = D <= 128 ? 2 : 1;     // KB: buffers of K
+    float* Kb = smem;                          // [KB][CH][DP]
+    float* Qs = Kb + KB * CH * DP;             // [CH][DP]
+    float* Ss = Qs + CH * DP;                  // [32][DP] the state slice, a value column per row
+    float* Ms = Ss + CW_COLS * DP;             // [CH][CP]
+    float* Ps = Ms + CH * CP;                  // [CH][CP]
+    float* Rs = Ps + CH * CP;                  // [32][CP] V - diag(Gamma) K S, a value column per row
+    float* Us = Rs + CW_COLS * CP;             // [32][CP] U
+    float* gam = Us + CW_COLS * CP;            // [CH] Gamma
+    float* last = gam + CH;                    // [CH] L[CH-1][.]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int col0 = blockIdx.x * CW_COLS, h = blockIdx.y, b = blockIdx.z, kvh = h / (H / G);
+    const int n = n_new != nullptr ? min(n_new[b], Tn) : Tn;
+    const long long row0 = (long long)b * Tn;
+    float* orow = out + (row0 * H + h) * Dv + col0;              // + t * H * Dv
+    for (int i = tid; i < (Tn - max(n, 0)) * CW_COLS; i += CW_THREADS)       // padding rows
+        orow[(long long)(max(n, 0) + i / CW_COLS) * H * Dv + i % CW_COLS] = 0.f;
+    if (n <= 0) return;
+    const int line = seq_ids != nullptr ? seq_ids[b] : b;
+    float* Sb = S + ((long long)line * H + h) * D * Dv + col0;
+    const bool fresh = q_start[b] == 0;
+    for (int i = tid; i < D * CW_COLS; i += CW_THREADS) {
+        const int d = i / CW_COLS, j = i % CW_COLS;
+        Ss[j * DP + d] = fresh ? 0.f : Sb[(long long)d * Dv + j];
+    }
+    const float* chunk0 = scratch + ((long long)b * H + h) * NC * CHUNK_FLOATS;
+    const int chunks = (n + CH - 1) / CH;
+    auto rows = [&](const float* src, float* dst, int c) {       // K or Q rows of chunk c
+        if (c < chunks)
+            for (int i = tid; i < CH * (D / 4); i += CW_THREADS) {
+                const int t = i / (D / 4), d = (i % (D / 4)) * 4;
+                const bool ok = c * CH + t < n;
+                mma::cp_async16((uint32_t)__cvta_generic_to_shared(dst + t * DP + d),
+                                src + ((row0 + (ok ? c * CH + t : 0)) * G + kvh) * D + d, ok);
+            }
+    };
+    auto square = [&](int off, float* dst, int c) {              // M or P of chunk c
+        if (c < chunks)
+            for (int i = tid; i < CH * (CH / 4); i += CW_THREADS) {
+                const int t = i / (CH / 4), x = (i % (CH / 4)) * 4;
+                mma::cp_async16((uint32_t)__cvta_generic_to_shared(dst + t * CP + x),
+                                chunk0 + (long long)c * CHUNK_FLOATS + off + t * CH + x, true);
+            }
+    };
+    rows(kn, Kb, 0);
+    rows(qn, Qs, 0);
+    square(0, Ms, 0);
+    mma::cp_async_commit();
+    square(CH * CH, Ps, 0);
+    mma::cp_async_commit();
+    const int rg = lane >> 3, cg = lane & 7, ra = 4 * warp + rg, rb = 60 - 4 * warp + rg;
+    for (int c = 0; c < chunks; ++c) {
+        const float* Ks = Kb + (KB == 2 ? (c & 1) * CH * DP : 0);
+        const int t0 = c * CH;
+        if (tid < 2 * CH) gam[tid] = chunk0[(long long)c * CHUNK_FLOATS + 2 * CH * CH + tid];      // and `last` behind it
+        float v[2][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[0][i] = t0 + ra < n ? vn[((row0 + t0 + ra) * H + h) * Dv + col0 + cg + 8 * i] : 0.f;
+            v[1][i] = t0 + rb < n ? vn[((row0 + t0 + rb) * H + h) * Dv + col0 + cg + 8 * i] : 0.f;
+        }
+        mma::cp_async_wait<1>();               // everything but P
+        __syncthreads();
+        if (KB == 2) {
+            rows(kn, Kb + ((c + 1) & 1) * CH * DP, c + 1);
+            mma::cp_async_commit();
+        }
+        uint64_t acc[4][4] = {};               // K S of rows ra, rb; Q S of rows ra, rb
+#pragma unroll 1
+        for (int d0 = 0; d0 < D; d0 += 16) {   // sums of 16 first: half the rounding error of one long chain
+            uint64_t part[4][4] = {};
+#pragma unroll
+            for (int d = d0; d < d0 + 16; d += 4) {
+                const ulonglong2 a[4] = {ld_pairs(Ks + ra * DP + d), ld_pairs(Ks + rb * DP + d), ld_pairs(Qs + ra * DP + d),
+                                         ld_pairs(Qs + rb * DP + d)};
+                ulonglong2 sb[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) sb[j] = ld_pairs(Ss + (cg + 8 * j) * DP + d);
+                dot_step(part, a, sb);
+            }
+            add_pairs(acc, part);
+        }
+        const float ga = gam[ra], gb = gam[rb];
+        float o[2][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            Rs[(cg + 8 * i) * CP + ra] = fmaf(-ga, lo2(acc[0][i]) + hi2(acc[0][i]), v[0][i]);
+            Rs[(cg + 8 * i) * CP + rb] = fmaf(-gb, lo2(acc[1][i]) + hi2(acc[1][i]), v[1][i]);
+            o[0][i] = ga * (lo2(acc[2][i]) + hi2(acc[2][i]));
+            o[1][i] = gb * (lo2(acc[3][i]) + hi2(acc[3][i]));
+        }
+        __syncthreads();
+        rows(qn, Qs, c + 1);                   // the queries of this chunk have been used
+        mma::cp_async_commit();
+        // rows ra and rb of a lower triangular 64 x 64 matrix times the columns of X [32][CP]
+        auto triangular = [&](const float* M, const float* X, uint64_t (&y)[2][4]) {
+            const int e = 4 * warp, f = 60 - 4 * warp;           // the blocks of the diagonal: [e, e + 4) and [f, f + 4)
+#pragma unroll 1
+            for (int s0 = 0; s0 < f; s0 += 16) {                 // sums of 16 first, as above
+                uint64_t part[2][4] = {};
+#pragma unroll
+                for (int s = s0; s < s0 + 16; s += 4) {
+                    if (s >= f) break;
+                    const ulonglong2 a = ld_pairs(M + rb * CP + s);
+                    ulonglong2 xb[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        xb[j] = ld_pairs(X + (cg + 8 * j) * CP + s);
+                        part[1][j] = fma2(a.y, xb[j].y, fma2(a.x, xb[j].x, part[1][j]));
+                    }
+                    if (s >= e) continue;
+                    const ulonglong2 c = ld_pairs(M + ra * CP + s);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) part[0][j] = fma2(c.y, xb[j].y, fma2(c.x, xb[j].x, part[0][j]));
+                }
+                add_pairs(y, part);
+            }
+            // on the diagonal the entries behind the row's own are left out, not multiplied by zero: a token that is not a
+            // number does not reach the tokens before it
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int row = half ? rb : ra, s = half ? f : e;
+                const float4 m = *reinterpret_cast<const float4*>(M + row * CP + s);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float4 x = *reinterpret_cast<const float4*>(X + (cg + 8 * j) * CP + s);
+                    float d = m.x * x.x;
+                    if (rg >= 1) d = fmaf(m.y, x.y, d);
+                    if (rg >= 2) d = fmaf(m.z, x.z, d);
+                    if (rg >= 3) d = fmaf(m.w, x.w, d);
+                    y[half][j] = pack2(lo2(y[half][j]) + d, hi2(y[half][j]));
+                }
+            }
+        };
+        uint64_t y[2][4] = {};
+        triangular(Ms, Rs, y);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            Us[(cg + 8 * i) * CP + ra] = lo2(y[0][i]) + hi2(y[0][i]);
+            Us[(cg + 8 * i) * CP + rb] = lo2(y[1][i]) + hi2(y[1][i]);
+        }
+        mma::cp_async_wait<KB>();              // P of this chunk (the groups behind it: Q and, with two buffers, K)
+        __syncthreads();
+        square(0, Ms, c + 1);
+        mma::cp_async_commit();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y[0][i] = y[1][i] = 0ull;
+        triangular(Ps, Us, y);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (t0 + ra < n) orow[(long long)(t0 + ra) * H * Dv + cg + 8 * i] = o[0][i] + (lo2(y[0][i]) + hi2(y[0][i]));
+            if (t0 + rb < n) orow[(long long)(t0 + rb) * H * Dv + cg + 8 * i] = o[1][i] + (lo2(y[1][i]) + hi2(y[1][i]));
+        }
+        // S[.][j] <- Gamma S + sum_s last_s U[s][j] K[s][.]: DT key channels x 4 value columns per thread
+        {
+            const int d0 = ((warp & 3) * 8 + cg) * DT, j0 = (warp >> 2) * 16 + rg;       // columns j0 + 4 i
+            const uint64_t gl = pack2(gam[CH - 1], gam[CH - 1]);
+            uint64_t st[4][DT / 2] = {};       // the chunk's own part; the decayed state joins it once
+#pragma unroll 1
+            for (int s0 = 0; s0 < CH; s0 += 16) {
+                uint64_t part[4][DT / 2] = {};
+#pragma unroll 2
+                for (int s = s0; s < s0 + 16; s += 4) {
+                    float u[4][4], lw[4];
+                    *reinterpret_cast<float4*>(lw) = *reinterpret_cast<const float4*>(last + s);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        *reinterpret_cast<float4*>(u[i]) = *reinterpret_cast<const float4*>(Us + (j0 + 4 * i) * CP + s);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        uint64_t kv[DT / 2];
+#pragma unroll
+                        for (int x = 0; x < DT / 2; ++x)
+                            kv[x] = *reinterpret_cast<const uint64_t*>(Ks + (s + q) * DP + d0 + 2 * x);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float w = u[i][q] * lw[q];
+                            const uint64_t ww = pack2(w, w);
+#pragma unroll
+                            for (int x = 0; x < DT / 2; ++x) part[i][x] = fma2(kv[x], ww, part[i][x]);
+                        }
+                    }
+                }
+                add_pairs(st, part);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int x = 0; x < DT / 2; ++x) {
+                    uint64_t* at = reinterpret_cast<uint64_t*>(Ss + (j0 + 4 * i) * DP + d0 + 2 * x);
+                    *at = fma2(*at, gl, st[i][x]);
+                }
+        }
+        __syncthreads();                       // K, P, U and the old state are free
+        if (KB == 1) rows(kn, Kb, c + 1);
+        mma::cp_async_commit();
+        square(CH * CH, Ps, c + 1);
+        mma::cp_async_commit();
+    }
+    for (int i = tid; i < D * CW_COLS; i += CW_THREADS) {
+        const int d = i / CW_COLS, j = i % CW_COLS;
+        Sb[(long long)d * Dv + j] = Ss[j * DP + d];
+    }
+}
+
+template <int D>
+int launch_chunks(const float* qn, const float* kn, const float* vn, const float* gate, long long ld_a, int a_off,
+                  const float* beta, long long ld_b, int b_off, float* S, float* out, float* scratch, const int* q_start,
+                  const int* n_new, const int* seq_ids, int B, int Tn, int H, int G, int Dv, cudaStream_t st) {
+    constexpr int DP = D + 4;
+    const int NC = (Tn + CH - 1) / CH;
+    const size_t sys = (size_t)4 * CH * CP * sizeof(float);
+    const size_t scan = (size_t)((D <= 128 ? 3 : 2) * CH * DP + CW_COLS * DP + 2 * CH * CP + 2 * CW_COLS * CP + 2 * CH) * sizeof(float);
+    static_assert((2 * CH * 260 + CW_COLS * 260 + 2 * CH * CP + 2 * CW_COLS * CP + 2 * CH) * 4 <= 232448, "shared memory");
+    NXD_CHECK_CUDA(cudaFuncSetAttribute(delta_chunk_system_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sys));
+    NXD_CHECK_CUDA(cudaFuncSetAttribute(delta_chunk_scan_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan));
+    delta_chunk_system_kernel<D><<<dim3(NC, H, B), CW_THREADS, sys, st>>>(qn, kn, gate, ld_a, a_off, beta, ld_b, b_off, scratch,
+                                                                          n_new, Tn, H, G);
+    NXD_LAUNCH_CHECK();
+    delta_chunk_scan_kernel<D><<<dim3(Dv / CW_COLS, H, B), CW_THREADS, scan, st>>>(qn, kn, vn, scratch, S, out, q_start, n_new,
+                                                                                  seq_ids, Tn, NC, H, G, Dv);
+    NXD_LAUNCH_CHECK();
+    return 0;
+}
+
 }  // namespace
 
 // dtype of proj: 0 bf16, 1 fp32.  proj [B * Tn, ld]: raw q (G * D channels) at column off_q, k (G * D) at off_k, v
@@ -361,6 +880,26 @@ NXD_API int nxd_delta_prep(int dtype, const void* proj, long long ld, int off_q,
     const int wpb = 8;
     const unsigned blocks = (unsigned)((units + wpb - 1) / wpb);
     cudaStream_t st = (cudaStream_t)stream;
+    {   // strips: V channels per lane, all rows and offsets multiples of V values, results and taps aligned
+        const int V = D / 32;
+        auto al = [](const void* p, size_t n) { return ((uintptr_t)p % n) == 0; };
+        if (taps == 4 && (D == 64 || D == 128 || D == 256) && Dv % D == 0 && ld % V == 0 && off_q % V == 0 && off_k % V == 0 &&
+            off_v % V == 0 && al(proj, 16) && al(conv_w, 16) && al(qn, 16) && al(kn, 16) && al(vn, 16) && B < 65536 &&
+            (Tn + PREP_STRIP - 1) / PREP_STRIP < 65536) {
+#define NXD_STRIP(T, V_)                                                                                                   \
+    return launch_prep_strip<T, V_>(proj, ld, off_q, off_k, off_v, conv_w, conv_state, qn, kn, vn, q_start, n_new, seq_ids, B, \
+                                    Tn, H, G, Dv, qscale, unit_eps, st)
+            if (dtype == 0) {
+                if (V == 2) NXD_STRIP(bf16, 2);
+                if (V == 4) NXD_STRIP(bf16, 4);
+                NXD_STRIP(bf16, 8);
+            }
+            if (V == 2) NXD_STRIP(float, 2);
+            if (V == 4) NXD_STRIP(float, 4);
+            NXD_STRIP(float, 8);
+#undef NXD_STRIP
+        }
+    }
     if (dtype == 0)
         delta_prep_kernel<bf16><<<blocks, wpb * 32, 0, st>>>((const bf16*)proj, ld, off_q, off_k, off_v, conv_w, conv_state, qn,
                                                             kn, vn, q_start, n_new, seq_ids, units, Tn, H, G, D, Dv, taps,
@@ -393,15 +932,24 @@ NXD_API int nxd_delta_conv_state(int dtype, const void* proj, long long ld, int 
     return 0;
 }
 
+// Floats of scratch with which nxd_delta_scan runs the chunk-wise form, 0 where it does not apply: one decay per head, key
+// sizes of 64 / 128 / 256, value sizes in whole slices of 32 columns, steps of at least three chunks (measured at 8 heads of 256 x
+// 512, token by token against chunks: 70 tokens 82 / 116 us, 128 tokens 113 / 117, 1024 tokens 610 / 374).
+NXD_API long long nxd_delta_scan_scratch(int B, int Tn, int H, int D, int Dv, int per_channel) {
+    if (per_channel || (D != 64 && D != 128 && D != 256) || Dv % CW_COLS != 0 || Tn < 3 * CH || B > 65535 || H > 65535) return 0;
+    return (long long)B * H * ((Tn + CH - 1) / CH) * CHUNK_FLOATS;
+}
+
 // qn, kn, vn as written by nxd_delta_prep.  apre fp32 [B * Tn, ld_a]: decay pre-activation of head h at column a_off + h
 // (per_channel == 0) or of (h, key channel i) at a_off + h * D + i; dt_bias [H] or [H * D], a_log [H]:
 // g = exp(-exp(a_log) softplus(apre + dt_bias)).  bpre fp32 [B * Tn, ld_b]: beta = sigmoid(bpre[b_off + h]).  Both are
 // OVERWRITTEN with g and beta (a first kernel, one thread per value; the recurrence then reads them).
-// S fp32 [lines, H, D, Dv], updated in place.  out fp32 [B * Tn, H, Dv].
+// S fp32 [lines, H, D, Dv], updated in place.  out fp32 [B * Tn, H, Dv].  scratch: nxd_delta_scan_scratch floats, or NULL
+// (token by token).
 NXD_API int nxd_delta_scan(const float* qn, const float* kn, const float* vn, float* apre, long long ld_a, int a_off,
                            float* bpre, long long ld_b, int b_off, const float* a_log, const float* dt_bias, float* S,
                            float* out, const int* q_start, const int* n_new, const int* seq_ids, int B, int Tn, int H, int G,
-                           int D, int Dv, int per_channel, void* stream) {
+                           int D, int Dv, int per_channel, float* scratch, void* stream) {
     if ((long long)B * Tn * H * Dv == 0) return 0;
     NXD_REQUIRE(G > 0 && H % G == 0, "delta rule: %d heads over %d query/key heads", H, G);
     NXD_REQUIRE(D >= 1 && D <= 1024, "delta rule: key size %d", D);
@@ -412,6 +960,16 @@ NXD_API int nxd_delta_scan(const float* qn, const float* kn, const float* vn, fl
     delta_gates_kernel<<<(unsigned)((vals + 255) / 256), 256, 0, st>>>(apre, ld_a, a_off, bpre, ld_b, b_off, a_log, dt_bias,
                                                                       N, H, per_head);
     NXD_LAUNCH_CHECK();
+    auto al = [](const void* p) { return ((uintptr_t)p % 16) == 0; };
+    if (scratch != nullptr && nxd_delta_scan_scratch(B, Tn, H, D, Dv, per_channel) > 0 && al(qn) && al(kn) && al(scratch)) {
+#define NXD_CHUNKS(D_)                                                                                                  \
+    return launch_chunks<D_>(qn, kn, vn, apre, ld_a, a_off, bpre, ld_b, b_off, S, out, scratch, q_start, n_new, seq_ids, B, Tn, \
+                             H, G, Dv, st)
+        if (D == 64) NXD_CHUNKS(64);
+        if (D == 128) NXD_CHUNKS(128);
+        NXD_CHUNKS(256);
+#undef NXD_CHUNKS
+    }
     // rows of a column per thread (NPT) and lanes per column (R, a power of two): the smallest slice that keeps R <= 4,
     // wider keys spread over more lanes (measured at 8 heads of 256 x 512, 2 x 4096 tokens: slices of 32 / 16 / 8 rows take
     // 4.5 / 7.8 / 13.8 ms -- fewer columns per CTA re-read the keys and queries more often)

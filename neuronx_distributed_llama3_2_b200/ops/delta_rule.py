@@ -128,11 +128,17 @@ def delta_scan(qn: torch.Tensor, kn: torch.Tensor, vn: torch.Tensor, a_pre: torc
         out = torch.empty(B, T, H, Dv, dtype=torch.float32, device=qn.device)
         qs, nn_, sid = _i32(q_start), _i32(n_new), _i32(seq_ids)
         L = _lib.lib(GROUP)
+        scratch = None
+        if not per_channel and T > 1:          # long steps run in chunks of 64 tokens
+            need = L.nxd_delta_scan_scratch
+            need.restype = _c.c_longlong
+            floats = need(_c.c_int(B), _c.c_int(T), _c.c_int(H), _c.c_int(D), _c.c_int(Dv), _c.c_int(0))
+            scratch = torch.empty(floats, dtype=torch.float32, device=qn.device) if floats else None
         rc = L.nxd_delta_scan(_lib.ptr(qn), _lib.ptr(kn), _lib.ptr(vn), _lib.ptr(a_pre), _c.c_longlong(a_pre.stride(0)),
                               _c.c_int(a_offset), _lib.ptr(b_pre), _c.c_longlong(b_pre.stride(0)), _c.c_int(b_offset),
                               _lib.ptr(a_log), _lib.ptr(dt_bias), _lib.ptr(S), _lib.ptr(out), _lib.ptr(qs), _lib.ptr(nn_),
                               _lib.ptr(sid), _c.c_int(B), _c.c_int(T), _c.c_int(H), _c.c_int(G), _c.c_int(D), _c.c_int(Dv),
-                              _c.c_int(int(per_channel)), _lib.stream_ptr())
+                              _c.c_int(int(per_channel)), _lib.ptr(scratch), _lib.stream_ptr())
         _lib.check(rc, "nxd_delta_scan", L)
         return out
     out = torch.zeros(B, T, H, Dv, dtype=torch.float32, device=qn.device)

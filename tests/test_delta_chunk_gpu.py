@@ -1,0 +1,113 @@
+"""Chunk-wise gated delta rule and the strip-wise short convolution ahead of it, against float64 token by token."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _oracle(q, k, v, g, beta, S):
+    """q, k [T, G, D], v [T, H, Dv], g, beta [T, H], S [H, D, Dv]."""
+    H, rep = v.shape[1], v.shape[1] // q.shape[1]
+    out = []
+    for t in range(q.shape[0]):
+        kt, qt = (x[t].repeat_interleave(rep, dim=0) for x in (k, q))
+        S = S * g[t].reshape(H, 1, 1)
+        u = beta[t].reshape(H, 1) * (v[t] - torch.einsum("hdv,hd->hv", S, kt))
+        S = S + kt.unsqueeze(-1) * u.unsqueeze(1)
+        out.append(torch.einsum("hdv,hd->hv", S, qt))
+    return torch.stack(out), S
+
+
+# steps around the 64-token chunk, ragged and empty rows, a second portion that continues the state; decays from none to total
+@pytest.mark.parametrize("D,H,G,Dv", [(64, 2, 2, 32), (64, 4, 2, 96), (128, 2, 1, 256), (256, 1, 1, 64)])
+@pytest.mark.parametrize("T,n_new", [(192, None), (257, [257, 1, 0]), (200, [129, 200, 64])])
+@pytest.mark.parametrize("strength", [-6.0, 0.0, 6.0])
+def test_chunks_match_float64(D, H, G, Dv, T, n_new, strength):
+    from neuronx_distributed_llama3_2_b200.ops import delta_rule as dr
+
+    B, lines = 3, 4
+    gen = torch.Generator(device="cuda").manual_seed(D + T)
+
+    def normal(*s):
+        return torch.randn(*s, generator=gen, device="cuda")
+
+    line = torch.tensor([2, 0, 3], dtype=torch.int32, device="cuda")
+    S = normal(lines, H, D, Dv)
+    a_log, dt_bias = normal(H) * 0.5 + strength, normal(H)
+    states, at = [None] * B, [0] * B
+    for _ in range(2):
+        q = F.normalize(normal(B, T, G, D), dim=-1) * D ** -0.5
+        k, v = F.normalize(normal(B, T, G, D), dim=-1), normal(B, T, H, Dv)
+        a_pre, b_pre = normal(B * T, H + 3), normal(B * T, H + 1)
+        new = None if n_new is None else torch.tensor(n_new, dtype=torch.int32, device="cuda")
+        g = torch.exp(-torch.exp(a_log.double()) * F.softplus(a_pre[:, 3:].double() + dt_bias.double())).reshape(B, T, H)
+        beta = torch.sigmoid(b_pre[:, 1:].double()).reshape(B, T, H)
+        before = S.clone()
+        out = dr.delta_scan(q, k, v, a_pre, 3, b_pre, 1, a_log, dt_bias, S, torch.tensor(at, dtype=torch.int32, device="cuda"),
+                            False, n_new=new, seq_ids=line)
+        assert torch.equal(S[1], before[1])              # a line that no row uses
+        for b in range(B):
+            n = T if n_new is None else n_new[b]
+            assert not out[b, n:].any()
+            if n == 0:
+                assert torch.equal(S[line[b]], before[line[b]])
+                continue
+            start = torch.zeros(H, D, Dv, dtype=torch.float64, device="cuda") if at[b] == 0 else states[b]
+            ref, states[b] = _oracle(q[b, :n].double(), k[b, :n].double(), v[b, :n].double(), g[b, :n], beta[b, :n], start)
+            at[b] += n
+            # per token a few roundings of 2^-24 (6e-8), each of which fades with the decay: the sums of exponentials that make
+            # g are off by 1e-7 of the decay's distance from one per step, which weak decays collect over all tokens so far
+            bound = (at[b] if strength < 0 else 8) ** 0.5 * 3e-7
+            assert (out[b, :n] - ref).norm() <= bound * ref.norm()
+            assert (S[line[b]] - states[b]).norm() <= bound * states[b].norm()
+
+
+def test_a_token_that_is_not_a_number_leaves_the_tokens_before_it_alone():
+    from neuronx_distributed_llama3_2_b200.ops import delta_rule as dr
+
+    T, D, Dv = 192, 64, 32
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    q, k = (F.normalize(torch.randn(1, T, 1, D, generator=gen, device="cuda"), dim=-1) for _ in range(2))
+    v = torch.randn(1, T, 1, Dv, generator=gen, device="cuda")
+    zero, start = torch.zeros(T, 1, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def run(value):
+        x = v.clone()
+        x[0, 70, 0, 3] = value
+        return dr.delta_scan(q, k, x, zero.clone(), 0, zero.clone(), 0, zero[0].clone(), zero[0].clone(),
+                             torch.zeros(1, 1, D, Dv, device="cuda"), start, False)[0, :, 0]
+
+    clean = run(0.5)
+    for bad in (float("nan"), float("inf")):
+        out = run(bad)
+        assert torch.equal(out[:70], clean[:70]) and not torch.isfinite(out[70:, 3]).any()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("D,H,G,Dv", [(64, 3, 1, 64), (128, 2, 2, 256), (256, 2, 1, 256)])
+def test_strips_of_the_short_convolution_match_float64(dtype, D, H, G, Dv):
+    from neuronx_distributed_llama3_2_b200.ops import delta_rule as dr
+
+    B, taps, C = 2, 4, 2 * G * D + H * Dv
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    total = 80
+    raw = torch.randn(B, total, C + 16, generator=gen, device="cuda").to(dtype)
+    w = torch.randn(C, taps, generator=gen, device="cuda") * 0.5
+    state = torch.randn(3, taps - 1, C, generator=gen, device="cuda")
+    line = torch.tensor([2, 0], dtype=torch.int32, device="cuda")
+    x = torch.cat([torch.zeros(B, taps - 1, C, dtype=torch.float64, device="cuda"), raw[..., 8:8 + C].double()], dim=1)
+    act = F.silu(sum(w[:, j].double() * x[:, j:j + total] for j in range(taps)))
+    q, k, v = act.split([G * D, G * D, H * Dv], dim=-1)
+    q, k = (t.unflatten(-1, (G, D)) for t in (q, k))
+    q, k = (t / torch.sqrt(t.square().sum(-1, keepdim=True) + 1e-6) for t in (q, k))
+    refs = (q * 0.25, k, v.unflatten(-1, (H, Dv)))
+    at = 0
+    for size in (1, 17, 3, 16, 43):                      # portions around the strips of 16
+        got = dr.delta_prep(raw[:, at:at + size].contiguous(), (8, 8 + G * D, 8 + 2 * G * D), w, state,
+                            torch.full((B,), at, dtype=torch.int32, device="cuda"), H, G, D, Dv, 0.25, seq_ids=line)
+        for x32, ref in zip(got, refs):
+            ref = ref[:, at:at + size]
+            assert (x32 - ref).norm() <= 1e-6 * ref.norm()          # four products and a silu in fp32
+        at += size
+    assert torch.equal(state[line.long()], raw[:, -3:, 8:8 + C].float())
