@@ -15,7 +15,8 @@
 //                      shared memory in blocks of 16.  A row that starts at position 0 starts from the zero state, any
 //                      other row continues from the state of its line; padding tokens (t >= n_new[b]) change nothing.
 //                      Serves token generation (one token), short steps and fp32 serving.
-//   retention_chunk_*  the chunk-wise form for long steps, three kernels (4 x 4 register tiles, value columns in tiles):
+//   retention_chunk_*  the chunk-wise form for long steps of the sizes and lengths that retention_tc.cu does not take, three
+//                      kernels (4 x 4 register tiles, value columns in tiles):
 //                        local   per (chunk, head, row, column tile): rotated q / k of the chunk in shared memory,
 //                                P[t][s] = decay^(t-s) (q_t . k_s) for s <= t, o_local = P v, and the chunk's own
 //                                contribution to the state U = sum_s decay^(L-1-s) k_s v_s^T

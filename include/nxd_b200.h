@@ -494,6 +494,12 @@ int nxd_retention_chunkwise(int dtype, const void* proj, long long ld, int q_off
                             float* state, float* out, float* U, float* qrot, const int* q_start, const int* n_new,
                             const int* seq_ids, int B, int Tn, int H, int D, int Dv, float kscale, const float* rope_cos,
                             const float* rope_sin, int rot, int halves, int max_pos, void* stream);
+/* the same on the tensor cores with fp32 accuracy (csrc/retention_tc.cu); workspace bytes, 0 where it does not apply */
+long long nxd_retention_tc_workspace(int dtype, int B, int Tn, int H, int D, int Dv);
+int nxd_retention_tc(int dtype, const void* proj, long long ld, int q_off, int k_off, int v_off, const float* decay,
+                     float* state, float* out, void* work, const int* q_start, const int* n_new, const int* seq_ids, int B,
+                     int Tn, int H, int D, int Dv, float kscale, const float* rope_cos, const float* rope_sin, int rot,
+                     int halves, int max_pos, void* stream);
 /* Hyper-connections (csrc/hyper_connection.cu): X [N, S, W] fp32 streams.  ya != NULL: x_t <- sum_s mix[s][t] x_s +
  * outw[t] * y with y = ya, or (yb != NULL) 0.5 * (rmsnorm(ya) * wa + rmsnorm(yb) * wb).  inw != NULL: h [N, W] = RMS norm
  * (weight wn) of sum_s inw[s] x_s, of the streams as the write left them.  y_dtype / h_dtype: 0 bf16, 1 fp32. */

@@ -22,6 +22,16 @@ from . import _lib
 
 GROUP = "retention_serving"
 CHUNK = 64
+
+# steps that run on the tensor cores (csrc/retention_tc.cu) where its sizes apply.  Measured against the fp32 kernels, one row, heads
+# x key x value size: 64 tokens 4 x 64 x 128 34 / 47 us, 4 x 128 x 256 67 / 60, 8 x 256 x 512 178 / 61; 128 tokens 50 / 48, 117 / 61,
+# 343 / 63; 4096 tokens 77 / 75, 225 / 108, 1942 / 317
+TC_MIN_TOKENS, TC_MIN_TOKENS_WIDE, TC_WIDE = 128, 64, 128
+
+
+def _tc_wanted(T: int, dim: int) -> bool:
+    return T >= (TC_MIN_TOKENS_WIDE if dim >= TC_WIDE else TC_MIN_TOKENS)
+
 _SMEM_LIMIT = 220 * 1024
 
 
@@ -95,6 +105,15 @@ def _launch(chunkwise: bool, proj, offsets, decay, state, q_start, heads, dim, v
     head = (_c.c_int(_code(proj.dtype)), _lib.ptr(proj), _c.c_longlong(ld), _c.c_int(offsets[0]), _c.c_int(offsets[1]),
             _c.c_int(offsets[2]), _lib.ptr(decay), _lib.ptr(state), _lib.ptr(out))
     L = _lib.lib(GROUP)
+    if chunkwise and _tc_wanted(T, dim):
+        need = L.nxd_retention_tc_workspace
+        need.restype = _c.c_longlong
+        size = need(_c.c_int(_code(proj.dtype)), _c.c_int(B), _c.c_int(T), _c.c_int(heads), _c.c_int(dim), _c.c_int(vdim))
+        if size and state.data_ptr() % 16 == 0:
+            work = torch.empty(size, dtype=torch.uint8, device=proj.device)
+            rc = L.nxd_retention_tc(*head, _lib.ptr(work), _lib.ptr(qs), _lib.ptr(nn_), _lib.ptr(sid), *tail)
+            _lib.check(rc, "nxd_retention_tc", L)
+            return out
     if chunkwise:
         nc = (T + CHUNK - 1) // CHUNK
         u = torch.empty(B, heads, nc, dim, vdim, dtype=torch.float32, device=proj.device)
