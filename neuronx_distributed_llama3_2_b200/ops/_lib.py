@@ -233,10 +233,16 @@ def _full_lib() -> ctypes.CDLL:
     return _lib
 
 
+_gpu_seen = False
+
+
 def available(group: Optional[str] = None) -> bool:
     """True when our CUDA kernels are usable (a GPU is present and the .so loads)."""
-    if not torch.cuda.is_available():
-        return False
+    global _gpu_seen
+    if not _gpu_seen:                # asked ahead of every op: a GPU that is there stays there
+        if not torch.cuda.is_available():
+            return False
+        _gpu_seen = True
     if os.environ.get("NXD_FORCE_TORCH", "0") == "1":
         return False
     try:
@@ -262,7 +268,8 @@ def kernel_launches() -> int:
 
 
 def stream_ptr() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream of the current device, without a ``Stream`` object in between (5 us of every launch)."""
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def check(code: int, what: str, handle: Optional[ctypes.CDLL] = None) -> None:
