@@ -99,6 +99,59 @@ __global__ void rope_kernel(bf16* __restrict__ x, const float* __restrict__ cos_
     }
 }
 
+// Prompt step: queries and keys rotated in place, and the step's rotated keys and values written to the cache, in one pass over the
+// projection.  Item = 8 columns of each half of a head.  Bound by memory; on 2048 tokens x 48 heads of 64 it replaces the rotation
+// (9.4 us), two transposing copies (8.8), the cache write (3.6) and four index conversions (8).
+__global__ void rope_cache_kernel(bf16* __restrict__ x, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                                  const int* __restrict__ positions, bf16* __restrict__ cache_k, bf16* __restrict__ cache_v,
+                                  const int* __restrict__ seq_ids, const int* __restrict__ block_table, long long stride_b,
+                                  long long stride_h, int page_size, int max_pages, int Tn, size_t rows, int n_q, int n_kv, int D) {
+    const int half_vec = D >> 4, heads = n_q + 2 * n_kv;
+    const size_t total = rows * (size_t)heads * half_vec;
+    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
+        const int c = (int)(idx % half_vec);
+        const size_t th = idx / half_vec;
+        const int h = (int)(th % heads);
+        const size_t row = th / heads;
+        bf16* base = x + (row * heads + h) * (size_t)D;
+        bf16x8 va = reinterpret_cast<bf16x8*>(base)[c], vb = reinterpret_cast<bf16x8*>(base + (D >> 1))[c];
+        if (h < n_q + n_kv) {
+            const int pos = positions[row];
+            float a[8], b[8], oa[8], ob[8];
+            unpack8(va, a);
+            unpack8(vb, b);
+            const float4* cp = reinterpret_cast<const float4*>(cos_t + (size_t)pos * (D >> 1) + c * 8);
+            const float4* sp = reinterpret_cast<const float4*>(sin_t + (size_t)pos * (D >> 1) + c * 8);
+            const float4 c0 = cp[0], c1 = cp[1], s0 = sp[0], s1 = sp[1];
+            const float cs[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+            const float sn[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                oa[k] = a[k] * cs[k] - b[k] * sn[k];
+                ob[k] = b[k] * cs[k] + a[k] * sn[k];
+            }
+            va = pack8(oa);
+            vb = pack8(ob);
+            reinterpret_cast<bf16x8*>(base)[c] = va;
+            reinterpret_cast<bf16x8*>(base + (D >> 1))[c] = vb;
+        }
+        if (h >= n_q) {
+            const int b = (int)(row / Tn), t = (int)(row % Tn);
+            const int line = seq_ids ? seq_ids[b] : b, at = positions[(size_t)b * Tn] + t;     // rows follow the first position
+            const int kv = h < n_q + n_kv ? h - n_q : h - n_q - n_kv;
+            size_t off;
+            if (block_table)
+                off = (size_t)block_table[(size_t)line * max_pages + at / page_size] * stride_b + (size_t)kv * stride_h +
+                      (size_t)(at % page_size) * D;
+            else
+                off = (size_t)line * stride_b + (size_t)kv * stride_h + (size_t)at * D;
+            bf16* dst = (h < n_q + n_kv ? cache_k : cache_v) + off;
+            reinterpret_cast<bf16x8*>(dst)[c] = va;
+            reinterpret_cast<bf16x8*>(dst + (D >> 1))[c] = vb;
+        }
+    }
+}
+
 inline int grid_for(size_t work_items, int threads) {
     size_t blocks = (work_items + threads - 1) / threads;
     const size_t cap = (size_t)nxd_num_sms() * 16;
@@ -143,6 +196,21 @@ NXD_API int nxd_rope_inplace(void* x, const float* cos_t, const float* sin_t, co
     rope_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
         (bf16*)x, cos_t, sin_t, positions, (size_t)T, heads_total, n_rot_heads, D, pos_div < 1 ? 1 : pos_div,
         pos_mod < 1 ? 1 : pos_mod, inverse ? -1.f : 1.f);
+    NXD_LAUNCH_CHECK();
+    return 0;
+}
+
+// qkv [B * Tn, n_q + 2 n_kv, D] bf16 (q | k | v heads): q and k rotated in place at positions [B * Tn] int32; row t of sequence b
+// goes to cache row positions[b * Tn] + t of line seq_ids[b] (NULL: b).  Cache as in nxd_kv_cache_update.  D a multiple of 16.
+NXD_API int nxd_rope_cache_write(void* qkv, const float* cos_t, const float* sin_t, const int* positions, void* cache_k,
+                                 void* cache_v, const int* seq_ids, const int* block_table, long long stride_b, long long stride_h,
+                                 int page_size, int max_pages, int B, int Tn, int n_q, int n_kv, int D, void* stream) {
+    NXD_REQUIRE(D % 16 == 0, "rope_cache: head dim %d must be a multiple of 16", D);
+    const size_t rows = (size_t)B * Tn;
+    if (rows == 0) return 0;
+    rope_cache_kernel<<<grid_for(rows * (n_q + 2 * n_kv) * (D / 16), 256), 256, 0, (cudaStream_t)stream>>>(
+        (bf16*)qkv, cos_t, sin_t, positions, (bf16*)cache_k, (bf16*)cache_v, seq_ids, block_table, stride_b, stride_h,
+        page_size > 0 ? page_size : 1, max_pages, Tn, rows, n_q, n_kv, D);
     NXD_LAUNCH_CHECK();
     return 0;
 }

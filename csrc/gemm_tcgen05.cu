@@ -56,14 +56,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     const uint32_t cta_rank = ptx::cluster_ctarank();
     const bool is_leader = cta_rank == 0;
 
-    constexpr int kOutN = SEG == kSegGlu ? BN / 2 : BN;      // output columns of a tile (gate and up share one)
+    constexpr bool kSorted = SEG == kSegPlain || SEG == kSegGlu || SEG == kSegRelu2, kGlu = SEG == kSegGlu || SEG == kDenseGlu;
+    constexpr int kOutN = kGlu ? BN / 2 : BN;                // output columns of a tile (gate and up share one)
     const int num_m_tiles = (M + kTileM - 1) / kTileM;
     const int num_n_tiles = (N + kOutN - 1) / kOutN;
     const int tiles_per_batch = num_m_tiles * num_n_tiles;
     int num_tiles = tiles_per_batch * (GROUPED ? batches : 1);
     int* seg_tile = reinterpret_cast<int*>(smem + L::kBarrierOffset + L::kBarrierBytes);   // first tile of every expert
     int* seg_row = seg_tile + kSegMaxExperts + 1;                                          // first row of every expert
-    if constexpr (SEG != kSegOff) {
+    if constexpr (kSorted) {
         if (warp == 3) segment_starts(seg.counts, batches, num_n_tiles, seg_row, seg_tile);
     }
     const int num_k_blocks = (K + kBlockK - 1) / kBlockK;
@@ -91,11 +92,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     ptx::cluster_sync();
     ptx::tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_ptr_smem;
-    if constexpr (SEG != kSegOff) num_tiles = seg_tile[batches];
+    if constexpr (kSorted) num_tiles = seg_tile[batches];
     // problem index, tile coordinates and first row of a tile
     auto locate = [&](int tile, int& e, int& tm, int& tn, int& row_base) {
         row_base = 0;
-        if constexpr (SEG != kSegOff) {
+        if constexpr (kSorted) {
             int lo = 0, hi = batches;                        // seg_tile[lo] <= tile < seg_tile[hi]
             while (hi - lo > 1) {
                 const int mid = (lo + hi) >> 1;
@@ -122,7 +123,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 const int m0 = row_base + tm * kTileM + (int)cta_rank * kBlockM;
                 // gate and up of the same columns meet in one tile: the pair's first CTA stages the gate half of B, the
                 // second the up half
-                const int n0 = SEG == kSegGlu ? (int)cta_rank * N + tn * kOutN : tn * BN + (int)cta_rank * (BN / 2);
+                const int n0 = kGlu ? (int)cta_rank * N + tn * kOutN : tn * BN + (int)cta_rank * (BN / 2);
                 for (int kb = 0; kb < num_k_blocks; ++kb) {
                     ptx::mbar_wait(&empty_bar[stage], phase ^ 1);
                     uint8_t* sa = smem + stage * L::kStageBytes;
@@ -130,7 +131,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                     const int k0 = kb * kBlockK;
                     if (is_leader) ptx::mbar_arrive_expect_tx(&full_bar[stage], 2 * L::kStageBytes);
                     auto load = [&](const CUtensorMap* map, void* dst, int c0, int c1) {
-                        if (SEG && map == &tmap_a) ptx::tma_load_2d_pair(map, &full_bar[stage], dst, c0, c1);
+                        if (kSorted && map == &tmap_a) ptx::tma_load_2d_pair(map, &full_bar[stage], dst, c0, c1);
                         else if constexpr (GROUPED) ptx::tma_load_3d_pair(map, &full_bar[stage], dst, c0, c1, e);
                         else ptx::tma_load_2d_pair(map, &full_bar[stage], dst, c0, c1);
                     };
@@ -201,7 +202,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             const int row0 = row_base + tm * kTileM + (int)cta_rank * kBlockM + q * 32;
             const int n0 = tn * kOutN;
             // experts start at multiples of 32 rows, so a warp's 32 rows never hold two experts' rows
-            const int row_end = SEG ? row_base + seg.counts[e] : M;
+            const int row_end = kSorted ? row_base + seg.counts[e] : M;
             ptx::mbar_wait(&tmem_full_bar[acc], acc_phase);
             ptx::tcgen05_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
@@ -212,7 +213,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 uint32_t r[kCols];
                 ptx::tmem_ld_32x32b_x32(taddr + c * kCols, r);
                 if constexpr (kCols == 64) ptx::tmem_ld_32x32b_x32(taddr + c * kCols + 32, r + 32);
-                if constexpr (SEG == kSegGlu) {
+                if constexpr (kGlu) {
 #pragma unroll
                     for (int half = 0; half < kCols / 32; ++half) {
                         uint32_t up[32];
@@ -259,7 +260,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 if (lane == 0) {
                     const int col0 = n0 + c * kCols;
                     if (col0 < N && row0 < row_end) {
-                        if constexpr (GROUPED && SEG == kSegOff) {
+                        if constexpr (GROUPED && !kSorted) {
                             if constexpr (OUT_MODE == kOutF32Acc)
                                 ptx::tma_reduce_add_3d(&tmap_d, stg + buf * (32 * 128), col0, row0, e);
                             else
@@ -498,6 +499,48 @@ NXD_API int nxd_experts_gemm_bf16(const void* a, const void* b, void* d, const i
                                   int K, int mode, float limit, float alpha, float up_shift, void* stream) {
     nxd_gemm::SegArgs seg{counts, limit, alpha, up_shift};
     return nxd_gemm::run_experts(a, b, d, seg, E, rows, pairs, N, K, mode, (cudaStream_t)stream);
+}
+
+namespace nxd_gemm {
+
+template <int BN>
+static int launch_glu(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, int M, int N, int K,
+                      const SegArgs& act, cudaStream_t stream) {
+    using L = SmemLayout<BN>;
+    auto kern = gemm_pair_kernel<BN, false, false, kOutBF16, false, kDenseGlu>;
+    static bool configured = false;
+    if (!configured) {
+        NXD_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes));
+        configured = true;
+    }
+    const long tiles = (long)((M + kTileM - 1) / kTileM) * ((N + BN / 2 - 1) / (BN / 2));
+    long clusters = nxd_num_sms() / 2;
+    if (clusters > tiles) clusters = tiles;
+    kern<<<dim3((unsigned)clusters * 2), dim3(kThreads), L::kSmemBytes, stream>>>(ta, tb, td, M, N, K, 1, act);
+    NXD_LAUNCH_CHECK();
+    return 0;
+}
+
+}  // namespace nxd_gemm
+
+// D[M, N] = glu(A W_gate^T, A W_up^T): A [M, K], W [2 N, K] (gate rows first), the gated activation (SegArgs::glu; limit = inf,
+// alpha = 1, up_shift = 0: silu(gate) * up) on the fp32 products in the epilogue, as in run_experts.  2048 x 8192 x 2048: the
+// product alone 79 us and an activation kernel of 17 us that reads 67 MB and writes 34; together in one launch 84 us.  K, N and the pitches multiples of 8 elements, bases 16-byte aligned.
+NXD_API int nxd_gemm_glu_bf16(const void* a, const void* w, void* d, int M, int N, int K, long long lda, long long ldw,
+                              long long ldd, float limit, float alpha, float up_shift, void* stream) {
+    using namespace nxd_gemm;
+    NXD_REQUIRE(M > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "gemm_glu: %d x %d x %d", M, N, K);
+    NXD_REQUIRE(lda % 8 == 0 && ldw % 8 == 0 && ldd % 8 == 0, "gemm_glu: pitches must be multiples of 8 elements (%lld)", lda);
+    NXD_REQUIRE((((uintptr_t)a | (uintptr_t)w | (uintptr_t)d) & 15) == 0, "gemm_glu: operands must be %s", "16-byte aligned");
+    const int bn = pick_block_n(M, 2 * N);
+    CUtensorMap ta, tb, td;
+    int rc;
+    if ((rc = make_tmap_2d(&ta, a, (uint64_t)K, (uint64_t)M, (uint64_t)lda, 64, kBlockM))) return rc;
+    if ((rc = make_tmap_2d(&tb, w, (uint64_t)K, (uint64_t)2 * N, (uint64_t)ldw, 64, bn / 2))) return rc;
+    if ((rc = make_tmap_2d(&td, d, (uint64_t)N, (uint64_t)M, (uint64_t)ldd, 64, 32, 2))) return rc;
+    const SegArgs act{nullptr, limit, alpha, up_shift};
+    return bn == 256 ? launch_glu<256>(ta, tb, td, M, N, K, act, (cudaStream_t)stream)
+                     : launch_glu<128>(ta, tb, td, M, N, K, act, (cudaStream_t)stream);
 }
 
 // Grouped (batched over experts) GEMM: E problems of one shape in ONE launch.  a / b / d point at problem 0, stride_*

@@ -51,7 +51,7 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m_tiles, int num_n
 }
 
 // Rows sorted by expert (sparse mixtures): what the GEMM kernel's SEG variants and the kernels that sort the rows agree on.
-enum { kSegOff = 0, kSegPlain = 1, kSegGlu = 2, kSegRelu2 = 3 };
+enum { kSegOff = 0, kSegPlain = 1, kSegGlu = 2, kSegRelu2 = 3, kDenseGlu = 4 };   // kDenseGlu: one dense problem, no sorting
 constexpr int kSegMaxExperts = 128;
 constexpr int kSegSmemBytes = 2 * (kSegMaxExperts + 1) * 4;
 constexpr int kSegAlign = 32;   // an expert's rows start at a multiple: the 32 rows of an epilogue warp's store

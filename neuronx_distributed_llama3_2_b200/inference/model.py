@@ -18,6 +18,7 @@ unchanged.  Differences from the training forward:
 """
 from __future__ import annotations
 
+import os
 from typing import Optional, Tuple
 
 import torch
@@ -275,7 +276,67 @@ class KVCacheInferenceMixin:
             x3 = mlp.down_proj(act.reshape(B, 1, -1)).reshape(B, -1) + x2
         return x3.reshape(B, 1, -1), None
 
+    # -- prompt layer on direct kernel calls (8 launches) ---------------------------------------------------------------
+    def _prompt_layer_ok(self, layer, hidden: torch.Tensor, residual) -> bool:
+        """The plain Llama layer (``_fused_decode_ok``) on one process with the native kernels, more rows than the
+        token-generation kernels take, and nothing hooked into the modules that are passed by."""
+        from ..ops import backend
+
+        B, T, H = hidden.shape
+        if (B * T <= 128 or not hidden.is_cuda or hidden.dtype != torch.bfloat16 or H % 8 or not hidden.is_contiguous()
+                or ps.get_tensor_model_parallel_size() > 1 or backend.attn_backend() != "nxd"
+                or os.environ.get("NXD_ATTN_FWD", "tc") != "tc"):
+            return False
+        self._fused_decode_ok(layer, hidden[:1, 0])            # fills the layer's flag
+        if not layer._nxd_fused_decode or backend.gemm_backend() != "tcgen05" or not attn_ops._lib.available():
+            return False
+        cls = type(self)
+        if (cls._attention is not KVCacheInferenceMixin._attention or cls._qkv_to_cache is not KVCacheInferenceMixin._qkv_to_cache
+                or cls._layer is not KVCacheInferenceMixin._layer or self.kv_cache.k[0].dtype != torch.bfloat16):
+            return False
+        attn, mlp = layer.self_attn, layer.mlp
+        mods = (layer.input_layernorm, layer.post_attention_layernorm, attn, attn.qkv_proj, attn.o_proj, mlp, mlp.gate_up_proj,
+                mlp.down_proj)
+        if any(m._forward_hooks or m._forward_pre_hooks for m in mods):
+            return False
+        norms = (layer.input_layernorm.weight, layer.post_attention_layernorm.weight)
+        ws = (attn.qkv_proj.weight_qkv, attn.o_proj.weight, mlp.gate_up_proj.weight, mlp.down_proj.weight)
+        return (all(w.dtype == torch.bfloat16 and w.is_contiguous() for w in norms)
+                and all(w.dtype == torch.bfloat16 and w.stride(1) == 1 and w.shape[0] % 16 == 0 and w.shape[1] % 8 == 0
+                        and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0 for w in ws)
+                and (residual is None or (residual.dtype == torch.bfloat16 and residual.is_contiguous())))
+
+    def _layer_prompt(self, i: int, layer, hidden, residual, positions, seq_ids):
+        """RMSNorm | QKV GEMM | rotation + cache write | attention | o_proj | RMSNorm | gate/up GEMM with the activation |
+        down_proj, each a direct kernel call: no autograd wrappers, transposing copies or index conversions per layer."""
+        from ..ops.flash_attn import flash_attn_forward
+        from ..ops.gemm import gemm, gemm_swiglu
+
+        B, T, H = hidden.shape
+        attn, mlp = layer.self_attn, layer.mlp
+        nq, nkv, D = attn.q_heads_local, attn.kv_heads_local, attn.head_dim
+        if "prompt_i32" not in self._step_kv:        # int32 copies once per step, not per layer
+            self._step_kv["prompt_i32"] = (positions.to(torch.int32).contiguous(),
+                                           seq_ids.to(torch.int32).contiguous() if seq_ids is not None else None)
+        pos, sid = self._step_kv["prompt_i32"]
+        cos, sin = self._rope(hidden.device)
+        kc = self.kv_cache
+        ck, cv = kc.layer(i)
+        xn, x = norm_ops.rms_norm_forward(hidden, layer.input_layernorm.weight, layer.input_layernorm.variance_epsilon, residual)
+        qkv = gemm(xn.view(B * T, H), attn.qkv_proj.weight_qkv, "nt").view(B, T, nq + 2 * nkv, D)
+        rope_ops.rope_cache_write_(qkv, cos, sin, pos, ck, cv, nq, nkv, seq_ids=sid,
+                                   block_table=kc.block_table if kc.paged else None, page_size=kc.page_size if kc.paged else 0)
+        heads = qkv.permute(0, 2, 1, 3)
+        o = flash_attn_forward(heads[:, :nq], heads[:, nq:nq + nkv], heads[:, nq + nkv:], D ** -0.5)
+        a = gemm(o.permute(0, 2, 1, 3).reshape(B * T, nq * D), attn.o_proj.weight, "nt").view(B, T, H)
+        norm = layer.post_attention_layernorm
+        xn, x = norm_ops.rms_norm_forward(a, norm.weight, norm.variance_epsilon, x)
+        act = gemm_swiglu(xn.view(B * T, H), mlp.gate_up_proj.weight)
+        return gemm(act, mlp.down_proj.weight, "nt").view(B, T, H), x
+
     def _layer(self, i: int, layer, hidden, residual, positions, seq_ids, lengths, prefill):
+        if prefill and not self._step_past_context and self._prompt_layer_ok(layer, hidden, residual):
+            return self._layer_prompt(i, layer, hidden, residual, positions, seq_ids)
         if not prefill and hidden.shape[1] == 1:
             if self._fused_decode_ok(layer, hidden):
                 return self._layer_fused_decode(i, layer, hidden, residual, positions, seq_ids, lengths)

@@ -34,6 +34,18 @@ def _strides(*ts) -> "_c.Array":
     return (_c.c_longlong * len(vals))(*vals)
 
 
+def flash_attn_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: float) -> torch.Tensor:
+    """Causal attention on the tcgen05 kernel without autograd or the log-sum-exp (serving): strided bf16 views with unit
+    stride on the last dimension and other strides multiples of 8."""
+    B, Hq, Sq, D = q.shape
+    o = torch.empty(B, Sq, Hq, D, dtype=q.dtype, device=q.device).permute(0, 2, 1, 3)
+    rc = _lib.lib().nxd_flash_attn_fwd_tc(
+        _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(o), _lib.ptr(None), _strides(q, k, v, o), _c.c_int(B), _c.c_int(Hq),
+        _c.c_int(k.shape[1]), _c.c_int(Sq), _c.c_int(k.shape[2]), _c.c_int(D), _c.c_float(scale), _c.c_int(1), _lib.stream_ptr())
+    _lib.check(rc, "nxd_flash_attn_fwd_tc")
+    return o
+
+
 class _FlashAttnFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, scale, causal, dropout_p=0.0, seed=0):

@@ -53,6 +53,21 @@ def gemm(a: torch.Tensor, b: torch.Tensor, layout: str, out: Optional[torch.Tens
     return out
 
 
+def gemm_swiglu(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """``silu(x W_gate^T) * (x W_up^T)`` in one launch: ``x [M, K]``, ``w [2 I, K]`` with the gate rows first -> ``[M, I]``;
+    the activation is applied to the fp32 products.  bf16, unit inner strides, ``K`` and ``I`` multiples of 8."""
+    m, k = x.shape
+    n = w.shape[0] // 2
+    assert w.shape[1] == k and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.stride(1) == 1 and w.stride(1) == 1
+    out = torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
+    rc = _lib.lib().nxd_gemm_glu_bf16(
+        _lib.ptr(x), _lib.ptr(w), _lib.ptr(out), _c.c_int(m), _c.c_int(n), _c.c_int(k), _c.c_longlong(x.stride(0)),
+        _c.c_longlong(w.stride(0)), _c.c_longlong(n), _c.c_float(float("inf")), _c.c_float(1.0), _c.c_float(0.0),
+        _lib.stream_ptr())
+    _lib.check(rc, "nxd_gemm_glu_bf16")
+    return out
+
+
 def gemm_grouped(a: torch.Tensor, b: torch.Tensor, layout: str, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``E`` GEMMs of one shape in ONE launch (``nxd_gemm_grouped_bf16``: 3-D tensor maps, the persistent tile loop runs
     over every expert's tiles; rows past an expert's extent are out of bounds of the map, so the row count needs no

@@ -19,6 +19,19 @@ def rms_norm_ref(x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
     return (y * w.float()).to(x.dtype)
 
 
+def rms_norm_forward(x: torch.Tensor, w: torch.Tensor, eps: float, residual: Optional[torch.Tensor] = None):
+    """``(rmsnorm(x + residual), x + residual)`` of contiguous bf16 rows on the GPU without autograd (serving); the second is
+    ``x`` itself without a residual."""
+    y = torch.empty_like(x)
+    s = torch.empty_like(x) if residual is not None else x
+    H = x.shape[-1]
+    rc = _lib.lib().nxd_rmsnorm_fwd(_lib.ptr(x), _lib.ptr(residual), _lib.ptr(w), _lib.ptr(y),
+                                    _lib.ptr(s if residual is not None else None), _lib.ptr(None), _c.c_int(x.numel() // H),
+                                    _c.c_int(H), _c.c_float(eps), _lib.stream_ptr())
+    _lib.check(rc, "nxd_rmsnorm_fwd")
+    return y, s
+
+
 class _RMSNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, eps, residual):

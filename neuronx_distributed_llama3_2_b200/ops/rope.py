@@ -159,3 +159,20 @@ def rope_inplace_(x: torch.Tensor, cos, sin, n_rot_heads: int, pos_div: int = 1,
         return x
     x.copy_(rope_ref(x, cos, sin, n_rot_heads, pos_div, pos_mod, positions))
     return x
+
+
+def rope_cache_write_(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, positions: torch.Tensor, cache_k: torch.Tensor,
+                      cache_v: torch.Tensor, n_q: int, n_kv: int, seq_ids: Optional[torch.Tensor] = None,
+                      block_table: Optional[torch.Tensor] = None, page_size: int = 0) -> torch.Tensor:
+    """Prompt step on the GPU: ``qkv [B, T, n_q + 2 n_kv, D]`` bf16, contiguous; queries and keys are rotated in place at
+    ``positions [B, T]`` and the step's keys and values written to rows ``positions[b, 0] + t`` of cache line ``seq_ids[b]``
+    (default ``b``), one launch.  ``positions`` / ``seq_ids`` / ``block_table`` int32."""
+    B, T, heads, D = qkv.shape
+    assert heads == n_q + 2 * n_kv and qkv.is_contiguous() and positions.dtype == torch.int32 and positions.is_contiguous()
+    rc = _lib.lib().nxd_rope_cache_write(
+        _lib.ptr(qkv), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(positions), _lib.ptr(cache_k), _lib.ptr(cache_v),
+        _lib.ptr(seq_ids), _lib.ptr(block_table), _c.c_longlong(cache_k.stride(0)), _c.c_longlong(cache_k.stride(1)),
+        _c.c_int(page_size), _c.c_int(block_table.shape[1] if block_table is not None else 0), _c.c_int(B), _c.c_int(T),
+        _c.c_int(n_q), _c.c_int(n_kv), _c.c_int(D), _lib.stream_ptr())
+    _lib.check(rc, "nxd_rope_cache_write")
+    return qkv
