@@ -216,18 +216,20 @@ __global__ void __launch_bounds__(128) decode_attn_split_kernel(
 // through a per-warp cp.async ring, so the next two tiles are in flight while the current one is multiplied (the FMA
 // kernel above issues its loads and then waits for them, every iteration).
 //
-//   grid = (B * n_kv, n_splits), 4 warps; warp w owns the 32-key tiles w, w + 4, ... of the split and keeps its own
+//   grid = (B * n_kv, n_splits), 4 warps; warp w owns the kTile-key tiles w, w + 4, ... of the split and keeps its own
 //   online-softmax state (m, l, O[16 x D]) in registers; the four states merge through shared memory at the end.
-//   Per tile: S[16 x 32] = Q K^T (D / 16 k-steps x 4 key blocks), P = exp2(scale * (S - m)), O += P V
-//   (2 k-steps x D / 8 channel blocks, V fragments through ldmatrix.trans).
+//   Per tile: S[16 x kTile] = Q K^T (D / 16 k-steps x kTile / 8 key blocks), P = exp2(scale * (S - m)), O += P V
+//   (kTile / 16 k-steps x D / 8 channel blocks, V fragments through ldmatrix.trans).
 template <int D>
 struct MmaDecodeCfg {
     static constexpr int kWarps = 4;
-    static constexpr int kTile = 32;                          // keys per warp step
+    // keys per warp step; at 128 columns 32 of them would fill the SM's shared memory with one CTA's rings, and a second CTA
+    // hides the first one's start and merge
+    static constexpr int kTile = D <= 64 ? 32 : 16;
     static constexpr int kStages = 3;
     static constexpr int kTileBytes = kTile * D * 2;          // one of K or V
     static constexpr int kWarpBytes = kStages * 2 * kTileBytes;
-    static constexpr int kSmemBytes = kWarps * kWarpBytes;    // 96 KB (D = 64) / 192 KB (D = 128)
+    static constexpr int kSmemBytes = kWarps * kWarpBytes;    // 96 KB: two CTAs per SM
     static_assert(kWarps * 16 * (D + 4) * 4 + kWarps * 32 * 4 <= kSmemBytes, "merge buffers alias the ring");
 };
 
@@ -274,18 +276,35 @@ __global__ void __launch_bounds__(128) decode_attn_mma_kernel(
 
     const int n_tiles = end > start ? (end - start + C::kTile - 1) / C::kTile : 0;
     const int my_tiles = n_tiles > warp ? (n_tiles - warp + C::kWarps - 1) / C::kWarps : 0;
+    const int line = cache.seq_ids ? cache.seq_ids[b] : b;
+    const bool whole_tiles = cache.block_table == nullptr || cache.page_size % C::kTile == 0;
+    auto tile_offset = [&](int key) {       // of key (a multiple of the tile) from the cache's start
+        const size_t head = (size_t)hk * cache.stride_h;
+        if (cache.block_table == nullptr) return (size_t)line * cache.stride_b + head + (size_t)key * D;
+        const int pg = key / cache.page_size;
+        return (size_t)cache.block_table[(size_t)line * cache.max_pages + pg] * cache.stride_b + head +
+               (size_t)(key - pg * cache.page_size) * D;
+    };
     auto issue = [&](int i) {       // tile i of this warp -> ring stage i % kStages (an empty group beyond the last tile)
         if (i < my_tiles) {
             const int key0 = start + (warp + i * C::kWarps) * C::kTile;
             const uint32_t sk = ring + (i % C::kStages) * 2 * C::kTileBytes, sv = sk + C::kTileBytes;
             constexpr int CH = D / 8;
+            // the tile's 32 keys are neighbours in memory (contiguous cache, or a page that holds whole tiles): one address
+            // per tile and a constant step per piece.  Looking every piece's row up (two integer divisions and a table read
+            // for 16 bytes) took 2.5 times as long as the memory on a paged cache.
+            const bool whole = whole_tiles;
+            const size_t base = whole ? tile_offset(key0) : 0;
+            const int r0 = lane / CH, c = lane % CH;
 #pragma unroll
             for (int j = 0; j < C::kTile * CH / 32; ++j) {
-                const int idx = lane + j * 32;
-                const int r = idx / CH, c = idx % CH;
+                const int r = r0 + j * (32 / CH);
                 const int pos = key0 + r;
                 const bool ok = pos < end;
-                const size_t off = row_ptr(cache.k, cache, b, hk, ok ? pos : start, D) - cache.k + c * 8;
+                size_t off;
+                if (whole) off = base + (ok ? r * D : 0);
+                else off = row_ptr(cache.k, cache, b, hk, ok ? pos : start, D) - cache.k;
+                off += c * 8;
                 mma::cp_async16(mma::tile_addr<D>(sk, r, c), cache.k + off, ok);
                 mma::cp_async16(mma::tile_addr<D>(sv, r, c), cache.v + off, ok);   // rows past the end: zeros (0 * NaN)
             }
@@ -301,13 +320,14 @@ __global__ void __launch_bounds__(128) decode_attn_mma_kernel(
         __syncwarp();
         const int key0 = start + (warp + i * C::kWarps) * C::kTile;
         const uint32_t sk = ring + (i % C::kStages) * 2 * C::kTileBytes, sv = sk + C::kTileBytes;
-        float s[4][4];
+        constexpr int NT = C::kTile / 8;
+        float s[NT][4];
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
+        for (int nt = 0; nt < NT; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
 #pragma unroll
-            for (int nb = 0; nb < 2; ++nb) {
+            for (int nb = 0; nb < NT / 2; ++nb) {
                 uint32_t kb[4];
                 mma::load_b<D>(kb, sk, nb * 16, kk, lane);
                 mma::mma16816(s[2 * nb], qa[kk], kb[0], kb[1]);
@@ -316,7 +336,7 @@ __global__ void __launch_bounds__(128) decode_attn_mma_kernel(
         }
         if (key0 + C::kTile > end) {      // the last tile of the split: keys past the end do not take part
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt)
+            for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
                     if (key0 + nt * 8 + 2 * t4 + (c & 1) >= end) s[nt][c] = -INFINITY;
@@ -326,7 +346,7 @@ __global__ void __launch_bounds__(128) decode_attn_mma_kernel(
         for (int r = 0; r < 2; ++r) {
             float mx = fmaxf(s[0][2 * r], s[0][2 * r + 1]);
 #pragma unroll
-            for (int nt = 1; nt < 4; ++nt) mx = fmaxf(mx, fmaxf(s[nt][2 * r], s[nt][2 * r + 1]));
+            for (int nt = 1; nt < NT; ++nt) mx = fmaxf(mx, fmaxf(s[nt][2 * r], s[nt][2 * r + 1]));
             mx = mma::quad_max(mx);
             const float m_new = fmaxf(m_run[r], mx);      // finite: the first key of a tile is always inside the split
             alpha[r] = exp2f((m_run[r] - m_new) * scale_log2);
@@ -334,9 +354,9 @@ __global__ void __launch_bounds__(128) decode_attn_mma_kernel(
             mneg[r] = -m_new * scale_log2;
             l_run[r] *= alpha[r];
         }
-        uint32_t pa[2][4];
+        uint32_t pa[NT / 2][4];
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
+        for (int nt = 0; nt < NT; ++nt) {
             const float p0 = exp2f(fmaf(s[nt][0], scale_log2, mneg[0])), p1 = exp2f(fmaf(s[nt][1], scale_log2, mneg[0]));
             const float p2 = exp2f(fmaf(s[nt][2], scale_log2, mneg[1])), p3 = exp2f(fmaf(s[nt][3], scale_log2, mneg[1]));
             l_run[0] += p0 + p1;
@@ -352,7 +372,7 @@ __global__ void __launch_bounds__(128) decode_attn_mma_kernel(
             o[j][3] *= alpha[1];
         }
 #pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
+        for (int ks = 0; ks < NT / 2; ++ks) {
 #pragma unroll
             for (int dj = 0; dj < D / 16; ++dj) {
                 uint32_t vb[4];
@@ -406,23 +426,37 @@ __global__ void __launch_bounds__(128) decode_attn_mma_kernel(
     }
 }
 
+// D threads per (sequence, query head).  A chain of loads: the weights of all splits come from one load per lane and a warp
+// reduction, the partial rows are read eight at a time (split by split, a merge of 16 splits took longer than the attention
+// of 128 keys).
+constexpr int kMaxSplits = 64;
+
 template <int D>
-__global__ void decode_attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                         bf16* __restrict__ out, int n_splits) {
+__global__ void __launch_bounds__(D) decode_attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
+                                                              bf16* __restrict__ out, int n_splits) {
+    __shared__ float wgt[kMaxSplits];
     pdl_trigger();
     pdl_wait();
     const size_t bh = blockIdx.x;  // b * n_q + h
     const int d = threadIdx.x;
-    float m = -INFINITY;
-    for (int s = 0; s < n_splits; ++s) m = fmaxf(m, part_ml[(bh * n_splits + s) * 2]);
-    float l = 0.f, o = 0.f;
-    for (int s = 0; s < n_splits; ++s) {
-        const float ms = part_ml[(bh * n_splits + s) * 2];
-        const float w = (ms == -INFINITY) ? 0.f : exp2f(ms - m);
-        l += part_ml[(bh * n_splits + s) * 2 + 1] * w;
-        o += part_o[(bh * n_splits + s) * D + d] * w;
+    if (d < 32) {
+        const float2* ml = reinterpret_cast<const float2*>(part_ml) + bh * n_splits;
+        float2 a = make_float2(-INFINITY, 0.f), b = a;
+        if (d < n_splits) a = ml[d];
+        if (d + 32 < n_splits) b = ml[d + 32];
+        const float m = warp_max(fmaxf(a.x, b.x));
+        const float wa = a.x == -INFINITY ? 0.f : exp2f(a.x - m), wb = b.x == -INFINITY ? 0.f : exp2f(b.x - m);
+        const float l = warp_sum(a.y * wa + b.y * wb);
+        const float inv = l > 0.f ? 1.f / l : 0.f;
+        wgt[d] = wa * inv;
+        wgt[d + 32] = wb * inv;
     }
-    out[bh * D + d] = __float2bfloat16(l > 0.f ? o / l : 0.f);
+    __syncthreads();
+    const float* po = part_o + bh * n_splits * D + d;
+    float o = 0.f;
+#pragma unroll 8
+    for (int s = 0; s < n_splits; ++s) o = fmaf(po[(size_t)s * D], wgt[s], o);
+    out[bh * D + d] = __float2bfloat16(o);
 }
 
 // new_k/new_v: [B, n_kv, T_new, D]; positions: [B] start position (rows t -> positions[b] + t)
@@ -459,12 +493,17 @@ __global__ void kv_cache_update_kernel(const bf16* __restrict__ new_k, const bf1
 }  // namespace
 
 NXD_API int nxd_decode_attn_num_splits(int B, int n_kv, int max_len) {
-    // enough CTAs to cover the machine, at least 128 keys per split (two iterations of the 64-key CTA step)
-    int want = (2 * nxd_num_sms() + B * n_kv - 1) / (B * n_kv);
+    // one wave of CTAs (two per SM) at least 128 keys each: a second, partial wave costs more than a longer loop (16 sequences of
+    // 2048 keys, 8 heads of 64: 12.2 us with 2 splits, 14.6 with 3; 4 sequences: 5.9 with 8, 6.8 with 10).  From half a wave of
+    // pairs on, sequences of different lengths want the finer split (12 of up to 2900 keys, heads of 128: 26.1 with 4, 29.8 with
+    // 2).
+    const int pairs = B * n_kv;
+    int want = 2 * nxd_num_sms() / (pairs > 0 ? pairs : 1);
+    if (want < 4 && want > 1 && pairs * 4 <= 3 * nxd_num_sms()) want = 4;
     int by_len = (max_len + 127) / 128;
     int s = want < by_len ? want : by_len;
     if (s < 1) s = 1;
-    if (s > 64) s = 64;
+    if (s > kMaxSplits) s = kMaxSplits;
     return s;
 }
 
@@ -477,6 +516,7 @@ static int decode_attn_impl(const void* q, const void* cache_k, const void* cach
     NXD_REQUIRE(D == 64 || D == 128, "decode_attn: head dim %d not in {64, 128}", D);
     NXD_REQUIRE(n_q % n_kv == 0 && n_q / n_kv <= kMaxGroup, "decode_attn: unsupported GQA group %d/%d", n_q, n_kv);
     NXD_REQUIRE(scratch != nullptr && n_splits >= 1, "decode_attn: scratch required");
+    if (n_splits > kMaxSplits) n_splits = kMaxSplits;      // the merge holds the weights of that many (scratch is larger then)
     if (B == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     CacheView cv{(const bf16*)cache_k, (const bf16*)cache_v, block_table, seq_ids, stride_b, stride_h,

@@ -89,9 +89,6 @@ nki_flash_attn_func = flash_attn_func  # reference-compatible alias
 # decode path
 # ---------------------------------------------------------------------------------------------
 
-_decode_scratch = {}
-
-
 def kv_cache_update(cache_k: torch.Tensor, cache_v: torch.Tensor, new_k: torch.Tensor, new_v: torch.Tensor,
                     positions: torch.Tensor, seq_ids: Optional[torch.Tensor] = None,
                     block_table: Optional[torch.Tensor] = None, page_size: int = 0) -> None:
@@ -139,13 +136,8 @@ def decode_attention(q: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Tens
         lens = lengths.to(torch.int32).contiguous()
         max_len = cache_k.shape[2] if block_table is None else block_table.shape[1] * page_size
         n_splits = _lib.lib().nxd_decode_attn_num_splits(_c.c_int(B), _c.c_int(Hkv), _c.c_int(max_len))
-        need = B * Hq * n_splits * (D + 2)
-        key = (q.device.index, need)
-        scratch = _decode_scratch.get(key)
-        if scratch is None:
-            scratch = torch.empty(need, dtype=torch.float32, device=q.device)
-            _decode_scratch.clear()
-            _decode_scratch[key] = scratch
+        # the call's own scratch: a captured graph keeps it in its pool, and calls on other streams have theirs
+        scratch = torch.empty(B * Hq * n_splits * (D + 2), dtype=torch.float32, device=q.device)
         out = torch.empty_like(q)
         bt = block_table.to(torch.int32).contiguous() if block_table is not None else None
         qc = q.contiguous()
