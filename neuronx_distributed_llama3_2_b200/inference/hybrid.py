@@ -47,6 +47,7 @@ from ..ops import rope as rope_ops
 from ..ops import state_space as ss_ops
 from ..ops import stream_norm as sn_ops
 from ..ops import window_attention as wa_ops
+from ..ops.gemm import streams_on_tensor_cores
 from ..ops.linear import gemm_nt
 from .config import InferenceConfig
 from .kv_cache import KVCache
@@ -728,7 +729,7 @@ class TidavikInferenceModel(CacheRowsMixin, KVCacheInferenceMixin, TidavikForCau
 
     def _feed_forward(self, mlp, h2: torch.Tensor) -> torch.Tensor:
         N, w = h2.shape[0], mlp.gate_up_proj.weight
-        if backend.gemm_backend() == "tcgen05" and decode_fused.qualifies(h2):
+        if backend.gemm_backend() == "tcgen05" and decode_fused.qualifies(h2) and not streams_on_tensor_cores(N, *w.shape):
             act = decode_fused.gate_up_swiglu(h2, None, 0.0, w)
         elif (backend.gemm_backend() == "tcgen05" and N <= decode_fused.BATCHED_SWIGLU_MAX_ROWS
               and decode_fused.qualifies_batched(h2)):

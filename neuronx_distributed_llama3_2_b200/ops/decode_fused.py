@@ -3,8 +3,8 @@ write in one launch, RMSNorm + gate/up GEMV + SwiGLU in one launch.  With the tw
 residual in their epilogue (``fused_comm.skinny_gemm``) and the decode attention (split + merge) a decoder layer of the
 token-generation graph is six launches (reference graph: ``examples/inference/modules/model_base.py:459-518``).
 
-Batches of 9 .. 128 sequences take the tensor-core counterparts (``csrc/gemm_smallm.cu``: weight rows as the UMMA M
-dimension, cluster split-K): fused QKV GEMM + RoPE + cache write, gate/up GEMM + SwiGLU (<= 64 rows), and the plain GEMM
+Batches of 2 to 128 sequences on one process take the tensor-core counterparts (``csrc/gemm_smallm.cu``: weight rows as the
+UMMA M dimension, cluster split-K) unless the weights are small (``gemm.streams_on_tensor_cores``): fused QKV GEMM + RoPE + cache write, gate/up GEMM + SwiGLU (<= 64 rows), and the plain GEMM
 with the residual in its epilogue; the two RMSNorms stay separate launches there (eight launches per layer)."""
 from __future__ import annotations
 
@@ -60,7 +60,7 @@ def gate_up_swiglu(x: torch.Tensor, norm_w: Optional[torch.Tensor], eps: float, 
 
 
 def qualifies_batched(x: torch.Tensor) -> bool:
-    return (x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and MAX_ROWS < x.shape[0] <= BATCHED_MAX_ROWS
+    return (x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and 1 <= x.shape[0] <= BATCHED_MAX_ROWS
             and x.shape[1] % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0 and _lib.available())
 
 
@@ -68,7 +68,7 @@ def qkv_rope_cache_batched(xn: torch.Tensor, w_qkv: torch.Tensor, cos: torch.Ten
                            positions: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Tensor, n_q: int, n_kv: int,
                            D: int, seq_ids: Optional[torch.Tensor] = None, block_table: Optional[torch.Tensor] = None,
                            page_size: int = 0, splits: int = 0) -> torch.Tensor:
-    """``xn [B, H]`` (already normalised, ``B <= 128``) -> ``q [B, n_q, D]`` rotated; rotated K rows and V rows go into
+    """``xn [B, H]`` (already normalised, ``1 <= B <= 128``) -> ``q [B, n_q, D]`` rotated; rotated K rows and V rows go into
     the cache at ``positions[b]`` -- ONE tensor-core launch (``nxd_smallm_qkv_rope_cache``)."""
     B, K = xn.shape
     assert w_qkv.shape == ((n_q + 2 * n_kv) * D, K) and w_qkv.stride(1) == 1

@@ -100,6 +100,15 @@ def gemm_grouped(a: torch.Tensor, b: torch.Tensor, layout: str, out: Optional[to
 SMALLM_MAX_ROWS = 128
 
 
+def streams_on_tensor_cores(rows: int, n: int, k: int) -> bool:
+    """Whether ``gemm_smallm`` beats the FMA GEMV (``fused_comm.skinny_gemm``, up to 8 rows).  Measured in captured graphs,
+    rows / ``[n, k]``: 1 / ``[2048, 2048]`` 5.9 us FMA, 3.9 tensor cores; 1 / ``[16384, 2048]`` 17.1 / 12.1; 4 / ``[2048, 8192]``
+    19.5 / 8.2; 8 / ``[16384, 8192]`` 209 / 42; below two million weights a cluster's start costs more than the FMA GEMV
+    (1 / ``[256, 1024]`` 2.7 / 2.6, 1 / ``[64, 4096]`` 2.7 / 4.4), except that its 8-row form reads the rows from shared memory
+    8 times (8 / ``[256, 2048]`` 7.4 / 3.5)."""
+    return rows > 8 or n * k >= 1 << 21 or (rows > 4 and k >= 1024)
+
+
 def gemm_smallm(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor] = None, splits: int = 0
                 ) -> Optional[torch.Tensor]:
     """``x[B, K] @ w[N, K]^T (+ residual)`` for ``B <= 128`` rows on the tensor cores with the WEIGHT rows as the UMMA M

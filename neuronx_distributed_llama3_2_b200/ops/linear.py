@@ -52,16 +52,15 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
     n = b.shape[0]
     if (m <= 128 and out is None and not accumulate and out_dtype in (None, torch.bfloat16) and a.is_cuda
             and a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and _backend() == "tcgen05" and _lib.available()):
-        # token generation: weight-streaming kernels instead of a 256-row tensor-core tile that is mostly padding --
-        # FMA GEMV up to 8 rows, above that the tensor-core kernel with the weight rows as the UMMA M dimension
-        if m <= 8:
+        # token generation: weight-streaming kernels instead of a 256-row tensor-core tile that is mostly padding -- the
+        # tensor-core kernel with the weight rows as the UMMA M dimension, or the FMA GEMV for few rows of small weights
+        from .gemm import gemm_smallm, streams_on_tensor_cores
+
+        res = gemm_smallm(a, b) if streams_on_tensor_cores(m, n, k) else None
+        if res is None and m <= 8:
             from .fused_comm import skinny_gemm
 
             res = skinny_gemm(a, b)
-        else:
-            from .gemm import gemm_smallm
-
-            res = gemm_smallm(a, b)
         if res is not None:
             return res
     if _use_kernel(a, b, m, n, k):

@@ -15,8 +15,8 @@ def test_gate_up_product_with_activation_matches_float64(M, K, I):
     x, w = wide[:, :K], (torch.randn(2 * I, K, generator=g, device="cuda") * K ** -0.5 * 2).bfloat16()
     gate, up = (x.double() @ w.double().t()).chunk(2, dim=-1)
     ref = torch.nn.functional.silu(gate) * up
-    # one rounding to bf16 (2^-9 of the value) and fp32 sums
-    assert (gemm_swiglu(x, w).double() - ref).norm() <= 2.0 ** -9 * ref.norm()
+    # one rounding to 8 significant bits (half a unit: up to 2^-8 of a value) of fp32 sums
+    assert (gemm_swiglu(x, w).double() - ref).norm() <= 2.0 ** -8 * ref.norm()
 
 
 @pytest.mark.parametrize("D,nq,nkv", [(16, 3, 1), (64, 8, 2), (128, 2, 2)])

@@ -1,0 +1,52 @@
+"""Token steps of 1 to 8 rows on the tensor-core weight-streaming kernels, against float64 and the FMA kernels."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows", [1, 2, 5, 8])
+# around the line between the kernels, ragged last weight slabs and contraction tails
+@pytest.mark.parametrize("n,k", [(1024, 2048), (2056, 1032), (264, 1024), (16, 8192)])
+def test_few_rows_match_float64(rows, n, k):
+    from neuronx_distributed_llama3_2_b200.ops.linear import gemm_nt
+
+    g = torch.Generator(device="cuda").manual_seed(n + rows)
+    x, w = (torch.randn(r, k, generator=g, device="cuda").bfloat16() for r in (rows, n))
+    ref = x.double() @ w.double().t()
+    # one rounding to 8 significant bits (half a unit: up to 2^-8 of a value) of an fp32 sum
+    assert (gemm_nt(x, w).double() - ref).norm() <= 2.0 ** -8 * ref.norm()
+
+
+@pytest.mark.parametrize("batch,paged", [(2, False), (3, True), (8, False)])
+def test_token_step_matches_the_fma_kernels(batch, paged, monkeypatch):
+    from neuronx_distributed_llama3_2_b200.inference.config import InferenceConfig
+    from neuronx_distributed_llama3_2_b200.inference.model import KVCacheInferenceMixin, LlamaInferenceModel
+    from neuronx_distributed_llama3_2_b200.models.llama import LlamaConfig
+
+    torch.manual_seed(0)
+    cfg = LlamaConfig(vocab_size=512, hidden_size=1536, intermediate_size=2048, num_hidden_layers=2, num_attention_heads=12,
+                      num_key_value_heads=4, head_dim=128, rope_scaling=None)
+    model = LlamaInferenceModel(cfg, InferenceConfig(batch_size=batch, max_context_length=64, seq_len=64, paged_kv=paged,
+                                                     page_size=32), device="cuda")
+    ids = torch.randint(0, 512, (batch, 1), device="cuda")
+    pos = torch.arange(5, 5 + batch, device="cuda").reshape(batch, 1)
+    taken = []
+    real = KVCacheInferenceMixin._layer_batched_decode
+    monkeypatch.setattr(KVCacheInferenceMixin, "_layer_batched_decode", lambda self, *a: taken.append(1) or real(self, *a))
+
+    def run():
+        cache = model.init_kv_cache(device="cuda")
+        g = torch.Generator(device="cuda").manual_seed(1)
+        for t in cache.k + cache.v:
+            t.normal_(generator=g)
+        logits = model.forward_infer(ids, pos, return_logits=True, sample=False)[1]
+        return [logits] + cache.k + cache.v
+
+    got = run()
+    assert len(taken) == 2
+    monkeypatch.setattr(KVCacheInferenceMixin, "_tensor_core_decode", lambda *a: False)
+    ref = run()
+    assert len(taken) == 2
+    for a, b in zip(got, ref):      # the same roundings to bf16 of fp32 sums in another order, two layers of them
+        assert (a.float() - b.float()).norm() <= 1e-2 * b.float().norm()
