@@ -203,6 +203,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             const int n0 = tn * kOutN;
             // experts start at multiples of 32 rows, so a warp's 32 rows never hold two experts' rows
             const int row_end = kSorted ? row_base + seg.counts[e] : M;
+            float row_scale = 1.f;
+            if (SEG == kSegGlu && seg.row_scale != nullptr && row0 + lane < row_end) row_scale = seg.row_scale[row0 + lane];
             ptx::mbar_wait(&tmem_full_bar[acc], acc_phase);
             ptx::tcgen05_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
@@ -222,7 +224,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 #pragma unroll
                         for (int j = 0; j < 32; ++j)
                             r[half * 32 + j] = __float_as_uint(
-                                seg.glu(__uint_as_float(r[half * 32 + j]), __uint_as_float(up[j])));
+                                SEG == kSegGlu ? seg.glu(__uint_as_float(r[half * 32 + j]) * row_scale,
+                                                         __uint_as_float(up[j]) * row_scale)
+                                               : seg.glu(__uint_as_float(r[half * 32 + j]), __uint_as_float(up[j])));
                     }
                 } else {
                     ptx::tmem_ld_wait();
@@ -432,12 +436,12 @@ int run_grouped(int layout, const void* a, const void* b, long long lda, long lo
 #undef NXD_GG_LAYOUT
 }
 
-template <int BN, int SEG>
+template <int BN, int SEG, int OUT_MODE = kOutBF16>
 static int launch_experts(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, int E, int rows, int N, int K,
                           const SegArgs& seg, cudaStream_t stream) {
     constexpr int kSmem = SmemLayout<BN>::kSmemBytes + kSegSmemBytes;
     static_assert(kSmem <= 232448, "shared memory budget exceeded");
-    auto kern = gemm_pair_kernel<BN, false, true, kOutBF16, true, SEG>;
+    auto kern = gemm_pair_kernel<BN, false, true, OUT_MODE, true, SEG>;
     static bool configured = false;
     if (!configured) {
         NXD_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
@@ -455,7 +459,8 @@ static int launch_experts(const CUtensorMap& ta, const CUtensorMap& tb, const CU
 
 // D[r, :] = act(A[r, :] @ B_e) for the rows r of expert e, all experts in one launch.  A [rows, K] holds the tokens sorted by
 // expert, expert e's counts[e] rows from segment_starts' row offset on (multiples of 32); B [E, K, Nb] row-major.
-//   mode kSegPlain: D [rows, N], Nb = N;  kSegRelu2: max(., 0)^2;  kSegGlu: Nb = 2 N, gate columns first, D = glu(gate, up)
+//   mode kSegPlain: D [rows, N], Nb = N, bf16 or (wide) fp32;  kSegRelu2: max(., 0)^2;
+//   kSegGlu: Nb = 2 N, gate columns first, D = glu(gate, up)
 // The gate / up products stay in fp32 up to the activation.  Rows between an expert's end and the next one's start are
 // computed along (whatever A holds there) and not stored unless they share a 32-row group with a real row.
 // 8190 tokens, top 2 of 8 experts, 2048 x 4096: 179 us (1540 TF) gate / up with the activation, 99 us (1390 TF) down; one
@@ -463,7 +468,8 @@ static int launch_experts(const CUtensorMap& ta, const CUtensorMap& tb, const CU
 // A tile is 256 rows: with few rows per expert the launch is the stream of the weights, and narrow column tiles give it
 // more clusters (pick_block_n on the expected number of tiles).
 static int run_experts(const void* a, const void* b, void* d, const SegArgs& seg, int E, int rows, int pairs, int N, int K,
-                       int mode, cudaStream_t stream) {
+                       int mode, bool wide, cudaStream_t stream) {
+    NXD_REQUIRE(!wide || mode == kSegPlain, "experts: %s", "fp32 results of plain products only");
     NXD_REQUIRE(E > 0 && E <= kSegMaxExperts, "experts: %d experts", E);
     NXD_REQUIRE(rows > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "experts: %d rows, %d x %d", rows, N, K);
     NXD_REQUIRE(((uintptr_t)a & 15) == 0 && ((uintptr_t)b & 15) == 0 && ((uintptr_t)d & 15) == 0,
@@ -476,8 +482,11 @@ static int run_experts(const void* a, const void* b, void* d, const SegArgs& seg
     if (rc) return rc;
     rc = make_tmap_3d(&tb, b, (uint64_t)nb, (uint64_t)K, (uint64_t)E, (uint64_t)nb, (uint64_t)K * nb, 64, kBlockK);
     if (rc) return rc;
-    rc = make_tmap_2d(&td, d, (uint64_t)N, (uint64_t)rows, (uint64_t)N, 64, 32, 2);
+    rc = make_tmap_2d(&td, d, (uint64_t)N, (uint64_t)rows, (uint64_t)N, wide ? 32 : 64, 32, wide ? 4 : 2);
     if (rc) return rc;
+    if (wide)
+        return bn == 256 ? launch_experts<256, kSegPlain, kOutF32>(ta, tb, td, E, rows, N, K, seg, stream)
+                         : launch_experts<128, kSegPlain, kOutF32>(ta, tb, td, E, rows, N, K, seg, stream);
 #define NXD_EXPERTS(MODE_)                                                                              \
     return bn == 256 ? launch_experts<256, MODE_>(ta, tb, td, E, rows, N, K, seg, stream)                \
                      : launch_experts<128, MODE_>(ta, tb, td, E, rows, N, K, seg, stream)
@@ -494,11 +503,13 @@ static int run_experts(const void* a, const void* b, void* d, const SegArgs& seg
 
 // Products of the sparse experts over rows sorted by expert (run_experts above): counts [E] int32 on the device, mode 1 plain,
 // 2 gate | up through the clamped gated activation, 3 max(., 0)^2.  `rows`: rows of a and d; `pairs`: real rows expected (picks
-// the tile width only).
-NXD_API int nxd_experts_gemm_bf16(const void* a, const void* b, void* d, const int* counts, int E, int rows, int pairs, int N,
-                                  int K, int mode, float limit, float alpha, float up_shift, void* stream) {
-    nxd_gemm::SegArgs seg{counts, limit, alpha, up_shift};
-    return nxd_gemm::run_experts(a, b, d, seg, E, rows, pairs, N, K, mode, (cudaStream_t)stream);
+// the tile width only).  row_scale [rows] fp32 or NULL: mode 2, factor of a row's products ahead of the activation.  wide: d is
+// fp32 (mode 1), else bf16.
+NXD_API int nxd_experts_gemm_bf16(const void* a, const void* b, void* d, const int* counts, const float* row_scale, int E,
+                                  int rows, int pairs, int N, int K, int mode, int wide, float limit, float alpha,
+                                  float up_shift, void* stream) {
+    nxd_gemm::SegArgs seg{counts, limit, alpha, up_shift, row_scale};
+    return nxd_gemm::run_experts(a, b, d, seg, E, rows, pairs, N, K, mode, wide != 0, (cudaStream_t)stream);
 }
 
 namespace nxd_gemm {
@@ -538,7 +549,7 @@ NXD_API int nxd_gemm_glu_bf16(const void* a, const void* w, void* d, int M, int 
     if ((rc = make_tmap_2d(&ta, a, (uint64_t)K, (uint64_t)M, (uint64_t)lda, 64, kBlockM))) return rc;
     if ((rc = make_tmap_2d(&tb, w, (uint64_t)K, (uint64_t)2 * N, (uint64_t)ldw, 64, bn / 2))) return rc;
     if ((rc = make_tmap_2d(&td, d, (uint64_t)N, (uint64_t)M, (uint64_t)ldd, 64, 32, 2))) return rc;
-    const SegArgs act{nullptr, limit, alpha, up_shift};
+    const SegArgs act{nullptr, limit, alpha, up_shift, nullptr};
     return bn == 256 ? launch_glu<256>(ta, tb, td, M, N, K, act, (cudaStream_t)stream)
                      : launch_glu<128>(ta, tb, td, M, N, K, act, (cudaStream_t)stream);
 }

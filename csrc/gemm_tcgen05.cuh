@@ -59,6 +59,8 @@ constexpr int kSegAlign = 32;   // an expert's rows start at a multiple: the 32 
 struct SegArgs {
     const int* counts;                // [E] rows per expert
     float limit, alpha, up_shift;     // of the gated activation
+    const float* row_scale;           // [rows] or NULL: factor of a row's products ahead of the activation (a weight on the
+                                      // expert's input, applied in fp32)
     __device__ __forceinline__ float glu(float g, float u) const {
         g = fminf(g, limit);
         u = fminf(fmaxf(u, -limit), limit);

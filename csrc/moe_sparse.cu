@@ -460,17 +460,18 @@ __global__ void glu_bias_vec_kernel(const bf16* __restrict__ src, long long ld, 
 
 // Bound by memory.  V = 8: a thread takes 8 consecutive columns (16-byte loads of bf16 rows, W a multiple of 8, aligned
 // rows); V = 1: any W.  8190 tokens x 2048, top 2 (134 MB): 61 us with one column per thread, 24 us (5.6 TB/s).
-template <typename T, int V>
-__global__ void moe_gather_combine_kernel(const T* __restrict__ ys, const int* __restrict__ slot,
+// TY: type of the experts' outputs (bf16 or fp32)
+template <typename T, int V, typename TY = T>
+__global__ void moe_gather_combine_kernel(const TY* __restrict__ ys, const int* __restrict__ slot,
                                           const int* __restrict__ idx, const float* __restrict__ wts,
-                                          const T* __restrict__ h, const T* __restrict__ shared_out,
+                                          const T* __restrict__ h, const TY* __restrict__ shared_out,
                                           const float* __restrict__ sgate, float* __restrict__ y, int top, int W, int E) {
     const long long t = blockIdx.x;
     for (int c = threadIdx.x * V; c < W; c += blockDim.x * V) {
         float a[V];
 #pragma unroll
         for (int i = 0; i < V; ++i) a[i] = 0.f;
-        auto add = [&](const T* row, float wgt) {
+        auto add = [&](const auto* row, float wgt) {
             float v[V];
             if constexpr (V == 8) ld8(row + c, v);
             else v[0] = ldf(row + c);
@@ -479,7 +480,9 @@ __global__ void moe_gather_combine_kernel(const T* __restrict__ ys, const int* _
         };
         for (int j = 0; j < top; ++j) {
             const int e = idx[t * top + j];
-            add((e < 0 || e >= E) ? h + t * W : ys + (long long)slot[t * top + j] * W, wts[t * top + j]);
+            const float wgt = wts[t * top + j];
+            if (e < 0 || e >= E) add(h + t * W, wgt);
+            else add(ys + (long long)slot[t * top + j] * W, wgt);
         }
         if (shared_out != nullptr) add(shared_out + t * W, sgate != nullptr ? sgate[t] : 1.f);
         if constexpr (V == 8) {
@@ -500,11 +503,12 @@ __global__ void moe_gather_combine_kernel(const T* __restrict__ ys, const int* _
 constexpr int CNT_THREADS = 256, CNT_PAIRS = 2048;      // pairs per block
 
 __global__ void __launch_bounds__(CNT_THREADS)
-moe_count_kernel(const int* __restrict__ idx, int* __restrict__ counts, int* __restrict__ place, long long P, int E) {
+moe_count_kernel(const int* __restrict__ idx, int* __restrict__ counts, int* __restrict__ place, long long P, int top, int E) {
     extern __shared__ int hist[];                       // [E] pairs of this block, then [E] the block's first place
     int* first = hist + E;
     for (int e = threadIdx.x; e < E; e += CNT_THREADS) hist[e] = 0;
     __syncthreads();
+    if (blockIdx.x == 0 && threadIdx.x == 0) counts[E] = (int)(P / top);      // the tokens: rows of a shared expert
     const long long p0 = (long long)blockIdx.x * CNT_PAIRS;
     int mine[CNT_PAIRS / CNT_THREADS];
 #pragma unroll
@@ -526,11 +530,11 @@ moe_count_kernel(const int* __restrict__ idx, int* __restrict__ counts, int* __r
 
 constexpr int GA_WARPS = 8;
 
-// slot [P] (in: place, out: row of the pair); x [rows, W] <- h[p / top] (times in_scale[p], rounded)
+// slot [P] (in: place, out: row of the pair); x [rows, W] <- h[p / top]; row_scale [rows] <- in_scale[p] (both NULL: none)
 __global__ void __launch_bounds__(GA_WARPS * 32)
 moe_gather_rows_kernel(const bf16* __restrict__ h, const int* __restrict__ idx, const int* __restrict__ counts,
-                       int* __restrict__ slot, const float* __restrict__ in_scale, bf16* __restrict__ x, long long P, int top,
-                       int W8, int E) {
+                       int* __restrict__ slot, const float* __restrict__ in_scale, float* __restrict__ row_scale,
+                       bf16* __restrict__ x, long long P, int top, int W8, int E) {
     __shared__ int row0[nxd_gemm::kSegMaxExperts + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp == 0) nxd_gemm::segment_starts(counts, E, 0, row0, nullptr);
@@ -541,22 +545,14 @@ moe_gather_rows_kernel(const bf16* __restrict__ h, const int* __restrict__ idx, 
     if (e < 0 || e >= E) return;                        // identity expert: the combination reads h itself
     const int row = row0[e] + slot[p];
     __syncwarp();                                       // every lane has read the place
-    if (lane == 0) slot[p] = row;
+    if (lane == 0) {
+        slot[p] = row;
+        if (in_scale != nullptr) row_scale[row] = in_scale[p];
+    }
     const bf16x8* src = reinterpret_cast<const bf16x8*>(h) + p / top * W8;
     bf16x8* dst = reinterpret_cast<bf16x8*>(x) + (long long)row * W8;
-    if (in_scale == nullptr) {
 #pragma unroll 4
-        for (int c = lane; c < W8; c += 32) dst[c] = src[c];
-    } else {
-        const float s = in_scale[p];
-        for (int c = lane; c < W8; c += 32) {
-            float v[8];
-            unpack8(src[c], v);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] *= s;
-            dst[c] = pack8(v);
-        }
-    }
+    for (int c = lane; c < W8; c += 32) dst[c] = src[c];
 }
 
 }  // namespace
@@ -594,19 +590,20 @@ NXD_API int nxd_moe_router(int dtype, const void* h, const float* wr, const floa
     return 0;
 }
 
-// Rows of the pairs sorted by expert.  counts [E] int32: ZEROED by the caller, out: pairs of every expert; slot [P] int32 out:
-// the pair's row in x (not written for identity experts); x [rows, W] bf16 with rows >= P + 32 E, W a multiple of 8.
-NXD_API int nxd_moe_sort_rows(const void* h, const int* idx, int* counts, int* slot, const float* in_scale, void* x, long long P,
-                              int top, int W, int E, void* stream) {
+// Rows of the pairs sorted by expert.  counts [E + 1] int32: ZEROED by the caller, out: pairs of every expert, then P / top;
+// slot [P] int32 out: the pair's row in x (not written for identity experts); x [rows, W] bf16 with rows >= P + 32 E, W a
+// multiple of 8; row_scale [rows] <- in_scale [P] of the row's pair (both fp32, or both NULL).
+NXD_API int nxd_moe_sort_rows(const void* h, const int* idx, int* counts, int* slot, const float* in_scale, float* row_scale,
+                              void* x, long long P, int top, int W, int E, void* stream) {
     if (P == 0) return 0;
     NXD_REQUIRE(E > 0 && E <= nxd_gemm::kSegMaxExperts && W % 8 == 0, "sort rows: %d experts, width %d", E, W);
     NXD_REQUIRE(((uintptr_t)h % 16) == 0 && ((uintptr_t)x % 16) == 0, "sort rows: rows must be 16-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
     moe_count_kernel<<<(unsigned)((P + CNT_PAIRS - 1) / CNT_PAIRS), CNT_THREADS, 2 * E * sizeof(int), st>>>(idx, counts, slot,
-                                                                                                           P, E);
+                                                                                                           P, top, E);
     NXD_LAUNCH_CHECK();
     moe_gather_rows_kernel<<<(unsigned)((P + GA_WARPS - 1) / GA_WARPS), GA_WARPS * 32, 0, st>>>(
-        (const bf16*)h, idx, counts, slot, in_scale, (bf16*)x, P, top, W / 8, E);
+        (const bf16*)h, idx, counts, slot, in_scale, row_scale, (bf16*)x, P, top, W / 8, E);
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -713,6 +710,7 @@ NXD_API int nxd_clamped_glu(int dtype, const void* gate_up, void* out, long long
 }
 
 // ys [pairs, W]: expert outputs in sorted order, slot [N, top]: row of ys of every (token, choice); identity experts read h.
+// dtype 0 bf16, 1 fp32, 2: bf16 h with fp32 ys and shared_out.
 NXD_API int nxd_moe_gather_combine(int dtype, const void* ys, const int* slot, const int* idx, const float* wts,
                                    const void* h, const void* shared_out, const float* sgate, float* y, long long N,
                                    int top, int W, int E, void* stream) {
@@ -723,7 +721,13 @@ NXD_API int nxd_moe_gather_combine(int dtype, const void* ys, const int* slot, c
 #define NXD_GC(T, V)                                                                                     \
     moe_gather_combine_kernel<T, V><<<(unsigned)N, 128, 0, (cudaStream_t)stream>>>(                      \
         (const T*)ys, slot, idx, wts, (const T*)h, (const T*)shared_out, sgate, y, top, W, E)
-    if (dtype == 0) {
+    if (dtype == 2) {
+#define NXD_GC_WIDE(V)                                                                                   \
+    moe_gather_combine_kernel<bf16, V, float><<<(unsigned)N, 128, 0, (cudaStream_t)stream>>>(            \
+        (const float*)ys, slot, idx, wts, (const bf16*)h, (const float*)shared_out, sgate, y, top, W, E)
+        if (vec) NXD_GC_WIDE(8); else NXD_GC_WIDE(1);
+#undef NXD_GC_WIDE
+    } else if (dtype == 0) {
         if (vec) NXD_GC(bf16, 8); else NXD_GC(bf16, 1);
     } else {
         if (vec) NXD_GC(float, 8); else NXD_GC(float, 1);

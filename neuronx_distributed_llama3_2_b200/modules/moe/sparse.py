@@ -78,9 +78,13 @@ class SparseMoE(torch.nn.Module):
 
     def _use_device_sorted(self, h: torch.Tensor) -> bool:
         """The sorted path without a host read: one process holds whole experts, ``sorted_forward_applies``."""
-        w_in = (self.experts.gate_up_proj if self.gated else self.experts.up_proj).weight
         return (h.is_cuda and ps.get_tensor_model_parallel_size() == 1 and ps.get_expert_model_parallel_size() == 1
-                and moe_sparse.sorted_forward_applies(h, w_in, self.experts.down_proj.weight))
+                and moe_sparse.sorted_forward_applies(h, *self._sorted_weights()))
+
+    def _sorted_weights(self):
+        """In and down weights of the experts, then those of the shared expert if there is one."""
+        return [w for ex in (self.experts, self.shared) if ex is not None
+                for w in ((ex.gate_up_proj if self.gated else ex.up_proj).weight, ex.down_proj.weight)]
 
     def forward(self, h: torch.Tensor, path: Optional[str] = None) -> torch.Tensor:
         """``h [N, W]`` (activation dtype) -> combined output ``[N, W]`` in fp32."""
@@ -119,10 +123,10 @@ class SparseMoE(torch.nn.Module):
         in_scale = None
         if self.weight_on_input:
             in_scale, wts = wts, self._ones_like(wts)
-        w_in = (self.experts.gate_up_proj if self.gated else self.experts.up_proj).weight
-        shared_out = self.shared(h.unsqueeze(0))[0] if self.shared is not None else None
-        return moe_sparse.sorted_forward(h, idx, wts, w_in, self.experts.down_proj.weight, self.gated, self.limit, self.alpha,
-                                         self.up_shift, in_scale, shared_out, sg)
+        w_in, w_down, *shared = self._sorted_weights()
+        return moe_sparse.sorted_forward(h, idx, wts, w_in, w_down, self.gated, self.limit, self.alpha, self.up_shift, in_scale,
+                                         *(shared or (None, None)), shared_limit=self.shared_limit if shared else 0.0,
+                                         shared_gate=sg)
 
     def _forward_sorted(self, h, idx, wts, sg):
         N, E, k = h.shape[0], self.num_experts, self.top_k

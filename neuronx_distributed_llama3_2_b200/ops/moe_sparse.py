@@ -228,36 +228,40 @@ def down_combine(act: torch.Tensor, w_down: torch.Tensor, idx: torch.Tensor, wts
 SORTED_MAX_EXPERTS = 128
 
 
-def sorted_forward_applies(h: torch.Tensor, w_in: torch.Tensor, w_down: torch.Tensor) -> bool:
-    """Whether ``sorted_forward`` takes these operands: bf16 on the GPU, widths that are multiples of 8 (TMA rows), at most
-    128 experts."""
-    return (_use_kernel(h) and h.dtype == torch.bfloat16 and w_in.dtype == h.dtype and w_down.dtype == h.dtype
-            and h.is_contiguous() and w_in.is_contiguous() and w_down.is_contiguous()
-            and w_in.shape[0] <= SORTED_MAX_EXPERTS and w_in.shape[1] % 8 == 0 and w_down.shape[1] % 8 == 0
-            and w_in.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0 and h.data_ptr() % 16 == 0)
+def sorted_forward_applies(h: torch.Tensor, *weights: torch.Tensor) -> bool:
+    """Whether ``sorted_forward`` takes these operands (``w_in, w_down`` and those of a shared expert): bf16 on the GPU, widths
+    that are multiples of 8 (TMA rows), at most 128 experts."""
+    return (_use_kernel(h) and h.dtype == torch.bfloat16 and h.is_contiguous() and h.data_ptr() % 16 == 0
+            and weights[0].shape[0] <= SORTED_MAX_EXPERTS
+            and all(w.dtype == h.dtype and w.is_contiguous() and w.data_ptr() % 16 == 0 and w.shape[1] % 8 == 0
+                    and w.shape[2] % 8 == 0 for w in weights))
 
 
 def sorted_forward(h: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, w_in: torch.Tensor, w_down: torch.Tensor, gated: bool,
                    limit: float = float("inf"), alpha: float = 1.0, up_shift: float = 0.0,
-                   in_scale: Optional[torch.Tensor] = None, shared_out: Optional[torch.Tensor] = None,
+                   in_scale: Optional[torch.Tensor] = None, shared_in: Optional[torch.Tensor] = None,
+                   shared_down: Optional[torch.Tensor] = None, shared_limit: float = float("inf"),
                    shared_gate: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The mixture of the chosen experts -> fp32 ``[N, W]``, on rows that are sorted by expert on the device: no host
     read, one call.  ``w_in [E, W, 2F]`` (``gated``: gate | up through the clamped activation, applied to the fp32
     products) or ``[E, W, F]`` (``max(., 0) ** 2``), ``w_down [E, F, W]``; ``in_scale [N, top]`` multiplies a pair's input
-    row; index ``>= E``: identity expert."""
+    row (in fp32, on its products); index ``>= E``: identity expert; ``shared_in [1, W, 2Fs]`` / ``shared_down [1, Fs, W]``: a
+    shared expert, times ``shared_gate [N]``."""
     N, W = h.shape
     E, F, _ = w_down.shape
+    Fs = shared_down.shape[1] if shared_down is not None else 0
     top = idx.shape[1]
     L = _lib.lib("window_moe_serving")
     size = L.nxd_moe_sorted_workspace
     size.restype = _c.c_longlong
-    work = torch.empty(size(_c.c_longlong(N), _c.c_int(top), _c.c_int(W), _c.c_int(F), _c.c_int(E)), dtype=torch.uint8,
-                       device=h.device)
+    work = torch.empty(size(_c.c_longlong(N), _c.c_int(top), _c.c_int(W), _c.c_int(F), _c.c_int(E), _c.c_int(Fs)),
+                       dtype=torch.uint8, device=h.device)
     y = torch.empty(N, W, dtype=torch.float32, device=h.device)
     rc = L.nxd_moe_sorted_forward(_lib.ptr(h), _lib.ptr(idx), _lib.ptr(wts), _lib.ptr(in_scale), _lib.ptr(w_in),
-                                  _lib.ptr(w_down), _lib.ptr(shared_out), _lib.ptr(shared_gate), _lib.ptr(y), _lib.ptr(work),
-                                  _c.c_longlong(N), _c.c_int(top), _c.c_int(W), _c.c_int(F), _c.c_int(E), _c.c_int(int(gated)),
-                                  _c.c_float(limit), _c.c_float(alpha), _c.c_float(up_shift), _lib.stream_ptr())
+                                  _lib.ptr(w_down), _lib.ptr(shared_in), _lib.ptr(shared_down), _lib.ptr(shared_gate), _lib.ptr(y),
+                                  _lib.ptr(work), _c.c_longlong(N), _c.c_int(top), _c.c_int(W), _c.c_int(F), _c.c_int(E),
+                                  _c.c_int(Fs), _c.c_int(int(gated)), _c.c_float(limit), _c.c_float(shared_limit),
+                                  _c.c_float(alpha), _c.c_float(up_shift), _lib.stream_ptr())
     _lib.check(rc, "nxd_moe_sorted_forward", L)
     return y
 
