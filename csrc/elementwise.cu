@@ -63,39 +63,62 @@ __global__ void swiglu_bwd_kernel(const bf16* __restrict__ gu, const bf16* __res
     }
 }
 
-// One thread rotates 8 (x1, x2) pairs: columns [8c, 8c+8) and [D/2 + 8c, ...).
-__global__ void rope_kernel(bf16* __restrict__ x, const float* __restrict__ cos_t,
-                            const float* __restrict__ sin_t, const int* __restrict__ positions, size_t T,
-                            int heads_total, int n_rot_heads, int D, int pos_div, int pos_mod, float sin_sign) {
+// One thread takes 8 (x1, x2) pairs, columns [8c, 8c+8) and [D/2 + 8c, ...), of kRopeHeads heads of a token: the table entries
+// and the position are read once for them and 2 kRopeHeads 16-byte loads are in flight.  Heads from n_rot on are copied
+// (n_heads = heads_total, x != y) or left alone (n_heads = n_rot, x == y).  Bound by memory: 8192 tokens x 40 heads of 128, 32 of
+// them rotated, 30 us on average for one launch out of place (168 MB) and one in place (134 MB), against 23 us of copy and 31 us of
+// rotation each with one head per thread.
+constexpr int kRopeHeads = 4;
+
+__global__ void rope_kernel(const bf16* x, bf16* y, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                            const int* __restrict__ positions, size_t T, int heads_total, int n_heads, int n_rot, int D,
+                            int pos_div, int pos_mod, float sin_sign) {
     const int half_vec = D >> 4;  // 16-byte vectors in half a head
-    const size_t total = T * (size_t)n_rot_heads * half_vec;
+    const int groups = (n_heads + kRopeHeads - 1) / kRopeHeads;
+    const size_t total = T * (size_t)groups * half_vec;
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x) {
         const int c = (int)(idx % half_vec);
-        const size_t th = idx / half_vec;
-        const int h = (int)(th % n_rot_heads);
-        const size_t t = th / n_rot_heads;
-        const int pos = positions ? positions[t] : (int)((t / pos_div) % pos_mod);
-        bf16* base = x + (t * heads_total + h) * (size_t)D;
-        bf16x8* p1 = reinterpret_cast<bf16x8*>(base) + c;
-        bf16x8* p2 = reinterpret_cast<bf16x8*>(base + (D >> 1)) + c;
-        float a[8], b[8], oa[8], ob[8];
-        bf16x8 va = *p1, vb = *p2;
-        unpack8(va, a);
-        unpack8(vb, b);
-        const float4* cp = reinterpret_cast<const float4*>(cos_t + (size_t)pos * (D >> 1) + c * 8);
-        const float4* sp = reinterpret_cast<const float4*>(sin_t + (size_t)pos * (D >> 1) + c * 8);
-        const float4 c0 = cp[0], c1 = cp[1], s0 = sp[0], s1 = sp[1];
-        const float cs[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-        const float sn[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+        const size_t tg = idx / half_vec;
+        const int h0 = (int)(tg % groups) * kRopeHeads;
+        const size_t t = tg / groups;
+        const size_t at = (t * heads_total + h0) * (size_t)D + c * 8;
+        bf16x8 va[kRopeHeads], vb[kRopeHeads];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const float s = sn[k] * sin_sign;
-            oa[k] = a[k] * cs[k] - b[k] * s;
-            ob[k] = b[k] * cs[k] + a[k] * s;
+        for (int j = 0; j < kRopeHeads; ++j) {
+            if (h0 + j < n_heads) {
+                va[j] = *reinterpret_cast<const bf16x8*>(x + at + (size_t)j * D);
+                vb[j] = *reinterpret_cast<const bf16x8*>(x + at + (size_t)j * D + (D >> 1));
+            }
         }
-        *p1 = pack8(oa);
-        *p2 = pack8(ob);
+        float cs[8], sn[8];
+        if (h0 < n_rot) {
+            const int pos = positions ? positions[t] : (int)((t / pos_div) % pos_mod);
+            const float4* cp = reinterpret_cast<const float4*>(cos_t + (size_t)pos * (D >> 1) + c * 8);
+            const float4* sp = reinterpret_cast<const float4*>(sin_t + (size_t)pos * (D >> 1) + c * 8);
+            const float4 c0 = cp[0], c1 = cp[1], s0 = sp[0], s1 = sp[1];
+            cs[0] = c0.x, cs[1] = c0.y, cs[2] = c0.z, cs[3] = c0.w, cs[4] = c1.x, cs[5] = c1.y, cs[6] = c1.z, cs[7] = c1.w;
+            sn[0] = s0.x, sn[1] = s0.y, sn[2] = s0.z, sn[3] = s0.w, sn[4] = s1.x, sn[5] = s1.y, sn[6] = s1.z, sn[7] = s1.w;
+        }
+#pragma unroll
+        for (int j = 0; j < kRopeHeads; ++j) {
+            if (h0 + j >= n_heads) break;
+            if (h0 + j < n_rot) {
+                float a[8], b[8], oa[8], ob[8];
+                unpack8(va[j], a);
+                unpack8(vb[j], b);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const float s = sn[k] * sin_sign;
+                    oa[k] = a[k] * cs[k] - b[k] * s;
+                    ob[k] = b[k] * cs[k] + a[k] * s;
+                }
+                va[j] = pack8(oa);
+                vb[j] = pack8(ob);
+            }
+            *reinterpret_cast<bf16x8*>(y + at + (size_t)j * D) = va[j];
+            *reinterpret_cast<bf16x8*>(y + at + (size_t)j * D + (D >> 1)) = vb[j];
+        }
     }
 }
 
@@ -186,18 +209,26 @@ NXD_API int nxd_swiglu_bwd(const void* gate_up, const void* dy, void* dgate_up, 
 // x: [T, heads_total, D] bf16 (in place).  cos/sin: [max_pos, D/2] fp32.
 // position of token t = positions[t] if given, else (t / pos_div) % pos_mod.
 // inverse != 0 applies the transpose rotation (backward).
+// x [T, heads_total, D] bf16 -> y (x itself, or another buffer): the first n_rot_heads heads rotated at positions[t] (int32) or
+// (t / pos_div) % pos_mod, the others copied.  D a multiple of 16, x and y 16-byte aligned.
+NXD_API int nxd_rope(const void* x, void* y, const float* cos_t, const float* sin_t, const int* positions, long long T,
+                     int heads_total, int n_rot_heads, int D, int pos_div, int pos_mod, int inverse, void* stream) {
+    NXD_REQUIRE(D % 16 == 0, "rope: head dim %d must be a multiple of 16", D);
+    NXD_REQUIRE(n_rot_heads <= heads_total, "rope: n_rot_heads > heads_total");
+    const int n_heads = x == y ? n_rot_heads : heads_total;
+    if (T == 0 || n_heads == 0) return 0;
+    const size_t work = (size_t)T * ((n_heads + kRopeHeads - 1) / kRopeHeads) * (D / 16);
+    rope_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
+        (const bf16*)x, (bf16*)y, cos_t, sin_t, positions, (size_t)T, heads_total, n_heads, n_rot_heads, D,
+        pos_div < 1 ? 1 : pos_div, pos_mod < 1 ? 1 : pos_mod, inverse ? -1.f : 1.f);
+    NXD_LAUNCH_CHECK();
+    return 0;
+}
+
 NXD_API int nxd_rope_inplace(void* x, const float* cos_t, const float* sin_t, const int* positions, long long T,
                              int heads_total, int n_rot_heads, int D, int pos_div, int pos_mod, int inverse,
                              void* stream) {
-    NXD_REQUIRE(D % 16 == 0, "rope: head dim %d must be a multiple of 16", D);
-    NXD_REQUIRE(n_rot_heads <= heads_total, "rope: n_rot_heads > heads_total");
-    if (T == 0 || n_rot_heads == 0) return 0;
-    const size_t work = (size_t)T * n_rot_heads * (D / 16);
-    rope_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
-        (bf16*)x, cos_t, sin_t, positions, (size_t)T, heads_total, n_rot_heads, D, pos_div < 1 ? 1 : pos_div,
-        pos_mod < 1 ? 1 : pos_mod, inverse ? -1.f : 1.f);
-    NXD_LAUNCH_CHECK();
-    return 0;
+    return nxd_rope(x, x, cos_t, sin_t, positions, T, heads_total, n_rot_heads, D, pos_div, pos_mod, inverse, stream);
 }
 
 // qkv [B * Tn, n_q + 2 n_kv, D] bf16 (q | k | v heads): q and k rotated in place at positions [B * Tn] int32; row t of sequence b

@@ -57,6 +57,8 @@ int nxd_rmsnorm_bwd_static(const void* dy, const void* x, const void* w, const f
  *      examples/inference/modules/attention/utils.py:27-41) ------------------------------------- */
 int nxd_swiglu_fwd(const void* gate_up, void* out, long long rows, int I, void* stream);
 int nxd_swiglu_bwd(const void* gate_up, const void* dy, void* dgate_up, long long rows, int I, void* stream);
+int nxd_rope(const void* x, void* y, const float* cos_t, const float* sin_t, const int* positions, long long T,
+             int heads_total, int n_rot_heads, int D, int pos_div, int pos_mod, int inverse, void* stream);
 int nxd_rope_inplace(void* x, const float* cos_t, const float* sin_t, const int* positions, long long T,
                      int heads_total, int n_rot_heads, int D, int pos_div, int pos_mod, int inverse,
                      void* stream);

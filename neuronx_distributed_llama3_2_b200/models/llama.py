@@ -280,14 +280,8 @@ class LlamaAttention(nn.Module):
         else:
             qkv = torch.cat(self.qkv_proj(x), dim=-1)
         S, B = qkv.shape[0], qkv.shape[1]
-        qkv = qkv.reshape(S * B, nq + 2 * nkv, D)
-        # rotate q and k heads (the first nq + nkv heads) in one pass; token t = s * B + b sits at position s
-        qkv = rope_ops.apply_rope(qkv, cos, sin, nq + nkv, pos_div=B, pos_mod=S)
-        qkv = qkv.reshape(S, B, nq + 2 * nkv, D)
-        q = qkv[:, :, :nq].permute(1, 2, 0, 3)                   # [B, nq, S, D] strided views, no copies
-        k = qkv[:, :, nq:nq + nkv].permute(1, 2, 0, 3)
-        v = qkv[:, :, nq + nkv:].permute(1, 2, 0, 3)
-        o = attn_ops.flash_attn_func(q, k, v, causal=True)       # [B, nq, S, D] stored as [S, B, nq, D]
+        # q and k heads are rotated in one pass (token s sits at position s); [B, nq, S, D] stored as [S, B, nq, D]
+        o = attn_ops.rope_flash_attn_func(qkv.reshape(S, B, nq + 2 * nkv, D), cos, sin, nq, nkv)
         o = o.permute(2, 0, 1, 3).reshape(S, B, nq * D)
         return self.o_proj(o)
 

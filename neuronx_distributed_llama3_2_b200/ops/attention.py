@@ -85,6 +85,21 @@ def flash_attn_func(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, dropout_p
 nki_flash_attn_func = flash_attn_func  # reference-compatible alias
 
 
+def rope_flash_attn_func(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, n_q: int, n_kv: int) -> torch.Tensor:
+    """Causal attention of a projection ``qkv [S, B, n_q + 2 n_kv, D]`` (q | k | v heads) whose queries and keys are first rotated
+    at position ``s`` -> ``[B, n_q, S, D]``."""
+    S, B, heads, D = qkv.shape
+    if qkv.is_cuda and qkv.dtype == torch.bfloat16 and D in (64, 128) and _backend(qkv) == "nxd":
+        from .flash_attn import rope_flash_attn
+
+        return rope_flash_attn(qkv, cos, sin, n_q, n_kv)
+    from .rope import apply_rope
+
+    x = apply_rope(qkv.reshape(S * B, heads, D), cos, sin, n_q + n_kv, pos_div=B, pos_mod=S).reshape(S, B, heads, D)
+    q, k, v = (x[:, :, a:b].permute(1, 2, 0, 3) for a, b in ((0, n_q), (n_q, n_q + n_kv), (n_q + n_kv, heads)))  # views
+    return flash_attn_func(q, k, v, causal=True)
+
+
 # ---------------------------------------------------------------------------------------------
 # decode path
 # ---------------------------------------------------------------------------------------------

@@ -111,34 +111,43 @@ def rope_ref(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, n_rot_heads:
     return torch.cat([out, x[:, n_rot_heads:]], dim=1)
 
 
+def _aligned(x: torch.Tensor) -> torch.Tensor:
+    """Contiguous, at a 16-byte boundary (the kernel's vectors)."""
+    x = x.contiguous()
+    return x if x.data_ptr() % 16 == 0 else x.clone()
+
+
 class _RopeFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, cos, sin, n_rot_heads, pos_div, pos_mod, positions):
         ctx.args = (n_rot_heads, pos_div, pos_mod)
         ctx.save_for_backward(cos, sin, positions if positions is not None else torch.empty(0))
         ctx.has_pos = positions is not None
-        out = x.contiguous().clone()
-        _launch(out, cos, sin, n_rot_heads, pos_div, pos_mod, positions, False)
+        x = _aligned(x)
+        out = torch.empty_like(x)
+        _launch(x, cos, sin, n_rot_heads, pos_div, pos_mod, positions, False, out)
         return out
 
     @staticmethod
     def backward(ctx, dy):
         cos, sin, positions = ctx.saved_tensors
         n_rot_heads, pos_div, pos_mod = ctx.args
-        dx = dy.contiguous().clone()
-        _launch(dx, cos, sin, n_rot_heads, pos_div, pos_mod, positions if ctx.has_pos else None, True)
+        dy = _aligned(dy)
+        dx = torch.empty_like(dy)
+        _launch(dy, cos, sin, n_rot_heads, pos_div, pos_mod, positions if ctx.has_pos else None, True, dx)
         return dx, None, None, None, None, None, None
 
 
-def _launch(x, cos, sin, n_rot_heads, pos_div, pos_mod, positions, inverse):
+def _launch(x, cos, sin, n_rot_heads, pos_div, pos_mod, positions, inverse, out=None):
+    """``x [T, heads, D]`` rotated into ``out`` (all heads written), or in place without one."""
     T, Hh, D = x.shape
     pos_t = None
     if positions is not None:
         pos_t = positions.reshape(-1).to(torch.int32).contiguous()
-    rc = _lib.lib().nxd_rope_inplace(_lib.ptr(x), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(pos_t), _c.c_longlong(T),
-                                     _c.c_int(Hh), _c.c_int(n_rot_heads), _c.c_int(D), _c.c_int(pos_div),
-                                     _c.c_int(pos_mod), _c.c_int(1 if inverse else 0), _lib.stream_ptr())
-    _lib.check(rc, "nxd_rope_inplace")
+    rc = _lib.lib().nxd_rope(_lib.ptr(x), _lib.ptr(x if out is None else out), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(pos_t),
+                             _c.c_longlong(T), _c.c_int(Hh), _c.c_int(n_rot_heads), _c.c_int(D), _c.c_int(pos_div),
+                             _c.c_int(pos_mod), _c.c_int(1 if inverse else 0), _lib.stream_ptr())
+    _lib.check(rc, "nxd_rope")
 
 
 def apply_rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, n_rot_heads: int, pos_div: int = 1,
