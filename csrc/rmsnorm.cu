@@ -13,6 +13,8 @@
 //           dw = sum_rows(dy * xhat)   -> persistent CTAs accumulate per-thread
 //           partials in registers, write [P, H] fp32 partials to scratch, and a
 //           second kernel reduces the P partial rows.
+#include <cuda_pipeline.h>
+
 #include "common.cuh"
 
 namespace {
@@ -73,82 +75,101 @@ __global__ void rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __res
     }
 }
 
+// Rows of up to kRingMaxH columns (the ring of wider ones doesn't fit).  Bound by memory (3 reads and a
+// write per element with a residual gradient).  A thread copies its own columns of the CTA's next rows into shared memory with
+// cp.async, kRing - 1 rows ahead, and reads only what it copied itself: no barrier for the data, one for the row's sum, and 160 to
+// 200 KB in flight per SM whatever the registers allow.  The grid is what is resident at once.  8192 x 3072 (201 MB): 71 us with
+// the next row prefetched into registers (113 of them: 3 CTAs per SM for a grid of 4), 44 us.
+constexpr int kRing = 3, kRingMaxH = 8192;
+
 template <int VPT>
-__global__ void rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
-                                   const bf16* __restrict__ w, const float* __restrict__ rstd,
-                                   const bf16* __restrict__ dres, bf16* __restrict__ dx,
-                                   float* __restrict__ dw_partial, int rows, int H) {
-    __shared__ float red[32];
-    const int nvec = H >> 3;
-    float wv[VPT][8], dwacc[VPT][8];
-    const bf16x8* wr = reinterpret_cast<const bf16x8*>(w);
+__global__ void __launch_bounds__(VPT == 1 ? 256 : 512)
+rmsnorm_bwd_ring_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w,
+                        const float* __restrict__ rstd, const bf16* __restrict__ dres, bf16* __restrict__ dx,
+                        float* __restrict__ dw_partial, int rows, int H) {
+    extern __shared__ __align__(16) bf16x8 ring[];       // [kRing][dy | x | dres][nvec]
+    __shared__ float red[2][32];
+    const int nvec = H >> 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
+    float dwacc[VPT][8];
+    bf16x8 wv[VPT];
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
         const int c = threadIdx.x + i * blockDim.x;
 #pragma unroll
         for (int k = 0; k < 8; ++k) dwacc[i][k] = 0.f;
-        if (c < nvec) {
-            bf16x8 p = wr[c];
-            unpack8(p, wv[i]);
-        }
+        if (c < nvec) wv[i] = reinterpret_cast<const bf16x8*>(w)[c];
     }
-    // software pipeline over the rows of this CTA: the loads of row i + 1 are issued before the block-wide reduction
-    // of row i, so the row loop is no longer one global-load latency plus two barriers per row (61 us -> see profiles)
-    bf16x8 ndy[VPT], nx[VPT];
-    auto fetch = [&](int row) {
-        const bf16x8* dyr = reinterpret_cast<const bf16x8*>(dy + (size_t)row * H);
-        const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + (size_t)row * H);
+    auto fetch = [&](int row, int slot) {
+        if (row < rows) {
+            bf16x8* dst = ring + (size_t)slot * 3 * nvec;
+            const size_t at = (size_t)row * H;
 #pragma unroll
-        for (int i = 0; i < VPT; ++i) {
-            const int c = threadIdx.x + i * blockDim.x;
-            if (c < nvec) {
-                ndy[i] = dyr[c];
-                nx[i] = xr[c];
+            for (int i = 0; i < VPT; ++i) {
+                const int c = threadIdx.x + i * blockDim.x;
+                if (c < nvec) {
+                    __pipeline_memcpy_async(dst + c, dy + at + c * 8, 16);
+                    __pipeline_memcpy_async(dst + nvec + c, x + at + c * 8, 16);
+                    if (dres != nullptr) __pipeline_memcpy_async(dst + 2 * nvec + c, dres + at + c * 8, 16);
+                }
             }
         }
+        __pipeline_commit();
     };
-    if ((int)blockIdx.x < rows) fetch(blockIdx.x);
+#pragma unroll
+    for (int j = 0; j < kRing - 1; ++j) fetch(blockIdx.x + j * gridDim.x, j);
+    int slot = 0, par = 0;
     for (int row = blockIdx.x; row < rows; row += gridDim.x) {
         const float rs = rstd[row];
-        float g[VPT][8], xh[VPT][8];
+        {   // the slot read in the last round is free: this thread alone uses its columns
+            const int ahead = slot == 0 ? kRing - 1 : slot - 1;
+            const long long next = row + (long long)(kRing - 1) * gridDim.x;
+            fetch(next < rows ? (int)next : rows, ahead);
+        }
+        __pipeline_wait_prior(kRing - 1);
+        const bf16x8* src = ring + (size_t)slot * 3 * nvec;
         float dot = 0.f;
 #pragma unroll
         for (int i = 0; i < VPT; ++i) {
             const int c = threadIdx.x + i * blockDim.x;
             if (c < nvec) {
-                float d[8], xv[8];
-                unpack8(ndy[i], d);
-                unpack8(nx[i], xv);
+                float d[8], xv[8], wf[8];
+                unpack8(src[c], d);
+                unpack8(src[nvec + c], xv);
+                unpack8(wv[i], wf);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
-                    xh[i][k] = xv[k] * rs;
-                    g[i][k] = d[k] * wv[i][k];
-                    dot += g[i][k] * xh[i][k];
-                    dwacc[i][k] += d[k] * xh[i][k];
+                    const float xh = xv[k] * rs;
+                    dot += d[k] * wf[k] * xh;
+                    dwacc[i][k] += d[k] * xh;
                 }
             }
         }
-        if (row + (int)gridDim.x < rows) fetch(row + gridDim.x);
-        dot = block_sum(dot, red) / (float)H;
+        dot = warp_sum(dot);
+        if (lane == 0) red[par][warp] = dot;
+        __syncthreads();                                 // red[par] is written again two rows on, behind the next row's barrier
+        dot = warp_sum(lane < nwarps ? red[par][lane] : 0.f) / (float)H;
         bf16x8* dxr = reinterpret_cast<bf16x8*>(dx + (size_t)row * H);
-        const bf16x8* drr = dres ? reinterpret_cast<const bf16x8*>(dres + (size_t)row * H) : nullptr;
 #pragma unroll
         for (int i = 0; i < VPT; ++i) {
             const int c = threadIdx.x + i * blockDim.x;
             if (c < nvec) {
-                float o[8];
+                float d[8], xv[8], wf[8], o[8];
+                unpack8(src[c], d);
+                unpack8(src[nvec + c], xv);
+                unpack8(wv[i], wf);
 #pragma unroll
-                for (int k = 0; k < 8; ++k) o[k] = rs * (g[i][k] - xh[i][k] * dot);
-                if (drr) {  // fused add of the gradient flowing through the residual branch
+                for (int k = 0; k < 8; ++k) o[k] = rs * (d[k] * wf[k] - xv[k] * rs * dot);
+                if (dres != nullptr) {                   // fused add of the gradient flowing through the residual branch
                     float r[8];
-                    bf16x8 q = drr[c];
-                    unpack8(q, r);
+                    unpack8(src[2 * nvec + c], r);
 #pragma unroll
                     for (int k = 0; k < 8; ++k) o[k] += r[k];
                 }
                 dxr[c] = pack8(o);
             }
         }
+        par ^= 1;
+        slot = slot + 1 == kRing ? 0 : slot + 1;
     }
     float* out = dw_partial + (size_t)blockIdx.x * H;
 #pragma unroll
@@ -162,14 +183,26 @@ __global__ void rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __re
     }
 }
 
-// dw[h] = sum_p partial[p, h]; optionally accumulates into an fp32 buffer.
-__global__ void colsum_partials_kernel(const float* __restrict__ partial, int P, int H,
-                                       bf16* __restrict__ dw_bf16, float* __restrict__ dw_f32,
-                                       int accumulate) {
-    const int h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= H) return;
+// dw[h] = sum_p partial[p, h]; optionally accumulates into an fp32 buffer.  32 columns per block (one 128-byte line of a
+// partial row per warp), kSumWarps warps take every kSumWarps-th row, 8 loads in flight each.  592 rows x 3072: 29 us with one
+// thread per column, 5 us.
+constexpr int kSumWarps = 16;
+
+__global__ void __launch_bounds__(32 * kSumWarps)
+colsum_partials_kernel(const float* __restrict__ partial, int P, int H, bf16* __restrict__ dw_bf16,
+                       float* __restrict__ dw_f32, int accumulate) {
+    __shared__ float part[kSumWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, h = blockIdx.x * 32 + lane;
     float s = 0.f;
-    for (int p = 0; p < P; ++p) s += partial[(size_t)p * H + h];
+    if (h < H) {
+#pragma unroll 8
+        for (int p = warp; p < P; p += kSumWarps) s += partial[(size_t)p * H + h];
+    }
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp != 0 || h >= H) return;
+#pragma unroll
+    for (int i = 1; i < kSumWarps; ++i) s += part[i][lane];
     if (dw_f32) dw_f32[h] = accumulate ? dw_f32[h] + s : s;
     if (dw_bf16) dw_bf16[h] = __float2bfloat16(s);
 }
@@ -230,23 +263,34 @@ NXD_API int nxd_rmsnorm_fwd(const void* x, const void* residual, const void* w, 
     return 0;
 }
 
-static int rmsnorm_bwd_impl(const void* dy, const void* x, const void* w, const float* rstd, const void* dresidual,
-                            void* dx, void* dw_bf16, float* dw_f32, int accumulate, float* scratch, int rows,
-                            int H, cudaStream_t s) {
-    NormCfg c = pick_cfg(H);
-    const int P = nxd_rmsnorm_bwd_num_partials(rows);
-#define LAUNCH(V)                                                                                        \
-    rmsnorm_bwd_kernel<V><<<P, c.threads, 0, s>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, \
-                                                  (const bf16*)dresidual, (bf16*)dx, scratch, rows, H)
-    switch (c.vpt) {
-        case 1: LAUNCH(1); break;
-        case 2: LAUNCH(2); break;
-        case 4: LAUNCH(4); break;
-        default: LAUNCH(8); break;
+template <int VPT>
+static int rmsnorm_bwd_ring(const void* dy, const void* x, const void* w, const float* rstd, const void* dresidual, void* dx,
+                            float* scratch, int& P, int rows, int H, cudaStream_t s) {
+    const int smem = kRing * 3 * H * 2, threads = ((H / 8 + VPT - 1) / VPT + 31) / 32 * 32;
+    static bool configured = false;
+    if (!configured) {
+        NXD_CHECK_CUDA(cudaFuncSetAttribute(rmsnorm_bwd_ring_kernel<VPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            kRing * 3 * kRingMaxH * 2));
+        configured = true;
     }
-#undef LAUNCH
+    // resident CTAs per SM: 227 KB of shared memory (1 KB of it reserved per CTA); 64 (VPT 1) and 80 registers a thread let 4 run
+    int per_sm = 232448 / (smem + 1024 + 256);
+    if (per_sm > 4) per_sm = 4;
+    if (P > per_sm * nxd_num_sms()) P = per_sm * nxd_num_sms();
+    rmsnorm_bwd_ring_kernel<VPT><<<P, threads, smem, s>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd,
+                                                          (const bf16*)dresidual, (bf16*)dx, scratch, rows, H);
     NXD_LAUNCH_CHECK();
-    colsum_partials_kernel<<<(H + 255) / 256, 256, 0, s>>>(scratch, P, H, (bf16*)dw_bf16, dw_f32, accumulate);
+    return 0;
+}
+
+// scratch: P * H floats
+static int rmsnorm_bwd_impl(const void* dy, const void* x, const void* w, const float* rstd, const void* dresidual,
+                            void* dx, void* dw_bf16, float* dw_f32, int accumulate, float* scratch, int P, int rows,
+                            int H, cudaStream_t s) {
+    const int rc = H <= 2048 ? rmsnorm_bwd_ring<1>(dy, x, w, rstd, dresidual, dx, scratch, P, rows, H, s)
+                             : rmsnorm_bwd_ring<2>(dy, x, w, rstd, dresidual, dx, scratch, P, rows, H, s);
+    if (rc) return rc;
+    colsum_partials_kernel<<<(H + 31) / 32, 32 * kSumWarps, 0, s>>>(scratch, P, H, (bf16*)dw_bf16, dw_f32, accumulate);
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -255,7 +299,7 @@ static int rmsnorm_bwd_impl(const void* dy, const void* x, const void* w, const 
 // (the column-sum kernel with no partial rows reads nothing and stores 0).
 static int rmsnorm_bwd_empty(void* dw_bf16, float* dw_f32, int accumulate, int H, cudaStream_t s) {
     if (accumulate || (dw_bf16 == nullptr && dw_f32 == nullptr)) return 0;
-    colsum_partials_kernel<<<(H + 255) / 256, 256, 0, s>>>(nullptr, 0, H, (bf16*)dw_bf16, dw_f32, 0);
+    colsum_partials_kernel<<<(H + 31) / 32, 32 * kSumWarps, 0, s>>>(nullptr, 0, H, (bf16*)dw_bf16, dw_f32, 0);
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -267,8 +311,9 @@ NXD_API int nxd_rmsnorm_bwd(const void* dy, const void* x, const void* w, const 
     NXD_REQUIRE(H % 8 == 0 && H <= 65536, "rmsnorm_bwd: H=%d must be a multiple of 8 and <= 65536", H);
     NXD_REQUIRE(scratch != nullptr, "rmsnorm_bwd: scratch buffer is required");
     if (rows == 0) return rmsnorm_bwd_empty(dw_bf16, dw_f32, accumulate, H, (cudaStream_t)stream);
-    return rmsnorm_bwd_impl(dy, x, w, rstd, dresidual, dx, dw_bf16, dw_f32, accumulate, scratch, rows, H,
-                            (cudaStream_t)stream);
+    NXD_REQUIRE(H <= kRingMaxH, "rmsnorm_bwd: H=%d, at most %d columns", H, kRingMaxH);
+    return rmsnorm_bwd_impl(dy, x, w, rstd, dresidual, dx, dw_bf16, dw_f32, accumulate, scratch,
+                            nxd_rmsnorm_bwd_num_partials(rows), rows, H, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -318,26 +363,6 @@ int static_scratch_for_current_device(float** out) {
     return 0;
 }
 
-int rmsnorm_bwd_static_launch(const void* dy, const void* x, const void* w, const float* rstd, const void* dresidual,
-                              void* dx, void* dw_bf16, float* dw_f32, int accumulate, float* scratch, int P, int rows,
-                              int H, cudaStream_t s) {
-    NormCfg c = pick_cfg(H);
-#define LAUNCH(V)                                                                                        \
-    rmsnorm_bwd_kernel<V><<<P, c.threads, 0, s>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, \
-                                                  (const bf16*)dresidual, (bf16*)dx, scratch, rows, H)
-    switch (c.vpt) {
-        case 1: LAUNCH(1); break;
-        case 2: LAUNCH(2); break;
-        case 4: LAUNCH(4); break;
-        default: LAUNCH(8); break;
-    }
-#undef LAUNCH
-    NXD_LAUNCH_CHECK();
-    colsum_partials_kernel<<<(H + 255) / 256, 256, 0, s>>>(scratch, P, H, (bf16*)dw_bf16, dw_f32, accumulate);
-    NXD_LAUNCH_CHECK();
-    return 0;
-}
-
 }  // namespace
 
 NXD_API int nxd_rmsnorm_bwd_static_max_h(void) { return kStaticMaxH; }
@@ -357,6 +382,6 @@ NXD_API int nxd_rmsnorm_bwd_static(const void* dy, const void* x, const void* w,
     int P = nxd_rmsnorm_bwd_num_partials(rows);
     const int fit = kStaticScratchFloats / H;
     if (P > fit) P = fit;
-    return rmsnorm_bwd_static_launch(dy, x, w, rstd, dresidual, dx, dw_bf16, dw_f32, accumulate, scratch, P, rows, H,
-                                     (cudaStream_t)stream);
+    return rmsnorm_bwd_impl(dy, x, w, rstd, dresidual, dx, dw_bf16, dw_f32, accumulate, scratch, P, rows, H,
+                            (cudaStream_t)stream);
 }
