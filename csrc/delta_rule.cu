@@ -482,8 +482,9 @@ int launch_scan(const float* qn, const float* kn, const float* vn, const float* 
 //                       contraction, so both operands are read as 16-byte pieces and nothing is shuffled)
 // Bound by the fp32 pipes of the second kernel: a token costs 3 D + CH multiply-adds per value column, like token by token, but
 // 64 tokens are independent, where delta_scan waits for two dot products and a shuffle tree per token.  Its own limit is the
-// shared memory that feeds them (0.4 floats read per multiply-add).  4 x 2048 tokens, 4 heads of 128 x 256: 69 + 348 us against
-// 779 us token by token.
+// chain of a chunk's phases: 4 x 2048 tokens, 4 heads of 128 x 256 take 69 + 344 us against 779 us token by token, of which the two
+// wide products cost 99 and 70 us, the triangular ones 78 and barriers, loads and stores the rest (360 us with a chunk's factors
+// loaded at its start instead of one chunk ahead); neither 8 x 8 tiles with half of the shared-memory loads nor 16 warps change it.
 constexpr int CH = 64, CP = CH + 4, CW_THREADS = 256, CW_COLS = 32;
 
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
@@ -646,8 +647,7 @@ delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ 
     float* Ps = Ms + CH * CP;                  // [CH][CP]
     float* Rs = Ps + CH * CP;                  // [32][CP] V - diag(Gamma) K S, a value column per row
     float* Us = Rs + CW_COLS * CP;             // [32][CP] U
-    float* gam = Us + CW_COLS * CP;            // [CH] Gamma
-    float* last = gam + CH;                    // [CH] L[CH-1][.]
+    float* gam2 = Us + CW_COLS * CP;           // [2][2 CH] Gamma and L[CH-1][.] of this chunk and the next
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int col0 = blockIdx.x * CW_COLS, h = blockIdx.y, b = blockIdx.z, kvh = h / (H / G);
     const int n = n_new != nullptr ? min(n_new[b], Tn) : Tn;
@@ -682,9 +682,15 @@ delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ 
                                 chunk0 + (long long)c * CHUNK_FLOATS + off + t * CH + x, true);
             }
     };
+    auto factors = [&](int c) {                                  // Gamma and L[CH-1][.] of chunk c
+        if (c < chunks && tid < 2 * CH / 4)
+            mma::cp_async16((uint32_t)__cvta_generic_to_shared(gam2 + (c & 1) * 2 * CH + tid * 4),
+                            chunk0 + (long long)c * CHUNK_FLOATS + 2 * CH * CH + tid * 4, true);
+    };
     rows(kn, Kb, 0);
     rows(qn, Qs, 0);
     square(0, Ms, 0);
+    factors(0);
     mma::cp_async_commit();
     square(CH * CH, Ps, 0);
     mma::cp_async_commit();
@@ -692,7 +698,7 @@ delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ 
     for (int c = 0; c < chunks; ++c) {
         const float* Ks = Kb + (KB == 2 ? (c & 1) * CH * DP : 0);
         const int t0 = c * CH;
-        if (tid < 2 * CH) gam[tid] = chunk0[(long long)c * CHUNK_FLOATS + 2 * CH * CH + tid];      // and `last` behind it
+        const float *gam = gam2 + (c & 1) * 2 * CH, *last = gam + CH;
         float v[2][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -782,6 +788,7 @@ delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ 
         mma::cp_async_wait<KB>();              // P of this chunk (the groups behind it: Q and, with two buffers, K)
         __syncthreads();
         square(0, Ms, c + 1);
+        factors(c + 1);
         mma::cp_async_commit();
 #pragma unroll
         for (int i = 0; i < 4; ++i) y[0][i] = y[1][i] = 0ull;
@@ -850,8 +857,8 @@ int launch_chunks(const float* qn, const float* kn, const float* vn, const float
     constexpr int DP = D + 4;
     const int NC = (Tn + CH - 1) / CH;
     const size_t sys = (size_t)4 * CH * CP * sizeof(float);
-    const size_t scan = (size_t)((D <= 128 ? 3 : 2) * CH * DP + CW_COLS * DP + 2 * CH * CP + 2 * CW_COLS * CP + 2 * CH) * sizeof(float);
-    static_assert((2 * CH * 260 + CW_COLS * 260 + 2 * CH * CP + 2 * CW_COLS * CP + 2 * CH) * 4 <= 232448, "shared memory");
+    const size_t scan = (size_t)((D <= 128 ? 3 : 2) * CH * DP + CW_COLS * DP + 2 * CH * CP + 2 * CW_COLS * CP + 4 * CH) * sizeof(float);
+    static_assert((2 * CH * 260 + CW_COLS * 260 + 2 * CH * CP + 2 * CW_COLS * CP + 4 * CH) * 4 <= 232448, "shared memory");
     NXD_CHECK_CUDA(cudaFuncSetAttribute(delta_chunk_system_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sys));
     NXD_CHECK_CUDA(cudaFuncSetAttribute(delta_chunk_scan_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan));
     delta_chunk_system_kernel<D><<<dim3(NC, H, B), CW_THREADS, sys, st>>>(qn, kn, gate, ld_a, a_off, beta, ld_b, b_off, scratch,
