@@ -494,12 +494,10 @@ __global__ void kv_cache_update_kernel(const bf16* __restrict__ new_k, const bf1
 
 NXD_API int nxd_decode_attn_num_splits(int B, int n_kv, int max_len) {
     // one wave of CTAs (two per SM) at least 128 keys each: a second, partial wave costs more than a longer loop (16 sequences of
-    // 2048 keys, 8 heads of 64: 12.2 us with 2 splits, 14.6 with 3; 4 sequences: 5.9 with 8, 6.8 with 10).  From half a wave of
-    // pairs on, sequences of different lengths want the finer split (12 of up to 2900 keys, heads of 128: 26.1 with 4, 29.8 with
-    // 2).
+    // 2048 keys, 8 heads of 64: 12.2 us with 2 splits, 14.6 with 3; 4 sequences: 5.9 with 8, 6.8 with 10; 12 of up to 2576 keys:
+    // 13.2 with 3, 14.9 with 4, and with heads of 128 20.8 with 3, 21.3 with 4).
     const int pairs = B * n_kv;
-    int want = 2 * nxd_num_sms() / (pairs > 0 ? pairs : 1);
-    if (want < 4 && want > 1 && pairs * 4 <= 3 * nxd_num_sms()) want = 4;
+    const int want = 2 * nxd_num_sms() / (pairs > 0 ? pairs : 1);
     int by_len = (max_len + 127) / 128;
     int s = want < by_len ? want : by_len;
     if (s < 1) s = 1;
