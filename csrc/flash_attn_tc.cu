@@ -390,10 +390,11 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                 mx3 = fmaxf(mx3, __uint_as_float(sr[c + 3]));
             }
             const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
-            // lazy rescale: keep the stale max unless it moved by more than 2^8 (in scaled log2 units)
+            // lazy rescale: keep the stale max unless it moved by more than 2^8 (in scaled log2 units).  CACHE follows every
+            // move, as the kernels it takes calls from do: the row's largest weight is then exactly 1 and not rounded.
             float alpha = 1.f;
             bool rescale = false;
-            if ((mx - m_run) * sc > kRescaleThreshold || m_run == -INFINITY) {
+            if ((mx - m_run) * sc > (CACHE ? 0.f : kRescaleThreshold) || m_run == -INFINITY) {
                 const float m_new = fmaxf(m_run, mx);
                 if (m_new != -INFINITY) {
                     alpha = ex2_approx((m_run - m_new) * sc);   // 0 when m_run was -inf

@@ -61,3 +61,29 @@ def test_portion_over_the_cache_matches_the_restatement(D, T, starts, n_new, pag
                                       D ** -0.5, window, keep, slopes, gate=None if gate is None else gate[b, :n], **kw)
         # the weights and the result are rounded to bf16: 2^-9 of each weight and of the value
         assert (out[b, :n].float() - ref).norm() <= 2.0 ** -7 * ref.norm()
+
+
+# weights are rounded to bf16: relative to the row's running maximum the largest one is 1 and keeps its value, relative to a stale
+# maximum it is rounded too.  Few keys that matter (distance bias, scores of a wide spread), and many
+@pytest.mark.parametrize("D,T,past,window,bias,spread", [(128, 300, 600, 512, True, 1.0), (64, 300, 100, None, False, 1.0),
+                                                         (64, 300, 600, 512, False, 3.0), (128, 200, 3000, None, True, 2.0)])
+def test_weights_are_no_further_off_than_on_the_mma_kernel(D, T, past, window, bias, spread):
+    from neuronx_distributed_llama3_2_b200.ops import window_attention as wa
+
+    B, H, G, S = 2, 16, 4, past + T
+    g = torch.Generator(device="cuda").manual_seed(D + T)
+    q, k, v = (torch.randn(*s, generator=g, device="cuda").bfloat16() for s in ((B, T, H, D), (B, G, S, D), (B, G, S, D)))
+    q = q * spread
+    slopes = wa.distance_slopes(H, device="cuda") if bias else None
+    start = torch.full((B,), past, dtype=torch.int32, device="cuda")
+    pos, key = torch.arange(past, S, device="cuda"), torch.arange(S, device="cuda")
+    dist = pos[:, None] - key[None]
+    s = torch.einsum("bthd,bhnd->bhtn", q.double(), k.double().repeat_interleave(H // G, 1)) * D ** -0.5
+    if bias:
+        s -= slopes.double()[:, None, None] * dist
+    s.masked_fill_((dist < 0) | (dist >= (window or S)), float("-inf"))
+    ref = torch.einsum("bhtn,bhnd->bthd", s.softmax(-1), v.double().repeat_interleave(H // G, 1))
+    tc, mma = ((wa.window_attention_prefill(q, k, v, start, D ** -0.5, window, slopes=slopes, impl=i).double() - ref).norm()
+               for i in ("tc", "mma"))
+    # both errors are sums over more than 6000 rows of independent roundings, their ratio scatters by less than 2 %
+    assert tc <= 1.02 * mma
