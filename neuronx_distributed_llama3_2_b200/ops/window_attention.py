@@ -260,7 +260,8 @@ def _out_rows(out: Optional[torch.Tensor], q: torch.Tensor, rows: int, H: int, D
 # tokens x cache rows from which the tcgen05 kernel over the cache serves a portion.  Measured against the mma.sync kernel at 16
 # and 32 heads of 64 / 128, 1 to 3 rows, portions of 16 .. 1024 after 1 .. 3000 tokens: below, both are bound by the call itself
 # (25 to 31 us); above, 31 .. 71 us against 32 .. 203 us without score changes and 61 .. 209 against 105 .. 815 us with them.
-TC_CACHE_MIN_WORK = 150_000
+# Fewer tokens than the mma.sync kernel takes (16) stay on the generic kernel, which does not round its weights to bf16.
+TC_CACHE_MIN_WORK, TC_CACHE_MIN_TOKENS = 150_000, 16
 
 
 def _tc_cache(L):
@@ -319,7 +320,7 @@ def window_attention_prefill(q: torch.Tensor, cache_k: torch.Tensor, cache_v: to
         cargs, bt = _cache_args(cache_k, cache_v, block_table, page_size, rows=True)
         sk = sinks.float().contiguous() if sinks is not None else None
         margs, _keep = _mod_args(softcap, log_bias, sigmoid_bias, gate, q, Dv if gate_elements else 0, gate_mul, out_ld)
-        if impl == "tc" or (impl == "auto" and not chunk and not value_heads and T * (
+        if impl == "tc" or (impl == "auto" and not chunk and not value_heads and T >= TC_CACHE_MIN_TOKENS and T * (
                 cache_k.shape[2] * (bt.shape[1] if bt is not None else 1)) >= TC_CACHE_MIN_WORK):
             tc = _tc_cache_applies(q, cache_k, cache_v, out, G, bt, page_size, gate, gate_elements)
             assert tc and not chunk and not value_heads or impl == "auto"

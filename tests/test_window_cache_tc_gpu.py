@@ -87,3 +87,16 @@ def test_weights_are_no_further_off_than_on_the_mma_kernel(D, T, past, window, b
                for i in ("tc", "mma"))
     # both errors are sums over more than 6000 rows of independent roundings, their ratio scatters by less than 2 %
     assert tc <= 1.02 * mma
+
+
+# on either side of the 16 tokens from which weights are rounded to bf16, over a cache that is long enough for any portion
+@pytest.mark.parametrize("T,kernel", [(2, "generic"), (15, "generic"), (16, "tc")])
+def test_few_tokens_over_a_long_cache_keep_fp32_weights(T, kernel):
+    from neuronx_distributed_llama3_2_b200.ops import window_attention as wa
+
+    g = torch.Generator(device="cuda").manual_seed(T)
+    q, k, v = (torch.randn(*s, generator=g, device="cuda").bfloat16() for s in ((1, T, 4, 128), (1, 2, 1 << 17, 128), (1, 2, 1 << 17, 128)))
+    start = torch.full((1,), 500, dtype=torch.int32, device="cuda")
+    assert T * k.shape[2] >= wa.TC_CACHE_MIN_WORK
+    auto, same = (wa.window_attention_prefill(q, k, v, start, 0.1, 300, impl=i) for i in ("auto", kernel))
+    assert torch.equal(auto, same)
