@@ -75,18 +75,29 @@ __global__ void rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __res
     }
 }
 
-// Rows of up to kRingMaxH columns (the ring of wider ones doesn't fit).  Bound by memory (3 reads and a
-// write per element with a residual gradient).  A thread copies its own columns of the CTA's next rows into shared memory with
-// cp.async, kRing - 1 rows ahead, and reads only what it copied itself: no barrier for the data, one for the row's sum, and 160 to
-// 200 KB in flight per SM whatever the registers allow.  The grid is what is resident at once.  8192 x 3072 (201 MB): 71 us with
-// the next row prefetched into registers (113 of them: 3 CTAs per SM for a grid of 4), 44 us.
-constexpr int kRing = 3, kRingMaxH = 8192;
+// Bound by memory (3 reads and a write per element with a residual gradient).  A thread copies its own columns of the CTA's next
+// rows into shared memory with cp.async, kRing - 1 rows ahead, and reads only what it copied itself: no barrier for the data, one
+// for the row's sum.  The grid is what is resident at once: up to 4 CTAs per SM, each with rings of 6 kRing H bytes (3072 columns:
+// 221 KB per SM, two thirds of it without a residual gradient).  8192 x 3072 (201 MB): 71 us with the next row prefetched into
+// registers (113 of them: 3 CTAs per SM for a grid of 4), 44 us.
+// 8 VPT columns per thread and at most 512 threads: 2048, 8192 and kRingMaxH columns with 1, 2 and 4 vectors.  Three rows of more
+// than 12842 columns do not fit shared memory, so the widest instance keeps two.
+constexpr int kRingMaxH = 16384;
+
+template <int VPT>
+struct RingCfg {
+    static constexpr int kRows = VPT == 4 ? 2 : 3;
+    static constexpr int kMaxH = VPT == 1 ? 2048 : VPT == 2 ? 8192 : kRingMaxH;
+    static constexpr int kCtas = VPT == 4 ? 2 : 4;           // per SM that the registers (48, 58 and 109 a thread) let run
+    static constexpr int smem(int H) { return kRows * 3 * H * 2; }
+};
 
 template <int VPT>
 __global__ void __launch_bounds__(VPT == 1 ? 256 : 512)
 rmsnorm_bwd_ring_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w,
                         const float* __restrict__ rstd, const bf16* __restrict__ dres, bf16* __restrict__ dx,
                         float* __restrict__ dw_partial, int rows, int H) {
+    constexpr int kRing = RingCfg<VPT>::kRows;
     extern __shared__ __align__(16) bf16x8 ring[];       // [kRing][dy | x | dres][nvec]
     __shared__ float red[2][32];
     const int nvec = H >> 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
@@ -266,16 +277,17 @@ NXD_API int nxd_rmsnorm_fwd(const void* x, const void* residual, const void* w, 
 template <int VPT>
 static int rmsnorm_bwd_ring(const void* dy, const void* x, const void* w, const float* rstd, const void* dresidual, void* dx,
                             float* scratch, int& P, int rows, int H, cudaStream_t s) {
-    const int smem = kRing * 3 * H * 2, threads = ((H / 8 + VPT - 1) / VPT + 31) / 32 * 32;
+    using C = RingCfg<VPT>;
+    const int smem = C::smem(H), threads = ((H / 8 + VPT - 1) / VPT + 31) / 32 * 32;
     static bool configured = false;
     if (!configured) {
         NXD_CHECK_CUDA(cudaFuncSetAttribute(rmsnorm_bwd_ring_kernel<VPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            kRing * 3 * kRingMaxH * 2));
+                                            C::smem(C::kMaxH)));
         configured = true;
     }
-    // resident CTAs per SM: 227 KB of shared memory (1 KB of it reserved per CTA); 64 (VPT 1) and 80 registers a thread let 4 run
+    // resident CTAs per SM: 227 KB of shared memory (1 KB of it reserved per CTA); the registers let C::kCtas run
     int per_sm = 232448 / (smem + 1024 + 256);
-    if (per_sm > 4) per_sm = 4;
+    if (per_sm > C::kCtas) per_sm = C::kCtas;
     if (P > per_sm * nxd_num_sms()) P = per_sm * nxd_num_sms();
     rmsnorm_bwd_ring_kernel<VPT><<<P, threads, smem, s>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd,
                                                           (const bf16*)dresidual, (bf16*)dx, scratch, rows, H);
@@ -287,8 +299,9 @@ static int rmsnorm_bwd_ring(const void* dy, const void* x, const void* w, const 
 static int rmsnorm_bwd_impl(const void* dy, const void* x, const void* w, const float* rstd, const void* dresidual,
                             void* dx, void* dw_bf16, float* dw_f32, int accumulate, float* scratch, int P, int rows,
                             int H, cudaStream_t s) {
-    const int rc = H <= 2048 ? rmsnorm_bwd_ring<1>(dy, x, w, rstd, dresidual, dx, scratch, P, rows, H, s)
-                             : rmsnorm_bwd_ring<2>(dy, x, w, rstd, dresidual, dx, scratch, P, rows, H, s);
+    const int rc = H <= RingCfg<1>::kMaxH   ? rmsnorm_bwd_ring<1>(dy, x, w, rstd, dresidual, dx, scratch, P, rows, H, s)
+                   : H <= RingCfg<2>::kMaxH ? rmsnorm_bwd_ring<2>(dy, x, w, rstd, dresidual, dx, scratch, P, rows, H, s)
+                                            : rmsnorm_bwd_ring<4>(dy, x, w, rstd, dresidual, dx, scratch, P, rows, H, s);
     if (rc) return rc;
     colsum_partials_kernel<<<(H + 31) / 32, 32 * kSumWarps, 0, s>>>(scratch, P, H, (bf16*)dw_bf16, dw_f32, accumulate);
     NXD_LAUNCH_CHECK();
@@ -329,7 +342,7 @@ NXD_API int nxd_rmsnorm_bwd(const void* dy, const void* x, const void* w, const 
 //
 //   * Limit: H <= kStaticMaxH (8192).  The number of partial rows is reduced to fit (at least 128 rows of partials
 //     remain at the largest H), which changes the summation order of dW slightly but not the result beyond fp32
-//     rounding.  Larger H is rejected with an error; use nxd_rmsnorm_bwd() with your own buffer instead.
+//     rounding.  Larger H is rejected with an error; use nxd_rmsnorm_bwd() (up to 16384 columns) with your own buffer instead.
 //   * The first call on each device resolves the array's device address (cudaGetSymbolAddress with that device
 //     current).  Make that first call before you start capturing a stream into a graph.
 //   * All calls share the one array.  Nothing in it has to start at zero -- every partial row that is read is

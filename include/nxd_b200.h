@@ -39,7 +39,7 @@ int nxd_gemm_bf16(int layout, const void* a, const void* b, void* d, int M, int 
 int nxd_rmsnorm_fwd(const void* x, const void* residual, const void* w, void* y, void* residual_out,
                     float* rstd, int rows, int H, float eps, void* stream);
 int nxd_rmsnorm_bwd_num_partials(int rows);
-/* scratch: nxd_rmsnorm_bwd_num_partials(rows) * H floats */
+/* scratch: nxd_rmsnorm_bwd_num_partials(rows) * H floats; H a multiple of 8, at most 16384 */
 int nxd_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dresidual,
                     void* dx, void* dw_bf16, float* dw_f32, int accumulate, float* scratch, int rows, int H,
                     void* stream);

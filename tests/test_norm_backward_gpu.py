@@ -5,8 +5,10 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# widths at the switch from one to two vectors per thread (2048) and the widest (8192), threads without a column, one vector; rows below and above the ring's depth and the grid
-@pytest.mark.parametrize("rows,H", [(1, 8), (3, 264), (700, 264), (2401, 2048), (5, 2056), (1501, 3072), (447, 8192)])
+# widths at the switches to two (2048) and four (8192) vectors per thread and the widest (16384), threads without a column, one
+# vector; rows below and above the ring's depth and the grid
+@pytest.mark.parametrize("rows,H", [(1, 8), (3, 264), (700, 264), (2401, 2048), (5, 2056), (1501, 3072), (447, 8192), (3, 8200),
+                                    (701, 9216), (1, 16384), (301, 16384)])
 @pytest.mark.parametrize("residual", [False, True])
 def test_rms_norm_backward_matches_float64(rows, H, residual):
     from neuronx_distributed_llama3_2_b200.ops import norm
@@ -39,6 +41,6 @@ def test_rms_norm_backward_matches_float64(rows, H, residual):
 def test_rows_wider_than_the_ring_are_refused():
     from neuronx_distributed_llama3_2_b200.ops import norm
 
-    x = torch.ones(2, 8200, device="cuda", dtype=torch.bfloat16).requires_grad_()
+    x = torch.ones(2, 16392, device="cuda", dtype=torch.bfloat16).requires_grad_()
     with pytest.raises(RuntimeError, match="rmsnorm_bwd"):
         norm.rms_norm(x, x.detach()[0], 1e-6).sum().backward()
