@@ -6,6 +6,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+
 #define NXD_API extern "C" __attribute__((visibility("default")))
 
 // ---- error reporting (host) -------------------------------------------------
@@ -43,6 +45,20 @@ void nxd_count_launches(int n);
             return (int)_e;                                                     \
         }                                                                       \
     } while (0)
+
+// Lets `Kernel` be launched with up to `bytes` of dynamic shared memory on the current device.  The attribute belongs to a kernel
+// on one device: it is set once for every device that the process launches from, not once per process.
+template <auto Kernel>
+inline cudaError_t nxd_allow_smem(int bytes) {
+    static std::atomic<unsigned long long> done{0};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+    if (e != cudaSuccess || (done.load(std::memory_order_relaxed) & bit)) return e;
+    e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+    return e;
+}
 
 // ---- programmatic dependent launch (PDL) ---------------------------------------
 // The token-generation graph is a chain of short kernels; launch latency and prologues (barrier init, tensor-memory

@@ -544,21 +544,11 @@ static int decode_attn_impl(const void* q, const void* cache_k, const void* cach
     if (use_mma) {
         dim3 mgrid(B * n_kv, n_splits);
         if (D == 64) {
-            static bool configured = false;
-            if (!configured) {
-                NXD_CHECK_CUDA(cudaFuncSetAttribute(decode_attn_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                    MmaDecodeCfg<64>::kSmemBytes));
-                configured = true;
-            }
+            NXD_CHECK_CUDA(nxd_allow_smem<decode_attn_mma_kernel<64>>(MmaDecodeCfg<64>::kSmemBytes));
             NXD_CHECK_CUDA(nxd_launch_pdl(decode_attn_mma_kernel<64>, mgrid, dim3(128), MmaDecodeCfg<64>::kSmemBytes, s,
                                           (const bf16*)q, cv, lengths, part_o, part_ml, n_q, n_kv, n_splits, scale_log2));
         } else {
-            static bool configured = false;
-            if (!configured) {
-                NXD_CHECK_CUDA(cudaFuncSetAttribute(decode_attn_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                    MmaDecodeCfg<128>::kSmemBytes));
-                configured = true;
-            }
+            NXD_CHECK_CUDA(nxd_allow_smem<decode_attn_mma_kernel<128>>(MmaDecodeCfg<128>::kSmemBytes));
             NXD_CHECK_CUDA(nxd_launch_pdl(decode_attn_mma_kernel<128>, mgrid, dim3(128), MmaDecodeCfg<128>::kSmemBytes, s,
                                           (const bf16*)q, cv, lengths, part_o, part_ml, n_q, n_kv, n_splits, scale_log2));
         }

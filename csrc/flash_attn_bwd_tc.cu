@@ -591,10 +591,9 @@ template <int kD, bool CAUSAL, bool DROP>
 int launch_bwd_tc(dim3 grid, cudaStream_t st, const CUtensorMap& tq, const CUtensorMap& tdo, const CUtensorMap& tk,
                   const CUtensorMap& tv, const CUtensorMap& tdk, const CUtensorMap& tdv, const CUtensorMap& tdq,
                   const CUtensorMap& tdka, const CUtensorMap& tdva, const BwdParams& p) {
-    static cudaError_t once = cudaFuncSetAttribute(fa_bwd_tc_kernel<kD, CAUSAL, DROP>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<kD>::kBytes);
-    NXD_CHECK_CUDA(once);
-    fa_bwd_tc_kernel<kD, CAUSAL, DROP><<<grid, kThreadsBwd, BwdSmem<kD>::kBytes, st>>>(tq, tdo, tk, tv, tdk, tdv, tdq, tdka, tdva, p);
+    constexpr auto kern = fa_bwd_tc_kernel<kD, CAUSAL, DROP>;
+    NXD_CHECK_CUDA(nxd_allow_smem<kern>(BwdSmem<kD>::kBytes));
+    kern<<<grid, kThreadsBwd, BwdSmem<kD>::kBytes, st>>>(tq, tdo, tk, tv, tdk, tdv, tdq, tdka, tdva, p);
     NXD_LAUNCH_CHECK();
     return 0;
 }

@@ -526,10 +526,9 @@ int launch_fwd_tc_one(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
                       const TcParams& p, cudaStream_t st) {
     using L = TcSmem<D>;
     dim3 grid(p.Hq, p.B, (p.Sq + kBM - 1) / kBM);
-    static cudaError_t once = cudaFuncSetAttribute(fa_fwd_tc_kernel<D, CAUSAL, DROP>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
-    NXD_CHECK_CUDA(once);
-    fa_fwd_tc_kernel<D, CAUSAL, DROP><<<grid, kThreadsTc, L::kBytes, st>>>(tq, tk, tv, to, p);
+    constexpr auto kern = fa_fwd_tc_kernel<D, CAUSAL, DROP>;
+    NXD_CHECK_CUDA(nxd_allow_smem<kern>(L::kBytes));
+    kern<<<grid, kThreadsTc, L::kBytes, st>>>(tq, tk, tv, to, p);
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -549,10 +548,9 @@ int launch_fwd_tc_win(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
                       const TcParams& p, cudaStream_t st) {
     using L = TcSmem<D>;
     dim3 grid(p.Hq, p.B, (p.Sq + kBM - 1) / kBM);
-    static cudaError_t once = cudaFuncSetAttribute(fa_fwd_tc_kernel<D, true, false, true, SCORE, CACHE>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
-    NXD_CHECK_CUDA(once);
-    fa_fwd_tc_kernel<D, true, false, true, SCORE, CACHE><<<grid, kThreadsTc, L::kBytes, st>>>(tq, tk, tv, to, p);
+    constexpr auto kern = fa_fwd_tc_kernel<D, true, false, true, SCORE, CACHE>;
+    NXD_CHECK_CUDA(nxd_allow_smem<kern>(L::kBytes));
+    kern<<<grid, kThreadsTc, L::kBytes, st>>>(tq, tk, tv, to, p);
     NXD_LAUNCH_CHECK();
     return 0;
 }

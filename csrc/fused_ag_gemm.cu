@@ -488,10 +488,9 @@ static int ag_gemm_impl(int layout, const void* x_local, const void* w, void* y,
 #define NXD_AG_LAUNCH(BN_, BMN_)                                                                              \
     {                                                                                                         \
         using L = SmemLayout<BN_>;                                                                            \
-        static cudaError_t once = cudaFuncSetAttribute(ag_gemm_kernel<BN_, BMN_>,                             \
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes); \
-        NXD_CHECK_CUDA(once);                                                                                 \
-        ag_gemm_kernel<BN_, BMN_><<<dim3(clusters * 2), dim3(kThreads), L::kSmemBytes, st>>>(ta_l, ta_t, tb, td, ag, M, \
+        constexpr auto kern = ag_gemm_kernel<BN_, BMN_>;                                                      \
+        NXD_CHECK_CUDA(nxd_allow_smem<kern>(L::kSmemBytes));                                                  \
+        kern<<<dim3(clusters * 2), dim3(kThreads), L::kSmemBytes, st>>>(ta_l, ta_t, tb, td, ag, M, \
                                                                                              N, K);           \
     }
     if (bn == 256) {

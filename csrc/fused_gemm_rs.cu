@@ -372,10 +372,9 @@ static int gemm_rs_impl(int layout, const void* x, const void* w, void* out, int
 #define NXD_RS_LAUNCH(BN_, BMN_)                                                                              \
     {                                                                                                         \
         using L = SmemLayout<BN_>;                                                                            \
-        static cudaError_t once = cudaFuncSetAttribute(gemm_rs_kernel<BN_, BMN_>,                             \
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes); \
-        NXD_CHECK_CUDA(once);                                                                                 \
-        gemm_rs_kernel<BN_, BMN_><<<dim3(clusters * 2), dim3(kThreads), L::kSmemBytes, st>>>(ta, tb, td, rs, M, N, K); \
+        constexpr auto kern = gemm_rs_kernel<BN_, BMN_>;                                                      \
+        NXD_CHECK_CUDA(nxd_allow_smem<kern>(L::kSmemBytes));                                                  \
+        kern<<<dim3(clusters * 2), dim3(kThreads), L::kSmemBytes, st>>>(ta, tb, td, rs, M, N, K); \
     }
     if (bn == 256) {
         if (layout == 0) NXD_RS_LAUNCH(256, false) else NXD_RS_LAUNCH(256, true)

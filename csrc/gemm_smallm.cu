@@ -425,12 +425,8 @@ template <int BT, int EPI>
 int launch(const CUtensorMap& tw, const CUtensorMap& tx, const EpiArgs& ep, int B, int N, int K, int splits,
            cudaStream_t stream) {
     using C = Cfg<BT, EPI>;
-    auto kern = gemm_smallm_kernel<BT, EPI>;
-    static bool configured = false;
-    if (!configured) {
-        NXD_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
-        configured = true;
-    }
+    constexpr auto kern = gemm_smallm_kernel<BT, EPI>;
+    NXD_CHECK_CUDA(nxd_allow_smem<kern>(C::kSmemBytes));
     const int n_tiles = (N + kWRows - 1) / kWRows;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(n_tiles * splits));

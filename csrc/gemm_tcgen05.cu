@@ -298,12 +298,8 @@ template <int BN, bool A_MN, bool B_MN, int OUT_MODE>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, int M, int N, int K,
                   cudaStream_t stream) {
     using L = SmemLayout<BN>;
-    auto kern = gemm_pair_kernel<BN, A_MN, B_MN, OUT_MODE>;
-    static bool configured = false;
-    if (!configured) {
-        NXD_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes));
-        configured = true;
-    }
+    constexpr auto kern = gemm_pair_kernel<BN, A_MN, B_MN, OUT_MODE>;
+    NXD_CHECK_CUDA(nxd_allow_smem<kern>(L::kSmemBytes));
     const int num_tiles = ((M + kTileM - 1) / kTileM) * ((N + BN - 1) / BN);
     int clusters = nxd_num_sms() / 2;
     if (clusters > num_tiles) clusters = num_tiles;
@@ -376,12 +372,8 @@ template <int BN, bool A_MN, bool B_MN, int OUT_MODE>
 static int launch_grouped(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, int E, int M, int N,
                           int K, cudaStream_t stream) {
     using L = SmemLayout<BN>;
-    auto kern = gemm_pair_kernel<BN, A_MN, B_MN, OUT_MODE, true>;
-    static bool configured = false;
-    if (!configured) {
-        NXD_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes));
-        configured = true;
-    }
+    constexpr auto kern = gemm_pair_kernel<BN, A_MN, B_MN, OUT_MODE, true>;
+    NXD_CHECK_CUDA(nxd_allow_smem<kern>(L::kSmemBytes));
     const long num_tiles = (long)E * ((M + kTileM - 1) / kTileM) * ((N + BN - 1) / BN);
     long clusters = nxd_num_sms() / 2;
     if (clusters > num_tiles) clusters = num_tiles;
@@ -441,12 +433,8 @@ static int launch_experts(const CUtensorMap& ta, const CUtensorMap& tb, const CU
                           const SegArgs& seg, cudaStream_t stream) {
     constexpr int kSmem = SmemLayout<BN>::kSmemBytes + kSegSmemBytes;
     static_assert(kSmem <= 232448, "shared memory budget exceeded");
-    auto kern = gemm_pair_kernel<BN, false, true, OUT_MODE, true, SEG>;
-    static bool configured = false;
-    if (!configured) {
-        NXD_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-        configured = true;
-    }
+    constexpr auto kern = gemm_pair_kernel<BN, false, true, OUT_MODE, true, SEG>;
+    NXD_CHECK_CUDA(nxd_allow_smem<kern>(kSmem));
     const int out_n = SEG == kSegGlu ? BN / 2 : BN;
     // tiles at most: every expert may end in a partial one
     const long most = ((long)rows / kTileM + E) * ((N + out_n - 1) / out_n);
@@ -518,12 +506,8 @@ template <int BN>
 static int launch_glu(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, int M, int N, int K,
                       const SegArgs& act, cudaStream_t stream) {
     using L = SmemLayout<BN>;
-    auto kern = gemm_pair_kernel<BN, false, false, kOutBF16, false, kDenseGlu>;
-    static bool configured = false;
-    if (!configured) {
-        NXD_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes));
-        configured = true;
-    }
+    constexpr auto kern = gemm_pair_kernel<BN, false, false, kOutBF16, false, kDenseGlu>;
+    NXD_CHECK_CUDA(nxd_allow_smem<kern>(L::kSmemBytes));
     const long tiles = (long)((M + kTileM - 1) / kTileM) * ((N + BN / 2 - 1) / (BN / 2));
     long clusters = nxd_num_sms() / 2;
     if (clusters > tiles) clusters = tiles;

@@ -279,12 +279,7 @@ static int rmsnorm_bwd_ring(const void* dy, const void* x, const void* w, const 
                             float* scratch, int& P, int rows, int H, cudaStream_t s) {
     using C = RingCfg<VPT>;
     const int smem = C::smem(H), threads = ((H / 8 + VPT - 1) / VPT + 31) / 32 * 32;
-    static bool configured = false;
-    if (!configured) {
-        NXD_CHECK_CUDA(cudaFuncSetAttribute(rmsnorm_bwd_ring_kernel<VPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            C::smem(C::kMaxH)));
-        configured = true;
-    }
+    NXD_CHECK_CUDA(nxd_allow_smem<rmsnorm_bwd_ring_kernel<VPT>>(C::smem(C::kMaxH)));
     // resident CTAs per SM: 227 KB of shared memory (1 KB of it reserved per CTA); the registers let C::kCtas run
     int per_sm = 232448 / (smem + 1024 + 256);
     if (per_sm > C::kCtas) per_sm = C::kCtas;
