@@ -428,12 +428,12 @@ int run_grouped(int layout, const void* a, const void* b, long long lda, long lo
 #undef NXD_GG_LAYOUT
 }
 
-template <int BN, int SEG, int OUT_MODE = kOutBF16>
+template <int BN, int SEG>
 static int launch_experts(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, int E, int rows, int N, int K,
                           const SegArgs& seg, cudaStream_t stream) {
     constexpr int kSmem = SmemLayout<BN>::kSmemBytes + kSegSmemBytes;
     static_assert(kSmem <= 232448, "shared memory budget exceeded");
-    constexpr auto kern = gemm_pair_kernel<BN, false, true, OUT_MODE, true, SEG>;
+    constexpr auto kern = gemm_pair_kernel<BN, false, true, SEG == kSegPlain ? kOutF32 : kOutBF16, true, SEG>;
     NXD_CHECK_CUDA(nxd_allow_smem<kern>(kSmem));
     const int out_n = SEG == kSegGlu ? BN / 2 : BN;
     // tiles at most: every expert may end in a partial one
@@ -447,17 +447,17 @@ static int launch_experts(const CUtensorMap& ta, const CUtensorMap& tb, const CU
 
 // D[r, :] = act(A[r, :] @ B_e) for the rows r of expert e, all experts in one launch.  A [rows, K] holds the tokens sorted by
 // expert, expert e's counts[e] rows from segment_starts' row offset on (multiples of 32); B [E, K, Nb] row-major.
-//   mode kSegPlain: D [rows, N], Nb = N, bf16 or (wide) fp32;  kSegRelu2: max(., 0)^2;
-//   kSegGlu: Nb = 2 N, gate columns first, D = glu(gate, up)
+//   mode kSegPlain: D [rows, N] fp32, Nb = N;  kSegRelu2: D bf16, max(., 0)^2;
+//   kSegGlu: Nb = 2 N, gate columns first, D bf16 = glu(gate, up)
 // The gate / up products stay in fp32 up to the activation.  Rows between an expert's end and the next one's start are
 // computed along (whatever A holds there) and not stored unless they share a 32-row group with a real row.
-// 8190 tokens, top 2 of 8 experts, 2048 x 4096: 179 us (1540 TF) gate / up with the activation, 99 us (1390 TF) down; one
+// 8190 tokens, top 2 of 8 experts, 2048 x 4096: 179 us (1540 TF) gate / up with the activation, 104 us (1330 TF) down; one
 // launch per expert with the activation in a kernel of its own took 470 us and a host read of the counts.
 // A tile is 256 rows: with few rows per expert the launch is the stream of the weights, and narrow column tiles give it
 // more clusters (pick_block_n on the expected number of tiles).
 static int run_experts(const void* a, const void* b, void* d, const SegArgs& seg, int E, int rows, int pairs, int N, int K,
-                       int mode, bool wide, cudaStream_t stream) {
-    NXD_REQUIRE(!wide || mode == kSegPlain, "experts: %s", "fp32 results of plain products only");
+                       int mode, cudaStream_t stream) {
+    const bool wide = mode == kSegPlain;
     NXD_REQUIRE(E > 0 && E <= kSegMaxExperts, "experts: %d experts", E);
     NXD_REQUIRE(rows > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "experts: %d rows, %d x %d", rows, N, K);
     NXD_REQUIRE(((uintptr_t)a & 15) == 0 && ((uintptr_t)b & 15) == 0 && ((uintptr_t)d & 15) == 0,
@@ -472,9 +472,6 @@ static int run_experts(const void* a, const void* b, void* d, const SegArgs& seg
     if (rc) return rc;
     rc = make_tmap_2d(&td, d, (uint64_t)N, (uint64_t)rows, (uint64_t)N, wide ? 32 : 64, 32, wide ? 4 : 2);
     if (rc) return rc;
-    if (wide)
-        return bn == 256 ? launch_experts<256, kSegPlain, kOutF32>(ta, tb, td, E, rows, N, K, seg, stream)
-                         : launch_experts<128, kSegPlain, kOutF32>(ta, tb, td, E, rows, N, K, seg, stream);
 #define NXD_EXPERTS(MODE_)                                                                              \
     return bn == 256 ? launch_experts<256, MODE_>(ta, tb, td, E, rows, N, K, seg, stream)                \
                      : launch_experts<128, MODE_>(ta, tb, td, E, rows, N, K, seg, stream)
@@ -491,13 +488,13 @@ static int run_experts(const void* a, const void* b, void* d, const SegArgs& seg
 
 // Products of the sparse experts over rows sorted by expert (run_experts above): counts [E] int32 on the device, mode 1 plain,
 // 2 gate | up through the clamped gated activation, 3 max(., 0)^2.  `rows`: rows of a and d; `pairs`: real rows expected (picks
-// the tile width only).  row_scale [rows] fp32 or NULL: mode 2, factor of a row's products ahead of the activation.  wide: d is
-// fp32 (mode 1), else bf16.
+// the tile width only).  row_scale [rows] fp32 or NULL: mode 2, factor of a row's products ahead of the activation.  d is fp32 in
+// mode 1, else bf16.
 NXD_API int nxd_experts_gemm_bf16(const void* a, const void* b, void* d, const int* counts, const float* row_scale, int E,
-                                  int rows, int pairs, int N, int K, int mode, int wide, float limit, float alpha,
-                                  float up_shift, void* stream) {
+                                  int rows, int pairs, int N, int K, int mode, float limit, float alpha, float up_shift,
+                                  void* stream) {
     nxd_gemm::SegArgs seg{counts, limit, alpha, up_shift, row_scale};
-    return nxd_gemm::run_experts(a, b, d, seg, E, rows, pairs, N, K, mode, wide != 0, (cudaStream_t)stream);
+    return nxd_gemm::run_experts(a, b, d, seg, E, rows, pairs, N, K, mode, (cudaStream_t)stream);
 }
 
 namespace nxd_gemm {

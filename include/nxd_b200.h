@@ -480,7 +480,7 @@ int nxd_moe_gather_combine(int dtype, const void* ys, const int* slot, const int
 int nxd_moe_sort_rows(const void* h, const int* idx, int* counts, int* slot, const float* in_scale, float* row_scale, void* x,
                       long long P, int top, int W, int E, void* stream);
 int nxd_experts_gemm_bf16(const void* a, const void* b, void* d, const int* counts, const float* row_scale, int E, int rows,
-                          int pairs, int N, int K, int mode, int wide, float limit, float alpha, float up_shift, void* stream);
+                          int pairs, int N, int K, int mode, float limit, float alpha, float up_shift, void* stream);
 /* the whole mixture after its router on sorted rows (csrc/moe_forward.cu) */
 long long nxd_moe_sorted_workspace(long long N, int top, int W, int F, int E, int Fs);
 int nxd_moe_sorted_forward(const void* h, const int* idx, const float* wts, const float* in_scale, const void* w_in,

@@ -79,3 +79,36 @@ def test_router_forms_match_float64(N, W, R, dtype):
     assert (p.gather(1, idx.long()) - top.values).abs().max() <= 1e-5
     assert (wts.double() - 1.5 * p.gather(1, idx.long())).abs().max() <= 1e-5
     assert (sg.double() - torch.sigmoid(h.double() @ gate.double()[0])).abs().max() <= 1e-5
+
+
+# below and above 16 pairs per expert (32 tokens), one and several row tiles; with and without a shared expert
+@pytest.mark.parametrize("N", [1, 31, 32, 200, 1000])
+@pytest.mark.parametrize("shared", [0, 72])
+def test_captured_step_repeats_and_is_as_exact_as_the_pairs(N, shared):
+    from neuronx_distributed_llama3_2_b200.modules.moe.sparse import SparseMoE
+
+    g = torch.Generator(device="cuda").manual_seed(N + shared)
+    m = SparseMoE(136, 4, 2, 200, 1.5, shared_intermediate_size=shared, dtype=torch.bfloat16, device="cuda").eval()
+    with torch.no_grad():
+        for p in m.parameters():
+            p.copy_(torch.randn(p.shape, generator=g, device="cuda") * p.shape[-2] ** -0.5 if p.dim() > 1 else torch.zeros_like(p))
+        h, first = (torch.randn(N, 136, generator=g, device="cuda").bfloat16() for _ in range(2))
+        assert m._use_device_sorted(h)
+        given = first.clone()
+        m(given)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = m(given)
+        for x in (first, h, first, h):                  # every replay reads its own input
+            given.copy_(x)
+            graph.replay()
+            assert torch.equal(out, m(x))
+        idx, wts, gate = m.router.select(h, m.shared_gate.weight if shared else None)
+        ref = _reference(h, idx, wts, m.experts.gate_up_proj.weight, m.experts.down_proj.weight, 1.5, 1.702, 1.0, False)
+        if shared:
+            ref += _reference(h, torch.zeros(N, 1, dtype=torch.int32, device="cuda"), gate.unsqueeze(1),
+                              m.shared.gate_up_proj.weight, m.shared.down_proj.weight, 1.5, 1.702, 1.0, False)
+        ours, pairs = ((y.double() - ref).norm() for y in (out, m(h, path="pairs")))
+    # both round the activation to bf16 and nothing else, at the same values but for those next to a rounding boundary (a second
+    # rounding, of the experts' outputs, would make it 1.4)
+    assert ours <= 1.1 * pairs
