@@ -226,7 +226,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                             r[half * 32 + j] = __float_as_uint(
                                 SEG == kSegGlu ? seg.glu(__uint_as_float(r[half * 32 + j]) * row_scale,
                                                          __uint_as_float(up[j]) * row_scale)
-                                               : seg.glu(__uint_as_float(r[half * 32 + j]), __uint_as_float(up[j])));
+                                               : SegArgs::swiglu(__uint_as_float(r[half * 32 + j]), __uint_as_float(up[j])));
                     }
                 } else {
                     ptx::tmem_ld_wait();
@@ -500,39 +500,38 @@ NXD_API int nxd_experts_gemm_bf16(const void* a, const void* b, void* d, const i
 namespace nxd_gemm {
 
 template <int BN>
-static int launch_glu(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, int M, int N, int K,
-                      const SegArgs& act, cudaStream_t stream) {
+static int launch_swiglu(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, int M, int N, int K,
+                         cudaStream_t stream) {
     using L = SmemLayout<BN>;
     constexpr auto kern = gemm_pair_kernel<BN, false, false, kOutBF16, false, kDenseGlu>;
     NXD_CHECK_CUDA(nxd_allow_smem<kern>(L::kSmemBytes));
     const long tiles = (long)((M + kTileM - 1) / kTileM) * ((N + BN / 2 - 1) / (BN / 2));
     long clusters = nxd_num_sms() / 2;
     if (clusters > tiles) clusters = tiles;
-    kern<<<dim3((unsigned)clusters * 2), dim3(kThreads), L::kSmemBytes, stream>>>(ta, tb, td, M, N, K, 1, act);
+    kern<<<dim3((unsigned)clusters * 2), dim3(kThreads), L::kSmemBytes, stream>>>(ta, tb, td, M, N, K, 1, SegArgs{});
     NXD_LAUNCH_CHECK();
     return 0;
 }
 
 }  // namespace nxd_gemm
 
-// D[M, N] = glu(A W_gate^T, A W_up^T): A [M, K], W [2 N, K] (gate rows first), the gated activation (SegArgs::glu; limit = inf,
-// alpha = 1, up_shift = 0: silu(gate) * up) on the fp32 products in the epilogue, as in run_experts.  2048 x 8192 x 2048: the
-// product alone 79 us and an activation kernel of 17 us that reads 67 MB and writes 34; together in one launch 84 us.  K, N and the pitches multiples of 8 elements, bases 16-byte aligned.
-NXD_API int nxd_gemm_glu_bf16(const void* a, const void* w, void* d, int M, int N, int K, long long lda, long long ldw,
-                              long long ldd, float limit, float alpha, float up_shift, void* stream) {
+// D[M, N] = silu(A W_gate^T) * (A W_up^T): A [M, K], W [2 N, K] (gate rows first), the activation on the fp32 products in the
+// epilogue, as in run_experts.  2048 x 8192 x 2048: the product alone 79 us and an activation kernel of 17 us that reads 67 MB and
+// writes 34; together in one launch 84 us.  K, N and the pitches multiples of 8 elements, bases 16-byte aligned.
+NXD_API int nxd_gemm_swiglu_bf16(const void* a, const void* w, void* d, int M, int N, int K, long long lda, long long ldw,
+                                 long long ldd, void* stream) {
     using namespace nxd_gemm;
-    NXD_REQUIRE(M > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "gemm_glu: %d x %d x %d", M, N, K);
-    NXD_REQUIRE(lda % 8 == 0 && ldw % 8 == 0 && ldd % 8 == 0, "gemm_glu: pitches must be multiples of 8 elements (%lld)", lda);
-    NXD_REQUIRE((((uintptr_t)a | (uintptr_t)w | (uintptr_t)d) & 15) == 0, "gemm_glu: operands must be %s", "16-byte aligned");
+    NXD_REQUIRE(M > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "gemm_swiglu: %d x %d x %d", M, N, K);
+    NXD_REQUIRE(lda % 8 == 0 && ldw % 8 == 0 && ldd % 8 == 0, "gemm_swiglu: pitches must be multiples of 8 elements (%lld)", lda);
+    NXD_REQUIRE((((uintptr_t)a | (uintptr_t)w | (uintptr_t)d) & 15) == 0, "gemm_swiglu: operands must be %s", "16-byte aligned");
     const int bn = pick_block_n(M, 2 * N);
     CUtensorMap ta, tb, td;
     int rc;
     if ((rc = make_tmap_2d(&ta, a, (uint64_t)K, (uint64_t)M, (uint64_t)lda, 64, kBlockM))) return rc;
     if ((rc = make_tmap_2d(&tb, w, (uint64_t)K, (uint64_t)2 * N, (uint64_t)ldw, 64, bn / 2))) return rc;
     if ((rc = make_tmap_2d(&td, d, (uint64_t)N, (uint64_t)M, (uint64_t)ldd, 64, 32, 2))) return rc;
-    const SegArgs act{nullptr, limit, alpha, up_shift, nullptr};
-    return bn == 256 ? launch_glu<256>(ta, tb, td, M, N, K, act, (cudaStream_t)stream)
-                     : launch_glu<128>(ta, tb, td, M, N, K, act, (cudaStream_t)stream);
+    return bn == 256 ? launch_swiglu<256>(ta, tb, td, M, N, K, (cudaStream_t)stream)
+                     : launch_swiglu<128>(ta, tb, td, M, N, K, (cudaStream_t)stream);
 }
 
 // Grouped (batched over experts) GEMM: E problems of one shape in ONE launch.  a / b / d point at problem 0, stride_*

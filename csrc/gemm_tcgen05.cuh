@@ -66,6 +66,8 @@ struct SegArgs {
         u = fminf(fmaxf(u, -limit), limit);
         return g / (1.f + expf(-alpha * g)) * (u + up_shift);
     }
+    // of a dense problem: no clamps, which would turn NaN into a number (the experts' clamps do, as in moe_sparse.cu)
+    static __device__ __forceinline__ float swiglu(float g, float u) { return g / (1.f + expf(-g)) * u; }
 };
 
 // One warp: first row and (for num_n_tiles > 0) first tile of every expert; entry E holds the totals.

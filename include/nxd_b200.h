@@ -244,8 +244,8 @@ int nxd_p2p_push_probe(int mode, const void* src, const void* const* dst_ptrs, i
 /* ---- MoE: grouped expert GEMM and token permutation (reference: modules/moe/moe_parallel_layers.py:78,94,108 einsum
  *      over e; modules/moe/expert_mlps.py:183-265 gather by token_assignments / weighted scatter-combine) -------------
  * E problems of one shape in one launch; stride_* = elements between consecutive problems; M needs no alignment. */
-int nxd_gemm_glu_bf16(const void* a, const void* w, void* d, int M, int N, int K, long long lda, long long ldw, long long ldd,
-                      float limit, float alpha, float up_shift, void* stream);
+int nxd_gemm_swiglu_bf16(const void* a, const void* w, void* d, int M, int N, int K, long long lda, long long ldw, long long ldd,
+                         void* stream);
 int nxd_rope_cache_write(void* qkv, const float* cos_t, const float* sin_t, const int* positions, void* cache_k, void* cache_v,
                          const int* seq_ids, const int* block_table, long long stride_b, long long stride_h, int page_size,
                          int max_pages, int B, int Tn, int n_q, int n_kv, int D, void* stream);

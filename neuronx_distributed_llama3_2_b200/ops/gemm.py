@@ -60,11 +60,10 @@ def gemm_swiglu(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     n = w.shape[0] // 2
     assert w.shape[1] == k and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.stride(1) == 1 and w.stride(1) == 1
     out = torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
-    rc = _lib.lib().nxd_gemm_glu_bf16(
+    rc = _lib.lib().nxd_gemm_swiglu_bf16(
         _lib.ptr(x), _lib.ptr(w), _lib.ptr(out), _c.c_int(m), _c.c_int(n), _c.c_int(k), _c.c_longlong(x.stride(0)),
-        _c.c_longlong(w.stride(0)), _c.c_longlong(n), _c.c_float(float("inf")), _c.c_float(1.0), _c.c_float(0.0),
-        _lib.stream_ptr())
-    _lib.check(rc, "nxd_gemm_glu_bf16")
+        _c.c_longlong(w.stride(0)), _c.c_longlong(n), _lib.stream_ptr())
+    _lib.check(rc, "nxd_gemm_swiglu_bf16")
     return out
 
 

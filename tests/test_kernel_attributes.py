@@ -78,7 +78,6 @@ def library(tmp_path_factory):
 
 
 P, L, F = (lambda n=1: c.c_void_p(n << 20)), c.c_longlong, c.c_float           # pointers are passed on, never followed
-INF = F(float("inf"))
 
 
 def _strides(n):
@@ -89,7 +88,7 @@ CALLS = {
     "rmsnorm_bwd": lambda lib: lib.nxd_rmsnorm_bwd(P(1), P(2), P(3), P(4), None, P(5), P(6), None, 0, P(7), 64, 8192, None),
     "rmsnorm_bwd_static": lambda lib: lib.nxd_rmsnorm_bwd_static(P(1), P(2), P(3), P(4), None, P(5), P(6), None, 0, 64, 4096, None),
     "gemm": lambda lib: lib.nxd_gemm_bf16(0, P(1), P(2), P(3), 256, 256, 256, L(256), L(256), L(256), 0, 0, None),
-    "gemm_glu": lambda lib: lib.nxd_gemm_glu_bf16(P(1), P(2), P(3), 256, 256, 256, L(256), L(256), L(256), INF, F(1), F(0), None),
+    "gemm_swiglu": lambda lib: lib.nxd_gemm_swiglu_bf16(P(1), P(2), P(3), 256, 256, 256, L(256), L(256), L(256), None),
     "experts": lambda lib: lib.nxd_moe_sorted_forward(P(1), P(2), P(3), None, P(4), P(5), None, None, None, P(6), P(7), L(64), 2, 256,
                                                       256, 4, 0, 1, F(1), F(1), F(1), F(0), None),
     "smallm": lambda lib: lib.nxd_gemm_smallm_bf16(P(1), P(2), None, P(3), 4, 2048, 2048, L(2048), L(2048), L(2048), L(0), 0, None),

@@ -19,6 +19,20 @@ def test_gate_up_product_with_activation_matches_float64(M, K, I):
     assert (gemm_swiglu(x, w).double() - ref).norm() <= 2.0 ** -8 * ref.norm()
 
 
+def test_gate_up_product_passes_values_that_are_no_numbers():
+    from neuronx_distributed_llama3_2_b200.ops import activation
+    from neuronx_distributed_llama3_2_b200.ops.gemm import gemm, gemm_swiglu
+
+    g = torch.Generator(device="cuda").manual_seed(0)
+    x, w = (torch.randn(n, 64, generator=g, device="cuda").bfloat16() for n in (300, 144))
+    x[5, 3] = w[7, 0] = w[72 + 9, 1] = float("nan")                   # a row, a gate column, an up column
+    w[11, 2] = w[72 + 13, 2] = float("inf")                           # infinities of both signs
+    out, ref = gemm_swiglu(x, w), activation.swiglu(gemm(x, w, "nt"))
+    assert ref[:, 7].isnan().all() and ref[:, 9].isnan().all() and ref.isinf().any()
+    for same in (torch.isnan, torch.isposinf, torch.isneginf):
+        assert torch.equal(same(out), same(ref))
+
+
 @pytest.mark.parametrize("D,nq,nkv", [(16, 3, 1), (64, 8, 2), (128, 2, 2)])
 @pytest.mark.parametrize("paged", [False, True])
 def test_rotation_and_cache_write_match_the_separate_kernels(D, nq, nkv, paged):
