@@ -329,7 +329,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                     }
                 };
                 if (p.bias_entries > 0) {
-                    const float* tb = dtab + d0;
+                    const float* tb = dtab + score::table_entry(d0, p.bias_entries);
                     if (MASK)
                         cap_and_bias([&](int c) { return f2_pack(dtab[min(max(d0 - c, 0), p.bias_entries - 1)],
                                                                  dtab[min(max(d0 - c - 1, 0), p.bias_entries - 1)]); });

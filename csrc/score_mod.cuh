@@ -65,6 +65,11 @@ __device__ __forceinline__ float tanh_fp32(float x) {
 __device__ __forceinline__ float sigmoid_log2(float x2) { return __fdividef(1.f, 1.f + exp2f(fminf(-x2, 100.f))); }
 __device__ __forceinline__ float sigmoid(float x) { return sigmoid_log2(x * kLog2e); }
 
+// Entry of a table of distances [0, entries) that a row reads first in a tile of 64 keys without a mask, and whose 63 predecessors
+// it reads next; d0: its distance from the tile's first key.  Rows of padding behind the sequence's end lie further off than the
+// table reaches and take its last entries (their results are dropped).
+__host__ __device__ inline int table_entry(int d0, int entries) { return d0 < entries ? d0 : entries - 1; }
+
 __device__ __forceinline__ float ldg(const float* p) { return *p; }
 __device__ __forceinline__ float ldg(const bf16* p) { return __bfloat162float(*p); }
 template <typename T>
