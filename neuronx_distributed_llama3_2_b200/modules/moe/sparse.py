@@ -87,10 +87,11 @@ class SparseMoE(torch.nn.Module):
                 for w in ((ex.gate_up_proj if self.gated else ex.up_proj).weight, ex.down_proj.weight)]
 
     def forward(self, h: torch.Tensor, path: Optional[str] = None) -> torch.Tensor:
-        """``h [N, W]`` (activation dtype) -> combined output ``[N, W]`` in fp32."""
+        """``h [N, W]`` (activation dtype) -> combined output ``[N, W]`` in fp32.  ``path``: ``"pairs"`` | ``"sorted"`` (counts read on
+        the host) | ``"device"`` (device-sorted), default: chosen by the sizes."""
         gated = self.shared is not None and self.shared_gate is not None
         idx, wts, sg = self.router.select(h, self.shared_gate.weight if gated else None)
-        if path != "pairs" and h.shape[0] and self._use_device_sorted(h):
+        if path == "device" or (path is None and h.shape[0] and self._use_device_sorted(h)):
             return self._forward_device_sorted(h, idx, wts, sg)
         sorted_path = self._use_sorted(h.shape[0]) if path is None else path == "sorted"
         if sorted_path:

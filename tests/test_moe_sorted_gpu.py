@@ -112,3 +112,23 @@ def test_captured_step_repeats_and_is_as_exact_as_the_pairs(N, shared):
     # both round the activation to bf16 and nothing else, at the same values but for those next to a rounding boundary (a second
     # rounding, of the experts' outputs, would make it 1.4)
     assert ours <= 1.1 * pairs
+
+
+def test_each_path_is_the_one_that_was_asked_for(monkeypatch):
+    from neuronx_distributed_llama3_2_b200.modules.moe.sparse import SparseMoE
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    m = SparseMoE(128, 4, 2, 64, 1.5, dtype=torch.bfloat16, device="cuda").eval()
+    taken = []
+    for name in ("_forward_sorted", "_forward_device_sorted"):
+        monkeypatch.setattr(m, name, lambda *a, name=name, call=getattr(m, name): (taken.append(name), call(*a))[1])
+    with torch.no_grad():
+        for p in m.parameters():
+            p.copy_(torch.randn(p.shape, generator=g, device="cuda") * 0.1)
+        h = torch.randn(90, 128, generator=g, device="cuda").bfloat16()
+        by_path = {path: m(h, path=path) for path in ("pairs", "sorted", "device", None)}
+    assert taken == ["_forward_sorted", "_forward_device_sorted", "_forward_device_sorted"]
+    assert torch.equal(by_path["device"], by_path[None])
+    # the host-counted path rounds the experts' outputs to bf16, all round the activation: 2^-8 of a value each
+    for y in by_path.values():
+        assert (y - by_path["pairs"]).norm() <= 3 * 2.0 ** -8 * by_path["pairs"].norm()
