@@ -473,18 +473,20 @@ int launch_scan(const float* qn, const float* kn, const float* vn, const float* 
 //   A[t][s] = beta_t L[t][s] (k_t . k_s), s < t;    (I + A) U = diag(beta) (V - diag(Gamma) K S)
 //   O = diag(Gamma) Q S + P U,  P[t][s] = L[t][s] (q_t . k_s), s <= t;    S <- Gamma_CH S + (diag(L[CH-1][.]) K)^T U
 //
+// With M = (I + A)^-1 diag(beta) and R = V - diag(Gamma) K S:  U = M R,  P U = (P M) R.
 // (the WY form of Householder products; Yang, Wang, Zhang, Shen, Kim, "Parallelizing Linear Transformers with the Delta Rule
 // over Sequence Length").  Decay ratios are products, never quotients or exponentials of sums, so a decay of any size is
-// exact to rounding and underflows to the right limit.  Two kernels, all fp32:
-//   delta_chunk_system  per (chunk, head, row), in parallel: (I + A)^-1 diag(beta), P, Gamma and L[CH-1][.] to scratch
-//   delta_chunk_scan    per (32 value columns, head, row), sequential over chunks with the state slice in shared memory:
+// exact to rounding and underflows to the right limit.  Two kernels:
+//   delta_chunk_system  per (chunk, head, row), in parallel, fp64: M, P M, Gamma and L[CH-1][.] to scratch
+//   delta_chunk_scan    fp32, per (32 value columns, head, row), sequential over chunks with the state slice in shared memory:
 //                       four products per chunk, register-tiled, on packed pairs of fp32 multiply-adds (pairs run along the
 //                       contraction, so both operands are read as 16-byte pieces and nothing is shuffled)
 // Bound by the fp32 pipes of the second kernel: a token costs 3 D + CH multiply-adds per value column, like token by token, but
 // 64 tokens are independent, where delta_scan waits for two dot products and a shuffle tree per token.  Its own limit is the
-// chain of a chunk's phases: 4 x 2048 tokens, 4 heads of 128 x 256 take 69 + 344 us against 779 us token by token, of which the two
-// wide products cost 99 and 70 us, the triangular ones 78 and barriers, loads and stores the rest (360 us with a chunk's factors
-// loaded at its start instead of one chunk ahead); neither 8 x 8 tiles with half of the shared-memory loads nor 16 warps change it.
+// chain of a chunk's phases: 4 x 2048 tokens, 4 heads of 128 x 256 take 53 us (69 us with fp32 products in the first kernel) + 345 us
+// against 779 us token by token; of the 345 us the two wide products cost 99 and 70, the triangular ones 78 and barriers, loads
+// and stores the rest (360 us with a chunk's factors loaded at its start instead of one chunk ahead); neither 8 x 8 tiles with half
+// of the shared-memory loads nor 16 warps change it.
 constexpr int CH = 64, CP = CH + 4, CW_THREADS = 256, CW_COLS = 32;
 
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
@@ -518,34 +520,59 @@ __device__ __forceinline__ void add_pairs(uint64_t (&acc)[R][C], const uint64_t 
         for (int j = 0; j < C; ++j) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc[i][j]) : "l"(part[i][j]));
 }
 
-// scratch per (row, head, chunk): M [CH][CH] = (I + A)^-1 diag(beta), P [CH][CH], Gamma [CH], L[CH-1][.] [CH]
-constexpr int CHUNK_FLOATS = 2 * CH * CH + 2 * CH;
+// scratch per (row, head, chunk): M [CH][CH] = (I + A)^-1 diag(beta), P M [CH][CH], Gamma [CH], L[CH-1][.] [CH]
+constexpr int CHUNK_FLOATS = 2 * CH * CH + 2 * CH, DPITCH = CH + 4;
 
+// c [8 x 8] += a [8 x 4] b [4 x 8]: a is row lane / 4, column lane % 4; b row lane % 4, column lane / 4; c row lane / 4, columns
+// 2 (lane % 4) and the next
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(c[0]), "+d"(c[1])
+        : "d"(a), "d"(b));
+}
+
+// All in fp64, rounded once at the end.  With neighbouring keys that are nearly parallel and decays near one, P sums errors u that
+// cancel: fp32 dot products, an fp32 inverse and P U as two products put 7e-7 into the output where token by token is off by 1.1e-7.
+// The entries of P M are small again where that happens, and the output is 1.0e-7 off.  (The state sums rounded u as well and
+// can be 1.7 times as far off as token by token: 3.4e-7 against 2.0e-7.)
 template <int D>
 __global__ void __launch_bounds__(CW_THREADS, 2)
 delta_chunk_system_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ gate,
                           long long ld_a, int a_off, const float* __restrict__ beta, long long ld_b, int b_off,
                           float* __restrict__ scratch, const int* __restrict__ n_new, int Tn, int H, int G) {
     extern __shared__ __align__(16) float smem[];
-    float* Ks = smem;                    // [CH][CP] 64 key channels at a time
-    float* Qs = Ks + CH * CP;            // [CH][CP]
-    float* As = Qs + CH * CP;            // [CH][CP] A
-    float* Ls = As + CH * CP;            // [CH][CP] L
-    float* Ts = Ks;                      // [CH][CP] columns of (I + A)^-1, once the products are done
+    double* Kd = reinterpret_cast<double*>(smem);      // [CH][DPITCH] 64 key channels at a time; then X = (I + A)^-1
+    double* Qd = Kd + CH * DPITCH;                     // [CH][DPITCH] the same of the queries; then P
+    double* Ad = Qd + CH * DPITCH;                     // [CH][DPITCH] L; then A
     __shared__ float gs[CH], bs[CH];
     const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, kvh = h / (H / G), tid = threadIdx.x;
-    const int lane = tid & 31, warp = tid >> 5;
+    const int lane = tid & 31, warp = tid >> 5, lr = lane >> 2, lc = lane & 3;
     const int n = n_new != nullptr ? min(n_new[b], Tn) : Tn;
     const int nt = min(CH, n - c * CH);  // real tokens; the others change nothing (k = q = 0, beta = 0, g = 1)
     if (nt <= 0) return;                 // the scan does not look at this chunk
     const long long row0 = (long long)b * Tn + c * CH;
+    float* out = scratch + (((long long)b * H + h) * gridDim.x + c) * CHUNK_FLOATS;
     if (tid < CH) {
         gs[tid] = tid < nt ? gate[(row0 + tid) * ld_a + a_off + h] : 1.f;
         bs[tid] = tid < nt ? beta[(row0 + tid) * ld_b + b_off + h] : 0.f;
     }
-    // rows of a thread: r and CH/2 + r of K and of Q; columns cg + 8 j, of which the upper half of the rows needs j < 4
-    const int r = warp * 4 + (lane >> 3), cg = lane & 7;
-    float lower[4][4] = {}, right[2][4] = {};                    // all four rows, j < 4; rows CH/2 + r, j >= 4
+    __syncthreads();
+    if (tid <= CH) {                     // column s = tid of L: running products of the decays behind s; the last thread: Gamma
+        const int s = tid < CH ? tid : -1;
+        double l = 1.;
+        for (int t = s + 1; t < CH; ++t) {
+            l *= gs[t];
+            if (s < 0) out[2 * CH * CH + t] = (float)l;
+            else Ad[t * DPITCH + s] = l;
+        }
+        if (s >= 0) {
+            Ad[s * DPITCH + s] = 1.;
+            out[2 * CH * CH + CH + s] = (float)l;
+        }
+    }
+    // eight rows of K and of Q per warp against the keys up to them (the sub-partitions' two warps: 2 x 9 tiles each)
+    const int rt = warp < 4 ? warp : 11 - warp;
+    double kk[8][2] = {}, qk[8][2] = {};
     for (int d0 = 0; d0 < D; d0 += 64) {
         __syncthreads();
         for (int i = tid; i < CH * 16; i += CW_THREADS) {
@@ -553,80 +580,82 @@ delta_chunk_system_kernel(const float* __restrict__ qn, const float* __restrict_
             const long long src = ((row0 + t) * G + kvh) * D + d0 + d;
             float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), qv = kv;
             if (t < nt) kv = *reinterpret_cast<const float4*>(kn + src), qv = *reinterpret_cast<const float4*>(qn + src);
-            *reinterpret_cast<float4*>(Ks + t * CP + d) = kv;
-            *reinterpret_cast<float4*>(Qs + t * CP + d) = qv;
+            double2* kd = reinterpret_cast<double2*>(Kd + t * DPITCH + d);
+            double2* qd = reinterpret_cast<double2*>(Qd + t * DPITCH + d);
+            kd[0] = make_double2(kv.x, kv.y), kd[1] = make_double2(kv.z, kv.w);
+            qd[0] = make_double2(qv.x, qv.y), qd[1] = make_double2(qv.z, qv.w);
         }
         __syncthreads();
 #pragma unroll 1
-        for (int d1 = 0; d1 < 64; d1 += 16) {                    // sums of 16, as in the scan
-            uint64_t p[4][4] = {}, q[2][4] = {};
+        for (int d = 0; d < 64; d += 4) {
+            const double ka = Kd[(rt * 8 + lr) * DPITCH + d + lc], qa = Qd[(rt * 8 + lr) * DPITCH + d + lc];
 #pragma unroll
-            for (int d = d1; d < d1 + 16; d += 4) {
-                const ulonglong2 a[4] = {ld_pairs(Ks + r * CP + d), ld_pairs(Qs + r * CP + d), ld_pairs(Ks + (r + CH / 2) * CP + d),
-                                         ld_pairs(Qs + (r + CH / 2) * CP + d)};
-                ulonglong2 kb[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) kb[j] = ld_pairs(Ks + (cg + 8 * j) * CP + d);
-                dot_step(p, a, kb);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) kb[j] = ld_pairs(Ks + (cg + 8 * j + 32) * CP + d);
-                const ulonglong2 a2[2] = {a[2], a[3]};
-                dot_step(q, a2, kb);
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) lower[i][j] += lo2(p[i][j]) + hi2(p[i][j]);
-#pragma unroll
-                for (int i = 0; i < 2; ++i) right[i][j] += lo2(q[i][j]) + hi2(q[i][j]);
+            for (int j = 0; j < 8; ++j) {
+                if (j > rt) break;
+                const double kb = Kd[(j * 8 + lr) * DPITCH + d + lc];
+                mma_f64(kk[j], ka, kb);
+                mma_f64(qk[j], qa, kb);
             }
         }
     }
-    if (tid < CH) {                      // column s of L: running products of the decays behind s
-        float l = 1.f;
-        for (int t = 0; t < CH; ++t) {
-            if (t > tid) l *= gs[t];
-            Ls[t * CP + tid] = t >= tid ? l : 0.f;
-        }
-    }
-    __syncthreads();
-    float* out = scratch + (((long long)b * H + h) * gridDim.x + c) * CHUNK_FLOATS;
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        const int t = r + half * (CH / 2);
+    __syncthreads();                     // keys and queries have been read: their places take X and P
+    {
+        const int t = rt * 8 + lr;
+        const double bt = bs[t];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const int s = cg + 8 * j;
-            const float l = Ls[t * CP + s], kk = j < 4 ? lower[2 * half][j & 3] : right[0][j & 3];
-            const float qk = j < 4 ? lower[2 * half + 1][j & 3] : right[1][j & 3];
-            As[t * CP + s] = s < t ? bs[t] * l * kk : 0.f;
-            out[CH * CH + t * CH + s] = s <= t ? l * qk : 0.f;
+            if (j > rt) break;
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {              // entries above the diagonal are never read
+                const int at = t * DPITCH + j * 8 + 2 * lc + x;
+                const double l = Ad[at];
+                Qd[at] = l * qk[j][x];
+                Ad[at] = bt * l * kk[j][x];
+            }
         }
     }
-    if (tid < CH) {
-        out[2 * CH * CH + tid] = Ls[tid * CP] * gs[0];
-        out[2 * CH * CH + CH + tid] = Ls[(CH - 1) * CP + tid];
-    }
     __syncthreads();
-    // columns of X = (I + A)^-1 by forward substitution, four lanes a column; Ts[col][t]
-    const int col = tid >> 2, part = tid & 3;
-    float* x = Ts + col * CP;
-    for (int t = part; t < CH; t += 4) x[t] = t == col ? 1.f : 0.f;
-    __syncwarp();
-    for (int t = 1; t < CH; ++t) {       // the lanes of a warp hold 8 neighbouring columns: rows above them stay zero
-        if (t <= (col & ~7)) continue;
-        float d = 0.f;
-#pragma unroll 4
-        for (int s = (col & ~7) + part; s < t; s += 4) d = fmaf(As[t * CP + s], x[s], d);
-        d += __shfl_xor_sync(0xffffffffu, d, 1);
-        d += __shfl_xor_sync(0xffffffffu, d, 2);
-        if (part == 0 && t > col) x[t] = -d;
+    // Eight columns of X and of P M per warp, eight rows at a time: matrix instructions for the blocks left of the diagonal one,
+    // single steps inside it that leave out what lies above the diagonal instead of multiplying it by zero (a token that is not a
+    // number does not reach the tokens before it).
+    const int c0 = warp * 8 + 2 * lc;
+    const double b0 = bs[c0], b1 = bs[c0 + 1];
+    auto put = [&](float* dst, int i, double v0, double v1) {
+        const int t = i * 8 + lr;
+        *reinterpret_cast<float2*>(dst + t * CH + c0) = make_float2(c0 <= t ? (float)(v0 * b0) : 0.f, c0 < t ? (float)(v1 * b1) : 0.f);
+    };
+    for (int i = 0; i < warp; ++i) {
+        put(out, i, 0., 0.);
+        put(out + CH * CH, i, 0., 0.);
+    }
+    for (int i = warp; i < 8; ++i) {
+        double v[2] = {}, y[2] = {};
+        for (int s = warp * 8; s < i * 8; s += 4) {
+            const double xb = Kd[(s + lc) * DPITCH + warp * 8 + lr];
+            mma_f64(v, Ad[(i * 8 + lr) * DPITCH + s + lc], xb);
+            mma_f64(y, Qd[(i * 8 + lr) * DPITCH + s + lc], xb);
+        }
+        v[0] = (i == warp && lr == 2 * lc ? 1. : 0.) - v[0];
+        v[1] = (i == warp && lr == 2 * lc + 1 ? 1. : 0.) - v[1];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const double x0 = __shfl_sync(0xffffffffu, v[0], r * 4 + lc), x1 = __shfl_sync(0xffffffffu, v[1], r * 4 + lc);
+            const int at = (i * 8 + lr) * DPITCH + i * 8 + r;
+            if (lr > r) {
+                const double a = Ad[at];
+                v[0] -= a * x0;
+                v[1] -= a * x1;
+            }
+            if (lr >= r) {
+                const double p = Qd[at];
+                y[0] += p * x0;
+                y[1] += p * x1;
+            }
+        }
+        *reinterpret_cast<double2*>(Kd + (i * 8 + lr) * DPITCH + c0) = make_double2(v[0], v[1]);
         __syncwarp();
-    }
-    __syncthreads();
-    for (int i = tid; i < CH * CH; i += CW_THREADS) {
-        const int t = i / CH, s = i % CH;
-        out[i] = s <= t ? Ts[s * CP + t] * bs[s] : 0.f;
+        put(out, i, v[0], v[1]);
+        put(out + CH * CH, i, y[0], y[1]);
     }
 }
 
@@ -644,7 +673,7 @@ delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ 
     float* Qs = Kb + KB * CH * DP;             // [CH][DP]
     float* Ss = Qs + CH * DP;                  // [32][DP] the state slice, a value column per row
     float* Ms = Ss + CW_COLS * DP;             // [CH][CP]
-    float* Ps = Ms + CH * CP;                  // [CH][CP]
+    float* Ps = Ms + CH * CP;                  // [CH][CP] P M
     float* Rs = Ps + CH * CP;                  // [32][CP] V - diag(Gamma) K S, a value column per row
     float* Us = Rs + CW_COLS * CP;             // [32][CP] U
     float* gam2 = Us + CW_COLS * CP;           // [2][2 CH] Gamma and L[CH-1][.] of this chunk and the next
@@ -792,7 +821,7 @@ delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ 
         mma::cp_async_commit();
 #pragma unroll
         for (int i = 0; i < 4; ++i) y[0][i] = y[1][i] = 0ull;
-        triangular(Ps, Us, y);
+        triangular(Ps, Rs, y);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             if (t0 + ra < n) orow[(long long)(t0 + ra) * H * Dv + cg + 8 * i] = o[0][i] + (lo2(y[0][i]) + hi2(y[0][i]));
@@ -856,7 +885,7 @@ int launch_chunks(const float* qn, const float* kn, const float* vn, const float
                   const int* n_new, const int* seq_ids, int B, int Tn, int H, int G, int Dv, cudaStream_t st) {
     constexpr int DP = D + 4;
     const int NC = (Tn + CH - 1) / CH;
-    const size_t sys = (size_t)4 * CH * CP * sizeof(float);
+    const size_t sys = (size_t)3 * CH * DPITCH * sizeof(double);
     const size_t scan = (size_t)((D <= 128 ? 3 : 2) * CH * DP + CW_COLS * DP + 2 * CH * CP + 2 * CW_COLS * CP + 4 * CH) * sizeof(float);
     static_assert((2 * CH * 260 + CW_COLS * 260 + 2 * CH * CP + 2 * CW_COLS * CP + 4 * CH) * 4 <= 232448, "shared memory");
     NXD_CHECK_CUDA(cudaFuncSetAttribute(delta_chunk_system_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sys));

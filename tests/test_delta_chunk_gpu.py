@@ -63,6 +63,41 @@ def test_chunks_match_float64(D, H, G, Dv, T, n_new, strength):
             assert (S[line[b]] - states[b]).norm() <= bound * states[b].norm()
 
 
+# keys from independent to nearly parallel, decays and learning rates from ordinary to next to one: where neighbouring tokens
+# overwrite one another, errors inside a chunk must not add up
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("common,strength,rate", [(0.0, 0.0, 0.0), (0.6, -6.0, 4.0), (0.9, -4.0, 4.0), (0.97, -7.0, 6.0)])
+def test_chunks_are_no_further_off_than_single_tokens(D, common, strength, rate):
+    from neuronx_distributed_llama3_2_b200.ops import delta_rule as dr
+
+    T, H, Dv, portion = 1024, 2, 64, 128                 # portions of 128 tokens run token by token
+    gen = torch.Generator(device="cuda").manual_seed(D)
+
+    def normal(*s):
+        return torch.randn(*s, generator=gen, device="cuda")
+
+    k, q = (F.normalize((1 - common) * normal(1, T, H, D) + common * x, dim=-1) for x in (normal(1, 1, H, D),) for _ in range(2))
+    q, v = q * D ** -0.5, normal(1, T, H, Dv)
+    a_pre, b_pre, start = normal(T, H), normal(T, H) + rate, normal(1, H, D, Dv)
+    a_log, dt_bias = normal(H) * 0.1 + strength, normal(H)
+    g = torch.exp(-torch.exp(a_log.double()) * F.softplus(a_pre.double() + dt_bias.double()))
+    want, state = _oracle(q[0].double(), k[0].double(), v[0].double(), g, torch.sigmoid(b_pre.double()), start[0].double())
+
+    def run(size):
+        S, outs = start.clone(), []
+        for t in range(0, T, size):
+            at = torch.full((1,), t + 1, dtype=torch.int32, device="cuda")          # not at a sequence's start: S is read
+            x, y, z = (r[:, t:t + size].contiguous() for r in (q, k, v))
+            outs.append(dr.delta_scan(x, y, z, a_pre[t:t + size].clone(), 0, b_pre[t:t + size].clone(), 0, a_log, dt_bias, S, at, False))
+        return (torch.cat(outs, 1)[0] - want).norm() / want.norm(), (S[0] - state).norm() / state.norm()
+
+    # both forms are fp32: a quarter for the scatter of sums of roundings.  The state also takes the sum of a chunk's 64 errors u times
+    # their keys: where it cancels, their roundings (2^-25 on average) do not, 8 x 2^-25 of a state that is about one u
+    (out, S), (out_tokens, S_tokens) = run(T), run(portion)
+    assert out <= 1.25 * out_tokens + 2.0 ** -24
+    assert S <= 1.25 * S_tokens + 2.0 ** -22
+
+
 def test_a_token_that_is_not_a_number_leaves_the_tokens_before_it_alone():
     from neuronx_distributed_llama3_2_b200.ops import delta_rule as dr
 
@@ -82,6 +117,8 @@ def test_a_token_that_is_not_a_number_leaves_the_tokens_before_it_alone():
     for bad in (float("nan"), float("inf")):
         out = run(bad)
         assert torch.equal(out[:70], clean[:70]) and not torch.isfinite(out[70:, 3]).any()
+    k[0, 69, 0, 5] = float("nan")                        # its row of the chunk's system
+    assert torch.equal(run(0.5)[:69], clean[:69])
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
