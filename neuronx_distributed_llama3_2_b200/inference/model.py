@@ -316,7 +316,9 @@ class KVCacheInferenceMixin:
         attn, mlp = layer.self_attn, layer.mlp
         mods = (layer.input_layernorm, layer.post_attention_layernorm, attn, attn.qkv_proj, attn.o_proj, mlp, mlp.gate_up_proj,
                 mlp.down_proj)
-        if any(m._forward_hooks or m._forward_pre_hooks for m in mods):
+        every = nn.modules.module
+        if (every._global_forward_hooks or every._global_forward_pre_hooks
+                or any(m._forward_hooks or m._forward_pre_hooks for m in mods)):
             return False
         norms = (layer.input_layernorm.weight, layer.post_attention_layernorm.weight)
         ws = (attn.qkv_proj.weight_qkv, attn.o_proj.weight, mlp.gate_up_proj.weight, mlp.down_proj.weight)

@@ -94,3 +94,29 @@ def test_prompt_layer_matches_the_general_path(D, B, T, paged, monkeypatch):
     # the general path rounds gate and up to bf16 ahead of the activation (2^-9 each); two layers of such differences
     for a, b in zip([got] + got_cache, [ref] + ref_cache):
         assert (a.float() - b.float()).norm() <= 2e-2 * b.float().norm()
+
+
+def test_hooks_on_every_module_see_the_prompt_layer(monkeypatch):
+    from neuronx_distributed_llama3_2_b200.inference.config import InferenceConfig
+    from neuronx_distributed_llama3_2_b200.inference.model import KVCacheInferenceMixin, LlamaInferenceModel
+    from neuronx_distributed_llama3_2_b200.models.llama import LlamaConfig
+
+    cfg = LlamaConfig(vocab_size=512, hidden_size=256, intermediate_size=512, num_hidden_layers=1, num_attention_heads=4,
+                      num_key_value_heads=2, head_dim=64, rope_scaling=None)
+    model = LlamaInferenceModel(cfg, InferenceConfig(batch_size=1, max_context_length=256, seq_len=256), device="cuda")
+    model.init_kv_cache(device="cuda")
+    ids, pos = torch.randint(0, 512, (1, 200), device="cuda"), torch.arange(200, device="cuda").unsqueeze(0)
+
+    def seen(register):
+        names, handle = [], register(lambda m, *a: names.append(type(m).__name__))
+        try:
+            model.forward_infer(ids, pos, sample=False)
+        finally:
+            handle.remove()
+        return names
+
+    every = torch.nn.modules.module
+    registers = (every.register_module_forward_hook, every.register_module_forward_pre_hook)
+    names = [seen(r) for r in registers]
+    monkeypatch.setattr(KVCacheInferenceMixin, "_prompt_layer_ok", lambda *a: False)
+    assert names == [seen(r) for r in registers] and "GQAQKVColumnParallelLinear" in names[0]
