@@ -489,18 +489,6 @@ int launch_scan(const float* qn, const float* kn, const float* vn, const float* 
 // of the shared-memory loads nor 16 warps change it.
 constexpr int CH = 64, CP = CH + 4, CW_THREADS = 256, CW_COLS = 32;
 
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ uint64_t pack2(float x, float y) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ float lo2(uint64_t v) { return __uint_as_float((uint32_t)v); }
-__device__ __forceinline__ float hi2(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
 __device__ __forceinline__ ulonglong2 ld_pairs(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
 
 // acc[i][j] += <a row i, b row j> over 4 values
@@ -509,7 +497,7 @@ __device__ __forceinline__ void dot_step(uint64_t (&acc)[R][C], const ulonglong2
 #pragma unroll
     for (int i = 0; i < R; ++i)
 #pragma unroll
-        for (int j = 0; j < C; ++j) acc[i][j] = fma2(a[i].y, b[j].y, fma2(a[i].x, b[j].x, acc[i][j]));
+        for (int j = 0; j < C; ++j) acc[i][j] = f2_fma(a[i].y, b[j].y, f2_fma(a[i].x, b[j].x, acc[i][j]));
 }
 
 template <int R, int C>
@@ -759,10 +747,10 @@ delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ 
         float o[2][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            Rs[(cg + 8 * i) * CP + ra] = fmaf(-ga, lo2(acc[0][i]) + hi2(acc[0][i]), v[0][i]);
-            Rs[(cg + 8 * i) * CP + rb] = fmaf(-gb, lo2(acc[1][i]) + hi2(acc[1][i]), v[1][i]);
-            o[0][i] = ga * (lo2(acc[2][i]) + hi2(acc[2][i]));
-            o[1][i] = gb * (lo2(acc[3][i]) + hi2(acc[3][i]));
+            Rs[(cg + 8 * i) * CP + ra] = fmaf(-ga, f2_lo(acc[0][i]) + f2_hi(acc[0][i]), v[0][i]);
+            Rs[(cg + 8 * i) * CP + rb] = fmaf(-gb, f2_lo(acc[1][i]) + f2_hi(acc[1][i]), v[1][i]);
+            o[0][i] = ga * (f2_lo(acc[2][i]) + f2_hi(acc[2][i]));
+            o[1][i] = gb * (f2_lo(acc[3][i]) + f2_hi(acc[3][i]));
         }
         __syncthreads();
         rows(qn, Qs, c + 1);                   // the queries of this chunk have been used
@@ -781,12 +769,12 @@ delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ 
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         xb[j] = ld_pairs(X + (cg + 8 * j) * CP + s);
-                        part[1][j] = fma2(a.y, xb[j].y, fma2(a.x, xb[j].x, part[1][j]));
+                        part[1][j] = f2_fma(a.y, xb[j].y, f2_fma(a.x, xb[j].x, part[1][j]));
                     }
                     if (s >= e) continue;
                     const ulonglong2 c = ld_pairs(M + ra * CP + s);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) part[0][j] = fma2(c.y, xb[j].y, fma2(c.x, xb[j].x, part[0][j]));
+                    for (int j = 0; j < 4; ++j) part[0][j] = f2_fma(c.y, xb[j].y, f2_fma(c.x, xb[j].x, part[0][j]));
                 }
                 add_pairs(y, part);
             }
@@ -803,7 +791,7 @@ delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ 
                     if (rg >= 1) d = fmaf(m.y, x.y, d);
                     if (rg >= 2) d = fmaf(m.z, x.z, d);
                     if (rg >= 3) d = fmaf(m.w, x.w, d);
-                    y[half][j] = pack2(lo2(y[half][j]) + d, hi2(y[half][j]));
+                    y[half][j] = f2_pack(f2_lo(y[half][j]) + d, f2_hi(y[half][j]));
                 }
             }
         };
@@ -811,8 +799,8 @@ delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ 
         triangular(Ms, Rs, y);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            Us[(cg + 8 * i) * CP + ra] = lo2(y[0][i]) + hi2(y[0][i]);
-            Us[(cg + 8 * i) * CP + rb] = lo2(y[1][i]) + hi2(y[1][i]);
+            Us[(cg + 8 * i) * CP + ra] = f2_lo(y[0][i]) + f2_hi(y[0][i]);
+            Us[(cg + 8 * i) * CP + rb] = f2_lo(y[1][i]) + f2_hi(y[1][i]);
         }
         mma::cp_async_wait<KB>();              // P of this chunk (the groups behind it: Q and, with two buffers, K)
         __syncthreads();
@@ -824,13 +812,13 @@ delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ 
         triangular(Ps, Rs, y);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            if (t0 + ra < n) orow[(long long)(t0 + ra) * H * Dv + cg + 8 * i] = o[0][i] + (lo2(y[0][i]) + hi2(y[0][i]));
-            if (t0 + rb < n) orow[(long long)(t0 + rb) * H * Dv + cg + 8 * i] = o[1][i] + (lo2(y[1][i]) + hi2(y[1][i]));
+            if (t0 + ra < n) orow[(long long)(t0 + ra) * H * Dv + cg + 8 * i] = o[0][i] + (f2_lo(y[0][i]) + f2_hi(y[0][i]));
+            if (t0 + rb < n) orow[(long long)(t0 + rb) * H * Dv + cg + 8 * i] = o[1][i] + (f2_lo(y[1][i]) + f2_hi(y[1][i]));
         }
         // S[.][j] <- Gamma S + sum_s last_s U[s][j] K[s][.]: DT key channels x 4 value columns per thread
         {
             const int d0 = ((warp & 3) * 8 + cg) * DT, j0 = (warp >> 2) * 16 + rg;       // columns j0 + 4 i
-            const uint64_t gl = pack2(gam[CH - 1], gam[CH - 1]);
+            const uint64_t gl = f2_pack(gam[CH - 1], gam[CH - 1]);
             uint64_t st[4][DT / 2] = {};       // the chunk's own part; the decayed state joins it once
 #pragma unroll 1
             for (int s0 = 0; s0 < CH; s0 += 16) {
@@ -851,9 +839,9 @@ delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ 
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const float w = u[i][q] * lw[q];
-                            const uint64_t ww = pack2(w, w);
+                            const uint64_t ww = f2_pack(w, w);
 #pragma unroll
-                            for (int x = 0; x < DT / 2; ++x) part[i][x] = fma2(kv[x], ww, part[i][x]);
+                            for (int x = 0; x < DT / 2; ++x) part[i][x] = f2_fma(kv[x], ww, part[i][x]);
                         }
                     }
                 }
@@ -864,7 +852,7 @@ delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ 
 #pragma unroll
                 for (int x = 0; x < DT / 2; ++x) {
                     uint64_t* at = reinterpret_cast<uint64_t*>(Ss + (j0 + 4 * i) * DP + d0 + 2 * x);
-                    *at = fma2(*at, gl, st[i][x]);
+                    *at = f2_fma(*at, gl, st[i][x]);
                 }
         }
         __syncthreads();                       // K, P, U and the old state are free

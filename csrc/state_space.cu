@@ -61,22 +61,7 @@ __device__ __forceinline__ float decay_exp(float y) {
 }
 constexpr float LOG2E = 1.4426950408889634f;
 // packed fp32 arithmetic on two neighbouring states
-__device__ __forceinline__ uint64_t pair2(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
 __device__ __forceinline__ void unpair2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
 
 // the decays of two states in the selective scan: fp32 serving rounds it as above, 16-bit serving takes the hardware's 2^x
 template <typename T>
@@ -85,8 +70,8 @@ struct ScanDecay {
     static __device__ __forceinline__ float at(float dt, float rate) { return exp2_ftz(dt * rate); }
     static __device__ __forceinline__ uint64_t at2(uint64_t dt, uint64_t rate) {
         float lo, hi;
-        unpair2(mul2(dt, rate), lo, hi);
-        return pair2(exp2_ftz(lo), exp2_ftz(hi));
+        unpair2(f2_mul(dt, rate), lo, hi);
+        return f2_pack(exp2_ftz(lo), exp2_ftz(hi));
     }
 };
 template <>
@@ -95,8 +80,8 @@ struct ScanDecay<float> {
     static __device__ __forceinline__ float at(float dt, float rate) { return decay_exp(dt * rate); }
     static __device__ __forceinline__ uint64_t at2(uint64_t dt, uint64_t rate) {
         float lo, hi;
-        unpair2(mul2(dt, rate), lo, hi);
-        return pair2(decay_exp(lo), decay_exp(hi));
+        unpair2(f2_mul(dt, rate), lo, hi);
+        return f2_pack(decay_exp(lo), decay_exp(hi));
     }
 };
 
@@ -429,8 +414,8 @@ selective_scan_kernel(const T* __restrict__ x, long long ld_x, const float* __re
                     sv[e] = (ok && !fresh) ? Sc[(long long)m * N + i] : 0.f;
                     av[e] = ok ? ScanDecay<T>::rate(-expf(a_log[(long long)(c0 + cl + m) * N + i])) : 0.f;
                 }
-                s[m][j] = pair2(sv[0], sv[1]);
-                a2[m][j] = pair2(av[0], av[1]);
+                s[m][j] = f2_pack(sv[0], sv[1]);
+                a2[m][j] = f2_pack(av[0], av[1]);
             }
         __syncthreads();
         for (int it = 0; it <= tiles + 1; ++it) {
@@ -445,7 +430,7 @@ selective_scan_kernel(const T* __restrict__ x, long long ld_x, const float* __re
 #pragma unroll
                         for (int m = 0; m < CPT; ++m) {
                             const float dvs = d.dt[g0 + q][cl + m], us = d.u[g0 + q][cl + m];
-                            dv[m] = pair2(dvs, dvs), u[m] = pair2(us, us), acc[m] = 0ull;
+                            dv[m] = f2_pack(dvs, dvs), u[m] = f2_pack(us, us), acc[m] = 0ull;
                         }
 #pragma unroll
                         for (int j = 0; j < NS; j += 4) {
@@ -455,10 +440,10 @@ selective_scan_kernel(const T* __restrict__ x, long long ld_x, const float* __re
                             for (int m = 0; m < CPT; ++m) {
                                 const uint64_t g01 = ScanDecay<T>::at2(dv[m], a2[m][j / 2]);
                                 const uint64_t g23 = ScanDecay<T>::at2(dv[m], a2[m][j / 2 + 1]);
-                                s[m][j / 2] = fma2(g01, s[m][j / 2], mul2(u[m], bv.x));
-                                s[m][j / 2 + 1] = fma2(g23, s[m][j / 2 + 1], mul2(u[m], bv.y));
-                                acc[m] = fma2(s[m][j / 2], cv.x, acc[m]);
-                                acc[m] = fma2(s[m][j / 2 + 1], cv.y, acc[m]);
+                                s[m][j / 2] = f2_fma(g01, s[m][j / 2], f2_mul(u[m], bv.x));
+                                s[m][j / 2 + 1] = f2_fma(g23, s[m][j / 2 + 1], f2_mul(u[m], bv.y));
+                                acc[m] = f2_fma(s[m][j / 2], cv.x, acc[m]);
+                                acc[m] = f2_fma(s[m][j / 2 + 1], cv.y, acc[m]);
                             }
                         }
 #pragma unroll
