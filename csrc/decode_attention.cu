@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(128) decode_attn_mma_kernel(
             const int key0 = start + (warp + i * C::kWarps) * C::kTile;
             const uint32_t sk = ring + (i % C::kStages) * 2 * C::kTileBytes, sv = sk + C::kTileBytes;
             constexpr int CH = D / 8;
-            // the tile's 32 keys are neighbours in memory (contiguous cache, or a page that holds whole tiles): one address
+            // the tile's kTile keys are neighbours in memory (contiguous cache, or a page that holds whole tiles): one address
             // per tile and a constant step per piece.  Looking every piece's row up (two integer divisions and a table read
             // for 16 bytes) took 2.5 times as long as the memory on a paged cache.
             const bool whole = whole_tiles;

@@ -483,8 +483,8 @@ int launch_scan(const float* qn, const float* kn, const float* vn, const float* 
 //                       contraction, so both operands are read as 16-byte pieces and nothing is shuffled)
 // Bound by the fp32 pipes of the second kernel: a token costs 3 D + CH multiply-adds per value column, like token by token, but
 // 64 tokens are independent, where delta_scan waits for two dot products and a shuffle tree per token.  Its own limit is the
-// chain of a chunk's phases: 4 x 2048 tokens, 4 heads of 128 x 256 take 53 us (69 us with fp32 products in the first kernel) + 345 us
-// against 779 us token by token; of the 345 us the two wide products cost 99 and 70, the triangular ones 78 and barriers, loads
+// chain of a chunk's phases: 4 x 2048 tokens, 4 heads of 128 x 256 take 53 us (67 us with fp32 products in the first kernel) + 346
+// us against 779 us token by token; of the 346 us the two wide products cost 99 and 70, the triangular ones 78 and barriers, loads
 // and stores the rest (360 us with a chunk's factors loaded at its start instead of one chunk ahead); neither 8 x 8 tiles with half
 // of the shared-memory loads nor 16 warps change it.
 constexpr int CH = 64, CP = CH + 4, CW_THREADS = 256, CW_COLS = 32;

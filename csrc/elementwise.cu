@@ -206,11 +206,9 @@ NXD_API int nxd_swiglu_bwd(const void* gate_up, const void* dy, void* dgate_up, 
     return 0;
 }
 
-// x: [T, heads_total, D] bf16 (in place).  cos/sin: [max_pos, D/2] fp32.
-// position of token t = positions[t] if given, else (t / pos_div) % pos_mod.
-// inverse != 0 applies the transpose rotation (backward).
-// x [T, heads_total, D] bf16 -> y (x itself, or another buffer): the first n_rot_heads heads rotated at positions[t] (int32) or
-// (t / pos_div) % pos_mod, the others copied.  D a multiple of 16, x and y 16-byte aligned.
+// x [T, heads_total, D] bf16 -> y (x itself, or another buffer): the first n_rot_heads heads rotated at positions[t] (int32; NULL:
+// (t / pos_div) % pos_mod), the others copied.  cos / sin [max_pos, D / 2] fp32; inverse != 0: the transpose rotation (backward).
+// D a multiple of 16, x and y 16-byte aligned.
 NXD_API int nxd_rope(const void* x, void* y, const float* cos_t, const float* sin_t, const int* positions, long long T,
                      int heads_total, int n_rot_heads, int D, int pos_div, int pos_mod, int inverse, void* stream) {
     NXD_REQUIRE(D % 16 == 0, "rope: head dim %d must be a multiple of 16", D);

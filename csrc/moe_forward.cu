@@ -1,7 +1,7 @@
 // The sparse mixture after its router in ONE call: rows sorted by expert, gate / up product with the activation, down product,
-// weighted combination, and a shared expert's two products -- six to eight launches that read the routing on the device.  One host call and one workspace instead of
-// four calls with an allocation each: at 64 tokens (width 1024, 16 experts) the launches take 36 us of GPU time and the four
-// calls from Python 80 us of host time.
+// weighted combination, and a shared expert's two products -- six to eight launches that read the routing on the device.  One host
+// call and one workspace instead of four calls with an allocation each: at 64 tokens (width 1024, 16 experts) the launches take
+// 36 us of GPU time and the four calls from Python 80 us of host time.
 #include "common.cuh"
 #include "gemm_tcgen05.cuh"
 
