@@ -331,7 +331,7 @@ def case_flag_protocol_stress(rank, world):
             assert _rel(got, ref) < 4e-3, f"oneshot iteration {it}"
 
 
-@pytest.mark.skipif(os.environ.get("NXD_STRESS", "0") != "1", reason="opt-in: NXD_STRESS=1 (see tools/run_sanitizers.sh)")
+@pytest.mark.skipif(os.environ.get("NXD_STRESS", "0") != "1", reason="opt-in: NXD_STRESS=1")
 def test_flag_protocol_stress():
     world = int(os.environ.get("NXD_STRESS_WORLD", "2"))
     if torch.cuda.device_count() < world:
