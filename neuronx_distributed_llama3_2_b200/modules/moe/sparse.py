@@ -17,9 +17,9 @@ Three execution paths over the same parameters:
             host;
   * device-sorted  the same in bf16 on the GPU with the counts read on the device: the sort, the two products (all experts
             in one launch each, the activation inside the first) and the combination are one call, capturable.  It
-            serves every number of tokens: in captured graphs of 1 .. 256 tokens at (width, experts, top, ff) = (2048, 8,
-            2, 2048) / (4096, 8, 2, 4096) / (1024, 16, 4, 512) it takes 49 .. 80 / 95 .. 202 / 38 .. 44 us where the pairs
-            take 82 .. 1948 / 402 .. 7539 / 45 .. 504 us.
+            serves every number of tokens but for small mixtures (``pairs_win``): in captured graphs of 1 .. 256 tokens at
+            (width, experts, top, ff) = (2048, 8, 2, 2048) / (4096, 8, 2, 4096) / (1024, 16, 4, 512) it takes 49 .. 80 / 95 .. 202 /
+            38 .. 44 us where the pairs take 82 .. 1948 / 402 .. 7539 / 45 .. 504 us.
 The combination (chosen experts, identity experts, shared expert times its sigmoid gate) is summed in fp32.
 """
 from __future__ import annotations
@@ -39,6 +39,17 @@ from .routing import RouterBiasedTopK
 SORTED_PATH_MIN_PAIRS_PER_EXPERT = 16.0
 
 
+def pairs_win(tokens: int, top: int, width: int, ff: int, shared_ff: int, gated: bool) -> bool:
+    """Whether the per-pair GEMVs beat the device-sorted path, whose six launches and 256-row tiles cost 20 to 25 us more at any
+    size.  A pair's products are two serial chains, over ``width`` (half as long without a gate) and over the chosen experts' ``ff``,
+    and the pairs together stream ``work`` million weights a matrix.  Fitted to captured graphs of 1 to 256 tokens, widths 256 to
+    2048, ff 64 to 1024, 4 to 64 experts, 1 to 4 chosen (1200 sizes): the form taken is 0.2 % slower than the faster one on average
+    and 13 % at most with a gate, 31 % in the worst of 300 sizes without one; with a shared expert 1.4 % and 31 %.  Sorted / pairs:
+    28 / 17 us (4 tokens, 256, 4 experts, 2, 256), 30 / 21 (512, 32, 1, 128), 39 / 48 (1, 1024, 16, 4, 512)."""
+    chain, work = top * ff + shared_ff, tokens * width * (top * ff + shared_ff) / 2 ** 20
+    return width + 0.5 * chain + 40 * work <= 1500 if gated else 0.2 * chain + 50 * work <= 1500
+
+
 class SparseMoE(torch.nn.Module):
     def __init__(self, hidden_size: int, num_experts: int, top_k: int, intermediate_size: int, limit: float,
                  num_identity_experts: int = 0, affinity_scale: float = 1.0, shared_intermediate_size: int = 0,
@@ -51,6 +62,7 @@ class SparseMoE(torch.nn.Module):
         self.weight_on_input, self.gated = weight_on_input, gated
         dev = device if device is not None else torch.device("cpu")
         self.hidden_size, self.num_experts, self.top_k = hidden_size, num_experts, top_k
+        self.intermediate_size, self.shared_intermediate_size = intermediate_size, shared_intermediate_size
         if limit is None:            # plain silu(gate) * up: no clamp, unit slope, no shift of the linear half
             limit, alpha, self.up_shift = float("inf"), 1.0, 0.0
         else:
@@ -76,10 +88,17 @@ class SparseMoE(torch.nn.Module):
             return False
         return n_tokens * self.top_k / max(self.num_experts, 1) >= SORTED_PATH_MIN_PAIRS_PER_EXPERT
 
-    def _use_device_sorted(self, h: torch.Tensor) -> bool:
-        """The sorted path without a host read: one process holds whole experts, ``sorted_forward_applies``."""
-        return (h.is_cuda and ps.get_tensor_model_parallel_size() == 1 and ps.get_expert_model_parallel_size() == 1
-                and moe_sparse.sorted_forward_applies(h, *self._sorted_weights()))
+    def _device_path(self, h: torch.Tensor):
+        """The path of a bf16 call on the GPU whose process holds whole experts: ``"pairs"`` or ``"device"`` with its weights, or
+        ``None`` where the device-sorted form does not apply.  The sizes are asked first: they cost the least."""
+        if (not h.is_cuda or h.dtype != torch.bfloat16 or not h.shape[0] or ps.get_tensor_model_parallel_size() > 1
+                or ps.get_expert_model_parallel_size() > 1):
+            return None, None
+        if (pairs_win(h.shape[0], self.top_k, h.shape[1], self.intermediate_size, self.shared_intermediate_size, self.gated)
+                and self.experts.down_proj.weight.dtype == h.dtype):
+            return "pairs", None
+        weights = self._sorted_weights()
+        return ("device", weights) if moe_sparse.sorted_forward_applies(h, *weights) else (None, None)
 
     def _sorted_weights(self):
         """In and down weights of the experts, then those of the shared expert if there is one."""
@@ -91,8 +110,11 @@ class SparseMoE(torch.nn.Module):
         the host) | ``"device"`` (device-sorted), default: chosen by the sizes."""
         gated = self.shared is not None and self.shared_gate is not None
         idx, wts, sg = self.router.select(h, self.shared_gate.weight if gated else None)
-        if path == "device" or (path is None and h.shape[0] and self._use_device_sorted(h)):
-            return self._forward_device_sorted(h, idx, wts, sg)
+        weights = None
+        if path is None:
+            path, weights = self._device_path(h)
+        if path == "device":
+            return self._forward_device_sorted(h, idx, wts, sg, weights or self._sorted_weights())
         sorted_path = self._use_sorted(h.shape[0]) if path is None else path == "sorted"
         if sorted_path:
             return self._forward_sorted(h, idx, wts, sg)
@@ -120,11 +142,11 @@ class SparseMoE(torch.nn.Module):
             ones = self._ones = torch.ones_like(wts)
         return ones
 
-    def _forward_device_sorted(self, h, idx, wts, sg):
+    def _forward_device_sorted(self, h, idx, wts, sg, weights):
         in_scale = None
         if self.weight_on_input:
             in_scale, wts = wts, self._ones_like(wts)
-        w_in, w_down, *shared = self._sorted_weights()
+        w_in, w_down, *shared = weights
         return moe_sparse.sorted_forward(h, idx, wts, w_in, w_down, self.gated, self.limit, self.alpha, self.up_shift, in_scale,
                                          *(shared or (None, None)), shared_limit=self.shared_limit if shared else 0.0,
                                          shared_gate=sg)

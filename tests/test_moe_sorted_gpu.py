@@ -92,16 +92,15 @@ def test_captured_step_repeats_and_is_as_exact_as_the_pairs(N, shared):
         for p in m.parameters():
             p.copy_(torch.randn(p.shape, generator=g, device="cuda") * p.shape[-2] ** -0.5 if p.dim() > 1 else torch.zeros_like(p))
         h, first = (torch.randn(N, 136, generator=g, device="cuda").bfloat16() for _ in range(2))
-        assert m._use_device_sorted(h)
         given = first.clone()
-        m(given)
+        m(given, path="device")
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
-            out = m(given)
+            out = m(given, path="device")
         for x in (first, h, first, h):                  # every replay reads its own input
             given.copy_(x)
             graph.replay()
-            assert torch.equal(out, m(x))
+            assert torch.equal(out, m(x, path="device"))
         idx, wts, gate = m.router.select(h, m.shared_gate.weight if shared else None)
         ref = _reference(h, idx, wts, m.experts.gate_up_proj.weight, m.experts.down_proj.weight, 1.5, 1.702, 1.0, False)
         if shared:
@@ -126,8 +125,10 @@ def test_each_path_is_the_one_that_was_asked_for(monkeypatch):
             p.copy_(torch.randn(p.shape, generator=g, device="cuda") * 0.1)
         h = torch.randn(90, 128, generator=g, device="cuda").bfloat16()
         by_path = {path: m(h, path=path) for path in ("pairs", "sorted", "device", None)}
-    assert taken == ["_forward_sorted", "_forward_device_sorted", "_forward_device_sorted"]
-    assert torch.equal(by_path["device"], by_path[None])
+        assert taken == ["_forward_sorted", "_forward_device_sorted"]
+        assert torch.equal(by_path["pairs"], by_path[None])                  # 90 tokens of a small mixture
+        many = torch.randn(3000, 128, generator=g, device="cuda").bfloat16()
+        assert torch.equal(m(many), m(many, path="device")) and taken[2:] == ["_forward_device_sorted"] * 2
     # the host-counted path rounds the experts' outputs to bf16, all round the activation: 2^-8 of a value each
     for y in by_path.values():
         assert (y - by_path["pairs"]).norm() <= 3 * 2.0 ** -8 * by_path["pairs"].norm()
