@@ -391,7 +391,9 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             }
             const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
             // lazy rescale: keep the stale max unless it moved by more than 2^8 (in scaled log2 units).  CACHE follows every
-            // move, as the kernels it takes calls from do: the row's largest weight is then exactly 1 and not rounded.
+            // move, as the kernels it takes calls from do: the row's largest weight is then exactly 1 and not rounded (the portion
+            // above: error 0.00188 instead of 0.00201 at the same time; without a bias the maximum moves in most tiles: 2100 tokens
+            // over a window of 1024 take 127 us instead of 110, 372 on the mma.sync kernel).
             float alpha = 1.f;
             bool rescale = false;
             if ((mx - m_run) * sc > (CACHE ? 0.f : kRescaleThreshold) || m_run == -INFINITY) {
