@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(128) decode_attn_mma_kernel(
 // D threads per (sequence, query head).  A chain of loads: the weights of all splits come from one load per lane and a warp
 // reduction, the partial rows are read eight at a time (split by split, a merge of 16 splits took longer than the attention
 // of 128 keys).
-constexpr int kMaxSplits = 64;
+constexpr int kMaxSplits = 64, kFewSplits = 4;
 
 template <int D>
 __global__ void __launch_bounds__(D) decode_attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
@@ -439,6 +439,27 @@ __global__ void __launch_bounds__(D) decode_attn_merge_kernel(const float* __res
     pdl_wait();
     const size_t bh = blockIdx.x;  // b * n_q + h
     const int d = threadIdx.x;
+    if (n_splits <= kFewSplits) {  // short contexts and many sequences: every thread weighs for itself, no barrier (0.5 us of 5)
+        const float2* ml = reinterpret_cast<const float2*>(part_ml) + bh * n_splits;
+        float2 a[kFewSplits];
+        float v[kFewSplits];
+#pragma unroll
+        for (int s = 0; s < kFewSplits; ++s) {
+            a[s] = s < n_splits ? ml[s] : make_float2(-INFINITY, 0.f);
+            v[s] = s < n_splits ? part_o[(bh * n_splits + s) * D + d] : 0.f;
+        }
+        float m = -INFINITY, l = 0.f, o = 0.f;
+#pragma unroll
+        for (int s = 0; s < kFewSplits; ++s) m = fmaxf(m, a[s].x);
+#pragma unroll
+        for (int s = 0; s < kFewSplits; ++s) {
+            const float w = a[s].x == -INFINITY ? 0.f : exp2f(a[s].x - m);
+            l = fmaf(a[s].y, w, l);
+            o = fmaf(v[s], w, o);
+        }
+        out[bh * D + d] = __float2bfloat16(l > 0.f ? o / l : 0.f);
+        return;
+    }
     if (d < 32) {
         const float2* ml = reinterpret_cast<const float2*>(part_ml) + bh * n_splits;
         float2 a = make_float2(-INFINITY, 0.f), b = a;
@@ -492,17 +513,38 @@ __global__ void kv_cache_update_kernel(const bf16* __restrict__ new_k, const bf1
 
 }  // namespace
 
-NXD_API int nxd_decode_attn_num_splits(int B, int n_kv, int max_len) {
-    // one wave of CTAs (two per SM) at least 128 keys each: a second, partial wave costs more than a longer loop (16 sequences of
-    // 2048 keys, 8 heads of 64: 12.2 us with 2 splits, 14.6 with 3; 4 sequences: 5.9 with 8, 6.8 with 10; 12 of up to 2576 keys:
-    // 13.2 with 3, 14.9 with 4, and with heads of 128 20.8 with 3, 21.3 with 4).
-    const int pairs = B * n_kv;
-    const int want = 2 * nxd_num_sms() / (pairs > 0 ? pairs : 1);
+static int decode_splits(int want, int max_len) {
     int by_len = (max_len + 127) / 128;
     int s = want < by_len ? want : by_len;
     if (s < 1) s = 1;
     if (s > kMaxSplits) s = kMaxSplits;
     return s;
+}
+
+// Whether the tensor-core kernel takes a group of query heads (NXD_DECODE_ATTN=fma keeps the FMA kernel for comparison)
+static bool decode_on_tensor_cores(int group) {
+    static const bool force_fma = [] {
+        const char* e = getenv("NXD_DECODE_ATTN");
+        return e != nullptr && e[0] == 'f';
+    }();
+    return group >= 2 && group <= 16 && !force_fma;
+}
+
+// Splits that any kernel fills the chip with (FMA kernel: several CTAs of little shared memory per SM, so more of them than two
+// per SM still run at once).
+NXD_API int nxd_decode_attn_num_splits(int B, int n_kv, int max_len) {
+    const int pairs = B * n_kv > 0 ? B * n_kv : 1;
+    return decode_splits((2 * nxd_num_sms() + pairs - 1) / pairs, max_len);
+}
+
+// The same for n_q query heads.  Tensor-core kernel: one wave of CTAs (two per SM) at least 128 keys each: a second, partial wave
+// costs more than a longer loop (16 sequences of 2048 keys, 8 heads of 64: 12.2 us with 2 splits, 14.6 with 3; 4 sequences: 5.9 with
+// 8, 6.8 with 10; 12 of up to 2576 keys: 13.2 with 3, 14.9 with 4, and with heads of 128 20.8 with 3, 21.3 with 4).  On the FMA kernel
+// the same rule halves what runs at once (12 sequences of 4000 keys, 16 heads of 64 without groups: 98 us with 2 splits, 185 with 1).
+NXD_API int nxd_decode_attn_splits(int B, int n_q, int n_kv, int max_len) {
+    const int pairs = B * n_kv > 0 ? B * n_kv : 1;
+    if (!decode_on_tensor_cores(n_kv > 0 ? n_q / n_kv : 1)) return nxd_decode_attn_num_splits(B, n_kv, max_len);
+    return decode_splits(2 * nxd_num_sms() / pairs, max_len);
 }
 
 // scratch: B * n_q * n_splits * (D + 2) floats.  seq_ids: [B] int32 cache line (contiguous cache) or block-table row
@@ -535,13 +577,7 @@ static int decode_attn_impl(const void* q, const void* cache_k, const void* cach
         case 3: NXD_DECODE_LAUNCH(DD, 3); break; \
         default: NXD_DECODE_LAUNCH(DD, 4); break; \
     }
-    // GQA groups of 2 .. 16 heads: tensor-core kernel (NXD_DECODE_ATTN=fma keeps the FMA kernel for comparison)
-    static const bool force_fma = [] {
-        const char* e = getenv("NXD_DECODE_ATTN");
-        return e != nullptr && e[0] == 'f';
-    }();
-    const bool use_mma = group >= 2 && group <= 16 && !force_fma;
-    if (use_mma) {
+    if (decode_on_tensor_cores(group)) {
         dim3 mgrid(B * n_kv, n_splits);
         if (D == 64) {
             NXD_CHECK_CUDA(nxd_allow_smem<decode_attn_mma_kernel<64>>(MmaDecodeCfg<64>::kSmemBytes));

@@ -88,6 +88,7 @@ int nxd_topk_sample(const void* logits, int dtype, int B, int V, long long row_s
 /* ---- decode attention + KV cache (reference: examples/inference/modules/attention/
  *      attention_base.py:141-170; modules/model_base.py:388-422) -------------------------------- */
 int nxd_decode_attn_num_splits(int B, int n_kv, int max_len);
+int nxd_decode_attn_splits(int B, int n_q, int n_kv, int max_len);      /* as chosen for that many query heads */
 /* scratch: B * n_q * n_splits * (D + 2) floats */
 int nxd_decode_attn(const void* q, const void* cache_k, const void* cache_v, const int* lengths,
                     const int* block_table, long long stride_b, long long stride_h, int page_size,

@@ -150,7 +150,7 @@ def decode_attention(q: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Tens
     if q.is_cuda and q.dtype == torch.bfloat16 and D in (64, 128) and _lib.available():
         lens = lengths.to(torch.int32).contiguous()
         max_len = cache_k.shape[2] if block_table is None else block_table.shape[1] * page_size
-        n_splits = _lib.lib().nxd_decode_attn_num_splits(_c.c_int(B), _c.c_int(Hkv), _c.c_int(max_len))
+        n_splits = _lib.lib().nxd_decode_attn_splits(_c.c_int(B), _c.c_int(Hq), _c.c_int(Hkv), _c.c_int(max_len))
         # the call's own scratch: a captured graph keeps it in its pool, and calls on other streams have theirs
         scratch = torch.empty(B * Hq * n_splits * (D + 2), dtype=torch.float32, device=q.device)
         out = torch.empty_like(q)

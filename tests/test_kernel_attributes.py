@@ -111,3 +111,10 @@ def test_every_device_is_given_its_shared_memory(library, name):
         rc = CALLS[name](library)
         assert rc == 0 and library.fake_refused() == 0, (device, rc, library.nxd_last_error())
         assert library.fake_launches() > 0
+
+
+# one wave of two CTAs per SM for groups of query heads, more where the FMA kernel serves (148 SMs)
+@pytest.mark.parametrize("B,n_q,n_kv,max_len,splits", [(12, 64, 16, 4000, 1), (12, 16, 16, 4000, 2), (5, 32, 32, 4000, 2), (1, 32, 8, 4000, 32),
+                                                       (1, 8, 8, 100000, 37), (64, 8, 1, 200, 2), (1, 32, 1, 100000, 64)])
+def test_splits_of_a_token_step(library, B, n_q, n_kv, max_len, splits):
+    assert library.nxd_decode_attn_splits(B, n_q, n_kv, max_len) == splits
