@@ -159,24 +159,24 @@ __device__ __forceinline__ void router_select(float* ps, float* cs, const float*
     }
 }
 
-// A CTA of RT_WARPS warps.  TOK == 1: one token, the warps share its experts (few tokens: the latency of one token counts).
-// TOK > 1: every warp takes TOK tokens and all experts, so a row of wr that is loaded serves TOK tokens (many tokens: the
-// fp32 rows of wr come from L1 / L2 and are the larger operand). 
-template <typename T, int V, int TOK>
+// A CTA of RT_WARPS warps.  SHARE: one token, the warps share its experts (few tokens: the latency of one token counts).  Else
+// every warp takes TOK tokens and all experts, so a row of wr that is loaded serves TOK tokens (many tokens: the fp32 rows of wr
+// come from L1 / L2 and are the larger operand).
+template <typename T, int V, int TOK, bool SHARE>
 __global__ void __launch_bounds__(RT_WARPS * 32)
 moe_router_kernel(const T* __restrict__ h, const float* __restrict__ wr, const float* __restrict__ corr,
                   const float* __restrict__ wsg, int* __restrict__ idx, float* __restrict__ wts,
                   float* __restrict__ sgate, long long N, int W, int R, int top, float out_scale,
                   const float* __restrict__ zbias, int mode) {
     extern __shared__ float smem[];
-    constexpr int G = TOK == 1 ? 4 : 8;
+    constexpr int G = SHARE ? 4 : 8;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long n0 = TOK == 1 ? blockIdx.x : ((long long)blockIdx.x * RT_WARPS + warp) * TOK;
-    if (n0 >= N) return;                            // TOK == 1: never; else whole warps, which share nothing
+    const long long n0 = SHARE ? blockIdx.x : ((long long)blockIdx.x * RT_WARPS + warp) * TOK;
+    if (n0 >= N) return;                            // SHARE: never; else whole warps, which share nothing
     const int nt = (int)min((long long)TOK, N - n0);
-    float* ps = smem + (TOK == 1 ? 0 : warp * (TOK + 1) * R);       // logits [TOK][R], then scratch [R]
+    float* ps = smem + (SHARE ? 0 : warp * (TOK + 1) * R);          // logits [TOK][R], then scratch [R]
     const T* hr = h + n0 * W;
-    for (int r0 = TOK == 1 ? warp * G : 0; r0 < R; r0 += TOK == 1 ? RT_WARPS * G : G) {
+    for (int r0 = SHARE ? warp * G : 0; r0 < R; r0 += SHARE ? RT_WARPS * G : G) {
         float acc[TOK][G];
         router_dots<T, V, TOK, G>(hr, wr + (long long)r0 * W, W, nt, R - r0, acc);
 #pragma unroll
@@ -187,7 +187,7 @@ moe_router_kernel(const T* __restrict__ h, const float* __restrict__ wr, const f
                 if (lane == 0 && r0 + i < R) ps[t * R + r0 + i] = z + (zbias != nullptr ? zbias[r0 + i] : 0.f);
             }
     }
-    if (wsg != nullptr && sgate != nullptr && (TOK > 1 || warp == RT_WARPS - 1)) {
+    if (wsg != nullptr && sgate != nullptr && (!SHARE || warp == RT_WARPS - 1)) {
         float acc[TOK][1];
         router_dots<T, V, TOK, 1>(hr, wsg, W, nt, 1, acc);
 #pragma unroll
@@ -196,7 +196,7 @@ moe_router_kernel(const T* __restrict__ h, const float* __restrict__ wr, const f
             if (lane == 0 && t < nt) sgate[n0 + t] = 1.f / (1.f + expf(-z));
         }
     }
-    if constexpr (TOK == 1) {
+    if constexpr (SHARE) {
         __syncthreads();
         if (warp == 0) router_select(ps, ps + R, corr, idx, wts, n0, R, top, out_scale, mode);
     } else {
@@ -567,18 +567,23 @@ NXD_API int nxd_moe_router(int dtype, const void* h, const float* wr, const floa
     if (N == 0) return 0;
     NXD_REQUIRE(top >= 1 && top <= R, "router: top %d of %d", top, R);
     NXD_REQUIRE((size_t)8 * R * sizeof(float) <= 48 * 1024, "router: %d outputs", R);
-    // one token per CTA while the tokens are too few to fill the chip with a warp per 4 tokens (or the logits of 16 tokens
-    // do not fit shared memory)
-    const bool single = N < 16ll * nxd_num_sms() || (size_t)RT_WARPS * 5 * R * sizeof(float) > 48 * 1024;
-    const size_t smem = (size_t)(single ? 2 : RT_WARPS * 5) * R * sizeof(float);
     const bool vec = W % 8 == 0 && ((uintptr_t)h % 16) == 0 && ((uintptr_t)wr % 16) == 0 && ((uintptr_t)wsg % 16) == 0;
-    const unsigned blocks = (unsigned)(single ? N : (N + RT_WARPS * 4 - 1) / (RT_WARPS * 4));
-#define NXD_RT(T, V, TOK)                                                                                               \
-    moe_router_kernel<T, V, TOK><<<blocks, RT_WARPS * 32, smem, (cudaStream_t)stream>>>(                                \
+    // A CTA per token (tok 0), a warp per token (1) or a warp per 4 tokens (4).  us at 1000 / 2400 / 4000 / 8000 tokens: 256 x 16 7 / 11 /
+    // 17 / 30, 7 / 10 / 12 / 21 and 16 / 17 / 17 / 21; 1024 x 64 26 / 56 / 94 / 178, 37 / 59 / 80 / 155 and 52 / 58 / 60 / 79; scalar
+    // loads (50 x 64) 10 / 20 / 25 / 42, 14 / 17 / 22 / 38 and 33 / 35 / 36 / 40.  The logits of 16 tokens must fit shared memory.
+    const long long sms = nxd_num_sms(), load = (long long)W * R;
+    const bool quad = (N >= (vec ? 24 : 64) * sms && N * load >= 1ll << 25) || (vec && N >= 16 * sms && load >= 1 << 16);
+    const int tok = N < 8 * sms ? 0 : quad && (size_t)RT_WARPS * 5 * R * sizeof(float) <= 48 * 1024 ? 4 : 1;
+    const size_t smem = (size_t)(tok == 0 ? 2 : RT_WARPS * (tok + 1)) * R * sizeof(float);
+    const unsigned blocks = (unsigned)(tok == 0 ? N : (N + RT_WARPS * tok - 1) / (RT_WARPS * tok));
+#define NXD_RT(T, V, TOK, SHARE)                                                                                        \
+    moe_router_kernel<T, V, TOK, SHARE><<<blocks, RT_WARPS * 32, smem, (cudaStream_t)stream>>>(                         \
         (const T*)h, wr, corr, wsg, idx, wts, sgate, N, W, R, top, out_scale, zbias, mode)
 #define NXD_RT_V(T, V)                                                                                                  \
     do {                                                                                                                \
-        if (single) NXD_RT(T, V, 1); else NXD_RT(T, V, 4);                                                              \
+        if (tok == 0) NXD_RT(T, V, 1, true);                                                                            \
+        else if (tok == 1) NXD_RT(T, V, 1, false);                                                                      \
+        else NXD_RT(T, V, 4, false);                                                                                    \
     } while (0)
     if (dtype == 0) {
         if (vec) NXD_RT_V(bf16, 8); else NXD_RT_V(bf16, 1);

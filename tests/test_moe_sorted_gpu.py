@@ -61,7 +61,9 @@ def test_sorted_experts_match_float64(N, E, top, W, F, form):
     assert (out.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
 
 
-@pytest.mark.parametrize("N,W,R", [(5, 72, 3), (5, 50, 37), (2400, 64, 37), (2401, 50, 9), (2369, 200, 700)])
+@pytest.mark.parametrize("N,W,R", [(5, 72, 3), (5, 50, 37), (2400, 64, 37), (2401, 50, 9), (2369, 200, 700)]
+                         # a CTA, a warp and a quarter of a warp per token, the last with vector and with scalar loads
+                         + [(1183, 72, 5), (1185, 72, 5), (3601, 256, 40), (9601, 50, 80)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_router_forms_match_float64(N, W, R, dtype):
     from neuronx_distributed_llama3_2_b200.ops import moe_sparse as ms
