@@ -96,7 +96,7 @@ __global__ void delta_prep_kernel(const T* __restrict__ proj, long long ld, int 
 // key or value piece and walks a strip of tokens with the last three inputs in registers, so every projection value is
 // read once (the general kernel reads it once per tap, 2 bytes at a time).  Bound by memory: 4 x 2048 tokens, 4 + 4 heads of
 // 128 and 4 of 256 (100 MB with the fp32 results): 44 us, 177 us with the general kernel.
-constexpr int PREP_STRIP = 16, PREP_AHEAD = 4;
+constexpr int PREP_STRIP = 16, PREP_SHORT = 4, PREP_AHEAD = 4;
 
 template <int V>
 __device__ __forceinline__ void ld_v(const float* p, float* f) {
@@ -134,13 +134,13 @@ delta_prep_strip_kernel(const T* __restrict__ proj, long long ld, int off_q, int
                         const float* __restrict__ conv_w, const float* __restrict__ conv_state, float* __restrict__ qn,
                         float* __restrict__ kn, float* __restrict__ vn, const int* __restrict__ q_start,
                         const int* __restrict__ n_new, const int* __restrict__ seq_ids, int units, int Tn, int H, int G, int Dv,
-                        float qscale, float unit_eps) {
+                        float qscale, float unit_eps, int strip) {
     constexpr int D = 32 * V, TAPS = 4, K = TAPS - 1;
     const int lane = threadIdx.x & 31, u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (u >= units) return;
-    const int b = blockIdx.z, s0 = blockIdx.y * PREP_STRIP;
+    const int b = blockIdx.z, s0 = blockIdx.y * strip;
     const int n = n_new != nullptr ? min(n_new[b], Tn) : Tn;
-    const int s_end = min(n, s0 + PREP_STRIP);
+    const int s_end = min(n, s0 + strip);
     if (s0 >= s_end) return;
     const int C = 2 * G * D + H * Dv;
     const int c = u * D + lane * V;                              // channel in q | k | v order
@@ -207,9 +207,12 @@ int launch_prep_strip(const void* proj, long long ld, int off_q, int off_k, int 
                       const float* conv_state, float* qn, float* kn, float* vn, const int* q_start, const int* n_new,
                       const int* seq_ids, int B, int Tn, int H, int G, int Dv, float qscale, float unit_eps, cudaStream_t st) {
     const int units = 2 * G + H * (Dv / (32 * V));
-    dim3 grid((units + 7) / 8, (Tn + PREP_STRIP - 1) / PREP_STRIP, B);
+    // short strips (every input read 1.75 times) while long ones would be too few warps: 1 x 64 tokens, 4 + 4 heads of 128 and 4 of
+    // 256: 13.1 us in strips of 16, 7.6 in strips of 4 (13.8 in the general kernel); 8 x 128 tokens, 3 x 16 heads of 128: 19.2 / 20.2
+    const int strip = (long long)units * ((Tn + PREP_STRIP - 1) / PREP_STRIP) * B < 1536 ? PREP_SHORT : PREP_STRIP;
+    dim3 grid((units + 7) / 8, (Tn + strip - 1) / strip, B);
     delta_prep_strip_kernel<T, V><<<grid, 256, 0, st>>>((const T*)proj, ld, off_q, off_k, off_v, conv_w, conv_state, qn, kn, vn,
-                                                        q_start, n_new, seq_ids, units, Tn, H, G, Dv, qscale, unit_eps);
+                                                        q_start, n_new, seq_ids, units, Tn, H, G, Dv, qscale, unit_eps, strip);
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -909,7 +912,7 @@ NXD_API int nxd_delta_prep(int dtype, const void* proj, long long ld, int off_q,
         auto al = [](const void* p, size_t n) { return ((uintptr_t)p % n) == 0; };
         if (taps == 4 && (D == 64 || D == 128 || D == 256) && Dv % D == 0 && ld % V == 0 && off_q % V == 0 && off_k % V == 0 &&
             off_v % V == 0 && al(proj, 16) && al(conv_w, 16) && al(qn, 16) && al(kn, 16) && al(vn, 16) && B < 65536 &&
-            (Tn + PREP_STRIP - 1) / PREP_STRIP < 65536) {
+            (Tn + PREP_SHORT - 1) / PREP_SHORT < 65536) {
 #define NXD_STRIP(T, V_)                                                                                                   \
     return launch_prep_strip<T, V_>(proj, ld, off_q, off_k, off_v, conv_w, conv_state, qn, kn, vn, q_start, n_new, seq_ids, B, \
                                     Tn, H, G, Dv, qscale, unit_eps, st)

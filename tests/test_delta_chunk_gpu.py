@@ -128,7 +128,8 @@ def test_strips_of_the_short_convolution_match_float64(dtype, D, H, G, Dv):
 
     B, taps, C = 2, 4, 2 * G * D + H * Dv
     gen = torch.Generator(device="cuda").manual_seed(D)
-    total = 80
+    long = 1 + 16 * (-(-1536 // (B * (2 * G + H * Dv // D))))        # enough of them for strips of 16
+    total = 80 + long
     raw = torch.randn(B, total, C + 16, generator=gen, device="cuda").to(dtype)
     w = torch.randn(C, taps, generator=gen, device="cuda") * 0.5
     state = torch.randn(3, taps - 1, C, generator=gen, device="cuda")
@@ -140,7 +141,7 @@ def test_strips_of_the_short_convolution_match_float64(dtype, D, H, G, Dv):
     q, k = (t / torch.sqrt(t.square().sum(-1, keepdim=True) + 1e-6) for t in (q, k))
     refs = (q * 0.25, k, v.unflatten(-1, (H, Dv)))
     at = 0
-    for size in (1, 17, 3, 16, 43):                      # portions around the strips of 16
+    for size in (1, 17, 3, 16, 43, long):                # portions around the strips of 4 (few tokens) and 16
         got = dr.delta_prep(raw[:, at:at + size].contiguous(), (8, 8 + G * D, 8 + 2 * G * D), w, state,
                             torch.full((B,), at, dtype=torch.int32, device="cuda"), H, G, D, Dv, 0.25, seq_ids=line)
         for x32, ref in zip(got, refs):
