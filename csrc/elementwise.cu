@@ -63,29 +63,28 @@ __global__ void swiglu_bwd_kernel(const bf16* __restrict__ gu, const bf16* __res
     }
 }
 
-// One thread takes 8 (x1, x2) pairs, columns [8c, 8c+8) and [D/2 + 8c, ...), of kRopeHeads heads of a token: the table entries
-// and the position are read once for them and 2 kRopeHeads 16-byte loads are in flight.  Heads from n_rot on are copied
+// One thread takes 8 (x1, x2) pairs, columns [8c, 8c+8) and [D/2 + 8c, ...), of kHeads heads of a token: the table entries
+// and the position are read once for them and 2 kHeads 16-byte loads are in flight.  Heads from n_rot on are copied
 // (n_heads = heads_total, x != y) or left alone (n_heads = n_rot, x == y).  Bound by memory: 8192 tokens x 40 heads of 128, 32 of
 // them rotated, 30 us on average for one launch out of place (168 MB) and one in place (134 MB), against 23 us of copy and 31 us of
 // rotation each with one head per thread.
-constexpr int kRopeHeads = 4;
-
+template <int kHeads>
 __global__ void rope_kernel(const bf16* x, bf16* y, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                             const int* __restrict__ positions, size_t T, int heads_total, int n_heads, int n_rot, int D,
                             int pos_div, int pos_mod, float sin_sign) {
     const int half_vec = D >> 4;  // 16-byte vectors in half a head
-    const int groups = (n_heads + kRopeHeads - 1) / kRopeHeads;
+    const int groups = (n_heads + kHeads - 1) / kHeads;
     const size_t total = T * (size_t)groups * half_vec;
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x) {
         const int c = (int)(idx % half_vec);
         const size_t tg = idx / half_vec;
-        const int h0 = (int)(tg % groups) * kRopeHeads;
+        const int h0 = (int)(tg % groups) * kHeads;
         const size_t t = tg / groups;
         const size_t at = (t * heads_total + h0) * (size_t)D + c * 8;
-        bf16x8 va[kRopeHeads], vb[kRopeHeads];
+        bf16x8 va[kHeads], vb[kHeads];
 #pragma unroll
-        for (int j = 0; j < kRopeHeads; ++j) {
+        for (int j = 0; j < kHeads; ++j) {
             if (h0 + j < n_heads) {
                 va[j] = *reinterpret_cast<const bf16x8*>(x + at + (size_t)j * D);
                 vb[j] = *reinterpret_cast<const bf16x8*>(x + at + (size_t)j * D + (D >> 1));
@@ -101,7 +100,7 @@ __global__ void rope_kernel(const bf16* x, bf16* y, const float* __restrict__ co
             sn[0] = s0.x, sn[1] = s0.y, sn[2] = s0.z, sn[3] = s0.w, sn[4] = s1.x, sn[5] = s1.y, sn[6] = s1.z, sn[7] = s1.w;
         }
 #pragma unroll
-        for (int j = 0; j < kRopeHeads; ++j) {
+        for (int j = 0; j < kHeads; ++j) {
             if (h0 + j >= n_heads) break;
             if (h0 + j < n_rot) {
                 float a[8], b[8], oa[8], ob[8];
@@ -215,8 +214,14 @@ NXD_API int nxd_rope(const void* x, void* y, const float* cos_t, const float* si
     NXD_REQUIRE(n_rot_heads <= heads_total, "rope: n_rot_heads > heads_total");
     const int n_heads = x == y ? n_rot_heads : heads_total;
     if (T == 0 || n_heads == 0) return 0;
-    const size_t work = (size_t)T * ((n_heads + kRopeHeads - 1) / kRopeHeads) * (D / 16);
-    rope_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
+    // four heads per thread where that leaves 2^16 threads and a warp reads 64 bytes or more of each half head: heads of 128, 40 of
+    // them: 1000 tokens in place 5.4 us with one head per thread, 4.6 with four, 8192 tokens 28.9 / 21.9, but 64 tokens 2.3 / 3.1;
+    // 48 heads of 64: 2048 tokens 8.4 / 11.0, 8192 tokens out of place 30.1 / 35.9
+    const size_t quads = (size_t)T * ((n_heads + 3) / 4) * (D / 16);
+    const bool four = D >= 128 && quads >= 1 << 16;
+    const size_t work = four ? quads : (size_t)T * n_heads * (D / 16);
+    auto kern = four ? rope_kernel<4> : rope_kernel<1>;
+    kern<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
         (const bf16*)x, (bf16*)y, cos_t, sin_t, positions, (size_t)T, heads_total, n_heads, n_rot_heads, D,
         pos_div < 1 ? 1 : pos_div, pos_mod < 1 ? 1 : pos_mod, inverse ? -1.f : 1.f);
     NXD_LAUNCH_CHECK();

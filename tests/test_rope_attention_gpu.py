@@ -12,7 +12,8 @@ def _tables(n, D):
 
 
 # heads around the four that a thread takes, with copied heads behind them; the smallest head size and one that is no power of two
-@pytest.mark.parametrize("T,heads,rot,D", [(1, 1, 1, 16), (7, 5, 3, 48), (33, 9, 8, 64), (130, 6, 0, 128), (1001, 40, 32, 128)])
+@pytest.mark.parametrize("T,heads,rot,D", [(1, 1, 1, 16), (7, 5, 3, 48), (33, 9, 8, 64), (130, 6, 0, 128), (1001, 40, 32, 128),
+                                             (1700, 19, 17, 128)])
 @pytest.mark.parametrize("offset", [0, 1])
 def test_rope_matches_fp32(T, heads, rot, D, offset):
     from neuronx_distributed_llama3_2_b200.ops import rope
