@@ -23,14 +23,18 @@ from . import _lib
 GROUP = "retention_serving"
 CHUNK = 64
 
-# steps that run on the tensor cores (csrc/retention_tc.cu) where its sizes apply.  Measured against the fp32 kernels, one row, heads
-# x key x value size: 64 tokens 4 x 64 x 128 34 / 47 us, 4 x 128 x 256 67 / 60, 8 x 256 x 512 178 / 61; 128 tokens 50 / 48, 117 / 61,
-# 343 / 63; 4096 tokens 77 / 75, 225 / 108, 1942 / 317
-TC_MIN_TOKENS, TC_MIN_TOKENS_WIDE, TC_WIDE = 128, 64, 128
+# steps that run on the tensor cores (csrc/retention_tc.cu) where its sizes apply.  Measured against the fp32 kernels at 1 and 64 pairs of a
+# row and a head, fp32 kernels / tensor cores: state 64 x 64 128 tokens 29 / 33 and 36 / 45 us, 1024 tokens 32 / 35 and 126 / 135;
+# 64 x 128 64 tokens 25 / 33 and 33 / 46, 128 tokens 41 / 33 and 51 / 47; 128 x 128 64 tokens 37 / 36 and 51 / 58, 96 tokens 55 / 36 and
+# 72 / 58; 128 x 256 64 tokens 56 / 37 and 81 / 77; 256 x 512 64 tokens 158 / 43 and 254 / 153
+TC_MIN_STATE, TC_WIDE_STATE = 64 * 128, 128 * 256
 
 
-def _tc_wanted(T: int, dim: int) -> bool:
-    return T >= (TC_MIN_TOKENS_WIDE if dim >= TC_WIDE else TC_MIN_TOKENS)
+def _tc_wanted(T: int, dim: int, vdim: int) -> bool:
+    state = dim * vdim
+    if state < TC_MIN_STATE:
+        return False
+    return T >= (128 if dim < 128 else 96 if state < TC_WIDE_STATE else 64)
 
 _SMEM_LIMIT = 220 * 1024
 
@@ -105,7 +109,7 @@ def _launch(chunkwise: bool, proj, offsets, decay, state, q_start, heads, dim, v
     head = (_c.c_int(_code(proj.dtype)), _lib.ptr(proj), _c.c_longlong(ld), _c.c_int(offsets[0]), _c.c_int(offsets[1]),
             _c.c_int(offsets[2]), _lib.ptr(decay), _lib.ptr(state), _lib.ptr(out))
     L = _lib.lib(GROUP)
-    if chunkwise and _tc_wanted(T, dim):
+    if chunkwise and _tc_wanted(T, dim, vdim):
         need = L.nxd_retention_tc_workspace
         need.restype = _c.c_longlong
         size = need(_c.c_int(_code(proj.dtype)), _c.c_int(B), _c.c_int(T), _c.c_int(heads), _c.c_int(dim), _c.c_int(vdim))
