@@ -99,6 +99,15 @@ def gemm_grouped(a: torch.Tensor, b: torch.Tensor, layout: str, out: Optional[to
 SMALLM_MAX_ROWS = 128
 
 
+def product_streams_on_tensor_cores(rows: int, n: int, k: int) -> bool:
+    """``streams_on_tensor_cores`` for a single product, whose FMA GEMV splits long rows over a CTA.  One row or two, in captured
+    graphs, FMA / tensor cores: 1 / ``[1024, 8192]`` 4.4 us / 6.9, 1 / ``[4096, 2048]`` 4.5 / 5.1, 1 / ``[2048, 8192]`` 7.9 / 7.2, 1 /
+    ``[16384, 512]`` 5.1 / 4.9; 2 / ``[512, 8192]`` 5.7 / 6.9, 2 / ``[2048, 2048]`` 3.7 / 4.0, 2 / ``[8192, 2048]`` 6.9 / 6.4."""
+    if rows > 2:
+        return streams_on_tensor_cores(rows, n, k)
+    return (n >= 2048 and k >= 4096) or n >= 16384 or (rows == 2 and n >= 8192 and k >= 2048)
+
+
 def streams_on_tensor_cores(rows: int, n: int, k: int) -> bool:
     """Whether ``gemm_smallm`` beats the FMA GEMV (``fused_comm.skinny_gemm``, up to 8 rows).  Measured in captured graphs,
     rows / ``[n, k]``: 1 / ``[2048, 2048]`` 5.9 us FMA, 3.9 tensor cores; 1 / ``[16384, 2048]`` 17.1 / 12.1; 4 / ``[2048, 8192]``

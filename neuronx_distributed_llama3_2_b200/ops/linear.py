@@ -54,9 +54,9 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
             and a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and _backend() == "tcgen05" and _lib.available()):
         # token generation: weight-streaming kernels instead of a 256-row tensor-core tile that is mostly padding -- the
         # tensor-core kernel with the weight rows as the UMMA M dimension, or the FMA GEMV for few rows of small weights
-        from .gemm import gemm_smallm, streams_on_tensor_cores
+        from .gemm import gemm_smallm, product_streams_on_tensor_cores
 
-        res = gemm_smallm(a, b) if streams_on_tensor_cores(m, n, k) else None
+        res = gemm_smallm(a, b) if product_streams_on_tensor_cores(m, n, k) else None
         if res is None and m <= 8:
             from .fused_comm import skinny_gemm
 

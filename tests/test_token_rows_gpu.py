@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("rows", [1, 2, 5, 8])
 # around the line between the kernels, ragged last weight slabs and contraction tails
-@pytest.mark.parametrize("n,k", [(1024, 2048), (2056, 1032), (264, 1024), (16, 8192)])
+@pytest.mark.parametrize("n,k", [(1024, 2048), (2056, 1032), (264, 1024), (16, 8192), (2056, 4104)])
 def test_few_rows_match_float64(rows, n, k):
     from neuronx_distributed_llama3_2_b200.ops.linear import gemm_nt
 
