@@ -6,7 +6,7 @@
 //   out[B, N] = x[B, K] @ w[N, K]^T (+ residual[B, N])          bf16 in, fp32 accumulation, bf16 out
 //
 // and two variants with the neighbouring element-wise work of a decoder layer in the epilogue (the batched counterparts of
-// decode_fused.cu, which covers single rows, and <= 8 rows of small weights or tensor-parallel shards, with FMA GEMVs):
+// decode_fused.cu, which covers <= 8 rows of small weights or tensor-parallel shards with FMA GEMVs):
 //
 //   QKV    w = fused [q | k | v] head-major rows: RoPE(q, k) at positions[b], q -> q_out, k / v -> KV cache (contiguous
 //          or paged).  A 128-row weight slab is one head (D = 128) or two (D = 64), so the rotation partner (d, d + D/2)

@@ -201,13 +201,12 @@ class KVCacheInferenceMixin:
                                          page_size=kc.page_size if kc.paged else 0, seq_ids=seq_ids)
 
     def _tensor_core_decode(self, layer, hidden) -> bool:
-        """More than 8 rows; or 2 to 8 on one process where every weight of the layer is large enough and aligned for the
-        tensor-core kernels (16 layers of the 1B model, context 2048, per token: 2 sequences 894 -> 816 us, 4 1279 -> 837, 8 2202 ->
-        893).  One sequence stays on the FMA kernels (842 us; 784 on the tensor cores): the two orders of the sums differ by
-        2.0e-2 of the logits after 16 layers, at errors of 3.35e-2 (FMA) and 3.24e-2 against float64."""
+        """More than 8 rows; or 1 to 8 on one process where every weight of the layer is large enough and aligned for the
+        tensor-core kernels (16 layers of the 1B model, context 2048, per token, FMA kernels / tensor cores: 1 sequence 841 / 795
+        us, 2 sequences 894 / 816, 4 1279 / 837, 8 2202 / 893; 4 layers of the 3B model, 1 sequence: 403 / 365)."""
         if hidden.shape[0] > 8:
             return True
-        if hidden.shape[0] == 1 or ps.get_tensor_model_parallel_size() > 1:
+        if ps.get_tensor_model_parallel_size() > 1:
             return False          # tensor parallel: the row-parallel GEMVs carry the one-shot all-reduce
         from ..ops.gemm import streams_on_tensor_cores
 

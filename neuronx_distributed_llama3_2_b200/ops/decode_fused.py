@@ -3,7 +3,7 @@ write in one launch, RMSNorm + gate/up GEMV + SwiGLU in one launch.  With the tw
 residual in their epilogue (``fused_comm.skinny_gemm``) and the decode attention (split + merge) a decoder layer of the
 token-generation graph is six launches (reference graph: ``examples/inference/modules/model_base.py:459-518``).
 
-Batches of 2 to 128 sequences on one process take the tensor-core counterparts (``csrc/gemm_smallm.cu``: weight rows as the
+Batches of 1 to 128 sequences on one process take the tensor-core counterparts (``csrc/gemm_smallm.cu``: weight rows as the
 UMMA M dimension, cluster split-K) unless the weights are small (``gemm.streams_on_tensor_cores``): fused QKV GEMM + RoPE + cache write, gate/up GEMM + SwiGLU (<= 64 rows), and the plain GEMM
 with the residual in its epilogue; the two RMSNorms stay separate launches there (eight launches per layer)."""
 from __future__ import annotations

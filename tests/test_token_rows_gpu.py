@@ -50,3 +50,8 @@ def test_token_step_matches_the_fma_kernels(batch, paged, monkeypatch):
     assert len(taken) == 2
     for a, b in zip(got, ref):      # the same roundings to bf16 of fp32 sums in another order, two layers of them
         assert (a.float() - b.float()).norm() <= 1e-2 * b.float().norm()
+
+
+@pytest.mark.parametrize("paged", [False, True])
+def test_one_sequence_matches_the_fma_kernels(paged, monkeypatch):
+    test_token_step_matches_the_fma_kernels(1, paged, monkeypatch)
