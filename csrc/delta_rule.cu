@@ -21,9 +21,14 @@
 //                      tokens (t >= n_new[b]) change nothing and come out as zeros.
 // This file is compiled without fast-math: the state lives for thousands of steps.
 #include "common.cuh"
+#include "delta_chunks.cuh"
 #include "mma_sync.cuh"
 
 namespace {
+
+using nxd_delta::CH;
+using nxd_delta::CHUNK_FLOATS;
+using nxd_delta::CW_COLS;
 
 __device__ __forceinline__ float ldf(const float* p) { return *p; }
 __device__ __forceinline__ float ldf(const bf16* p) { return __bfloat162float(*p); }
@@ -479,40 +484,9 @@ int launch_scan(const float* qn, const float* kn, const float* vn, const float* 
 // With M = (I + A)^-1 diag(beta) and R = V - diag(Gamma) K S:  U = M R,  P U = (P M) R.
 // (the WY form of Householder products; Yang, Wang, Zhang, Shen, Kim, "Parallelizing Linear Transformers with the Delta Rule
 // over Sequence Length").  Decay ratios are products, never quotients or exponentials of sums, so a decay of any size is
-// exact to rounding and underflows to the right limit.  Two kernels:
-//   delta_chunk_system  per (chunk, head, row), in parallel, fp64: M, P M, Gamma and L[CH-1][.] to scratch
-//   delta_chunk_scan    fp32, per (32 value columns, head, row), sequential over chunks with the state slice in shared memory:
-//                       four products per chunk, register-tiled, on packed pairs of fp32 multiply-adds (pairs run along the
-//                       contraction, so both operands are read as 16-byte pieces and nothing is shuffled)
-// Bound by the fp32 pipes of the second kernel: a token costs 3 D + CH multiply-adds per value column, like token by token, but
-// 64 tokens are independent, where delta_scan waits for two dot products and a shuffle tree per token.  Its own limit is the
-// chain of a chunk's phases: 4 x 2048 tokens, 4 heads of 128 x 256 take 53 us (67 us with fp32 products in the first kernel) + 346
-// us against 779 us token by token; of the 346 us the two wide products cost 99 and 70, the triangular ones 78 and barriers, loads
-// and stores the rest (360 us with a chunk's factors loaded at its start instead of one chunk ahead); neither 8 x 8 tiles with half
-// of the shared-memory loads nor 16 warps change it.
-constexpr int CH = 64, CP = CH + 4, CW_THREADS = 256, CW_COLS = 32;
-
-__device__ __forceinline__ ulonglong2 ld_pairs(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
-
-// acc[i][j] += <a row i, b row j> over 4 values
-template <int R, int C>
-__device__ __forceinline__ void dot_step(uint64_t (&acc)[R][C], const ulonglong2 (&a)[R], const ulonglong2 (&b)[C]) {
-#pragma unroll
-    for (int i = 0; i < R; ++i)
-#pragma unroll
-        for (int j = 0; j < C; ++j) acc[i][j] = f2_fma(a[i].y, b[j].y, f2_fma(a[i].x, b[j].x, acc[i][j]));
-}
-
-template <int R, int C>
-__device__ __forceinline__ void add_pairs(uint64_t (&acc)[R][C], const uint64_t (&part)[R][C]) {
-#pragma unroll
-    for (int i = 0; i < R; ++i)
-#pragma unroll
-        for (int j = 0; j < C; ++j) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc[i][j]) : "l"(part[i][j]));
-}
-
-// scratch per (row, head, chunk): M [CH][CH] = (I + A)^-1 diag(beta), P M [CH][CH], Gamma [CH], L[CH-1][.] [CH]
-constexpr int CHUNK_FLOATS = 2 * CH * CH + 2 * CH, DPITCH = CH + 4;
+// exact to rounding and underflows to the right limit.  delta_chunk_system makes M, P M, Gamma and L[CH-1][.] of every (chunk, head,
+// row) in parallel, in fp64; delta_chunks.cu has the rest, on the tensor cores.
+constexpr int CW_THREADS = 256, DPITCH = CH + 4;
 
 // c [8 x 8] += a [8 x 4] b [4 x 8]: a is row lane / 4, column lane % 4; b row lane % 4, column lane / 4; c row lane / 4, columns
 // 2 (lane % 4) and the next
@@ -530,19 +504,31 @@ template <int D>
 __global__ void __launch_bounds__(CW_THREADS, 2)
 delta_chunk_system_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ gate,
                           long long ld_a, int a_off, const float* __restrict__ beta, long long ld_b, int b_off,
-                          float* __restrict__ scratch, const int* __restrict__ n_new, int Tn, int H, int G) {
+                          float* __restrict__ scratch, const int* __restrict__ n_new, int Tn, int chunk0, int H, int G) {
     extern __shared__ __align__(16) float smem[];
     double* Kd = reinterpret_cast<double*>(smem);      // [CH][DPITCH] 64 key channels at a time; then X = (I + A)^-1
     double* Qd = Kd + CH * DPITCH;                     // [CH][DPITCH] the same of the queries; then P
     double* Ad = Qd + CH * DPITCH;                     // [CH][DPITCH] L; then A
     __shared__ float gs[CH], bs[CH];
-    const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, kvh = h / (H / G), tid = threadIdx.x;
+    const int c = chunk0 + blockIdx.x, h = blockIdx.y, b = blockIdx.z, kvh = h / (H / G), tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5, lr = lane >> 2, lc = lane & 3;
     const int n = n_new != nullptr ? min(n_new[b], Tn) : Tn;
     const int nt = min(CH, n - c * CH);  // real tokens; the others change nothing (k = q = 0, beta = 0, g = 1)
     if (nt <= 0) return;                 // the scan does not look at this chunk
     const long long row0 = (long long)b * Tn + c * CH;
-    float* out = scratch + (((long long)b * H + h) * gridDim.x + c) * CHUNK_FLOATS;
+    float* out = scratch + (((long long)b * H + h) * gridDim.x + blockIdx.x) * CHUNK_FLOATS;
+    // keys and queries of 64 channels on their way: the first ones while the decays are multiplied up, the others behind the products
+    float4 kv[4], qv[4];
+    auto fetch = [&](int d0) {
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const int i = tid + x * CW_THREADS, t = i >> 4, d = (i & 15) * 4;
+            const long long src = ((row0 + min(t, nt - 1)) * G + kvh) * D + d0 + d;
+            kv[x] = *reinterpret_cast<const float4*>(kn + src), qv[x] = *reinterpret_cast<const float4*>(qn + src);
+            if (t >= nt) kv[x] = qv[x] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    fetch(0);
     if (tid < CH) {
         gs[tid] = tid < nt ? gate[(row0 + tid) * ld_a + a_off + h] : 1.f;
         bs[tid] = tid < nt ? beta[(row0 + tid) * ld_b + b_off + h] : 0.f;
@@ -566,16 +552,15 @@ delta_chunk_system_kernel(const float* __restrict__ qn, const float* __restrict_
     double kk[8][2] = {}, qk[8][2] = {};
     for (int d0 = 0; d0 < D; d0 += 64) {
         __syncthreads();
-        for (int i = tid; i < CH * 16; i += CW_THREADS) {
-            const int t = i >> 4, d = (i & 15) * 4;
-            const long long src = ((row0 + t) * G + kvh) * D + d0 + d;
-            float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), qv = kv;
-            if (t < nt) kv = *reinterpret_cast<const float4*>(kn + src), qv = *reinterpret_cast<const float4*>(qn + src);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const int i = tid + x * CW_THREADS, t = i >> 4, d = (i & 15) * 4;
             double2* kd = reinterpret_cast<double2*>(Kd + t * DPITCH + d);
             double2* qd = reinterpret_cast<double2*>(Qd + t * DPITCH + d);
-            kd[0] = make_double2(kv.x, kv.y), kd[1] = make_double2(kv.z, kv.w);
-            qd[0] = make_double2(qv.x, qv.y), qd[1] = make_double2(qv.z, qv.w);
+            kd[0] = make_double2(kv[x].x, kv[x].y), kd[1] = make_double2(kv[x].z, kv[x].w);
+            qd[0] = make_double2(qv[x].x, qv[x].y), qd[1] = make_double2(qv[x].z, qv[x].w);
         }
+        if (d0 + 64 < D) fetch(d0 + 64);
         __syncthreads();
 #pragma unroll 1
         for (int d = 0; d < 64; d += 4) {
@@ -650,243 +635,29 @@ delta_chunk_system_kernel(const float* __restrict__ qn, const float* __restrict_
     }
 }
 
-// grid (Dv / 32, H, B).  Rows of a thread in the 64-row products: 4 w + rg and 60 - 4 w + rg (w the warp, rg = lane / 8), so
-// that the triangular products cost every warp the same; columns cg + 8 i (cg = lane % 8).
-template <int D>
-__global__ void __launch_bounds__(CW_THREADS, D == 64 ? 2 : 1)
-delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vn,
-                        const float* __restrict__ scratch, float* __restrict__ S, float* __restrict__ out,
-                        const int* __restrict__ q_start, const int* __restrict__ n_new, const int* __restrict__ seq_ids, int Tn,
-                        int NC, int H, int G, int Dv) {
-    extern __shared__ __align__(16) float smem[];
-    constexpr int DP = D + 4, DT = D / 32, KB = D <= 128 ? 2 : 1;     // KB: buffers of K
-    float* Kb = smem;                          // [KB][CH][DP]
-    float* Qs = Kb + KB * CH * DP;             // [CH][DP]
-    float* Ss = Qs + CH * DP;                  // [32][DP] the state slice, a value column per row
-    float* Ms = Ss + CW_COLS * DP;             // [CH][CP]
-    float* Ps = Ms + CH * CP;                  // [CH][CP] P M
-    float* Rs = Ps + CH * CP;                  // [32][CP] V - diag(Gamma) K S, a value column per row
-    float* Us = Rs + CW_COLS * CP;             // [32][CP] U
-    float* gam2 = Us + CW_COLS * CP;           // [2][2 CH] Gamma and L[CH-1][.] of this chunk and the next
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int col0 = blockIdx.x * CW_COLS, h = blockIdx.y, b = blockIdx.z, kvh = h / (H / G);
-    const int n = n_new != nullptr ? min(n_new[b], Tn) : Tn;
-    const long long row0 = (long long)b * Tn;
-    float* orow = out + (row0 * H + h) * Dv + col0;              // + t * H * Dv
-    for (int i = tid; i < (Tn - max(n, 0)) * CW_COLS; i += CW_THREADS)       // padding rows
-        orow[(long long)(max(n, 0) + i / CW_COLS) * H * Dv + i % CW_COLS] = 0.f;
-    if (n <= 0) return;
-    const int line = seq_ids != nullptr ? seq_ids[b] : b;
-    float* Sb = S + ((long long)line * H + h) * D * Dv + col0;
-    const bool fresh = q_start[b] == 0;
-    for (int i = tid; i < D * CW_COLS; i += CW_THREADS) {
-        const int d = i / CW_COLS, j = i % CW_COLS;
-        Ss[j * DP + d] = fresh ? 0.f : Sb[(long long)d * Dv + j];
-    }
-    const float* chunk0 = scratch + ((long long)b * H + h) * NC * CHUNK_FLOATS;
-    const int chunks = (n + CH - 1) / CH;
-    auto rows = [&](const float* src, float* dst, int c) {       // K or Q rows of chunk c
-        if (c < chunks)
-            for (int i = tid; i < CH * (D / 4); i += CW_THREADS) {
-                const int t = i / (D / 4), d = (i % (D / 4)) * 4;
-                const bool ok = c * CH + t < n;
-                mma::cp_async16((uint32_t)__cvta_generic_to_shared(dst + t * DP + d),
-                                src + ((row0 + (ok ? c * CH + t : 0)) * G + kvh) * D + d, ok);
-            }
-    };
-    auto square = [&](int off, float* dst, int c) {              // M or P of chunk c
-        if (c < chunks)
-            for (int i = tid; i < CH * (CH / 4); i += CW_THREADS) {
-                const int t = i / (CH / 4), x = (i % (CH / 4)) * 4;
-                mma::cp_async16((uint32_t)__cvta_generic_to_shared(dst + t * CP + x),
-                                chunk0 + (long long)c * CHUNK_FLOATS + off + t * CH + x, true);
-            }
-    };
-    auto factors = [&](int c) {                                  // Gamma and L[CH-1][.] of chunk c
-        if (c < chunks && tid < 2 * CH / 4)
-            mma::cp_async16((uint32_t)__cvta_generic_to_shared(gam2 + (c & 1) * 2 * CH + tid * 4),
-                            chunk0 + (long long)c * CHUNK_FLOATS + 2 * CH * CH + tid * 4, true);
-    };
-    rows(kn, Kb, 0);
-    rows(qn, Qs, 0);
-    square(0, Ms, 0);
-    factors(0);
-    mma::cp_async_commit();
-    square(CH * CH, Ps, 0);
-    mma::cp_async_commit();
-    const int rg = lane >> 3, cg = lane & 7, ra = 4 * warp + rg, rb = 60 - 4 * warp + rg;
-    for (int c = 0; c < chunks; ++c) {
-        const float* Ks = Kb + (KB == 2 ? (c & 1) * CH * DP : 0);
-        const int t0 = c * CH;
-        const float *gam = gam2 + (c & 1) * 2 * CH, *last = gam + CH;
-        float v[2][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            v[0][i] = t0 + ra < n ? vn[((row0 + t0 + ra) * H + h) * Dv + col0 + cg + 8 * i] : 0.f;
-            v[1][i] = t0 + rb < n ? vn[((row0 + t0 + rb) * H + h) * Dv + col0 + cg + 8 * i] : 0.f;
-        }
-        mma::cp_async_wait<1>();               // everything but P
-        __syncthreads();
-        if (KB == 2) {
-            rows(kn, Kb + ((c + 1) & 1) * CH * DP, c + 1);
-            mma::cp_async_commit();
-        }
-        uint64_t acc[4][4] = {};               // K S of rows ra, rb; Q S of rows ra, rb
-#pragma unroll 1
-        for (int d0 = 0; d0 < D; d0 += 16) {   // sums of 16 first: half the rounding error of one long chain
-            uint64_t part[4][4] = {};
-#pragma unroll
-            for (int d = d0; d < d0 + 16; d += 4) {
-                const ulonglong2 a[4] = {ld_pairs(Ks + ra * DP + d), ld_pairs(Ks + rb * DP + d), ld_pairs(Qs + ra * DP + d),
-                                         ld_pairs(Qs + rb * DP + d)};
-                ulonglong2 sb[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) sb[j] = ld_pairs(Ss + (cg + 8 * j) * DP + d);
-                dot_step(part, a, sb);
-            }
-            add_pairs(acc, part);
-        }
-        const float ga = gam[ra], gb = gam[rb];
-        float o[2][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            Rs[(cg + 8 * i) * CP + ra] = fmaf(-ga, f2_lo(acc[0][i]) + f2_hi(acc[0][i]), v[0][i]);
-            Rs[(cg + 8 * i) * CP + rb] = fmaf(-gb, f2_lo(acc[1][i]) + f2_hi(acc[1][i]), v[1][i]);
-            o[0][i] = ga * (f2_lo(acc[2][i]) + f2_hi(acc[2][i]));
-            o[1][i] = gb * (f2_lo(acc[3][i]) + f2_hi(acc[3][i]));
-        }
-        __syncthreads();
-        rows(qn, Qs, c + 1);                   // the queries of this chunk have been used
-        mma::cp_async_commit();
-        // rows ra and rb of a lower triangular 64 x 64 matrix times the columns of X [32][CP]
-        auto triangular = [&](const float* M, const float* X, uint64_t (&y)[2][4]) {
-            const int e = 4 * warp, f = 60 - 4 * warp;           // the blocks of the diagonal: [e, e + 4) and [f, f + 4)
-#pragma unroll 1
-            for (int s0 = 0; s0 < f; s0 += 16) {                 // sums of 16 first, as above
-                uint64_t part[2][4] = {};
-#pragma unroll
-                for (int s = s0; s < s0 + 16; s += 4) {
-                    if (s >= f) break;
-                    const ulonglong2 a = ld_pairs(M + rb * CP + s);
-                    ulonglong2 xb[4];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        xb[j] = ld_pairs(X + (cg + 8 * j) * CP + s);
-                        part[1][j] = f2_fma(a.y, xb[j].y, f2_fma(a.x, xb[j].x, part[1][j]));
-                    }
-                    if (s >= e) continue;
-                    const ulonglong2 c = ld_pairs(M + ra * CP + s);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) part[0][j] = f2_fma(c.y, xb[j].y, f2_fma(c.x, xb[j].x, part[0][j]));
-                }
-                add_pairs(y, part);
-            }
-            // on the diagonal the entries behind the row's own are left out, not multiplied by zero: a token that is not a
-            // number does not reach the tokens before it
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const int row = half ? rb : ra, s = half ? f : e;
-                const float4 m = *reinterpret_cast<const float4*>(M + row * CP + s);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float4 x = *reinterpret_cast<const float4*>(X + (cg + 8 * j) * CP + s);
-                    float d = m.x * x.x;
-                    if (rg >= 1) d = fmaf(m.y, x.y, d);
-                    if (rg >= 2) d = fmaf(m.z, x.z, d);
-                    if (rg >= 3) d = fmaf(m.w, x.w, d);
-                    y[half][j] = f2_pack(f2_lo(y[half][j]) + d, f2_hi(y[half][j]));
-                }
-            }
-        };
-        uint64_t y[2][4] = {};
-        triangular(Ms, Rs, y);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            Us[(cg + 8 * i) * CP + ra] = f2_lo(y[0][i]) + f2_hi(y[0][i]);
-            Us[(cg + 8 * i) * CP + rb] = f2_lo(y[1][i]) + f2_hi(y[1][i]);
-        }
-        mma::cp_async_wait<KB>();              // P of this chunk (the groups behind it: Q and, with two buffers, K)
-        __syncthreads();
-        square(0, Ms, c + 1);
-        factors(c + 1);
-        mma::cp_async_commit();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) y[0][i] = y[1][i] = 0ull;
-        triangular(Ps, Rs, y);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            if (t0 + ra < n) orow[(long long)(t0 + ra) * H * Dv + cg + 8 * i] = o[0][i] + (f2_lo(y[0][i]) + f2_hi(y[0][i]));
-            if (t0 + rb < n) orow[(long long)(t0 + rb) * H * Dv + cg + 8 * i] = o[1][i] + (f2_lo(y[1][i]) + f2_hi(y[1][i]));
-        }
-        // S[.][j] <- Gamma S + sum_s last_s U[s][j] K[s][.]: DT key channels x 4 value columns per thread
-        {
-            const int d0 = ((warp & 3) * 8 + cg) * DT, j0 = (warp >> 2) * 16 + rg;       // columns j0 + 4 i
-            const uint64_t gl = f2_pack(gam[CH - 1], gam[CH - 1]);
-            uint64_t st[4][DT / 2] = {};       // the chunk's own part; the decayed state joins it once
-#pragma unroll 1
-            for (int s0 = 0; s0 < CH; s0 += 16) {
-                uint64_t part[4][DT / 2] = {};
-#pragma unroll 2
-                for (int s = s0; s < s0 + 16; s += 4) {
-                    float u[4][4], lw[4];
-                    *reinterpret_cast<float4*>(lw) = *reinterpret_cast<const float4*>(last + s);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        *reinterpret_cast<float4*>(u[i]) = *reinterpret_cast<const float4*>(Us + (j0 + 4 * i) * CP + s);
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        uint64_t kv[DT / 2];
-#pragma unroll
-                        for (int x = 0; x < DT / 2; ++x)
-                            kv[x] = *reinterpret_cast<const uint64_t*>(Ks + (s + q) * DP + d0 + 2 * x);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const float w = u[i][q] * lw[q];
-                            const uint64_t ww = f2_pack(w, w);
-#pragma unroll
-                            for (int x = 0; x < DT / 2; ++x) part[i][x] = f2_fma(kv[x], ww, part[i][x]);
-                        }
-                    }
-                }
-                add_pairs(st, part);
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int x = 0; x < DT / 2; ++x) {
-                    uint64_t* at = reinterpret_cast<uint64_t*>(Ss + (j0 + 4 * i) * DP + d0 + 2 * x);
-                    *at = f2_fma(*at, gl, st[i][x]);
-                }
-        }
-        __syncthreads();                       // K, P, U and the old state are free
-        if (KB == 1) rows(kn, Kb, c + 1);
-        mma::cp_async_commit();
-        square(CH * CH, Ps, c + 1);
-        mma::cp_async_commit();
-    }
-    for (int i = tid; i < D * CW_COLS; i += CW_THREADS) {
-        const int d = i / CW_COLS, j = i % CW_COLS;
-        Sb[(long long)d * Dv + j] = Ss[j * DP + d];
-    }
+// chunks of a step that are worked on at once: the operand tiles (147 to 344 KB per row, head and chunk) take half a gigabyte at most,
+// longer steps run in several launches
+int segment_chunks(int B, int Tn, int H, int D) {
+    const long long each = (long long)B * H * nxd_delta::chunk_tiles(D) * nxd_delta::TILE_BYTES;
+    const long long fit = (512ll << 20) / each;
+    return (int)max(1ll, min((long long)(Tn + CH - 1) / CH, fit));
 }
 
 template <int D>
-int launch_chunks(const float* qn, const float* kn, const float* vn, const float* gate, long long ld_a, int a_off,
-                  const float* beta, long long ld_b, int b_off, float* S, float* out, float* scratch, const int* q_start,
-                  const int* n_new, const int* seq_ids, int B, int Tn, int H, int G, int Dv, cudaStream_t st) {
-    constexpr int DP = D + 4;
-    const int NC = (Tn + CH - 1) / CH;
-    const size_t sys = (size_t)3 * CH * DPITCH * sizeof(double);
-    const size_t scan = (size_t)((D <= 128 ? 3 : 2) * CH * DP + CW_COLS * DP + 2 * CH * CP + 2 * CW_COLS * CP + 4 * CH) * sizeof(float);
-    static_assert((2 * CH * 260 + CW_COLS * 260 + 2 * CH * CP + 2 * CW_COLS * CP + 4 * CH) * 4 <= 232448, "shared memory");
-    NXD_CHECK_CUDA(cudaFuncSetAttribute(delta_chunk_system_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sys));
-    NXD_CHECK_CUDA(cudaFuncSetAttribute(delta_chunk_scan_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan));
-    delta_chunk_system_kernel<D><<<dim3(NC, H, B), CW_THREADS, sys, st>>>(qn, kn, gate, ld_a, a_off, beta, ld_b, b_off, scratch,
-                                                                          n_new, Tn, H, G);
-    NXD_LAUNCH_CHECK();
-    delta_chunk_scan_kernel<D><<<dim3(Dv / CW_COLS, H, B), CW_THREADS, scan, st>>>(qn, kn, vn, scratch, S, out, q_start, n_new,
-                                                                                  seq_ids, Tn, NC, H, G, Dv);
-    NXD_LAUNCH_CHECK();
+int launch_chunks(const nxd_delta::Step& p, const float* gate, long long ld_a, int a_off, const float* beta, long long ld_b, int b_off,
+                  float* scratch, cudaStream_t st) {
+    const int NC = (p.Tn + CH - 1) / CH, seg = segment_chunks(p.B, p.Tn, p.H, D);
+    const size_t smem = (size_t)3 * CH * DPITCH * sizeof(double);
+    uint8_t* tiles = reinterpret_cast<uint8_t*>(scratch);
+    float* systems = scratch + (long long)p.B * p.H * seg * (nxd_delta::chunk_tiles(D) * nxd_delta::TILE_BYTES / 4);
+    NXD_CHECK_CUDA(nxd_allow_smem<delta_chunk_system_kernel<D>>((int)smem));
+    for (int c0 = 0; c0 < NC; c0 += seg) {
+        const int count = min(seg, NC - c0);
+        delta_chunk_system_kernel<D><<<dim3(count, p.H, p.B), CW_THREADS, smem, st>>>(p.qn, p.kn, gate, ld_a, a_off, beta, ld_b, b_off,
+                                                                                     systems, p.n_new, p.Tn, c0, p.H, p.G);
+        NXD_LAUNCH_CHECK();
+        if (int rc = nxd_delta::launch_chunks_tc(p, systems, tiles, c0, count, st)) return rc;
+    }
     return 0;
 }
 
@@ -960,11 +731,10 @@ NXD_API int nxd_delta_conv_state(int dtype, const void* proj, long long ld, int 
 }
 
 // Floats of scratch with which nxd_delta_scan runs the chunk-wise form, 0 where it does not apply: one decay per head, key
-// sizes of 64 / 128 / 256, value sizes in whole slices of 32 columns, steps of at least three chunks (measured at 8 heads of 256 x
-// 512, token by token against chunks: 70 tokens 82 / 116 us, 128 tokens 113 / 117, 1024 tokens 610 / 374).
+// sizes of 64 / 128 / 256, value sizes in whole slices of 32 columns, steps of at least three chunks.
 NXD_API long long nxd_delta_scan_scratch(int B, int Tn, int H, int D, int Dv, int per_channel) {
     if (per_channel || (D != 64 && D != 128 && D != 256) || Dv % CW_COLS != 0 || Tn < 3 * CH || B > 65535 || H > 65535) return 0;
-    return (long long)B * H * ((Tn + CH - 1) / CH) * CHUNK_FLOATS;
+    return (long long)B * H * segment_chunks(B, Tn, H, D) * (CHUNK_FLOATS + nxd_delta::chunk_tiles(D) * nxd_delta::TILE_BYTES / 4);
 }
 
 // qn, kn, vn as written by nxd_delta_prep.  apre fp32 [B * Tn, ld_a]: decay pre-activation of head h at column a_off + h
@@ -988,14 +758,12 @@ NXD_API int nxd_delta_scan(const float* qn, const float* kn, const float* vn, fl
                                                                       N, H, per_head);
     NXD_LAUNCH_CHECK();
     auto al = [](const void* p) { return ((uintptr_t)p % 16) == 0; };
-    if (scratch != nullptr && nxd_delta_scan_scratch(B, Tn, H, D, Dv, per_channel) > 0 && al(qn) && al(kn) && al(scratch)) {
-#define NXD_CHUNKS(D_)                                                                                                  \
-    return launch_chunks<D_>(qn, kn, vn, apre, ld_a, a_off, bpre, ld_b, b_off, S, out, scratch, q_start, n_new, seq_ids, B, Tn, \
-                             H, G, Dv, st)
-        if (D == 64) NXD_CHUNKS(64);
-        if (D == 128) NXD_CHUNKS(128);
-        NXD_CHUNKS(256);
-#undef NXD_CHUNKS
+    if (scratch != nullptr && nxd_delta_scan_scratch(B, Tn, H, D, Dv, per_channel) > 0 && al(qn) && al(kn) && al(vn) && al(S) &&
+        al(out) && al(scratch)) {
+        const nxd_delta::Step step{qn, kn, vn, S, out, q_start, n_new, seq_ids, B, Tn, H, G, D, Dv};
+        if (D == 64) return launch_chunks<64>(step, apre, ld_a, a_off, bpre, ld_b, b_off, scratch, st);
+        if (D == 128) return launch_chunks<128>(step, apre, ld_a, a_off, bpre, ld_b, b_off, scratch, st);
+        return launch_chunks<256>(step, apre, ld_a, a_off, bpre, ld_b, b_off, scratch, st);
     }
     // rows of a column per thread (NPT) and lanes per column (R, a power of two): the smallest slice that keeps R <= 4,
     // wider keys spread over more lanes (measured at 8 heads of 256 x 512, 2 x 4096 tokens: slices of 32 / 16 / 8 rows take

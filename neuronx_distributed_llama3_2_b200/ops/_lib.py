@@ -58,7 +58,7 @@ GROUPS["hybrid_serving"] = ["window_attention.cu", "post_norm.cu", "latent_atten
 # the delta-rule hybrids (gated delta rule, differential window attention, dense and sparse gated feed-forward on a
 # gated parallel residual): the attention-over-cache, norm, sparse-MoE and recurrent-output kernels, the recurrence's
 # own source and the GEMM kernels behind the linear layers
-GROUPS["delta_serving"] = ["window_attention.cu", "post_norm.cu", "moe_sparse.cu", "moe_forward.cu", "mlstm.cu", "delta_rule.cu",
+GROUPS["delta_serving"] = ["window_attention.cu", "post_norm.cu", "moe_sparse.cu", "moe_forward.cu", "mlstm.cu", "delta_rule.cu", "delta_chunks.cu",
                            "runtime.cu", "gemm_tcgen05.cu", "gemm_smallm.cu", "fused_gemm_ar.cu", "tma_host.cu"]
 
 # the retention hybrids (softmax attention with sinks next to fixed-decay linear attention, several residual streams,
@@ -84,7 +84,7 @@ GROUPS["state_space_serving"] = ["window_attention.cu", "state_space.cu", "strea
                                  "flash_attn_tc.cu", "attn_tc_host.cu"]
 
 # sources whose fp32 state is carried over thousands of steps: no approximate exp / tanh / division
-PRECISE_SOURCES = {"mlstm.cu", "delta_rule.cu", "retention.cu", "retention_tc.cu", "hyper_connection.cu", "stream_norm.cu",
+PRECISE_SOURCES = {"mlstm.cu", "delta_rule.cu", "delta_chunks.cu", "retention.cu", "retention_tc.cu", "hyper_connection.cu", "stream_norm.cu",
                    "state_space.cu"}
 
 _lib: Optional[ctypes.CDLL] = None

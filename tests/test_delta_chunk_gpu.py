@@ -149,3 +149,27 @@ def test_strips_of_the_short_convolution_match_float64(dtype, D, H, G, Dv):
             assert (x32 - ref).norm() <= 1e-6 * ref.norm()          # four products and a silu in fp32
         at += size
     assert torch.equal(state[line.long()], raw[:, -3:, 8:8 + C].float())
+
+
+# operand tiles of half a gigabyte at most: eight rows of 32 heads take their seven chunks in two launches, a row alone in one
+def test_steps_in_several_launches_are_the_same():
+    from neuronx_distributed_llama3_2_b200.ops import delta_rule as dr
+
+    B, T, H, D, Dv = 8, 421, 32, 256, 32
+    gen = torch.Generator(device="cuda").manual_seed(2)
+
+    def normal(*s):
+        return torch.randn(*s, generator=gen, device="cuda")
+
+    q, k = (F.normalize(normal(B, T, H, D), dim=-1) for _ in range(2))
+    v, a_pre, b_pre, S = normal(B, T, H, Dv), normal(B * T, H), normal(B * T, H), normal(B, H, D, Dv)
+    a_log, dt_bias = normal(H) - 2, normal(H)
+    start = torch.ones(B, dtype=torch.int32, device="cuda")
+    new = torch.tensor([T, 400, 384, 385, 1, 0, 64, 200], dtype=torch.int32, device="cuda")
+    state = S.clone()
+    out = dr.delta_scan(q, k, v, a_pre.clone(), 0, b_pre.clone(), 0, a_log, dt_bias, state, start, False, n_new=new)
+    for b in range(B):
+        rows, one = slice(b * T, (b + 1) * T), S[b:b + 1].clone()
+        ref = dr.delta_scan(q[b:b + 1], k[b:b + 1], v[b:b + 1], a_pre[rows].clone(), 0, b_pre[rows].clone(), 0, a_log, dt_bias, one,
+                            start[:1], False, n_new=new[b:b + 1])
+        assert torch.equal(out[b], ref[0]) and torch.equal(state[b], one[0])
