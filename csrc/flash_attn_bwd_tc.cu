@@ -108,7 +108,7 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     uint64_t* dq_empty = st_full + 5;
     uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + L::kNumBars);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     // grid = (kv heads x splits, batch, K/V blocks): the block index is the SLOWEST launch dimension, so with a causal mask
     // the CTAs are handed to the SMs longest first (K/V block 0 meets every query tile, the last one only two)
     const int nbk = blockIdx.z, hkv = blockIdx.x / p.nsplit, split = blockIdx.x % p.nsplit, b = blockIdx.y;
@@ -148,7 +148,7 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     ptx::tcgen05_fence_before();
     __syncthreads();
     ptx::tcgen05_fence_after();
-    const uint32_t tmem_base = *tmem_ptr_smem;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_smem, 0);
 
     if (warp == 0) {
         // ============================ TMA producer ============================
@@ -187,7 +187,7 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         }
     } else if (warp == 1) {
         // ============================ MMA issuer ============================
-        if (lane == 0 && total > 0) {
+        if (total > 0 && ptx::elect_one()) {
             constexpr uint32_t idesc_st = ptx::make_idesc_bf16(kBN, kBM, 0, 0);   // S^T, dP^T: 128 x 64, K-major A/B
             constexpr uint32_t idesc_kv = ptx::make_idesc_bf16(kBN, kD, 0, 1);    // dV, dK: 128 x 128, B MN-major
             constexpr uint32_t idesc_dq = ptx::make_idesc_bf16(128, kBM, 1, 1);   // dQ^T: 128 x 64, A and B MN-major

@@ -104,7 +104,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     uint64_t* pv_done = p_full + 1;
     uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(pv_done + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     // grid = (q heads, batch, q blocks): the q block is the slowest launch dimension and counted from the end, so the
     // long causal rows of EVERY head are scheduled before any short one (longest-first list scheduling)
     const int mb = gridDim.z - 1 - blockIdx.z;
@@ -158,7 +158,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     ptx::tcgen05_fence_before();
     __syncthreads();
     ptx::tcgen05_fence_after();
-    const uint32_t tmem_base = *tmem_ptr_smem;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_smem, 0);
     const uint32_t tmem_o = tmem_base;
     const uint32_t tmem_s = tmem_base + D;
     const uint32_t tmem_p = tmem_base + D + kBN;   // 128 lanes x 64 keys bf16 = 32 packed columns
@@ -224,7 +224,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         }
     } else if (warp == 1) {
         // ============================ MMA issuer ============================
-        if (lane == 0 && n_tiles > 0) {
+        if (n_tiles > 0 && ptx::elect_one()) {
             constexpr uint32_t idesc_s = ptx::make_idesc_bf16(kBM, kBN, 0, 0);
             constexpr uint32_t idesc_o = ptx::make_idesc_bf16(kBM, D, 0, 1);
             const uint32_t q_addr = ptx::smem_u32(sQ), ring_addr = ptx::smem_u32(sRing);

@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
     float* staging = reinterpret_cast<float*>(smem + C::kPipeBytes);      // receive buffer
     float* sendbuf = reinterpret_cast<float*>(smem);                      // aliases the pipeline
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int split = splits > 1 ? (int)ptx::cluster_ctarank() : 0;
     const int n0 = (blockIdx.x / splits) * kWRows;      // first weight row of the slab (SwiGLU: of the gate slab)
     const int nkb = (K + kBK - 1) / kBK;
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
     // now and waits for it after its main loop (measured: a full cluster barrier here costs ~1 us of start-up)
     if (splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     ptx::tcgen05_fence_after();
-    const uint32_t tmem_base = *tmem_ptr_smem;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_smem, 0);
     TRACE_STAMP(1, threadIdx.x == 0);
 
     if (warp == 0) {
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
         __syncwarp();
         if (splits > 1) cluster_wait();
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (ptx::elect_one()) {
             constexpr uint32_t idesc = ptx::make_idesc_bf16(kWRows, BT, 0, 0);
             int stage = 0;
             uint32_t phase = 0;

@@ -51,7 +51,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     uint64_t* tmem_empty_bar = tmem_full_bar + kAccStages;
     uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(tmem_empty_bar + kAccStages);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const int lane = threadIdx.x & 31;
     const uint32_t cta_rank = ptx::cluster_ctarank();
     const bool is_leader = cta_rank == 0;
@@ -91,7 +91,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     ptx::tcgen05_fence_before();
     ptx::cluster_sync();
     ptx::tcgen05_fence_after();
-    const uint32_t tmem_base = *tmem_ptr_smem;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_smem, 0);
     if constexpr (kSorted) num_tiles = seg_tile[batches];
     // problem index, tile coordinates and first row of a tile
     auto locate = [&](int tile, int& e, int& tm, int& tn, int& row_base) {
@@ -153,7 +153,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
     } else if (warp == 1) {
         // ======================= MMA issuer (leader CTA) =======================
-        if (is_leader && lane == 0) {
+        if (is_leader && ptx::elect_one()) {
             constexpr uint32_t idesc = ptx::make_idesc_bf16(kTileM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
             // K-major: 8-row groups 1024 B apart; step 32 B per UMMA_K inside the 128 B swizzle row.
             // MN-major: 64-element MN groups kBlockK*128 B apart (LBO), 8-k-row groups 1024 B apart

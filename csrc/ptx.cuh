@@ -20,6 +20,9 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// One thread of a converged warp.  A role that issues MMAs takes it, in a branch on a warp number that the compiler knows to be uniform
+// (__shfl_sync): under `threadIdx.x == n` every tcgen05.mma costs 50 to 100 clocks of issue, here 35 or less (an MMA of 128 x 64 x
+// 16 runs for 49).  Attention backward, 8192 tokens, 24 heads of 128: 1079 -> 904 us; forward 356 -> 333.
 __device__ __forceinline__ bool elect_one() {
     uint32_t pred = 0;
     asm volatile(
