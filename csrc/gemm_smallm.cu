@@ -61,24 +61,34 @@ struct EpiArgs {
     CacheDst cache;
     int n_q, n_kv, D;
     int up_row0;               // SwiGLU: first "up" row of w (= I)
+    // NORM: the activations before their RMSNorm, its weight and epsilon
+    const bf16* raw;
+    long long ld_raw;
+    const bf16* norm_w;
+    float eps;
 };
 
-template <int BT, int EPI>
+// NORM: the epilogue warps, which have nothing to do while the weights stream, normalise the CTA's slice of the activations into
+// shared memory themselves (every CTA sums the squares of the whole rows: 4 KB a row from L2), instead of a kernel between this one and
+// the one before.  A norm launch costs a token step 2.6 us; 16 rows of 2048 are the most that cost less here.
+template <int BT, int EPI, bool NORM>
 struct Cfg {
     static constexpr int kAcc = EPI == kEpiSwiglu ? 2 : 1;           // accumulators (weight slabs) per CTA
     static constexpr int kWBytes = kAcc * kWRows * kBK * 2;          // 16 / 32 KB
-    static constexpr int kXBytes = BT * kBK * 2;                     // 2 .. 16 KB
+    static constexpr int kXBytes = NORM ? 0 : BT * kBK * 2;          // 2 .. 16 KB
     static constexpr int kStageBytes = kWBytes + kXBytes;
     // one accumulator: pipeline + staging <= ~110 KB -> two CTAs per SM (BT = 128: one CTA, deeper pipeline);
     // two accumulators: one CTA per SM with 128-160 KB of weights in flight
-    static constexpr int kStages = kAcc == 2 ? (BT <= 32 ? 5 : 4) : (BT == 16 ? 5 : BT == 32 ? 4 : BT == 64 ? 3 : 4);
+    static constexpr int kStages = kAcc == 2 ? (BT <= 32 ? 5 : 4) : (BT == 16 ? (NORM ? 4 : 5) : BT == 32 ? 4 : BT == 64 ? 3 : 4);
     static constexpr int kPipeBytes = kStages * kStageBytes;
     // receive buffer, fp32 [accumulator][slot = source rank * tokens_per_rank + local token][128]; NOT aliased with the
     // pipeline: peers copy into it while this CTA may still be streaming.  The send buffer (same size, [accumulator]
     // [owner][local token][128]) aliases the pipeline stages, which are dead once the last MMA has retired.
     static constexpr int kStagingBytes = kAcc * BT * kWRows * 4;
     static constexpr int kBarOffset = kPipeBytes + kStagingBytes;
-    static constexpr int kSmemBytes = kBarOffset + (2 * kStages + 2) * 8 + 16 + 1024;
+    static constexpr int kNormOffset = kBarOffset + 1024;            // NORM: the slice, 64 columns of all rows after one another
+    static constexpr int kSmemBytes = NORM ? kNormOffset + 1024 : kBarOffset + (2 * kStages + 2) * 8 + 16 + 1024;
+    static constexpr int kNormBlocks = NORM ? (232448 - kSmemBytes) / (BT * kBK * 2) : 0;
     static_assert(kStagingBytes <= kPipeBytes, "the send buffer aliases the pipeline stages");
     static constexpr int kTmemCols = kAcc * BT < 32 ? 32 : kAcc * BT;
     static_assert(kStageBytes % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
@@ -113,18 +123,19 @@ __device__ long long g_smallm_trace[16];
 #define TRACE_STAMP(i, cond) do { } while (0)
 #endif
 
-template <int BT, int EPI>
+template <int BT, int EPI, bool NORM>
 __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w,
                                                               const __grid_constant__ CUtensorMap tmap_x,
                                                               const EpiArgs ep, int B, int N, int K, int splits) {
-    using C = Cfg<BT, EPI>;
+    using C = Cfg<BT, EPI, NORM>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = ptx::align_smem_1024(smem_raw);
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + C::kBarOffset);
     uint64_t* empty_bar = full_bar + C::kStages;
     uint64_t* acc_bar = empty_bar + C::kStages;
     uint64_t* recv_bar = acc_bar + 1;
-    uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(recv_bar + 1);
+    uint64_t* norm_bar = recv_bar + 1;
+    uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(norm_bar + (NORM ? 1 : 0));
     float* staging = reinterpret_cast<float*>(smem + C::kPipeBytes);      // receive buffer
     float* sendbuf = reinterpret_cast<float*>(smem);                      // aliases the pipeline
 
@@ -150,7 +161,7 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
             ptx::tma_load_2d(&tmap_w, &full_bar[stage], sw + kWRows * kBK * 2, kb * kBK, ep.up_row0 + n0);
     };
     auto load_x = [&](int kb, int stage) {
-        ptx::tma_load_2d(&tmap_x, &full_bar[stage], smem + stage * C::kStageBytes + C::kWBytes, kb * kBK, 0);
+        if (!NORM) ptx::tma_load_2d(&tmap_x, &full_bar[stage], smem + stage * C::kStageBytes + C::kWBytes, kb * kBK, 0);
     };
     const int pre = min(C::kStages, kb_end - kb_begin);
     if (warp == 0 && lane == 0) {
@@ -162,6 +173,7 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
         }
         ptx::mbar_init(acc_bar, 1);
         ptx::mbar_init(recv_bar, 1);
+        if (NORM) ptx::mbar_init(norm_bar, 128);
         ptx::fence_barrier_init();
         // every CTA of the cluster sends this one a [tpr][128] fp32 block per accumulator
         if (splits > 1 && split * tpr < B) ptx::mbar_arrive_expect_tx(recv_bar, (uint32_t)(splits * C::kAcc * tpr * kWRows * 4));
@@ -179,7 +191,7 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
 
     if (warp == 0) {
         if (lane == 0) {
-            pdl_wait();         // the activations come from the previous kernel (programmatic dependent launch)
+            if (!NORM) pdl_wait();      // the activations come from the previous kernel (programmatic dependent launch)
             TRACE_STAMP(2, true);
             for (int i = 0; i < pre; ++i) load_x(kb_begin + i, i);
             int stage = pre == C::kStages ? 0 : pre;
@@ -196,6 +208,7 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
     } else if (warp == 1) {
         if (ptx::elect_one()) {
             constexpr uint32_t idesc = ptx::make_idesc_bf16(kWRows, BT, 0, 0);
+            if (NORM) ptx::mbar_wait(norm_bar, 0);
             int stage = 0;
             uint32_t phase = 0;
             for (int kb = kb_begin; kb < kb_end; ++kb) {
@@ -203,7 +216,7 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
                 TRACE_STAMP(3, kb == kb_begin);
                 ptx::tcgen05_fence_after();
                 const uint32_t sw = ptx::smem_u32(smem + stage * C::kStageBytes);
-                const uint32_t sx = sw + C::kWBytes;
+                const uint32_t sx = NORM ? ptx::smem_u32(smem + C::kNormOffset) + (kb - kb_begin) * (BT * kBK * 2) : sw + C::kWBytes;
 #pragma unroll
                 for (int k = 0; k < kBK / 16; ++k) {
                     const uint64_t db = ptx::make_smem_desc(sx + k * 32, 16, 1024);
@@ -227,7 +240,52 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
         // no split-K, else into the send buffer [owner][local token][128]; consecutive lanes = consecutive n:
         // conflict-free 128-byte rows per warp store
         const int q = warp & 3;
+        const int row8 = (kb_end - kb_begin) * (kBK / 8), t = threadIdx.x - 64;     // NORM: vectors of a row in this CTA's slice
+        auto norm_w = [&](int c) {                                             // (zeros behind the end of the rows)
+            const int k = kb_begin * kBK + c * 8;
+            return c < row8 && k < K ? *reinterpret_cast<const uint4*>(ep.norm_w + k) : make_uint4(0u, 0u, 0u, 0u);
+        };
+        uint4 w0, w1;                                                          // the first ones do not wait for the kernel before
+        if constexpr (NORM) w0 = norm_w(t), w1 = norm_w(t + 128);
         pdl_wait();     // the epilogue reads the residual / positions and writes global memory
+        if constexpr (NORM) {
+            float (*red)[BT] = reinterpret_cast<float (*)[BT]>(smem + C::kBarOffset + 512);
+            float ss[BT] = {};
+            for (int c = t; c < K / 8; c += 128) {
+#pragma unroll
+                for (int b = 0; b < BT; ++b) {
+                    if (b >= B) break;
+                    float f[8];
+                    unpack8(*reinterpret_cast<const bf16x8*>(ep.raw + b * ep.ld_raw + c * 8), f);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) ss[b] = fmaf(f[e], f[e], ss[b]);
+                }
+            }
+#pragma unroll
+            for (int b = 0; b < BT; ++b) {
+                if (b >= B) break;
+                ss[b] = warp_sum(ss[b]);
+                if (lane == 0) red[q][b] = ss[b];
+            }
+            epilogue_bar();
+            for (int c = t, i = 0; c < row8; c += 128, ++i) {
+                const uint4 wv = i == 0 ? w0 : i == 1 ? w1 : norm_w(c);
+                const int k = min(kb_begin * kBK + c * 8, K - 8);
+                float w[8];
+                unpack8(*reinterpret_cast<const bf16x8*>(&wv), w);
+                for (int b = 0; b < B; ++b) {
+                    const float rstd = rsqrtf((red[0][b] + red[1][b] + red[2][b] + red[3][b]) / (float)K + ep.eps);
+                    float f[8];
+                    unpack8(*reinterpret_cast<const bf16x8*>(ep.raw + b * ep.ld_raw + k), f);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) f[e] = kb_begin * kBK + c * 8 < K ? f[e] * rstd * w[e] : 0.f;
+                    *reinterpret_cast<bf16x8*>(smem + C::kNormOffset + (c >> 3) * (BT * kBK * 2) + b * 128 +
+                                               (((c & 7) ^ (b & 7)) << 4)) = pack8(f);
+                }
+            }
+            ptx::fence_proxy_async();
+            ptx::mbar_arrive(norm_bar);
+        }
         ptx::mbar_wait(acc_bar, 0);
         TRACE_STAMP(5, threadIdx.x == 64);
         ptx::tcgen05_fence_after();
@@ -421,17 +479,18 @@ int pick_splits(int n_tiles, int nkb, int ctas_per_sm) {
     return s;
 }
 
-template <int BT, int EPI>
+template <int BT, int EPI, bool NORM = false>
 int launch(const CUtensorMap& tw, const CUtensorMap& tx, const EpiArgs& ep, int B, int N, int K, int splits,
            cudaStream_t stream) {
-    using C = Cfg<BT, EPI>;
-    constexpr auto kern = gemm_smallm_kernel<BT, EPI>;
-    NXD_CHECK_CUDA(nxd_allow_smem<kern>(C::kSmemBytes));
+    using C = Cfg<BT, EPI, NORM>;
+    constexpr auto kern = gemm_smallm_kernel<BT, EPI, NORM>;
+    NXD_CHECK_CUDA(nxd_allow_smem<kern>(NORM ? 232448 : C::kSmemBytes));
     const int n_tiles = (N + kWRows - 1) / kWRows;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(n_tiles * splits));
     cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = C::kSmemBytes;
+    const int slice = NORM ? (((K + kBK - 1) / kBK + splits - 1) / splits) * BT * kBK * 2 : 0;
+    cfg.dynamicSmemBytes = C::kSmemBytes + slice;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -447,6 +506,17 @@ int launch(const CUtensorMap& tw, const CUtensorMap& tx, const EpiArgs& ep, int 
     return 0;
 }
 
+int choose_splits(int splits, int bt, int epi, int n_tiles, int nkb) {
+    if (splits > 0) return splits;
+    static const int forced = [] {      // NXD_SMALLM_SPLITS=1|2|4|8: debugging / tuning override of the heuristic
+        const char* e = getenv("NXD_SMALLM_SPLITS");
+        return e != nullptr ? atoi(e) : 0;
+    }();
+    splits = forced > 0 ? forced : pick_splits(n_tiles, nkb, (epi == kEpiSwiglu || bt == 128) ? 1 : 2);
+    while (splits > 1 && nkb / splits < 1) splits >>= 1;
+    return splits;
+}
+
 // n_rows: weight rows covered by the grid (N, or I for SwiGLU); w_rows: rows of the weight tensor map
 template <int EPI>
 int run(const void* x, const void* w, const EpiArgs& ep, int B, int n_rows, int w_rows, int K, long long ldx,
@@ -458,14 +528,7 @@ int run(const void* x, const void* w, const EpiArgs& ep, int B, int n_rows, int 
     NXD_REQUIRE(((uintptr_t)x & 15) == 0 && ((uintptr_t)w & 15) == 0, "gemm_smallm: operands must be 16-byte aligned");
     const int bt = B <= 16 ? 16 : B <= 32 ? 32 : B <= 64 ? 64 : 128;
     const int n_tiles = (n_rows + kWRows - 1) / kWRows, nkb = (K + kBK - 1) / kBK;
-    if (splits <= 0) {
-        static const int forced = [] {      // NXD_SMALLM_SPLITS=1|2|4|8: debugging / tuning override of the heuristic
-            const char* e = getenv("NXD_SMALLM_SPLITS");
-            return e != nullptr ? atoi(e) : 0;
-        }();
-        splits = forced > 0 ? forced : pick_splits(n_tiles, nkb, (EPI == kEpiSwiglu || bt == 128) ? 1 : 2);
-        while (splits > 1 && nkb / splits < 1) splits >>= 1;
-    }
+    splits = choose_splits(splits, bt, EPI, n_tiles, nkb);
     NXD_REQUIRE(splits == 1 || splits == 2 || splits == 4 || splits == 8, "gemm_smallm: splits=%d", splits);
     CUtensorMap tw, tx;
     int rc = make_tmap_2d(&tw, w, (uint64_t)K, (uint64_t)w_rows, (uint64_t)ldw, kBK, kWRows);
@@ -480,6 +543,49 @@ int run(const void* x, const void* w, const EpiArgs& ep, int B, int n_rows, int 
             if constexpr (EPI == kEpiSwiglu) return -1;
             else return launch<128, EPI>(tw, tx, ep, B, n_rows, K, splits, st);
     }
+}
+
+int qkv_args(EpiArgs& ep, const float* cos_t, const float* sin_t, const int* positions, void* q_out, void* cache_k, void* cache_v,
+             const int* seq_ids, const int* block_table, long long stride_b, long long stride_h, int page_size, int max_pages, int n_q,
+             int n_kv, int D) {
+    NXD_REQUIRE(D == 64 || D == 128, "smallm_qkv: head dim %d not in {64, 128}", D);
+    NXD_REQUIRE(((uintptr_t)q_out & 15) == 0 && ((uintptr_t)cache_k & 15) == 0 && ((uintptr_t)cache_v & 15) == 0 &&
+                    stride_b % 8 == 0 && stride_h % 8 == 0,
+                "smallm_qkv: q_out / cache must be 16-byte aligned with strides that are multiples of 8");
+    ep.cos_t = cos_t;
+    ep.sin_t = sin_t;
+    ep.positions = positions;
+    ep.q_out = (bf16*)q_out;
+    ep.cache = CacheDst{(bf16*)cache_k, (bf16*)cache_v, block_table, seq_ids, stride_b, stride_h,
+                        page_size > 0 ? page_size : 1, max_pages};
+    ep.n_q = n_q;
+    ep.n_kv = n_kv;
+    ep.D = D;
+    return 0;
+}
+
+// Behind an RMSNorm of up to 16 rows: the splits, 0 where a CTA's slice of the rows does not fit shared memory
+template <int EPI>
+int norm_splits(int B, int n_rows, int K) {
+    if (B > 16) return 0;
+    const int nkb = (K + kBK - 1) / kBK, s = choose_splits(0, 16, EPI, (n_rows + kWRows - 1) / kWRows, nkb);
+    return (nkb + s - 1) / s <= Cfg<16, EPI, true>::kNormBlocks ? s : 0;
+}
+
+template <int EPI>
+int run_norm(const void* x, long long ldx, const void* norm_w, float eps, const void* w, EpiArgs& ep, int B, int n_rows, int w_rows,
+             int K, long long ldw, cudaStream_t st) {
+    const int splits = B >= 1 ? norm_splits<EPI>(B, n_rows, K) : 0;
+    NXD_REQUIRE(splits > 0, "gemm_smallm: %d rows of %d columns do not fit behind a norm", B, K);
+    NXD_REQUIRE(K % 8 == 0 && ldx % 8 == 0 && ldw % 8 == 0 && (((uintptr_t)x | (uintptr_t)w | (uintptr_t)norm_w) & 15) == 0,
+                "gemm_smallm: K=%d and the row pitches must be multiples of 8, operands 16-byte aligned", K);
+    ep.raw = (const bf16*)x;
+    ep.ld_raw = ldx;
+    ep.norm_w = (const bf16*)norm_w;
+    ep.eps = eps;
+    CUtensorMap tw;
+    if (int rc = make_tmap_2d(&tw, w, (uint64_t)K, (uint64_t)w_rows, (uint64_t)ldw, kBK, kWRows)) return rc;
+    return launch<16, EPI, true>(tw, tw, ep, B, n_rows, K, splits, st);
 }
 
 }  // namespace
@@ -504,22 +610,42 @@ NXD_API int nxd_smallm_qkv_rope_cache(const void* x, long long ldx, const void* 
                                       void* cache_v, const int* seq_ids, const int* block_table, long long stride_b,
                                       long long stride_h, int page_size, int max_pages, int B, int K, int n_q, int n_kv,
                                       int D, int splits, void* stream) {
-    NXD_REQUIRE(D == 64 || D == 128, "smallm_qkv: head dim %d not in {64, 128}", D);
-    NXD_REQUIRE(((uintptr_t)q_out & 15) == 0 && ((uintptr_t)cache_k & 15) == 0 && ((uintptr_t)cache_v & 15) == 0 &&
-                    stride_b % 8 == 0 && stride_h % 8 == 0,
-                "smallm_qkv: q_out / cache must be 16-byte aligned with strides that are multiples of 8");
     EpiArgs ep = {};
-    ep.cos_t = cos_t;
-    ep.sin_t = sin_t;
-    ep.positions = positions;
-    ep.q_out = (bf16*)q_out;
-    ep.cache = CacheDst{(bf16*)cache_k, (bf16*)cache_v, block_table, seq_ids, stride_b, stride_h,
-                        page_size > 0 ? page_size : 1, max_pages};
-    ep.n_q = n_q;
-    ep.n_kv = n_kv;
-    ep.D = D;
+    if (int rc = qkv_args(ep, cos_t, sin_t, positions, q_out, cache_k, cache_v, seq_ids, block_table, stride_b, stride_h, page_size,
+                          max_pages, n_q, n_kv, D))
+        return rc;
     const int N = (n_q + 2 * n_kv) * D;
     return run<kEpiQkvRope>(x, w, ep, B, N, N, K, ldx, ldw, splits, (cudaStream_t)stream);
+}
+
+// Whether the two entries below take B rows before an RMSNorm over K columns: q | k | v rows (gate_up 0) or I gate rows (1).
+NXD_API int nxd_smallm_norm_applies(int gate_up, int B, int K, int n_rows) {
+    return (gate_up ? norm_splits<kEpiSwiglu>(B, n_rows, K) : norm_splits<kEpiQkvRope>(B, n_rows, K)) > 0;
+}
+
+// nxd_smallm_qkv_rope_cache and nxd_smallm_gate_up_swiglu of rmsnorm(x) * norm_w, the norm inside: 1 <= B <= 16.
+NXD_API int nxd_smallm_norm_qkv_rope_cache(const void* x, long long ldx, const void* norm_w, float eps, const void* w,
+                                           long long ldw, const float* cos_t, const float* sin_t, const int* positions,
+                                           void* q_out, void* cache_k, void* cache_v, const int* seq_ids,
+                                           const int* block_table, long long stride_b, long long stride_h, int page_size,
+                                           int max_pages, int B, int K, int n_q, int n_kv, int D, void* stream) {
+    EpiArgs ep = {};
+    if (int rc = qkv_args(ep, cos_t, sin_t, positions, q_out, cache_k, cache_v, seq_ids, block_table, stride_b, stride_h, page_size,
+                          max_pages, n_q, n_kv, D))
+        return rc;
+    const int N = (n_q + 2 * n_kv) * D;
+    return run_norm<kEpiQkvRope>(x, ldx, norm_w, eps, w, ep, B, N, N, K, ldw, (cudaStream_t)stream);
+}
+
+NXD_API int nxd_smallm_norm_gate_up_swiglu(const void* x, long long ldx, const void* norm_w, float eps, const void* w,
+                                           long long ldw, void* out, long long ldo, int B, int K, int I, void* stream) {
+    NXD_REQUIRE(I % 8 == 0 && ldo % 8 == 0 && ((uintptr_t)out & 15) == 0,
+                "smallm_gate_up: I=%d and ldo must be multiples of 8, out 16-byte aligned", I);
+    EpiArgs ep = {};
+    ep.out = (bf16*)out;
+    ep.ldo = ldo;
+    ep.up_row0 = I;
+    return run_norm<kEpiSwiglu>(x, ldx, norm_w, eps, w, ep, B, I, 2 * I, K, ldw, (cudaStream_t)stream);
 }
 
 // out[B, I] = silu(x W_gate^T) * (x W_up^T); w: [2 I, K] with the gate rows first.  B <= 64, I % 8 == 0.

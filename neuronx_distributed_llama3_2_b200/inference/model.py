@@ -219,7 +219,8 @@ class KVCacheInferenceMixin:
                    and streams_on_tensor_cores(hidden.shape[0], *w.shape) for w in ws)
 
     def _layer_batched_decode(self, i: int, layer, hidden, residual, positions, seq_ids, lengths):
-        """One token per sequence for up to 128 sequences on the small-M tensor-core kernels (``csrc/gemm_smallm.cu``):
+        """One token per sequence for up to 128 sequences on the small-M tensor-core kernels (``csrc/gemm_smallm.cu``); up to 16
+        sequences have both RMSNorms inside the projections behind them, six launches.  More of them:
         RMSNorm | QKV GEMM+RoPE+cache write | attention (split, merge) | o_proj+residual | RMSNorm | gate/up+SwiGLU |
         down_proj+residual -- eight launches, no copies between them.  Tensor parallel: the two row-parallel GEMMs are
         followed by the one-shot all-reduce and the residual moves into the fused add+RMSNorm (ten launches)."""
@@ -241,16 +242,27 @@ class KVCacheInferenceMixin:
         ck, cv = self.kv_cache.layer(i)
         kc = self.kv_cache
         pos, sid = self._decode_i32(positions, seq_ids)
-        xn, x = self._add_norm(layer.input_layernorm, hidden.reshape(B, -1),
-                               residual.reshape(B, -1) if residual is not None else None)
-        q = decode_fused.qkv_rope_cache_batched(xn, attn.qkv_proj.weight_qkv, cos, sin, pos, ck, cv, nq, nkv, D,
-                                                seq_ids=sid, block_table=kc.block_table if kc.paged else None,
-                                                page_size=kc.page_size if kc.paged else 0)
+        place = dict(seq_ids=sid, block_table=kc.block_table if kc.paged else None, page_size=kc.page_size if kc.paged else 0)
+
+        def norm_inside(norm, y, w, gate_up):
+            return (tp == 1 and norm.weight.dtype == torch.bfloat16 and norm.weight.is_contiguous()
+                    and norm.weight.data_ptr() % 16 == 0 and decode_fused.norm_fits(y, w, gate_up))
+
+        norm, x = layer.input_layernorm, hidden.reshape(B, -1)
+        if residual is None and norm_inside(norm, x, attn.qkv_proj.weight_qkv, False):
+            q = decode_fused.norm_qkv_rope_cache(x, norm.weight, norm.variance_epsilon, attn.qkv_proj.weight_qkv, cos, sin, pos, ck,
+                                                 cv, nq, nkv, D, **place)
+        else:
+            xn, x = self._add_norm(norm, x, residual.reshape(B, -1) if residual is not None else None)
+            q = decode_fused.qkv_rope_cache_batched(xn, attn.qkv_proj.weight_qkv, cos, sin, pos, ck, cv, nq, nkv, D, **place)
         o = self._decode_attention(q, ck, cv, seq_ids, lengths).reshape(B, nq * D)
         if tp == 1:
             x2 = gemm_smallm(o, attn.o_proj.weight, residual=x)
-            xn2 = norm_ops.rms_norm(x2, layer.post_attention_layernorm.weight,
-                                    layer.post_attention_layernorm.variance_epsilon)
+            norm = layer.post_attention_layernorm
+            if norm_inside(norm, x2, mlp.gate_up_proj.weight, True):
+                act = decode_fused.norm_gate_up_swiglu(x2, norm.weight, norm.variance_epsilon, mlp.gate_up_proj.weight)
+                return gemm_smallm(act, mlp.down_proj.weight, residual=x2).reshape(B, 1, -1), None
+            xn2 = norm_ops.rms_norm(x2, norm.weight, norm.variance_epsilon)
         else:
             xn2, x2 = self._add_norm(layer.post_attention_layernorm, all_reduce(gemm_smallm(o, attn.o_proj.weight)), x)
         if B <= decode_fused.BATCHED_SWIGLU_MAX_ROWS:

@@ -84,6 +84,49 @@ def qkv_rope_cache_batched(xn: torch.Tensor, w_qkv: torch.Tensor, cos: torch.Ten
     return q
 
 
+def norm_fits(x: torch.Tensor, w: torch.Tensor, gate_up: bool) -> bool:
+    """Whether ``norm_qkv_rope_cache`` / ``norm_gate_up_swiglu`` take these rows: at most 16, a CTA's slice of them in its shared
+    memory (all widths up to 3072, wider ones where the contraction is split further)."""
+    B, K = x.shape
+    return (B <= 16 and K % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and bool(
+        _lib.lib().nxd_smallm_norm_applies(_c.c_int(int(gate_up)), _c.c_int(B), _c.c_int(K),
+                                           _c.c_int(w.shape[0] // 2 if gate_up else w.shape[0]))))
+
+
+def norm_qkv_rope_cache(x: torch.Tensor, norm_w: torch.Tensor, eps: float, w_qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor,
+                        positions: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Tensor, n_q: int, n_kv: int, D: int,
+                        seq_ids: Optional[torch.Tensor] = None, block_table: Optional[torch.Tensor] = None,
+                        page_size: int = 0) -> torch.Tensor:
+    """``qkv_rope_cache_batched`` of ``rmsnorm(x) * norm_w`` for up to 16 rows: the projection's kernel normalises its rows itself
+    (``nxd_smallm_norm_qkv_rope_cache``)."""
+    B, K = x.shape
+    assert w_qkv.shape == ((n_q + 2 * n_kv) * D, K) and w_qkv.stride(1) == 1 and norm_w.is_contiguous()
+    assert positions.dtype == torch.int32 and cos.dtype == torch.float32 and cos.shape[1] == D // 2
+    q = torch.empty((B, n_q, D), dtype=torch.bfloat16, device=x.device)
+    rc = _lib.lib().nxd_smallm_norm_qkv_rope_cache(
+        _lib.ptr(x), _c.c_longlong(x.stride(0)), _lib.ptr(norm_w), _c.c_float(eps), _lib.ptr(w_qkv),
+        _c.c_longlong(w_qkv.stride(0)), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(positions), _lib.ptr(q), _lib.ptr(cache_k),
+        _lib.ptr(cache_v), _lib.ptr(seq_ids), _lib.ptr(block_table), _c.c_longlong(cache_k.stride(0)),
+        _c.c_longlong(cache_k.stride(1)), _c.c_int(page_size), _c.c_int(block_table.shape[1] if block_table is not None else 0),
+        _c.c_int(B), _c.c_int(K), _c.c_int(n_q), _c.c_int(n_kv), _c.c_int(D), _lib.stream_ptr())
+    _lib.check(rc, "nxd_smallm_norm_qkv_rope_cache")
+    return q
+
+
+def norm_gate_up_swiglu(x: torch.Tensor, norm_w: torch.Tensor, eps: float, w_gate_up: torch.Tensor) -> torch.Tensor:
+    """``gate_up_swiglu_batched`` of ``rmsnorm(x) * norm_w`` for up to 16 rows (``nxd_smallm_norm_gate_up_swiglu``)."""
+    B, K = x.shape
+    I = w_gate_up.shape[0] // 2
+    assert w_gate_up.shape[1] == K and w_gate_up.stride(1) == 1 and I % 8 == 0 and norm_w.is_contiguous()
+    out = torch.empty((B, I), dtype=torch.bfloat16, device=x.device)
+    rc = _lib.lib().nxd_smallm_norm_gate_up_swiglu(
+        _lib.ptr(x), _c.c_longlong(x.stride(0)), _lib.ptr(norm_w), _c.c_float(eps), _lib.ptr(w_gate_up),
+        _c.c_longlong(w_gate_up.stride(0)), _lib.ptr(out), _c.c_longlong(out.stride(0)), _c.c_int(B), _c.c_int(K), _c.c_int(I),
+        _lib.stream_ptr())
+    _lib.check(rc, "nxd_smallm_norm_gate_up_swiglu")
+    return out
+
+
 def gate_up_swiglu_batched(xn: torch.Tensor, w_gate_up: torch.Tensor, splits: int = 0) -> torch.Tensor:
     """``silu(xn W_gate^T) * (xn W_up^T)`` for ``xn [B, H]``, ``B <= 64``; ``w_gate_up [2 I, H]`` gate rows first: one
     launch with two accumulators per CTA (``nxd_smallm_gate_up_swiglu``)."""

@@ -55,3 +55,29 @@ def test_token_step_matches_the_fma_kernels(batch, paged, monkeypatch):
 @pytest.mark.parametrize("paged", [False, True])
 def test_one_sequence_matches_the_fma_kernels(paged, monkeypatch):
     test_token_step_matches_the_fma_kernels(1, paged, monkeypatch)
+
+
+@pytest.mark.parametrize("rows", [1, 3, 16])
+# widths whose last block of 64 columns is not full, a contraction that is split unevenly, heads of both sizes
+@pytest.mark.parametrize("K,n_q,n_kv,D,I", [(2048, 8, 2, 64, 1024), (1032, 4, 4, 128, 264), (3072, 24, 8, 128, 8192)])
+def test_norm_inside_the_projections(rows, K, n_q, n_kv, D, I):
+    from neuronx_distributed_llama3_2_b200.ops import decode_fused as df, norm, rope
+
+    g = torch.Generator(device="cuda").manual_seed(K + rows)
+    x = torch.randn(rows, 2 * K, generator=g, device="cuda").bfloat16()[:, :K] * 3          # a row pitch of its own
+    nw = (torch.randn(K, generator=g, device="cuda") * 0.1 + 1).bfloat16()
+    w_qkv = torch.randn((n_q + 2 * n_kv) * D, K, generator=g, device="cuda").bfloat16() * 0.02
+    w_gu = torch.randn(2 * I, K, generator=g, device="cuda").bfloat16() * 0.02
+    cos, sin = rope.build_rope_cache(64, D, 1e4, None, device="cuda")
+    pos = torch.arange(3, 3 + rows, device="cuda").int()
+    assert df.norm_fits(x, w_qkv, False) and df.norm_fits(x, w_gu, True)
+    assert not df.norm_fits(torch.empty(17, K, dtype=torch.bfloat16, device="cuda"), w_qkv, False)
+    caches = [torch.zeros(4, rows, n_kv, 32, D, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    xn = norm.rms_norm(x.contiguous(), nw, 1e-5)
+    got = [df.norm_qkv_rope_cache(x, nw, 1e-5, w_qkv, cos, sin, pos, caches[0][0], caches[0][1], n_q, n_kv, D), caches[0],
+           df.norm_gate_up_swiglu(x, nw, 1e-5, w_gu)]
+    ref = [df.qkv_rope_cache_batched(xn, w_qkv, cos, sin, pos, caches[1][0], caches[1][1], n_q, n_kv, D), caches[1],
+           df.gate_up_swiglu_batched(xn, w_gu)]
+    # the same roundings; only the sum of squares is in another order, which moves some activations to the neighbouring bf16 value
+    for a, b in zip(got, ref):
+        assert (a.float() - b.float()).norm() <= 1e-3 * b.float().norm()
