@@ -31,6 +31,8 @@
 // cluster barrier after start-up, one launch.
 #include <stdlib.h>
 
+#include <type_traits>
+
 #include "decode_common.cuh"
 #include "gemm_tcgen05.cuh"
 #include "ptx.cuh"
@@ -70,7 +72,11 @@ struct EpiArgs {
 
 // NORM: the epilogue warps, which have nothing to do while the weights stream, normalise the CTA's slice of the activations into
 // shared memory themselves (every CTA sums the squares of the whole rows: 4 KB a row from L2), instead of a kernel between this one and
-// the one before.  A norm launch costs a token step 2.6 us; 16 rows of 2048 are the most that cost less here.
+// the one before (2.6 us of launch and latency).  Four layers and the head, norms inside / of their own: width 2048, 1 sequence 249 / 267
+// us, 2 258 / 270, 4 261 / 271, 8 (with rows in turn) 285 / 282; width 3072, where the weights take longer than the chain, 348 / 348 and
+// 4 sequences 358 / 352.
+constexpr int kNormRows = 4, kNormWidth = 2048;
+
 template <int BT, int EPI, bool NORM>
 struct Cfg {
     static constexpr int kAcc = EPI == kEpiSwiglu ? 2 : 1;           // accumulators (weight slabs) per CTA
@@ -240,49 +246,69 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
         // no split-K, else into the send buffer [owner][local token][128]; consecutive lanes = consecutive n:
         // conflict-free 128-byte rows per warp store
         const int q = warp & 3;
-        const int row8 = (kb_end - kb_begin) * (kBK / 8), t = threadIdx.x - 64;     // NORM: vectors of a row in this CTA's slice
-        auto norm_w = [&](int c) {                                             // (zeros behind the end of the rows)
-            const int k = kb_begin * kBK + c * 8;
-            return c < row8 && k < K ? *reinterpret_cast<const uint4*>(ep.norm_w + k) : make_uint4(0u, 0u, 0u, 0u);
-        };
-        uint4 w0, w1;                                                          // the first ones do not wait for the kernel before
-        if constexpr (NORM) w0 = norm_w(t), w1 = norm_w(t + 128);
+        if constexpr (NORM) {           // the norm's weights do not wait for the kernel before
+            const int k = kb_begin * kBK + (threadIdx.x - 64) * 64;
+            if (k < min(kb_end * kBK, K)) asm volatile("prefetch.global.L1 [%0];" ::"l"(ep.norm_w + k));
+        }
         pdl_wait();     // the epilogue reads the residual / positions and writes global memory
         if constexpr (NORM) {
-            float (*red)[BT] = reinterpret_cast<float (*)[BT]>(smem + C::kBarOffset + 512);
-            float ss[BT] = {};
-            for (int c = t; c < K / 8; c += 128) {
+            // two round trips to L2, whatever the number of rows: the warps share one row or two and take a row each of more, with all
+            // loads in flight; then every thread takes eight columns of a row at a time
+            float (*red)[4] = reinterpret_cast<float (*)[4]>(smem + C::kBarOffset + 512);      // [row][share]
+            const int t = threadIdx.x - 64;
+            auto normalise = [&](auto tag) {
+                constexpr int kShares = decltype(tag)::value, kLoads = kNormWidth / 8 / (32 * kShares), kItems = 4 / kShares;
+                const int share = q % kShares, own = q / kShares;
+                if (own < B) {
+                    const bf16x8* row = reinterpret_cast<const bf16x8*>(ep.raw + own * ep.ld_raw);
+                    bf16x8 v[kLoads] = {};
 #pragma unroll
-                for (int b = 0; b < BT; ++b) {
-                    if (b >= B) break;
-                    float f[8];
-                    unpack8(*reinterpret_cast<const bf16x8*>(ep.raw + b * ep.ld_raw + c * 8), f);
+                    for (int i = 0; i < kLoads; ++i)
+                        if ((i * kShares + share) * 32 + lane < K / 8) v[i] = row[(i * kShares + share) * 32 + lane];
+                    float ss = 0.f;
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) ss[b] = fmaf(f[e], f[e], ss[b]);
+                    for (int i = 0; i < kLoads; ++i) {
+                        float f[8];
+                        unpack8(v[i], f);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) ss = fmaf(f[e], f[e], ss);
+                    }
+                    ss = warp_sum(ss);
+                    if (lane == 0) red[own][share] = ss;
                 }
-            }
+                epilogue_bar();
+                const int row8 = (kb_end - kb_begin) * (kBK / 8);              // vectors of a row in this CTA's slice
+                for (int i0 = t; i0 < B * row8; i0 += 128 * kItems) {
+                    bf16x8 fv[kItems] = {}, wv[kItems] = {};
 #pragma unroll
-            for (int b = 0; b < BT; ++b) {
-                if (b >= B) break;
-                ss[b] = warp_sum(ss[b]);
-                if (lane == 0) red[q][b] = ss[b];
-            }
-            epilogue_bar();
-            for (int c = t, i = 0; c < row8; c += 128, ++i) {
-                const uint4 wv = i == 0 ? w0 : i == 1 ? w1 : norm_w(c);
-                const int k = min(kb_begin * kBK + c * 8, K - 8);
-                float w[8];
-                unpack8(*reinterpret_cast<const bf16x8*>(&wv), w);
-                for (int b = 0; b < B; ++b) {
-                    const float rstd = rsqrtf((red[0][b] + red[1][b] + red[2][b] + red[3][b]) / (float)K + ep.eps);
-                    float f[8];
-                    unpack8(*reinterpret_cast<const bf16x8*>(ep.raw + b * ep.ld_raw + k), f);
+                    for (int u = 0; u < kItems; ++u) {
+                        const int i = i0 + 128 * u, b = kShares == 4 ? 0 : i / row8, k = kb_begin * kBK + (i - b * row8) * 8;
+                        if (i < B * row8 && k < K) {                           // zeros behind the end, where the weights are zeros too
+                            fv[u] = *reinterpret_cast<const bf16x8*>(ep.raw + b * ep.ld_raw + k);
+                            wv[u] = *reinterpret_cast<const bf16x8*>(ep.norm_w + k);
+                        }
+                    }
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) f[e] = kb_begin * kBK + c * 8 < K ? f[e] * rstd * w[e] : 0.f;
-                    *reinterpret_cast<bf16x8*>(smem + C::kNormOffset + (c >> 3) * (BT * kBK * 2) + b * 128 +
-                                               (((c & 7) ^ (b & 7)) << 4)) = pack8(f);
+                    for (int u = 0; u < kItems; ++u) {
+                        const int i = i0 + 128 * u, b = kShares == 4 ? 0 : i / row8, c = i - b * row8;
+                        if (i >= B * row8) break;
+                        float sum = red[b][0];
+#pragma unroll
+                        for (int x = 1; x < kShares; ++x) sum += red[b][x];
+                        const float rstd = rsqrtf(sum / (float)K + ep.eps);
+                        float f[8], w[8];
+                        unpack8(fv[u], f);
+                        unpack8(wv[u], w);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) f[e] = f[e] * rstd * w[e];
+                        *reinterpret_cast<bf16x8*>(smem + C::kNormOffset + (c >> 3) * (BT * kBK * 2) + b * 128 +
+                                                   (((c & 7) ^ (b & 7)) << 4)) = pack8(f);
+                    }
                 }
-            }
+            };
+            if (B == 1) normalise(std::integral_constant<int, 4>());
+            else if (B == 2) normalise(std::integral_constant<int, 2>());
+            else normalise(std::integral_constant<int, 1>());
             ptx::fence_proxy_async();
             ptx::mbar_arrive(norm_bar);
         }
@@ -564,10 +590,10 @@ int qkv_args(EpiArgs& ep, const float* cos_t, const float* sin_t, const int* pos
     return 0;
 }
 
-// Behind an RMSNorm of up to 16 rows: the splits, 0 where a CTA's slice of the rows does not fit shared memory
+// Behind an RMSNorm: the splits, 0 where a norm of its own is faster or a CTA's slice of the rows does not fit shared memory
 template <int EPI>
 int norm_splits(int B, int n_rows, int K) {
-    if (B > 16) return 0;
+    if (B > kNormRows || K > kNormWidth) return 0;
     const int nkb = (K + kBK - 1) / kBK, s = choose_splits(0, 16, EPI, (n_rows + kWRows - 1) / kWRows, nkb);
     return (nkb + s - 1) / s <= Cfg<16, EPI, true>::kNormBlocks ? s : 0;
 }
@@ -576,7 +602,7 @@ template <int EPI>
 int run_norm(const void* x, long long ldx, const void* norm_w, float eps, const void* w, EpiArgs& ep, int B, int n_rows, int w_rows,
              int K, long long ldw, cudaStream_t st) {
     const int splits = B >= 1 ? norm_splits<EPI>(B, n_rows, K) : 0;
-    NXD_REQUIRE(splits > 0, "gemm_smallm: %d rows of %d columns do not fit behind a norm", B, K);
+    NXD_REQUIRE(splits > 0, "gemm_smallm: no norm over %d rows of %d columns inside", B, K);
     NXD_REQUIRE(K % 8 == 0 && ldx % 8 == 0 && ldw % 8 == 0 && (((uintptr_t)x | (uintptr_t)w | (uintptr_t)norm_w) & 15) == 0,
                 "gemm_smallm: K=%d and the row pitches must be multiples of 8, operands 16-byte aligned", K);
     ep.raw = (const bf16*)x;
@@ -623,7 +649,7 @@ NXD_API int nxd_smallm_norm_applies(int gate_up, int B, int K, int n_rows) {
     return (gate_up ? norm_splits<kEpiSwiglu>(B, n_rows, K) : norm_splits<kEpiQkvRope>(B, n_rows, K)) > 0;
 }
 
-// nxd_smallm_qkv_rope_cache and nxd_smallm_gate_up_swiglu of rmsnorm(x) * norm_w, the norm inside: 1 <= B <= 16.
+// nxd_smallm_qkv_rope_cache and nxd_smallm_gate_up_swiglu of rmsnorm(x) * norm_w, the norm inside.
 NXD_API int nxd_smallm_norm_qkv_rope_cache(const void* x, long long ldx, const void* norm_w, float eps, const void* w,
                                            long long ldw, const float* cos_t, const float* sin_t, const int* positions,
                                            void* q_out, void* cache_k, void* cache_v, const int* seq_ids,

@@ -219,8 +219,8 @@ class KVCacheInferenceMixin:
                    and streams_on_tensor_cores(hidden.shape[0], *w.shape) for w in ws)
 
     def _layer_batched_decode(self, i: int, layer, hidden, residual, positions, seq_ids, lengths):
-        """One token per sequence for up to 128 sequences on the small-M tensor-core kernels (``csrc/gemm_smallm.cu``); up to 16
-        sequences have both RMSNorms inside the projections behind them, six launches.  More of them:
+        """One token per sequence for up to 128 sequences on the small-M tensor-core kernels (``csrc/gemm_smallm.cu``); a few
+        sequences of a narrow model have both RMSNorms inside the projections behind them, six launches.  Else:
         RMSNorm | QKV GEMM+RoPE+cache write | attention (split, merge) | o_proj+residual | RMSNorm | gate/up+SwiGLU |
         down_proj+residual -- eight launches, no copies between them.  Tensor parallel: the two row-parallel GEMMs are
         followed by the one-shot all-reduce and the residual moves into the fused add+RMSNorm (ten launches)."""

@@ -85,10 +85,10 @@ def qkv_rope_cache_batched(xn: torch.Tensor, w_qkv: torch.Tensor, cos: torch.Ten
 
 
 def norm_fits(x: torch.Tensor, w: torch.Tensor, gate_up: bool) -> bool:
-    """Whether ``norm_qkv_rope_cache`` / ``norm_gate_up_swiglu`` take these rows: at most 16, a CTA's slice of them in its shared
-    memory (all widths up to 3072, wider ones where the contraction is split further)."""
+    """Whether ``norm_qkv_rope_cache`` / ``norm_gate_up_swiglu`` take these rows (few and narrow: ``csrc/gemm_smallm.cu`` has the
+    measurements)."""
     B, K = x.shape
-    return (B <= 16 and K % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and bool(
+    return (1 <= B <= MAX_ROWS and K % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and bool(
         _lib.lib().nxd_smallm_norm_applies(_c.c_int(int(gate_up)), _c.c_int(B), _c.c_int(K),
                                            _c.c_int(w.shape[0] // 2 if gate_up else w.shape[0]))))
 
@@ -97,7 +97,7 @@ def norm_qkv_rope_cache(x: torch.Tensor, norm_w: torch.Tensor, eps: float, w_qkv
                         positions: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Tensor, n_q: int, n_kv: int, D: int,
                         seq_ids: Optional[torch.Tensor] = None, block_table: Optional[torch.Tensor] = None,
                         page_size: int = 0) -> torch.Tensor:
-    """``qkv_rope_cache_batched`` of ``rmsnorm(x) * norm_w`` for up to 16 rows: the projection's kernel normalises its rows itself
+    """``qkv_rope_cache_batched`` of ``rmsnorm(x) * norm_w``: the projection's kernel normalises its rows itself
     (``nxd_smallm_norm_qkv_rope_cache``)."""
     B, K = x.shape
     assert w_qkv.shape == ((n_q + 2 * n_kv) * D, K) and w_qkv.stride(1) == 1 and norm_w.is_contiguous()
@@ -114,7 +114,7 @@ def norm_qkv_rope_cache(x: torch.Tensor, norm_w: torch.Tensor, eps: float, w_qkv
 
 
 def norm_gate_up_swiglu(x: torch.Tensor, norm_w: torch.Tensor, eps: float, w_gate_up: torch.Tensor) -> torch.Tensor:
-    """``gate_up_swiglu_batched`` of ``rmsnorm(x) * norm_w`` for up to 16 rows (``nxd_smallm_norm_gate_up_swiglu``)."""
+    """``gate_up_swiglu_batched`` of ``rmsnorm(x) * norm_w`` (``nxd_smallm_norm_gate_up_swiglu``)."""
     B, K = x.shape
     I = w_gate_up.shape[0] // 2
     assert w_gate_up.shape[1] == K and w_gate_up.stride(1) == 1 and I % 8 == 0 and norm_w.is_contiguous()

@@ -57,9 +57,9 @@ def test_one_sequence_matches_the_fma_kernels(paged, monkeypatch):
     test_token_step_matches_the_fma_kernels(1, paged, monkeypatch)
 
 
-@pytest.mark.parametrize("rows", [1, 3, 16])
+@pytest.mark.parametrize("rows", [1, 2, 3, 4])
 # widths whose last block of 64 columns is not full, a contraction that is split unevenly, heads of both sizes
-@pytest.mark.parametrize("K,n_q,n_kv,D,I", [(2048, 8, 2, 64, 1024), (1032, 4, 4, 128, 264), (3072, 24, 8, 128, 8192)])
+@pytest.mark.parametrize("K,n_q,n_kv,D,I", [(2048, 32, 8, 64, 8192), (1032, 4, 4, 128, 264), (520, 24, 8, 128, 4096)])
 def test_norm_inside_the_projections(rows, K, n_q, n_kv, D, I):
     from neuronx_distributed_llama3_2_b200.ops import decode_fused as df, norm, rope
 
@@ -71,7 +71,7 @@ def test_norm_inside_the_projections(rows, K, n_q, n_kv, D, I):
     cos, sin = rope.build_rope_cache(64, D, 1e4, None, device="cuda")
     pos = torch.arange(3, 3 + rows, device="cuda").int()
     assert df.norm_fits(x, w_qkv, False) and df.norm_fits(x, w_gu, True)
-    assert not df.norm_fits(torch.empty(17, K, dtype=torch.bfloat16, device="cuda"), w_qkv, False)
+    assert not df.norm_fits(torch.empty(5, K, dtype=torch.bfloat16, device="cuda"), w_qkv, False)
     caches = [torch.zeros(4, rows, n_kv, 32, D, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
     xn = norm.rms_norm(x.contiguous(), nw, 1e-5)
     got = [df.norm_qkv_rope_cache(x, nw, 1e-5, w_qkv, cos, sin, pos, caches[0][0], caches[0][1], n_q, n_kv, D), caches[0],
