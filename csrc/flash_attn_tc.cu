@@ -82,7 +82,8 @@ struct TcSmem {
 // one.  Rows of the last V tile past the sequence's end may hold anything (0 * NaN is NaN), so the producer warp copies that
 // one tile itself with zeros behind the end; every other tile is a TMA load.
 // Bound by the softmax like the other instantiations; portion of 2048 after 2048 tokens, 2 rows, 32 heads of 128 over 8,
-// window 2048 (138 GF): 207 us (665 TF) against 587 us on the mma.sync kernel over the cache (window_attention.cu).
+// window 2048 (138 GF): 168 us (820 TF) against 587 us on the mma.sync kernel over the cache (window_attention.cu).  A tile takes its
+// softmax warp 2400 clocks: 1050 exponentials, 460 bias, 430 waiting for scores; without bias 530 more for the accumulator.
 template <int D, bool CAUSAL, bool DROP, bool WIN = false, int SCORE = 0, bool CACHE = false>
 __global__ void __launch_bounds__(kThreadsTc, 2)
 fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -123,7 +124,13 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         n_sink = min((p.keep_first + kBN - 1) / kBN, t_win);
         n_tiles = n_tiles - t_win + n_sink;
     }
-    auto tile = [&](int j) { return WIN ? (j < n_sink ? j : t_win + (j - n_sink)) : j; };
+    // WIN visits its tiles from the diagonal back: where scores fall with the distance the running maximum is found at once, and the
+    // accumulator is not rescaled in every tile
+    auto tile = [&](int j) {
+        if (!WIN) return j;
+        const int i = SCORE == 2 ? j : n_tiles - 1 - j;
+        return i < n_sink ? i : t_win + (i - n_sink);
+    };
 
     if (warp == 0 && lane == 0) {
         ptx::prefetch_tensormap(&tmap_q);
@@ -344,9 +351,17 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             } else if (WIN) {
                 // log2 units: s * scale - slope * (query position - key position)
                 const float base = -slope2 * (float)(grow + offset - n0);
+                const uint64_t scale = f2_pack(p.scale_log2, p.scale_log2), slope = f2_pack(slope2, slope2), start = f2_pack(base, base);
+                auto log2_units = [&](auto bias) {
 #pragma unroll
-                for (int c = 0; c < kBN; ++c)
-                    sr[c] = __float_as_uint(fmaf(__uint_as_float(sr[c]), p.scale_log2, fmaf(slope2, (float)c, base)));
+                    for (int c = 0; c < kBN; c += 2) {
+                        const uint64_t x = f2_fma(f2_pack(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])), scale, bias(c));
+                        sr[c] = (uint32_t)x;
+                        sr[c + 1] = (uint32_t)(x >> 32);
+                    }
+                };
+                if (p.slopes != nullptr) log2_units([&](int c) { return f2_fma(slope, f2_pack((float)c, (float)(c + 1)), start); });
+                else log2_units([](int) { return 0ull; });
             }
             if (MASK) {
                 // columns c >= first_bad are masked: beyond the causal diagonal of this row, or beyond the sequence end
@@ -355,9 +370,14 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                 // WIN: columns below the window that are not kept first keys are masked as well
                 const int first_good = (WIN && p.window > 0) ? grow + offset - p.window + 1 - n0 : 0;
                 const int kept = WIN ? p.keep_first - n0 : 0;
+                // columns kept .. first_good - 1 as one unsigned comparison, without a branch: written as c < first_good && c >= kept
+                // behind an || a masked tile took 5900 clocks, three times the rest of a tile
+                const unsigned gap = (unsigned)max(first_good - kept, 0);
 #pragma unroll
-                for (int c = 0; c < kBN; ++c)
-                    if (c >= first_bad || (WIN && c < first_good && c >= kept)) sr[c] = SCORE == 2 ? 0x7f800000u : 0xff800000u;   // -inf
+                for (int c = 0; c < kBN; ++c) {
+                    const bool hidden = (c >= first_bad) | (WIN && (unsigned)(c - kept) < gap);
+                    sr[c] = hidden ? (SCORE == 2 ? 0x7f800000u : 0xff800000u) : sr[c];   // -inf
+                }
             }
             uint32_t pk[kBN / 2];
             if constexpr (SCORE == 2) {
@@ -392,8 +412,8 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
             // lazy rescale: keep the stale max unless it moved by more than 2^8 (in scaled log2 units).  CACHE follows every
             // move, as the kernels it takes calls from do: the row's largest weight is then exactly 1 and not rounded (the portion
-            // above: error 0.00188 instead of 0.00201 at the same time; without a bias the maximum moves in most tiles: 2100 tokens
-            // over a window of 1024 take 127 us instead of 110, 372 on the mma.sync kernel).
+            // above: error 0.00188 instead of 0.00201; without a bias the maximum of one of a warp's rows moves in most tiles, which
+            // costs a fifth of the time).
             float alpha = 1.f;
             bool rescale = false;
             if ((mx - m_run) * sc > (CACHE ? 0.f : kRescaleThreshold) || m_run == -INFINITY) {
@@ -405,13 +425,13 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                 }
             }
             const float neg_m = (m_run == -INFINITY) ? 0.f : -m_run * sc;
-            float rs0 = 0.f, rs1 = 0.f;
+            const uint64_t sc2 = f2_pack(sc, sc), neg_m2 = f2_pack(neg_m, neg_m);
+            uint64_t rs = 0ull;
 #pragma unroll
             for (int c = 0; c < kBN; c += 2) {
-                const float p0 = ex2_approx(fmaf(__uint_as_float(sr[c]), sc, neg_m));
-                const float p1 = ex2_approx(fmaf(__uint_as_float(sr[c + 1]), sc, neg_m));
-                rs0 += p0;
-                rs1 += p1;
+                const uint64_t x = f2_fma(f2_pack(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])), sc2, neg_m2);
+                const float p0 = ex2_approx(f2_lo(x)), p1 = ex2_approx(f2_hi(x));
+                asm("add.rn.f32x2 %0, %0, %1;" : "+l"(rs) : "l"(f2_pack(p0, p1)));
                 if (DROP) {   // the row sum (softmax denominator) is taken before dropout, the PV operand after it
                     const uint32_t hs = drop_head_seed(p.drop.seed, (uint32_t)(b * p.Hq + hq));
                     const bool k0 = drop_keep(hs, (uint32_t)grow, (uint32_t)(n0 + c), p.drop.threshold);
@@ -421,20 +441,27 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                     pk[c >> 1] = pack_bf16x2(p0, p1);
                 }
             }
-            l_run = l_run * alpha + (rs0 + rs1);
+            l_run = l_run * alpha + (f2_lo(rs) + f2_hi(rs));
             if (j > 0) {
                 ptx::mbar_wait(pv_done, ((uint32_t)(j - 1)) & 1u);  // P buffer free, O up to date
                 ptx::tcgen05_fence_after();
                 if (__any_sync(0xffffffffu, rescale)) {
 #pragma unroll 1
-                    for (int c = 0; c < D / 32; ++c) {
-                        uint32_t o[32];
-                        ptx::tmem_ld_32x32b_x32(tmem_o + lane_off + c * 32, o);
+                    for (int c = 0; c < D / 64; ++c) {
+                        uint32_t o[64];
+                        ptx::tmem_ld_32x32b_x32(tmem_o + lane_off + c * 64, o);
+                        ptx::tmem_ld_32x32b_x32(tmem_o + lane_off + c * 64 + 32, o + 32);
                         ptx::tmem_ld_wait();
                         const float a_o = rescale ? alpha : 1.f;
+                        const uint64_t a_o2 = f2_pack(a_o, a_o);
 #pragma unroll
-                        for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * a_o);
-                        tmem_st_32x32b_x32(tmem_o + lane_off + c * 32, o);
+                        for (int e = 0; e < 64; e += 2) {
+                            const uint64_t x = f2_mul(f2_pack(__uint_as_float(o[e]), __uint_as_float(o[e + 1])), a_o2);
+                            o[e] = (uint32_t)x;
+                            o[e + 1] = (uint32_t)(x >> 32);
+                        }
+                        tmem_st_32x32b_x32(tmem_o + lane_off + c * 64, o);
+                        tmem_st_32x32b_x32(tmem_o + lane_off + c * 64 + 32, o + 32);
                     }
                     tmem_st_wait();
                 }
