@@ -499,9 +499,12 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
 int pick_splits(int n_tiles, int nkb, int ctas_per_sm) {
     // the largest power of two <= 8 that keeps the grid within one resident wave and leaves two k blocks per slice
     // (measured at the Llama-3.2 decode shapes: 16-24 slabs -> 8, 64 -> 4, 128 -> 2, the 1002 slabs of the LM head -> 1)
-    const int slots = nxd_num_sms() * ctas_per_sm;
+    // With one CTA per SM more than 12 clusters of 8 do not all find 8 free SMs of one GPC, and the last wait for a second wave.  Slabs /
+    // contraction, 8 slices / 4: 100 rows, 16 / 8192 20.4 us / 15.0; 65 rows, 16 / 2048 10.6 / 6.3; 128 rows, 12 / 2048 8.2 / 8.4 and
+    // 8 / 4096 9.0 / 10.3; gate/up of 4 rows, 16 / 2048 9.7 / 6.0, 10 / 2048 4.8 / 5.3.
+    const int slots = nxd_num_sms() * ctas_per_sm, most = ctas_per_sm == 1 && n_tiles > 12 ? kMaxSplits / 2 : kMaxSplits;
     int s = 1;
-    while (s < kMaxSplits && n_tiles * s * 2 <= slots && nkb / (s * 2) >= 2) s *= 2;
+    while (s < most && n_tiles * s * 2 <= slots && nkb / (s * 2) >= 2) s *= 2;
     return s;
 }
 

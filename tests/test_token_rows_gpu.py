@@ -18,6 +18,12 @@ def test_few_rows_match_float64(rows, n, k):
     assert (gemm_nt(x, w).double() - ref).norm() <= 2.0 ** -8 * ref.norm()
 
 
+# one CTA per SM: 12 weight slabs in clusters of 8, 13 in clusters of 4
+@pytest.mark.parametrize("n", [1536, 1544])
+def test_many_rows_match_float64(n):
+    test_few_rows_match_float64(100, n, 2048)
+
+
 @pytest.mark.parametrize("batch,paged", [(2, False), (3, True), (8, False)])
 def test_token_step_matches_the_fma_kernels(batch, paged, monkeypatch):
     from neuronx_distributed_llama3_2_b200.inference.config import InferenceConfig
