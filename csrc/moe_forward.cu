@@ -1,10 +1,14 @@
-// The sparse mixture after its router in ONE call: rows sorted by expert, gate / up product with the activation, down product,
-// weighted combination, and a shared expert's two products -- six to eight launches that read the routing on the device.  One host
-// call and one workspace instead of four calls with an allocation each: at 64 tokens (width 1024, 16 experts) the launches take
-// 36 us of GPU time and the four calls from Python 80 us of host time.
+// The sparse mixture in ONE call, after its router or with it: rows sorted by expert, gate / up product with the activation, down
+// product, weighted combination, and a shared expert's two products -- launches that read the routing on the device.  One host call and
+// one workspace instead of five calls with allocations: 64 tokens (width 1024, 4 of 16 experts) are five launches, 37 us of GPU time
+// and 43 eagerly; with the router in a call of its own, a memset and separate counting 41 and 62, in calls of their own 80.
 #include "common.cuh"
 #include "gemm_tcgen05.cuh"
 
+NXD_API int nxd_moe_router(int dtype, const void* h, const float* wr, const float* corr, const float* wsg, int* idx, float* wts,
+                           float* sgate, long long N, int W, int R, int top, float out_scale, const float* zbias, int mode,
+                           void* stream);
+NXD_API int nxd_moe_sort_counts_itself(long long P);
 NXD_API int nxd_moe_sort_rows(const void* h, const int* idx, int* counts, int* slot, const float* in_scale, float* row_scale,
                               void* x, long long P, int top, int W, int E, void* stream);
 NXD_API int nxd_experts_gemm_bf16(const void* a, const void* b, void* d, const int* counts, const float* row_scale, int E,
@@ -17,7 +21,7 @@ NXD_API int nxd_moe_gather_combine(int dtype, const void* ys, const int* slot, c
 namespace {
 
 struct Layout {      // byte offsets into the workspace
-    long long rows, counts, slot, scale, x, act, ys, s_act, s_out, bytes;
+    long long rows, counts, slot, scale, x, act, ys, s_act, s_out, idx, wts, sgate, bytes;
 };
 
 // The experts' outputs are kept in fp32 up to the weighted sum, as the per-pair GEMVs keep them, at every size: a captured step
@@ -35,7 +39,10 @@ Layout layout(long long N, int top, int W, int F, int E, int Fs) {
     l.ys = up(l.act + 2 * l.rows * F);
     l.s_act = up(l.ys + 4 * l.rows * W);
     l.s_out = up(l.s_act + 2 * N * Fs);
-    l.bytes = up(l.s_out + (Fs > 0 ? 4 * N * W : 0));
+    l.idx = up(l.s_out + (Fs > 0 ? 4 * N * W : 0));      // nxd_moe_routed_forward
+    l.wts = up(l.idx + 4 * N * top);
+    l.sgate = up(l.wts + 4 * N * top);
+    l.bytes = up(l.sgate + (Fs > 0 ? 4 * N : 0));
     return l;
 }
 
@@ -61,7 +68,7 @@ NXD_API int nxd_moe_sorted_forward(const void* h, const int* idx, const float* w
     int* slot = reinterpret_cast<int*>(base + l.slot);
     void *x = base + l.x, *act = base + l.act, *ys = base + l.ys;
     const int rows = (int)l.rows, pairs = (int)(N * top);
-    NXD_CHECK_CUDA(cudaMemsetAsync(counts, 0, 4ll * (E + 1), (cudaStream_t)stream));
+    if (!nxd_moe_sort_counts_itself(N * top)) NXD_CHECK_CUDA(cudaMemsetAsync(counts, 0, 4ll * (E + 1), (cudaStream_t)stream));
     NXD_REQUIRE(in_scale == nullptr || gated, "sorted experts: %s", "a weight on the input needs gated experts");
     float* scale = in_scale != nullptr ? reinterpret_cast<float*>(base + l.scale) : nullptr;
     int rc = nxd_moe_sort_rows(h, idx, counts, slot, in_scale, scale, x, N * top, top, W, E, stream);
@@ -83,4 +90,21 @@ NXD_API int nxd_moe_sorted_forward(const void* h, const int* idx, const float* w
         if (rc) return rc;
     }
     return nxd_moe_gather_combine(2, ys, slot, idx, wts, h, s_out, sgate, y, N, top, W, E, stream);
+}
+
+// The same with its router in front (see nxd_moe_router: R outputs, wr [R, W], corr / zbias [R] or NULL, wsg [W] or NULL), the weight on
+// the expert's output.  The routing stays in the workspace.
+NXD_API int nxd_moe_routed_forward(const void* h, const float* wr, const float* corr, const float* wsg, const float* zbias, int R,
+                                   float out_scale, int mode, const void* w_in, const void* w_down, const void* s_in,
+                                   const void* s_down, float* y, void* work, long long N, int top, int W, int F, int E, int Fs,
+                                   int gated, float limit, float s_limit, float alpha, float up_shift, void* stream) {
+    if (N == 0) return 0;
+    const Layout l = layout(N, top, W, F, E, Fs);
+    char* base = static_cast<char*>(work);
+    int* idx = reinterpret_cast<int*>(base + l.idx);
+    float *wts = reinterpret_cast<float*>(base + l.wts), *sgate = wsg != nullptr && Fs > 0 ? reinterpret_cast<float*>(base + l.sgate) : nullptr;
+    const int rc = nxd_moe_router(0, h, wr, corr, wsg, idx, wts, sgate, N, W, R, top, out_scale, zbias, mode, stream);
+    if (rc) return rc;
+    return nxd_moe_sorted_forward(h, idx, wts, nullptr, w_in, w_down, s_in, s_down, sgate, y, work, N, top, W, F, E, Fs, gated, limit,
+                                  s_limit, alpha, up_shift, stream);
 }

@@ -556,6 +556,48 @@ moe_gather_rows_kernel(const bf16* __restrict__ h, const int* __restrict__ idx, 
     for (int c = lane; c < W8; c += 32) dst[c] = src[c];
 }
 
+// Both of the above for few pairs, in one launch and without zeroed counts: every block counts all pairs itself, a warp finds its
+// pair's place by counting the earlier ones of its expert.  A captured step, width 1024, 4 of 16 experts: 64 tokens 41.0 -> 36.9 us, 512
+// (2048 pairs) 49.2 -> 41.1.
+constexpr int FEW_PAIRS = 2048;
+
+__global__ void __launch_bounds__(GA_WARPS * 32)
+moe_sort_few_kernel(const bf16* __restrict__ h, const int* __restrict__ idx, int* __restrict__ counts, int* __restrict__ slot,
+                    const float* __restrict__ in_scale, float* __restrict__ row_scale, bf16* __restrict__ x, int P, int top, int W8,
+                    int E) {
+    __shared__ int expert[FEW_PAIRS], cnt[nxd_gemm::kSegMaxExperts], row0[nxd_gemm::kSegMaxExperts + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int e = threadIdx.x; e < E; e += GA_WARPS * 32) cnt[e] = 0;
+    __syncthreads();
+    for (int p = threadIdx.x; p < P; p += GA_WARPS * 32) {
+        const int e = idx[p];
+        expert[p] = e;
+        if (e >= 0 && e < E) atomicAdd(cnt + e, 1);
+    }
+    __syncthreads();
+    if (blockIdx.x == 0) {
+        for (int e = threadIdx.x; e < E; e += GA_WARPS * 32) counts[e] = cnt[e];
+        if (threadIdx.x == 0) counts[E] = P / top;      // the tokens: rows of a shared expert
+    }
+    if (warp == 0) nxd_gemm::segment_starts(cnt, E, 0, row0, nullptr);
+    __syncthreads();
+    const int p = blockIdx.x * GA_WARPS + warp;
+    if (p >= P) return;
+    const int e = expert[p];
+    if (e < 0 || e >= E) return;                        // identity expert: the combination reads h itself
+    int before = 0;
+    for (int q = lane; q < p; q += 32) before += expert[q] == e;
+    const int row = row0[e] + __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) {
+        slot[p] = row;
+        if (in_scale != nullptr) row_scale[row] = in_scale[p];
+    }
+    const bf16x8* src = reinterpret_cast<const bf16x8*>(h) + (long long)(p / top) * W8;
+    bf16x8* dst = reinterpret_cast<bf16x8*>(x) + (long long)row * W8;
+#pragma unroll 4
+    for (int c = lane; c < W8; c += 32) dst[c] = src[c];
+}
+
 }  // namespace
 
 // dtype: 0 bf16, 1 fp32 (activations and expert weights).  R = router outputs (experts + identity experts).
@@ -596,15 +638,24 @@ NXD_API int nxd_moe_router(int dtype, const void* h, const float* wr, const floa
     return 0;
 }
 
-// Rows of the pairs sorted by expert.  counts [E + 1] int32: ZEROED by the caller, out: pairs of every expert, then P / top;
+// Rows of the pairs sorted by expert.  counts [E + 1] int32: ZEROED by the caller (unless nxd_moe_sort_counts_itself(P)), out: pairs
+// of every expert, then P / top;
 // slot [P] int32 out: the pair's row in x (not written for identity experts); x [rows, W] bf16 with rows >= P + 32 E, W a
 // multiple of 8; row_scale [rows] <- in_scale [P] of the row's pair (both fp32, or both NULL).
+NXD_API int nxd_moe_sort_counts_itself(long long P) { return P <= FEW_PAIRS; }
+
 NXD_API int nxd_moe_sort_rows(const void* h, const int* idx, int* counts, int* slot, const float* in_scale, float* row_scale,
                               void* x, long long P, int top, int W, int E, void* stream) {
     if (P == 0) return 0;
     NXD_REQUIRE(E > 0 && E <= nxd_gemm::kSegMaxExperts && W % 8 == 0, "sort rows: %d experts, width %d", E, W);
     NXD_REQUIRE(((uintptr_t)h % 16) == 0 && ((uintptr_t)x % 16) == 0, "sort rows: rows must be 16-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
+    if (nxd_moe_sort_counts_itself(P)) {
+        moe_sort_few_kernel<<<(unsigned)((P + GA_WARPS - 1) / GA_WARPS), GA_WARPS * 32, 0, st>>>(
+            (const bf16*)h, idx, counts, slot, in_scale, row_scale, (bf16*)x, (int)P, top, W / 8, E);
+        NXD_LAUNCH_CHECK();
+        return 0;
+    }
     moe_count_kernel<<<(unsigned)((P + CNT_PAIRS - 1) / CNT_PAIRS), CNT_THREADS, 2 * E * sizeof(int), st>>>(idx, counts, slot,
                                                                                                            P, top, E);
     NXD_LAUNCH_CHECK();

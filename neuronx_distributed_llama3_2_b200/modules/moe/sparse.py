@@ -109,10 +109,14 @@ class SparseMoE(torch.nn.Module):
         """``h [N, W]`` (activation dtype) -> combined output ``[N, W]`` in fp32.  ``path``: ``"pairs"`` | ``"sorted"`` (counts read on
         the host) | ``"device"`` (device-sorted), default: chosen by the sizes."""
         gated = self.shared is not None and self.shared_gate is not None
-        idx, wts, sg = self.router.select(h, self.shared_gate.weight if gated else None)
+        shared_gate_w = self.shared_gate.weight if gated else None
         weights = None
         if path is None:
             path, weights = self._device_path(h)
+            if (path == "device" and not self.weight_on_input and type(self.router).select is RouterBiasedTopK.select
+                    and "select" not in self.router.__dict__ and moe_sparse.router_fits(self.router, shared_gate_w)):
+                return self._forward_device_sorted(h, None, None, shared_gate_w, weights)
+        idx, wts, sg = self.router.select(h, shared_gate_w)
         if path == "device":
             return self._forward_device_sorted(h, idx, wts, sg, weights or self._sorted_weights())
         sorted_path = self._use_sorted(h.shape[0]) if path is None else path == "sorted"
@@ -143,6 +147,10 @@ class SparseMoE(torch.nn.Module):
         return ones
 
     def _forward_device_sorted(self, h, idx, wts, sg, weights):
+        """``idx`` ``None``: the router runs in the same call, ``sg`` is its weight for the shared expert's gate."""
+        if idx is None:
+            return moe_sparse.routed_forward(h, self.router, sg, weights, self.gated, self.limit, self.alpha, self.up_shift,
+                                             self.shared_limit if self.shared is not None else 0.0)
         in_scale = None
         if self.weight_on_input:
             in_scale, wts = wts, self._ones_like(wts)

@@ -266,6 +266,43 @@ def sorted_forward(h: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, w_in: 
     return y
 
 
+_P, _I, _L, _F = _c.c_void_p, _c.c_int, _c.c_longlong, _c.c_float
+_ROUTED = [_P] * 5 + [_I, _F, _I] + [_P] * 6 + [_L] + [_I] * 6 + [_F] * 4 + [_P]
+_WORKSPACE = [_L] + [_I] * 5
+
+
+def routed_forward(h: torch.Tensor, router, shared_gate_w: Optional[torch.Tensor], weights, gated: bool, limit: float, alpha: float,
+                   up_shift: float, shared_limit: float) -> torch.Tensor:
+    """``route`` and ``sorted_forward`` in one call with one workspace (the weight on the expert's output).  ``router``: the module that
+    ``route`` gets its arguments from; its parameters are contiguous fp32 (``router_fits``)."""
+    N, W = h.shape
+    w_in, w_down, *shared = weights
+    E, F, _ = w_down.shape
+    Fs = shared[1].shape[1] if shared else 0
+    R, top = router.linear_router.weight.shape[0], router.top_k
+    L = _lib.lib("window_moe_serving")
+    size, call = L.nxd_moe_sorted_workspace, L.nxd_moe_routed_forward
+    if call.argtypes is None:                      # declared types: plain numbers go over without an object each
+        size.restype, size.argtypes, call.argtypes = _L, _WORKSPACE, _ROUTED
+    work = torch.empty(size(N, top, W, F, E, Fs), dtype=torch.uint8, device=h.device)
+    y = torch.empty(N, W, dtype=torch.float32, device=h.device)
+    mode = 3 if router.normalize else (2 if router.score == "sigmoid" else int(router.renormalize))
+    rc = call(h.data_ptr(), router.linear_router.weight.data_ptr(), router.correction.data_ptr(),
+              None if shared_gate_w is None else shared_gate_w.data_ptr(),
+              None if router.logit_bias is None else router.logit_bias.data_ptr(), R, router.affinity_scale, mode, w_in.data_ptr(),
+              w_down.data_ptr(), shared[0].data_ptr() if shared else None, shared[1].data_ptr() if shared else None, y.data_ptr(),
+              work.data_ptr(), N, top, W, F, E, Fs, int(gated), limit, shared_limit if shared else 0.0, alpha, up_shift,
+              _lib.stream_ptr())
+    _lib.check(rc, "nxd_moe_routed_forward", L)
+    return y
+
+
+def router_fits(router, shared_gate_w: Optional[torch.Tensor]) -> bool:
+    """Whether ``routed_forward`` can read the router's parameters as they are (``route`` converts what is not contiguous fp32)."""
+    return all(t is None or (t.dtype == torch.float32 and t.is_cuda and t.is_contiguous())
+               for t in (router.linear_router.weight, router.correction, router.logit_bias, shared_gate_w))
+
+
 def gather_combine(ys: torch.Tensor, slot: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, h: torch.Tensor,
                    num_experts: int, shared_out: Optional[torch.Tensor] = None,
                    shared_gate: Optional[torch.Tensor] = None) -> torch.Tensor:

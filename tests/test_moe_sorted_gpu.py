@@ -134,3 +134,27 @@ def test_each_path_is_the_one_that_was_asked_for(monkeypatch):
     # the host-counted path rounds the experts' outputs to bf16, all round the activation: 2^-8 of a value each
     for y in by_path.values():
         assert (y - by_path["pairs"]).norm() <= 3 * 2.0 ** -8 * by_path["pairs"].norm()
+
+
+# around the pairs that one launch sorts (2048), identity experts, a shared expert with its gate, every form of the scores
+@pytest.mark.parametrize("tokens", [64, 511, 512, 513])
+@pytest.mark.parametrize("kw", [dict(), dict(num_identity_experts=3, shared_intermediate_size=128, normalize=True),
+                                dict(score="sigmoid", router_bias=True, shared_intermediate_size=64, shared_gated=False),
+                                dict(renormalize=True, gated=False)])
+def test_router_and_experts_in_one_call(tokens, kw):
+    from neuronx_distributed_llama3_2_b200.modules.moe.sparse import SparseMoE
+
+    torch.manual_seed(tokens)
+    m = SparseMoE(512, 12, 4, 256, 7.0, dtype=torch.bfloat16, device="cuda", **kw).eval()
+    with torch.no_grad():
+        for p in m.parameters():
+            p.normal_(0, 0.05)
+        h = torch.randn(tokens, 512, device="cuda").bfloat16()
+        calls, select = [], m.router.select
+        whole = m(h)
+        m.router.select = lambda *a: calls.append(1) or select(*a)      # a replaced router is asked
+        assert torch.equal(m(h), whole) and len(calls) == 1
+        assert torch.equal(m(h, path="device"), whole)
+        pairs = m(h, path="pairs")
+    # the per-pair kernels: bf16 activations of fp32 sums in another order
+    assert (whole - pairs).norm() <= 2.0 ** -8 * pairs.norm()
