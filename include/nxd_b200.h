@@ -100,6 +100,11 @@ int nxd_decode_attn_lines(const void* q, const void* cache_k, const void* cache_
                           const int* block_table, const int* seq_ids, long long stride_b, long long stride_h,
                           int page_size, int max_pages, void* out, float* scratch, int B, int n_q, int n_kv, int D,
                           int n_splits, float scale, void* stream);
+/* Same with 64-bit lengths. */
+int nxd_decode_attn_lines64(const void* q, const void* cache_k, const void* cache_v, const long long* lengths,
+                            const int* block_table, const int* seq_ids, long long stride_b, long long stride_h,
+                            int page_size, int max_pages, void* out, float* scratch, int B, int n_q, int n_kv, int D,
+                            int n_splits, float scale, void* stream);
 int nxd_kv_cache_update(const void* new_k, const void* new_v, void* cache_k, void* cache_v, const int* positions,
                         const int* seq_ids, const int* block_table, long long stride_b, long long stride_h,
                         int page_size, int max_pages, int B, int n_kv, int T_new, int D, void* stream);
@@ -223,6 +228,15 @@ int nxd_smallm_qkv_rope_cache(const void* x, long long ldx, const void* w, long 
                               void* stream);
 int nxd_smallm_gate_up_swiglu(const void* x, long long ldx, const void* w, long long ldw, void* out, long long ldo, int B,
                               int K, int I, int splits, void* stream);
+/* The two behind an RMSNorm of few narrow rows, the norm inside the kernel; whether a shape is taken. */
+int nxd_smallm_norm_applies(int gate_up, int B, int K, int n_rows);
+int nxd_smallm_norm_qkv_rope_cache(const void* x, long long ldx, const void* norm_w, float eps, const void* w, long long ldw,
+                                   const float* cos_t, const float* sin_t, const int* positions, void* q_out, void* cache_k,
+                                   void* cache_v, const int* seq_ids, const int* block_table, long long stride_b,
+                                   long long stride_h, int page_size, int max_pages, int B, int K, int n_q, int n_kv, int D,
+                                   void* stream);
+int nxd_smallm_norm_gate_up_swiglu(const void* x, long long ldx, const void* norm_w, float eps, const void* w, long long ldw,
+                                   void* out, long long ldo, int B, int K, int I, void* stream);
 /* Weight-only int8 skinny GEMM (reference: quantization_layers.py:444-478 dequantise + matmul): out[B, N] (+ residual) =
  * (x[B, K] bf16 * w[N, K]^T int8) * scale, fp32 accumulation; scale_n == 1 (per tensor) or N (per output channel).
  * B <= 8, K % 16 == 0, ldw (bytes) % 16 == 0.  Streams half the bytes of the bf16 skinny GEMM. */

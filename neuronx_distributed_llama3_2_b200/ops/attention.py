@@ -148,7 +148,8 @@ def decode_attention(q: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Tens
     Hkv = cache_k.shape[1]
     scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(D)
     if q.is_cuda and q.dtype == torch.bfloat16 and D in (64, 128) and _lib.available():
-        lens = lengths.to(torch.int32).contiguous()
+        wide = lengths.dtype == torch.int64 and lengths.is_contiguous()          # read as they are
+        lens = lengths if wide else lengths.to(torch.int32).contiguous()
         max_len = cache_k.shape[2] if block_table is None else block_table.shape[1] * page_size
         n_splits = _lib.lib().nxd_decode_attn_splits(_c.c_int(B), _c.c_int(Hq), _c.c_int(Hkv), _c.c_int(max_len))
         # the call's own scratch: a captured graph keeps it in its pool, and calls on other streams have theirs
@@ -157,7 +158,7 @@ def decode_attention(q: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Tens
         bt = block_table.to(torch.int32).contiguous() if block_table is not None else None
         qc = q.contiguous()
         sid = seq_ids.to(torch.int32).contiguous() if seq_ids is not None else None
-        rc = _lib.lib().nxd_decode_attn_lines(
+        rc = (_lib.lib().nxd_decode_attn_lines64 if wide else _lib.lib().nxd_decode_attn_lines)(
             _lib.ptr(qc), _lib.ptr(cache_k), _lib.ptr(cache_v), _lib.ptr(lens), _lib.ptr(bt), _lib.ptr(sid),
             _c.c_longlong(cache_k.stride(0)), _c.c_longlong(cache_k.stride(1)), _c.c_int(page_size),
             _c.c_int(bt.shape[1] if bt is not None else 0), _lib.ptr(out), _lib.ptr(scratch), _c.c_int(B),

@@ -63,3 +63,17 @@ def test_captured_steps_of_different_sizes_keep_their_scratch():
             torch.full((1 << 22,), float("nan"), device="cuda")       # memory that a freed scratch buffer would share
             graph.replay()
             assert torch.equal(out, decode_attention(q, k, v, lens))
+
+
+# one query head per key head (multiply-add kernel) and four (tensor cores)
+@pytest.mark.parametrize("n_q", [2, 8])
+def test_lengths_of_64_bits_are_read_as_they_are(n_q):
+    from neuronx_distributed_llama3_2_b200.ops.attention import decode_attention
+
+    g = torch.Generator(device="cuda").manual_seed(n_q)
+    q = torch.randn(5, n_q, 64, generator=g, device="cuda").bfloat16()
+    k, v = (torch.randn(5, 2, 640, 64, generator=g, device="cuda").bfloat16() for _ in range(2))
+    lens = torch.tensor([1, 640, 129, 17, 128], device="cuda")
+    ref = decode_attention(q, k, v, lens.int())
+    assert torch.equal(decode_attention(q, k, v, lens), ref)
+    assert torch.equal(decode_attention(q, k, v, lens.repeat_interleave(2)[::2]), ref)      # not contiguous: converted
