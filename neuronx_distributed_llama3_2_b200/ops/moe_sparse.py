@@ -87,6 +87,13 @@ def glu_bias(src: torch.Tensor, gate_offset: int, up_offset: int, width: int, ga
     return clamped_glu_ref(g, u, limit, alpha, up_shift, act).to(src.dtype)
 
 
+def _router_mode(renormalize: bool, score: str, normalize: bool) -> int:
+    """``nxd_moe_router``'s form of the scores; what no form serves is refused here, whatever calls the kernel."""
+    assert score in ("softmax", "sigmoid") and not (renormalize and score == "sigmoid")
+    assert not normalize or (score == "softmax" and not renormalize)
+    return 3 if normalize else (2 if score == "sigmoid" else int(renormalize))
+
+
 def route(h: torch.Tensor, router_w: torch.Tensor, correction: Optional[torch.Tensor], top: int, scale: float,
           shared_gate_w: Optional[torch.Tensor] = None, logit_bias: Optional[torch.Tensor] = None,
           renormalize: bool = False, score: str = "softmax", normalize: bool = False) -> Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor]]:
@@ -95,8 +102,7 @@ def route(h: torch.Tensor, router_w: torch.Tensor, correction: Optional[torch.Te
     over the chosen logits only (``correction`` does not apply); ``score="sigmoid"``: every expert's score is the sigmoid
     of its own logit instead of the softmax over all of them; ``normalize`` (softmax scores): the chosen experts' scores are
     divided by their sum."""
-    assert score in ("softmax", "sigmoid") and not (renormalize and score == "sigmoid")
-    assert not normalize or (score == "softmax" and not renormalize)
+    mode = _router_mode(renormalize, score, normalize)
     N, W = h.shape
     R = router_w.shape[0]
     if _use_kernel(h) and router_w.dtype == torch.float32:
@@ -111,7 +117,7 @@ def route(h: torch.Tensor, router_w: torch.Tensor, correction: Optional[torch.Te
         rc = L.nxd_moe_router(_c.c_int(_code(h.dtype)), _lib.ptr(h), _lib.ptr(router_w.contiguous()), _lib.ptr(corr),
                               _lib.ptr(wsg), _lib.ptr(idx), _lib.ptr(wts), _lib.ptr(sg), _c.c_longlong(N), _c.c_int(W),
                               _c.c_int(R), _c.c_int(top), _c.c_float(scale), _lib.ptr(zb),
-                              _c.c_int(3 if normalize else (2 if score == "sigmoid" else int(renormalize))), _lib.stream_ptr())
+                              _c.c_int(mode), _lib.stream_ptr())
         _lib.check(rc, "nxd_moe_router", L)
         return idx, wts, sg
     hf = h.float()
@@ -275,6 +281,7 @@ def routed_forward(h: torch.Tensor, router, shared_gate_w: Optional[torch.Tensor
                    up_shift: float, shared_limit: float) -> torch.Tensor:
     """``route`` and ``sorted_forward`` in one call with one workspace (the weight on the expert's output).  ``router``: the module that
     ``route`` gets its arguments from; its parameters are contiguous fp32 (``router_fits``)."""
+    mode = _router_mode(router.renormalize, router.score, router.normalize)
     N, W = h.shape
     w_in, w_down, *shared = weights
     E, F, _ = w_down.shape
@@ -286,7 +293,6 @@ def routed_forward(h: torch.Tensor, router, shared_gate_w: Optional[torch.Tensor
         size.restype, size.argtypes, call.argtypes = _L, _WORKSPACE, _ROUTED
     work = torch.empty(size(N, top, W, F, E, Fs), dtype=torch.uint8, device=h.device)
     y = torch.empty(N, W, dtype=torch.float32, device=h.device)
-    mode = 3 if router.normalize else (2 if router.score == "sigmoid" else int(router.renormalize))
     rc = call(h.data_ptr(), router.linear_router.weight.data_ptr(), router.correction.data_ptr(),
               None if shared_gate_w is None else shared_gate_w.data_ptr(),
               None if router.logit_bias is None else router.logit_bias.data_ptr(), R, router.affinity_scale, mode, w_in.data_ptr(),

@@ -153,3 +153,18 @@ def _build_full_weights():
 
 def test_moe_expert_parallel_matches_golden():
     run_distributed(_ep_worker, 2)
+
+
+# scores that no form of the router serves: every way to the experts refuses them, the call that holds the router too
+@pytest.mark.parametrize("kw", [dict(score="sigmoid", normalize=True), dict(score="sigmoid", renormalize=True),
+                                dict(normalize=True, renormalize=True)])
+def test_router_forms_that_do_not_exist_are_refused(kw, monkeypatch):
+    from neuronx_distributed_llama3_2_b200.modules.moe.sparse import SparseMoE
+    from neuronx_distributed_llama3_2_b200.ops import _lib, moe_sparse
+
+    m, h = SparseMoE(16, 4, 2, 8, 7.0, **kw), torch.randn(3, 16)
+    with pytest.raises(AssertionError):
+        m(h)
+    monkeypatch.setattr(_lib, "lib", lambda *a: pytest.fail("the kernels were called"))
+    with pytest.raises(AssertionError):
+        moe_sparse.routed_forward(h, m.router, None, m._sorted_weights(), True, 7.0, 1.0, 1.0, 0.0)

@@ -158,3 +158,13 @@ def test_router_and_experts_in_one_call(tokens, kw):
         pairs = m(h, path="pairs")
     # the per-pair kernels: bf16 activations of fp32 sums in another order
     assert (whole - pairs).norm() <= 2.0 ** -8 * pairs.norm()
+
+
+@pytest.mark.parametrize("path", [None, "device", "pairs", "sorted"])
+@pytest.mark.parametrize("kw", [dict(score="sigmoid", normalize=True), dict(score="sigmoid", renormalize=True)])
+def test_router_forms_that_do_not_exist_are_refused_on_every_path(path, kw):
+    from neuronx_distributed_llama3_2_b200.modules.moe.sparse import SparseMoE
+
+    m = SparseMoE(512, 12, 4, 256, 7.0, dtype=torch.bfloat16, device="cuda", **kw).eval()
+    with torch.no_grad(), pytest.raises(AssertionError):
+        m(torch.zeros(64, 512, device="cuda").bfloat16(), path=path)
