@@ -293,7 +293,8 @@ def routed_forward(h: torch.Tensor, router, shared_gate_w: Optional[torch.Tensor
         size.restype, size.argtypes, call.argtypes = _L, _WORKSPACE, _ROUTED
     work = torch.empty(size(N, top, W, F, E, Fs), dtype=torch.uint8, device=h.device)
     y = torch.empty(N, W, dtype=torch.float32, device=h.device)
-    rc = call(h.data_ptr(), router.linear_router.weight.data_ptr(), router.correction.data_ptr(),
+    rc = call(h.data_ptr(), router.linear_router.weight.data_ptr(),
+              None if router.correction is None else router.correction.data_ptr(),
               None if shared_gate_w is None else shared_gate_w.data_ptr(),
               None if router.logit_bias is None else router.logit_bias.data_ptr(), R, router.affinity_scale, mode, w_in.data_ptr(),
               w_down.data_ptr(), shared[0].data_ptr() if shared else None, shared[1].data_ptr() if shared else None, y.data_ptr(),

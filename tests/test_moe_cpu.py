@@ -168,3 +168,29 @@ def test_router_forms_that_do_not_exist_are_refused(kw, monkeypatch):
     monkeypatch.setattr(_lib, "lib", lambda *a: pytest.fail("the kernels were called"))
     with pytest.raises(AssertionError):
         moe_sparse.routed_forward(h, m.router, None, m._sorted_weights(), True, 7.0, 1.0, 1.0, 0.0)
+
+
+def test_a_router_without_a_correction_goes_over_as_none(monkeypatch):
+    from types import SimpleNamespace
+
+    from neuronx_distributed_llama3_2_b200.modules.moe.sparse import SparseMoE
+    from neuronx_distributed_llama3_2_b200.ops import _lib, moe_sparse
+
+    m, h, calls = SparseMoE(16, 4, 2, 8, 7.0), torch.randn(3, 16), []
+
+    class Call:
+        argtypes = None
+
+        def __call__(self, *args):
+            calls.append(args)
+            return 0
+
+    class Size:
+        def __call__(self, *args):
+            return 64
+
+    monkeypatch.setattr(_lib, "lib", lambda *a: SimpleNamespace(nxd_moe_routed_forward=Call(), nxd_moe_sorted_workspace=Size()))
+    monkeypatch.setattr(_lib, "stream_ptr", lambda: None)
+    m.router.correction = None
+    moe_sparse.routed_forward(h, m.router, None, m._sorted_weights(), True, 7.0, 1.0, 1.0, 0.0)
+    assert calls[0][0] == h.data_ptr() and calls[0][2] is None
