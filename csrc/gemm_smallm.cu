@@ -97,6 +97,11 @@ struct Cfg {
     static constexpr int kNormBlocks = NORM ? (232448 - kSmemBytes) / (BT * kBK * 2) : 0;
     static_assert(kStagingBytes <= kPipeBytes, "the send buffer aliases the pipeline stages");
     static constexpr int kTmemCols = kAcc * BT < 32 ? 32 : kAcc * BT;
+    // columns of one tensor-memory load of the epilogue: a load of 32 from the second of two accumulators of 16 would read 16 columns
+    // that belong to nobody, or to the CTA beside
+    static constexpr int kLoadCols = BT < 32 ? BT : 32;
+    static_assert(kLoadCols == 16 || kLoadCols == 32, "width of a tensor-memory load");
+    static_assert((kAcc - 1) * BT + (BT + kLoadCols - 1) / kLoadCols * kLoadCols <= kTmemCols, "loads beyond the allocation");
     static_assert(kStageBytes % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
     static_assert(kSmemBytes <= 232448, "shared memory budget exceeded");
 };
@@ -316,24 +321,27 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
         TRACE_STAMP(5, threadIdx.x == 64);
         ptx::tcgen05_fence_after();
         const int nl = q * 32 + lane;
+        constexpr int kLoad = C::kLoadCols;
 #pragma unroll
         for (int a = 0; a < C::kAcc; ++a) {
             float* region = (splits == 1 ? staging : sendbuf) + a * (BT * kWRows);
 #pragma unroll
-            for (int c = 0; c < (BT + 31) / 32; ++c) {
-                if (c * 32 >= B) break;
-                uint32_t r[32];
+            for (int c = 0; c < BT / kLoad; ++c) {
+                if (c * kLoad >= B) break;
+                uint32_t r[kLoad];
                 if (has_k) {
-                    ptx::tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + a * BT + c * 32, r);
+                    const uint32_t at = tmem_base + ((uint32_t)(q * 32) << 16) + a * BT + c * kLoad;
+                    if constexpr (kLoad == 16) ptx::tmem_ld_32x32b_x16(at, r);
+                    else ptx::tmem_ld_32x32b_x32(at, r);
                     ptx::tmem_ld_wait();
                 } else {
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) r[j] = 0u;
+                    for (int j = 0; j < kLoad; ++j) r[j] = 0u;
                 }
                 // token b sits at row b of the buffer in both cases: owner * tpr + local = b
 #pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    if (c * 32 + j < B) region[(c * 32 + j) * kWRows + nl] = __uint_as_float(r[j]);
+                for (int j = 0; j < kLoad; ++j)
+                    if (c * kLoad + j < B) region[(c * kLoad + j) * kWRows + nl] = __uint_as_float(r[j]);
             }
         }
         TRACE_STAMP(6, threadIdx.x == 64);
