@@ -218,18 +218,31 @@ __device__ __forceinline__ uint64_t desc_b(uint32_t addr, uint32_t piece) {
            (uint64_t)4 << 61;
 }
 
-// Waits end: a kernel of this file that has waited for two seconds of clock gives up (no wait takes microseconds unless the device
-// is broken), its blocks put NaN where results are missing and return.
-__device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, volatile int* dead) {
+// Waits end.  One that has taken `limit` clocks (kWaitClocks is two seconds; the longest ones take some microseconds) gives up: `dead`
+// ends the other waits of the block, nxd_delta_scan_status tells the host, and NaN goes where results are missing.  A limit of zero
+// gives up without asking.
+constexpr long long kWaitClocks = 4000000000ll;
+
+__device__ int scan_gave_up;
+
+__device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, long long limit, volatile int* dead) {
     long long start = 0;
     for (int i = 1;; ++i) {
-        if (ptx::mbar_try_wait(bar, parity)) return true;
-        if ((i & 255) != 0) continue;
+        if (limit > 0 && ptx::mbar_try_wait(bar, parity)) return true;
+        if (limit > 0 && (i & 63) != 0) continue;        // the rest asked after every try: 227 us instead of 216 (4 heads of 64 x 128, 2 x 3497)
         if (*dead) return false;
         const long long now = clock64();
         if (start == 0) start = now;
-        else if (now - start > 4000000000ll) *dead = 1;
+        if (now - start < limit) continue;
+        *dead = 1;
+        scan_gave_up = 1;
+        return false;
     }
+}
+
+// the same for whole warps: the lanes leave it together and with one answer, as barriers and tensor-memory loads behind it want them
+__device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity, long long limit, volatile int* dead) {
+    return __all_sync(0xffffffffu, wait(bar, parity, limit, dead));
 }
 
 constexpr int kPairs = CW_COLS / 4;                      // pairs of columns of an epilogue thread (half of the columns)
@@ -265,14 +278,16 @@ __device__ __forceinline__ void put_row(uint8_t* base, int piece, int row, int g
 // of the products and half of the columns)
 template <int D>
 __global__ void __launch_bounds__(kThreads, 1)
-delta_chunk_scan_kernel(const Step p, const float* __restrict__ systems, const uint8_t* __restrict__ tiles, int c0, int count) {
+delta_chunk_scan_kernel(const Step p, const float* __restrict__ systems, const uint8_t* __restrict__ tiles, int c0, int count,
+                        long long limit) {
     using C = Cfg<D>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = ptx::align_smem_1024(smem_raw);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::kOffBar);
     uint64_t *empty = full + C::kSlots, *s_full = empty + C::kSlots, *u_full = s_full + 1, *v_full = u_full + 1, *accv = v_full + 1;
     uint64_t *acc1 = accv + 1, *acc3 = acc1 + C::kA1;    // accumulators: V, each 64 terms of the state, the state's update
-    uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc3 + 1);
+    uint64_t* drained = acc3 + 1;                        // every MMA has run
+    uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(drained + 1);
     __shared__ int bad[2][CW_COLS], any_bad[2];          // first token of a column whose value is not finite
     __shared__ int dead;
     // the warp's number as a value that the compiler knows to be the warp's: an MMA issued under a branch on threadIdx takes 60 clocks,
@@ -301,6 +316,7 @@ delta_chunk_scan_kernel(const Step p, const float* __restrict__ systems, const u
         ptx::mbar_init(accv, 1);
         for (int i = 0; i < C::kA1; ++i) ptx::mbar_init(&acc1[i], 1);
         ptx::mbar_init(acc3, 1);
+        ptx::mbar_init(drained, 1);
         dead = 0;
         ptx::fence_barrier_init();
     }
@@ -317,7 +333,7 @@ delta_chunk_scan_kernel(const Step p, const float* __restrict__ systems, const u
             int i = 0;
             for (; i < total; ++i) {
                 const int st = i % C::kSlots;
-                if (!wait(&empty[st], (uint32_t)(i / C::kSlots + 1) & 1, &dead)) break;
+                if (!wait(&empty[st], (uint32_t)(i / C::kSlots + 1) & 1, limit, &dead)) break;
                 // D = 64: the decayed keys are the first half of their tile (what the other rows multiply is not read)
                 const uint32_t bytes = D == 64 && i % (C::kTiles * 3) >= (C::kTiles - 1) * 3 ? PIECE_BYTES / 2 : PIECE_BYTES;
                 ptx::mbar_arrive_expect_tx(&full[st], bytes);
@@ -326,10 +342,9 @@ delta_chunk_scan_kernel(const Step p, const float* __restrict__ systems, const u
                              "l"(src + (long long)i * PIECE_BYTES), "r"(bytes), "r"(ptx::smem_u32(&full[st]))
                              : "memory");
             }
-            if (i < total) {                             // given up: the copies in flight still land in this block's memory
-                int none = 0;
-                for (int j = max(0, i - C::kSlots); j < i; ++j) wait(&full[j % C::kSlots], (uint32_t)(j / C::kSlots) & 1, &none);
-            }
+            int none = 0;                                // copies that no MMA has waited for still land in this block's memory
+            for (int j = max(0, i - C::kSlots); j < i; ++j)
+                wait(&full[j % C::kSlots], (uint32_t)(j / C::kSlots) & 1, kWaitClocks, &none);
         }
     } else if (warp == 1) {
         if (ptx::elect_one()) {
@@ -342,7 +357,7 @@ delta_chunk_scan_kernel(const Step p, const float* __restrict__ systems, const u
                 constexpr int kPer = 4 / decltype(halves)::value, kStep = (kKeys ? 2048 : 32) >> 4;
 #pragma unroll
                 for (int x = 0; x < 3; ++x) {
-                    if (!wait(&full[st], st_ph, &dead)) return false;
+                    if (!wait(&full[st], st_ph, limit, &dead)) return false;
                     ptx::tcgen05_fence_after();
                     const uint64_t da0 = ptx::make_smem_desc(ptx::smem_u32(smem + st * PIECE_BYTES), kKeys ? 8192 : 16, 1024);
                     constexpr uint32_t major = kKeys ? 1u << 15 : 0u;
@@ -363,21 +378,24 @@ delta_chunk_scan_kernel(const Step p, const float* __restrict__ systems, const u
             const uint64_t dv = desc_b(ptx::smem_u32(smem + C::kOffV), kSmall);
             for (int c = 0; c < chunks; ++c) {
                 const uint32_t ph = c & 1;
-                if (!wait(v_full, ph, &dead) || !product(std::false_type(), HV(), C::kAccV, dv)) break;
+                if (!wait(v_full, ph, limit, &dead) || !product(std::false_type(), HV(), C::kAccV, dv)) break;
                 ptx::umma_commit(accv);
-                if (!wait(s_full, ph, &dead)) break;
+                if (!wait(s_full, ph, limit, &dead)) break;
                 bool ok = true;
                 for (int kb = 0; kb < C::kA1 && ok; ++kb) {
                     ok = product(std::false_type(), H1(), kb * C::kHalves1 * C::kAccCols, ds + kb * (64 * kRow >> 4));
-                    ptx::umma_commit(&acc1[kb]);
+                    if (ok) ptx::umma_commit(&acc1[kb]);
                 }
                 if (!ok) break;
-                if (!wait(u_full, ph, &dead)) break;
+                if (!wait(u_full, ph, limit, &dead)) break;
                 // the state's update takes the accumulators that the epilogue has just read
                 for (int db = 0; db < C::kA3 && ok; ++db) ok = product(std::true_type(), Two(), 2 * db * C::kAccCols, du);
                 if (!ok) break;
                 ptx::umma_commit(acc3);
             }
+            int none = 0;                                // tensor memory is given back behind the last MMA
+            ptx::umma_commit(drained);
+            wait(drained, 0, kWaitClocks, &none);
         }
     } else if (warp < 4) {
         const int t = tid - 64;
@@ -391,8 +409,10 @@ delta_chunk_scan_kernel(const Step p, const float* __restrict__ systems, const u
                                                        : make_float4(0.f, 0.f, 0.f, 0.f);
         };
         fetch(0);
+        bool live = true;
         for (int c = 0; c < chunks; ++c) {
-            if (c > 0 && !wait(accv, (uint32_t)(c - 1) & 1, &dead)) break;      // the last V has been used
+            // the last V has been used.  What gives up runs on to the end: the barrier below wants both warps
+            if (c > 0 && live) live = wait_warp(accv, (uint32_t)(c - 1) & 1, limit, &dead);
             // A value that is not finite would reach the tokens before it through 0 * value: it goes over as zero, and the epilogue puts
             // NaN where it would have arrived
             if (t < CW_COLS) bad[c & 1][t] = CH;
@@ -435,20 +455,22 @@ delta_chunk_scan_kernel(const Step p, const float* __restrict__ systems, const u
         ptx::fence_proxy_async();
         ptx::mbar_arrive(s_full);
         const uint64_t nan = f2_pack(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff));
+        const volatile int* gone = &dead;
         int c = 0;
         for (; c < chunks; ++c) {
             const uint32_t ph = c & 1;
             const float gamma = systems[(e0 + c) * CHUNK_FLOATS + 2 * CH * CH + CH - 1];
             uint64_t r[kPairs] = {}, small[kPairs] = {}, rv[kPairs] = {};        // sums of their own for V and for the state
-            if (!wait(accv, ph, &dead)) break;
+            if (!wait_warp(accv, ph, limit, &dead)) break;
             ptx::tcgen05_fence_after();
 #pragma unroll
             for (int a = 0; a < C::kHalvesV; ++a) add_acc(at + C::kAccV + a * C::kAccCols, rv, small);
             bool ok = true;
 #pragma unroll
             for (int kb = 0; kb < C::kA1; ++kb) {
-                ok = ok && wait(&acc1[kb], ph, &dead);
+                ok = ok && wait_warp(&acc1[kb], ph, limit, &dead);
                 ptx::tcgen05_fence_after();
+                if (!ok) continue;
 #pragma unroll
                 for (int a = 0; a < C::kHalves1; ++a) add_acc(at + (kb * C::kHalves1 + a) * C::kAccCols, r, small);
             }
@@ -466,12 +488,13 @@ delta_chunk_scan_kernel(const Step p, const float* __restrict__ systems, const u
             ptx::fence_proxy_async();
             ptx::mbar_arrive(u_full);
             const int tok = (c0 + c) * CH + t;
+            if (__any_sync(0xffffffffu, *gone != 0)) break;     // another role gave up: the products may be of anything
             if (row >= CH && tok < n) {
 #pragma unroll
                 for (int j = 0; j < kPairs; j += 2)
                     *reinterpret_cast<ulonglong2*>(orow + tok * pitch + j0 + 2 * j) = make_ulonglong2(r[j], r[j + 1]);
             }
-            if (!wait(acc3, ph, &dead)) break;
+            if (!wait_warp(acc3, ph, limit, &dead)) break;
             ptx::tcgen05_fence_after();
             const uint64_t gamma2 = f2_pack(gamma, gamma);
 #pragma unroll
@@ -490,7 +513,7 @@ delta_chunk_scan_kernel(const Step p, const float* __restrict__ systems, const u
                 ptx::mbar_arrive(s_full);
             }
         }
-        if (c < chunks) {                                // given up
+        if (c < chunks || *gone != 0) {                  // given up
 #pragma unroll
             for (int i = 0; i < C::kBlocks; ++i)
 #pragma unroll
@@ -514,21 +537,37 @@ delta_chunk_scan_kernel(const Step p, const float* __restrict__ systems, const u
 }
 
 template <int D>
-int launch(const Step& s, const float* systems, uint8_t* tiles, int c0, int count, cudaStream_t st) {
+int launch(const Step& s, const float* systems, uint8_t* tiles, int c0, int count, long long limit, cudaStream_t st) {
     constexpr int factors = (CH * D + CH * MTP) * 4;
     NXD_CHECK_CUDA(nxd_allow_smem<delta_chunk_factors_kernel<D>>(factors));
     NXD_CHECK_CUDA(nxd_allow_smem<delta_chunk_scan_kernel<D>>(Cfg<D>::kSmem));
     delta_chunk_factors_kernel<D><<<dim3(count, s.H, s.B), FT, factors, st>>>(s.qn, s.kn, systems, tiles, s.n_new, s.Tn, c0, s.H, s.G);
     NXD_LAUNCH_CHECK();
-    delta_chunk_scan_kernel<D><<<dim3(s.Dv / CW_COLS, s.H, s.B), kThreads, Cfg<D>::kSmem, st>>>(s, systems, tiles, c0, count);
+    delta_chunk_scan_kernel<D><<<dim3(s.Dv / CW_COLS, s.H, s.B), kThreads, Cfg<D>::kSmem, st>>>(s, systems, tiles, c0, count,
+                                                                                                   limit);
     NXD_LAUNCH_CHECK();
     return 0;
 }
 
 }  // namespace
 
-int nxd_delta::launch_chunks_tc(const Step& s, const float* systems, uint8_t* tiles, int c0, int count, cudaStream_t st) {
-    if (s.D == 64) return launch<64>(s, systems, tiles, c0, count, st);
-    if (s.D == 128) return launch<128>(s, systems, tiles, c0, count, st);
-    return launch<256>(s, systems, tiles, c0, count, st);
+int nxd_delta::launch_chunks_tc(const Step& s, const float* systems, uint8_t* tiles, int c0, int count, long long wait_clocks,
+                                cudaStream_t st) {
+    const long long limit = wait_clocks < 0 ? kWaitClocks : wait_clocks;
+    if (s.D == 64) return launch<64>(s, systems, tiles, c0, count, limit, st);
+    if (s.D == 128) return launch<128>(s, systems, tiles, c0, count, limit, st);
+    return launch<256>(s, systems, tiles, c0, count, limit, st);
+}
+
+// *gave_up <- whether a scan on this device gave up a wait since the last call (its outputs and states are NaN from there on).  Waits
+// for the stream.
+NXD_API int nxd_delta_scan_status(int* gave_up, void* stream) {
+    const cudaStream_t st = (cudaStream_t)stream;
+    const int none = 0;
+    NXD_CHECK_CUDA(cudaMemcpyFromSymbolAsync(gave_up, scan_gave_up, sizeof(int), 0, cudaMemcpyDeviceToHost, st));
+    NXD_CHECK_CUDA(cudaStreamSynchronize(st));
+    if (*gave_up == 0) return 0;
+    NXD_CHECK_CUDA(cudaMemcpyToSymbolAsync(scan_gave_up, &none, sizeof(int), 0, cudaMemcpyHostToDevice, st));
+    NXD_CHECK_CUDA(cudaStreamSynchronize(st));
+    return 0;
 }

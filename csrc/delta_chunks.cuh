@@ -22,7 +22,8 @@ struct Step {
     int B, Tn, H, G, D, Dv;
 };
 
-// factors and scan of the chunks [c0, c0 + count), whose systems are in `systems`
-int launch_chunks_tc(const Step& s, const float* systems, uint8_t* tiles, int c0, int count, cudaStream_t st);
+// factors and scan of the chunks [c0, c0 + count), whose systems are in `systems`; wait_clocks: the clocks after which a wait inside
+// the scan gives up, -1: two seconds
+int launch_chunks_tc(const Step& s, const float* systems, uint8_t* tiles, int c0, int count, long long wait_clocks, cudaStream_t st);
 
 }  // namespace nxd_delta

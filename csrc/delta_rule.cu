@@ -645,7 +645,7 @@ int segment_chunks(int B, int Tn, int H, int D) {
 
 template <int D>
 int launch_chunks(const nxd_delta::Step& p, const float* gate, long long ld_a, int a_off, const float* beta, long long ld_b, int b_off,
-                  float* scratch, cudaStream_t st) {
+                  float* scratch, long long wait_clocks, cudaStream_t st) {
     const int NC = (p.Tn + CH - 1) / CH, seg = segment_chunks(p.B, p.Tn, p.H, D);
     const size_t smem = (size_t)3 * CH * DPITCH * sizeof(double);
     uint8_t* tiles = reinterpret_cast<uint8_t*>(scratch);
@@ -656,7 +656,7 @@ int launch_chunks(const nxd_delta::Step& p, const float* gate, long long ld_a, i
         delta_chunk_system_kernel<D><<<dim3(count, p.H, p.B), CW_THREADS, smem, st>>>(p.qn, p.kn, gate, ld_a, a_off, beta, ld_b, b_off,
                                                                                      systems, p.n_new, p.Tn, c0, p.H, p.G);
         NXD_LAUNCH_CHECK();
-        if (int rc = nxd_delta::launch_chunks_tc(p, systems, tiles, c0, count, st)) return rc;
+        if (int rc = nxd_delta::launch_chunks_tc(p, systems, tiles, c0, count, wait_clocks, st)) return rc;
     }
     return 0;
 }
@@ -743,10 +743,11 @@ NXD_API long long nxd_delta_scan_scratch(int B, int Tn, int H, int D, int Dv, in
 // OVERWRITTEN with g and beta (a first kernel, one thread per value; the recurrence then reads them).
 // S fp32 [lines, H, D, Dv], updated in place.  out fp32 [B * Tn, H, Dv].  scratch: nxd_delta_scan_scratch floats, or NULL
 // (token by token).
-NXD_API int nxd_delta_scan(const float* qn, const float* kn, const float* vn, float* apre, long long ld_a, int a_off,
-                           float* bpre, long long ld_b, int b_off, const float* a_log, const float* dt_bias, float* S,
-                           float* out, const int* q_start, const int* n_new, const int* seq_ids, int B, int Tn, int H, int G,
-                           int D, int Dv, int per_channel, float* scratch, void* stream) {
+// wait_clocks: the clocks after which a wait inside the chunk-wise form gives up (nxd_delta_scan_status), -1: two seconds.
+NXD_API int nxd_delta_scan_limited(const float* qn, const float* kn, const float* vn, float* apre, long long ld_a, int a_off,
+                                   float* bpre, long long ld_b, int b_off, const float* a_log, const float* dt_bias, float* S,
+                                   float* out, const int* q_start, const int* n_new, const int* seq_ids, int B, int Tn, int H, int G,
+                                   int D, int Dv, int per_channel, float* scratch, long long wait_clocks, void* stream) {
     if ((long long)B * Tn * H * Dv == 0) return 0;
     NXD_REQUIRE(G > 0 && H % G == 0, "delta rule: %d heads over %d query/key heads", H, G);
     NXD_REQUIRE(D >= 1 && D <= 1024, "delta rule: key size %d", D);
@@ -761,9 +762,9 @@ NXD_API int nxd_delta_scan(const float* qn, const float* kn, const float* vn, fl
     if (scratch != nullptr && nxd_delta_scan_scratch(B, Tn, H, D, Dv, per_channel) > 0 && al(qn) && al(kn) && al(vn) && al(S) &&
         al(out) && al(scratch)) {
         const nxd_delta::Step step{qn, kn, vn, S, out, q_start, n_new, seq_ids, B, Tn, H, G, D, Dv};
-        if (D == 64) return launch_chunks<64>(step, apre, ld_a, a_off, bpre, ld_b, b_off, scratch, st);
-        if (D == 128) return launch_chunks<128>(step, apre, ld_a, a_off, bpre, ld_b, b_off, scratch, st);
-        return launch_chunks<256>(step, apre, ld_a, a_off, bpre, ld_b, b_off, scratch, st);
+        if (D == 64) return launch_chunks<64>(step, apre, ld_a, a_off, bpre, ld_b, b_off, scratch, wait_clocks, st);
+        if (D == 128) return launch_chunks<128>(step, apre, ld_a, a_off, bpre, ld_b, b_off, scratch, wait_clocks, st);
+        return launch_chunks<256>(step, apre, ld_a, a_off, bpre, ld_b, b_off, scratch, wait_clocks, st);
     }
     // rows of a column per thread (NPT) and lanes per column (R, a power of two): the smallest slice that keeps R <= 4,
     // wider keys spread over more lanes (measured at 8 heads of 256 x 512, 2 x 4096 tokens: slices of 32 / 16 / 8 rows take
@@ -778,4 +779,12 @@ NXD_API int nxd_delta_scan(const float* qn, const float* kn, const float* vn, fl
     if (npt == 16) NXD_SCAN(16);
     NXD_SCAN(32);
 #undef NXD_SCAN
+}
+
+NXD_API int nxd_delta_scan(const float* qn, const float* kn, const float* vn, float* apre, long long ld_a, int a_off,
+                           float* bpre, long long ld_b, int b_off, const float* a_log, const float* dt_bias, float* S,
+                           float* out, const int* q_start, const int* n_new, const int* seq_ids, int B, int Tn, int H, int G,
+                           int D, int Dv, int per_channel, float* scratch, void* stream) {
+    return nxd_delta_scan_limited(qn, kn, vn, apre, ld_a, a_off, bpre, ld_b, b_off, a_log, dt_bias, S, out, q_start, n_new, seq_ids, B,
+                                  Tn, H, G, D, Dv, per_channel, scratch, -1, stream);
 }

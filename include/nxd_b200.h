@@ -463,6 +463,12 @@ int nxd_delta_scan(const float* qn, const float* kn, const float* vn, float* apr
                    float* bpre, long long ld_b, int b_off, const float* a_log, const float* dt_bias, float* S,
                    float* out, const int* q_start, const int* n_new, const int* seq_ids, int B, int Tn, int H, int G, int D,
                    int Dv, int per_channel, float* scratch, void* stream);
+/* the same with the clocks after which a wait inside it gives up (-1: two seconds); whether one did since the last call */
+int nxd_delta_scan_limited(const float* qn, const float* kn, const float* vn, float* apre, long long ld_a, int a_off,
+                           float* bpre, long long ld_b, int b_off, const float* a_log, const float* dt_bias, float* S,
+                           float* out, const int* q_start, const int* n_new, const int* seq_ids, int B, int Tn, int H, int G,
+                           int D, int Dv, int per_channel, float* scratch, long long wait_clocks, void* stream);
+int nxd_delta_scan_status(int* gave_up, void* stream);
 /* gate and up columns of a wider row (+ fp32 biases or NULL) -> gated activation as in nxd_clamped_glu, out [rows, F];
  * act_kind 1: the gate goes through the tanh form of gelu instead of g * sigmoid(alpha g) */
 int nxd_glu_bias(int dtype, const void* src, long long ld, int gate_off, int up_off, const float* gate_bias,

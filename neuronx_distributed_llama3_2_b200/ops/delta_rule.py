@@ -123,24 +123,7 @@ def delta_scan(qn: torch.Tensor, kn: torch.Tensor, vn: torch.Tensor, a_pre: torc
     B, T, G, D = qn.shape
     H, Dv = vn.shape[2], vn.shape[3]
     if qn.is_cuda and _lib.available(GROUP):
-        assert qn.is_contiguous() and kn.is_contiguous() and vn.is_contiguous() and S.is_contiguous()
-        assert a_pre.dtype == torch.float32 and b_pre.dtype == torch.float32 and a_pre.stride(1) == 1 and b_pre.stride(1) == 1
-        out = torch.empty(B, T, H, Dv, dtype=torch.float32, device=qn.device)
-        qs, nn_, sid = _i32(q_start), _i32(n_new), _i32(seq_ids)
-        L = _lib.lib(GROUP)
-        scratch = None
-        if not per_channel and T > 1:          # long steps run in chunks of 64 tokens
-            need = L.nxd_delta_scan_scratch
-            need.restype = _c.c_longlong
-            floats = need(_c.c_int(B), _c.c_int(T), _c.c_int(H), _c.c_int(D), _c.c_int(Dv), _c.c_int(0))
-            scratch = torch.empty(floats, dtype=torch.float32, device=qn.device) if floats else None
-        rc = L.nxd_delta_scan(_lib.ptr(qn), _lib.ptr(kn), _lib.ptr(vn), _lib.ptr(a_pre), _c.c_longlong(a_pre.stride(0)),
-                              _c.c_int(a_offset), _lib.ptr(b_pre), _c.c_longlong(b_pre.stride(0)), _c.c_int(b_offset),
-                              _lib.ptr(a_log), _lib.ptr(dt_bias), _lib.ptr(S), _lib.ptr(out), _lib.ptr(qs), _lib.ptr(nn_),
-                              _lib.ptr(sid), _c.c_int(B), _c.c_int(T), _c.c_int(H), _c.c_int(G), _c.c_int(D), _c.c_int(Dv),
-                              _c.c_int(int(per_channel)), _lib.ptr(scratch), _lib.stream_ptr())
-        _lib.check(rc, "nxd_delta_scan", L)
-        return out
+        return _scan_on_gpu(qn, kn, vn, a_pre, a_offset, b_pre, b_offset, a_log, dt_bias, S, q_start, per_channel, n_new, seq_ids)
     out = torch.zeros(B, T, H, Dv, dtype=torch.float32, device=qn.device)
     na = H * D if per_channel else H
     a = a_pre.reshape(B, T, -1)[..., a_offset: a_offset + na].float() + dt_bias.float()
@@ -162,3 +145,36 @@ def delta_scan(qn: torch.Tensor, kn: torch.Tensor, vn: torch.Tensor, a_pre: torc
             out[b, t] = torch.einsum("hdv,hd->hv", Sb, q)
         S[line] = Sb
     return out
+
+
+def _scan_on_gpu(qn, kn, vn, a_pre, a_offset, b_pre, b_offset, a_log, dt_bias, S, q_start, per_channel, n_new=None, seq_ids=None,
+                 wait_clocks: int = -1) -> torch.Tensor:
+    """``wait_clocks``: clocks after which a wait inside the chunk-wise kernel gives up, -1: two seconds (``scan_gave_up``)."""
+    B, T, G, D = qn.shape
+    H, Dv = vn.shape[2], vn.shape[3]
+    assert qn.is_contiguous() and kn.is_contiguous() and vn.is_contiguous() and S.is_contiguous()
+    assert a_pre.dtype == torch.float32 and b_pre.dtype == torch.float32 and a_pre.stride(1) == 1 and b_pre.stride(1) == 1
+    out = torch.empty(B, T, H, Dv, dtype=torch.float32, device=qn.device)
+    qs, nn_, sid = _i32(q_start), _i32(n_new), _i32(seq_ids)
+    L = _lib.lib(GROUP)
+    scratch = None
+    if not per_channel and T > 1:          # long steps run in chunks of 64 tokens
+        need = L.nxd_delta_scan_scratch
+        need.restype = _c.c_longlong
+        floats = need(_c.c_int(B), _c.c_int(T), _c.c_int(H), _c.c_int(D), _c.c_int(Dv), _c.c_int(0))
+        scratch = torch.empty(floats, dtype=torch.float32, device=qn.device) if floats else None
+    rc = L.nxd_delta_scan_limited(_lib.ptr(qn), _lib.ptr(kn), _lib.ptr(vn), _lib.ptr(a_pre), _c.c_longlong(a_pre.stride(0)),
+                                  _c.c_int(a_offset), _lib.ptr(b_pre), _c.c_longlong(b_pre.stride(0)), _c.c_int(b_offset),
+                                  _lib.ptr(a_log), _lib.ptr(dt_bias), _lib.ptr(S), _lib.ptr(out), _lib.ptr(qs), _lib.ptr(nn_),
+                                  _lib.ptr(sid), _c.c_int(B), _c.c_int(T), _c.c_int(H), _c.c_int(G), _c.c_int(D), _c.c_int(Dv),
+                                  _c.c_int(int(per_channel)), _lib.ptr(scratch), _c.c_longlong(wait_clocks), _lib.stream_ptr())
+    _lib.check(rc, "nxd_delta_scan", L)
+    return out
+
+
+def scan_gave_up() -> bool:
+    """Whether a ``delta_scan`` on the current device gave up waiting inside its kernel since the last call of this function: its
+    outputs and states are NaN from there on.  Waits for the current stream."""
+    flag, L = _c.c_int(0), _lib.lib(GROUP)
+    _lib.check(L.nxd_delta_scan_status(_c.byref(flag), _lib.stream_ptr()), "nxd_delta_scan_status", L)
+    return bool(flag.value)

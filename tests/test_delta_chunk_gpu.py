@@ -173,3 +173,36 @@ def test_steps_in_several_launches_are_the_same():
         ref = dr.delta_scan(q[b:b + 1], k[b:b + 1], v[b:b + 1], a_pre[rows].clone(), 0, b_pre[rows].clone(), 0, a_log, dt_bias, one,
                             start[:1], False, n_new=new[b:b + 1])
         assert torch.equal(out[b], ref[0]) and torch.equal(state[b], one[0])
+
+
+# limits from "at once" to "never": what gives up says so and leaves NaN behind its last good chunk, and the next call is sound
+@pytest.mark.parametrize("D,Dv", [(64, 64), (128, 96), (256, 64)])
+def test_a_wait_that_runs_out_is_reported(D, Dv):
+    from neuronx_distributed_llama3_2_b200.ops import delta_rule as dr
+
+    B, T, H = 2, 421, 3
+    gen = torch.Generator(device="cuda").manual_seed(D)
+
+    def normal(*s):
+        return torch.randn(*s, generator=gen, device="cuda")
+
+    q, k = (F.normalize(normal(B, T, H, D), dim=-1) for _ in range(2))
+    v, a_pre, b_pre, S = normal(B, T, H, Dv), normal(B * T, H), normal(B * T, H), normal(B, H, D, Dv)
+    a_log, dt_bias = normal(H) - 2, normal(H)
+    start = torch.ones(B, dtype=torch.int32, device="cuda")
+
+    def run(clocks):
+        state = S.clone()
+        out = dr._scan_on_gpu(q, k, v, a_pre.clone(), 0, b_pre.clone(), 0, a_log, dt_bias, state, start, False, wait_clocks=clocks)
+        return out, state, dr.scan_gave_up()
+
+    dr.scan_gave_up()
+    out, state, gave_up = run(-1)
+    assert not gave_up and torch.isfinite(state).all()
+    for clocks in (0, 100, 1000, 10000, 100000, -1):
+        x, s, gave_up = run(clocks)
+        assert (s.isnan() | (s == state)).all() and (x.isnan() | (x == out)).all()
+        assert gave_up or not (s.isnan().any() or x.isnan().any())
+        assert gave_up != (clocks == -1) or 0 < clocks   # in between it depends on the clock
+        if clocks == 0:
+            assert s.isnan().all() and x.isnan().all()
