@@ -98,6 +98,29 @@ def test_chunks_are_no_further_off_than_single_tokens(D, common, strength, rate)
     assert S <= 1.25 * S_tokens + 2.0 ** -22
 
 
+# decays of a half and of a fifth per token: few tokens count, and every value is a handful of roundings -- of the factors, of U's and the
+# state's three sums each, 2^-25.5 of a value on average: 6 + 2 of them in square 0.6e-7, a quarter more for the scatter
+@pytest.mark.parametrize("strength", [0.0, 1.0])
+@pytest.mark.parametrize("D", [64, 128, 256])
+def test_chunks_with_strong_decays_are_off_by_their_last_roundings(D, strength):
+    from neuronx_distributed_llama3_2_b200.ops import delta_rule as dr
+
+    T, H, Dv = 640, 4, 128
+    gen = torch.Generator(device="cuda").manual_seed(D)
+
+    def normal(*s):
+        return torch.randn(*s, generator=gen, device="cuda")
+
+    q, k = (F.normalize(normal(1, T, H, D), dim=-1) for _ in range(2))
+    q, v, S = q * D ** -0.5, normal(1, T, H, Dv), normal(1, H, D, Dv)
+    g, beta, before = normal(T, H), normal(T, H), S[0].double()
+    out = dr.delta_scan(q, k, v, g, 0, beta, 0, normal(H) * 0.1 + strength, normal(H) * 0.1, S,
+                        torch.ones(1, dtype=torch.int32, device="cuda"), False)
+    want, state = _oracle(q[0].double(), k[0].double(), v[0].double(), g.double(), beta.double(), before)     # the rounded gates
+    assert (out[0] - want).norm() <= 1.25 * 2.0 ** -24 * want.norm()
+    assert (S[0] - state).norm() <= 1.25 * 2.0 ** -24 * state.norm()
+
+
 def test_a_token_that_is_not_a_number_leaves_the_tokens_before_it_alone():
     from neuronx_distributed_llama3_2_b200.ops import delta_rule as dr
 
