@@ -16,11 +16,8 @@
 // room), x0 y0 shares its accumulator with nothing, the rest is added in fp32.  (With x1 y0 and x2 y0 in it the output was 1.5e-7
 // off instead of 0.8e-7.)
 //
-// 4 x 2048 tokens, 4 heads of 128 x 256: factors 39 us, scan 100 us, against 350 us for the whole in fp32 on the multiply-add pipes;
-// output 1.28e-7 and state 1.59e-7 off from float64 against 1.32e-7 and 1.59e-7.  A chunk takes the scan 3.1 us: 48 MMAs of 41 to 57
-// clocks (41 with 32 columns, 57 with 96), the rest latencies of its four hand-overs.  With 64 key channels and many heads of 64
-// columns the left operands (120 KB per head and chunk, read twice) cost what the faster scan wins: 16 x 2048 tokens, 32 heads of 64 x
-// 64 2576 us, 2502 before; 4 heads of 64 x 128, 2 x 3497 tokens 237 us, 515 before.
+// 4 x 2048 tokens, 4 heads of 128 x 256: factors 39 us, scan 100 us, against 350 us for the whole in fp32 on the multiply-add pipes.  A
+// chunk takes the scan 3.1 us: 48 MMAs of 41 to 57 clocks (41 with 32 columns, 57 with 96), the rest latencies of its four hand-overs.
 #include <type_traits>
 
 #include "delta_chunks.cuh"

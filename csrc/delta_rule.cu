@@ -485,8 +485,9 @@ int launch_scan(const float* qn, const float* kn, const float* vn, const float* 
 // (the WY form of Householder products; Yang, Wang, Zhang, Shen, Kim, "Parallelizing Linear Transformers with the Delta Rule
 // over Sequence Length").  Decay ratios are products, never quotients or exponentials of sums, so a decay of any size is
 // exact to rounding and underflows to the right limit.  delta_chunk_system makes M, P M, Gamma and L[CH-1][.] of every (chunk, head,
-// row) in parallel, in fp64; delta_chunks.cu has the rest, on the tensor cores.
-constexpr int CW_THREADS = 256, DPITCH = CH + 4;
+// row) in parallel, in fp64; delta_chunks.cu has the rest, on the tensor cores; delta_chunk_scan_fp32 serves where its operand tiles cost
+// more than they save (tensor_core_scan).
+constexpr int CW_THREADS = 256, DPITCH = CH + 4, CP = CH + 4;
 
 // c [8 x 8] += a [8 x 4] b [4 x 8]: a is row lane / 4, column lane % 4; b row lane % 4, column lane / 4; c row lane / 4, columns
 // 2 (lane % 4) and the next
@@ -635,6 +636,261 @@ delta_chunk_system_kernel(const float* __restrict__ qn, const float* __restrict_
     }
 }
 
+// The rest in fp32, per (32 value columns, head, row), sequential over chunks with the state slice in shared memory: four products per
+// chunk, register-tiled, on packed pairs of fp32 multiply-adds (pairs run along the contraction, so both operands are read as 16-byte
+// pieces and nothing is shuffled).  Bound by the fp32 pipes and the chain of a chunk's phases (11 us of 128 x 256 alone on an SM).
+__device__ __forceinline__ ulonglong2 ld_pairs(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
+
+// acc[i][j] += <a row i, b row j> over 4 values
+template <int R, int C>
+__device__ __forceinline__ void dot_step(uint64_t (&acc)[R][C], const ulonglong2 (&a)[R], const ulonglong2 (&b)[C]) {
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < C; ++j) acc[i][j] = f2_fma(a[i].y, b[j].y, f2_fma(a[i].x, b[j].x, acc[i][j]));
+}
+
+template <int R, int C>
+__device__ __forceinline__ void add_pairs(uint64_t (&acc)[R][C], const uint64_t (&part)[R][C]) {
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < C; ++j) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc[i][j]) : "l"(part[i][j]));
+}
+
+// grid (Dv / 32, H, B).  Rows of a thread in the 64-row products: 4 w + rg and 60 - 4 w + rg (w the warp, rg = lane / 8), so
+// that the triangular products cost every warp the same; columns cg + 8 i (cg = lane % 8).
+template <int D>
+__global__ void __launch_bounds__(CW_THREADS, D == 64 ? 2 : 1)
+delta_chunk_scan_fp32_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vn,
+                             const float* __restrict__ scratch, float* __restrict__ S, float* __restrict__ out,
+                             const int* __restrict__ q_start, const int* __restrict__ n_new, const int* __restrict__ seq_ids, int Tn,
+                             int NC, int H, int G, int Dv) {
+    extern __shared__ __align__(16) float smem[];
+    constexpr int DP = D + 4, DT = D / 32, KB = D <= 128 ? 2 : 1;     // KB: buffers of K
+    float* Kb = smem;                          // [KB][CH][DP]
+    float* Qs = Kb + KB * CH * DP;             // [CH][DP]
+    float* Ss = Qs + CH * DP;                  // [32][DP] the state slice, a value column per row
+    float* Ms = Ss + CW_COLS * DP;             // [CH][CP]
+    float* Ps = Ms + CH * CP;                  // [CH][CP] P M
+    float* Rs = Ps + CH * CP;                  // [32][CP] V - diag(Gamma) K S, a value column per row
+    float* Us = Rs + CW_COLS * CP;             // [32][CP] U
+    float* gam2 = Us + CW_COLS * CP;           // [2][2 CH] Gamma and L[CH-1][.] of this chunk and the next
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int col0 = blockIdx.x * CW_COLS, h = blockIdx.y, b = blockIdx.z, kvh = h / (H / G);
+    const int n = n_new != nullptr ? min(n_new[b], Tn) : Tn;
+    const long long row0 = (long long)b * Tn;
+    float* orow = out + (row0 * H + h) * Dv + col0;              // + t * H * Dv
+    for (int i = tid; i < (Tn - max(n, 0)) * CW_COLS; i += CW_THREADS)       // padding rows
+        orow[(long long)(max(n, 0) + i / CW_COLS) * H * Dv + i % CW_COLS] = 0.f;
+    if (n <= 0) return;
+    const int line = seq_ids != nullptr ? seq_ids[b] : b;
+    float* Sb = S + ((long long)line * H + h) * D * Dv + col0;
+    const bool fresh = q_start[b] == 0;
+    for (int i = tid; i < D * CW_COLS; i += CW_THREADS) {
+        const int d = i / CW_COLS, j = i % CW_COLS;
+        Ss[j * DP + d] = fresh ? 0.f : Sb[(long long)d * Dv + j];
+    }
+    const float* chunk0 = scratch + ((long long)b * H + h) * NC * CHUNK_FLOATS;
+    const int chunks = (n + CH - 1) / CH;
+    auto rows = [&](const float* src, float* dst, int c) {       // K or Q rows of chunk c
+        if (c < chunks)
+            for (int i = tid; i < CH * (D / 4); i += CW_THREADS) {
+                const int t = i / (D / 4), d = (i % (D / 4)) * 4;
+                const bool ok = c * CH + t < n;
+                mma::cp_async16((uint32_t)__cvta_generic_to_shared(dst + t * DP + d),
+                                src + ((row0 + (ok ? c * CH + t : 0)) * G + kvh) * D + d, ok);
+            }
+    };
+    auto square = [&](int off, float* dst, int c) {              // M or P of chunk c
+        if (c < chunks)
+            for (int i = tid; i < CH * (CH / 4); i += CW_THREADS) {
+                const int t = i / (CH / 4), x = (i % (CH / 4)) * 4;
+                mma::cp_async16((uint32_t)__cvta_generic_to_shared(dst + t * CP + x),
+                                chunk0 + (long long)c * CHUNK_FLOATS + off + t * CH + x, true);
+            }
+    };
+    auto factors = [&](int c) {                                  // Gamma and L[CH-1][.] of chunk c
+        if (c < chunks && tid < 2 * CH / 4)
+            mma::cp_async16((uint32_t)__cvta_generic_to_shared(gam2 + (c & 1) * 2 * CH + tid * 4),
+                            chunk0 + (long long)c * CHUNK_FLOATS + 2 * CH * CH + tid * 4, true);
+    };
+    rows(kn, Kb, 0);
+    rows(qn, Qs, 0);
+    square(0, Ms, 0);
+    factors(0);
+    mma::cp_async_commit();
+    square(CH * CH, Ps, 0);
+    mma::cp_async_commit();
+    const int rg = lane >> 3, cg = lane & 7, ra = 4 * warp + rg, rb = 60 - 4 * warp + rg;
+    for (int c = 0; c < chunks; ++c) {
+        const float* Ks = Kb + (KB == 2 ? (c & 1) * CH * DP : 0);
+        const int t0 = c * CH;
+        const float *gam = gam2 + (c & 1) * 2 * CH, *last = gam + CH;
+        float v[2][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[0][i] = t0 + ra < n ? vn[((row0 + t0 + ra) * H + h) * Dv + col0 + cg + 8 * i] : 0.f;
+            v[1][i] = t0 + rb < n ? vn[((row0 + t0 + rb) * H + h) * Dv + col0 + cg + 8 * i] : 0.f;
+        }
+        mma::cp_async_wait<1>();               // everything but P
+        __syncthreads();
+        if (KB == 2) {
+            rows(kn, Kb + ((c + 1) & 1) * CH * DP, c + 1);
+            mma::cp_async_commit();
+        }
+        uint64_t acc[4][4] = {};               // K S of rows ra, rb; Q S of rows ra, rb
+#pragma unroll 1
+        for (int d0 = 0; d0 < D; d0 += 16) {   // sums of 16 first: half the rounding error of one long chain
+            uint64_t part[4][4] = {};
+#pragma unroll
+            for (int d = d0; d < d0 + 16; d += 4) {
+                const ulonglong2 a[4] = {ld_pairs(Ks + ra * DP + d), ld_pairs(Ks + rb * DP + d), ld_pairs(Qs + ra * DP + d),
+                                         ld_pairs(Qs + rb * DP + d)};
+                ulonglong2 sb[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) sb[j] = ld_pairs(Ss + (cg + 8 * j) * DP + d);
+                dot_step(part, a, sb);
+            }
+            add_pairs(acc, part);
+        }
+        const float ga = gam[ra], gb = gam[rb];
+        float o[2][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            Rs[(cg + 8 * i) * CP + ra] = fmaf(-ga, f2_lo(acc[0][i]) + f2_hi(acc[0][i]), v[0][i]);
+            Rs[(cg + 8 * i) * CP + rb] = fmaf(-gb, f2_lo(acc[1][i]) + f2_hi(acc[1][i]), v[1][i]);
+            o[0][i] = ga * (f2_lo(acc[2][i]) + f2_hi(acc[2][i]));
+            o[1][i] = gb * (f2_lo(acc[3][i]) + f2_hi(acc[3][i]));
+        }
+        __syncthreads();
+        rows(qn, Qs, c + 1);                   // the queries of this chunk have been used
+        mma::cp_async_commit();
+        // rows ra and rb of a lower triangular 64 x 64 matrix times the columns of X [32][CP]
+        auto triangular = [&](const float* M, const float* X, uint64_t (&y)[2][4]) {
+            const int e = 4 * warp, f = 60 - 4 * warp;           // the blocks of the diagonal: [e, e + 4) and [f, f + 4)
+#pragma unroll 1
+            for (int s0 = 0; s0 < f; s0 += 16) {                 // sums of 16 first, as above
+                uint64_t part[2][4] = {};
+#pragma unroll
+                for (int s = s0; s < s0 + 16; s += 4) {
+                    if (s >= f) break;
+                    const ulonglong2 a = ld_pairs(M + rb * CP + s);
+                    ulonglong2 xb[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        xb[j] = ld_pairs(X + (cg + 8 * j) * CP + s);
+                        part[1][j] = f2_fma(a.y, xb[j].y, f2_fma(a.x, xb[j].x, part[1][j]));
+                    }
+                    if (s >= e) continue;
+                    const ulonglong2 c = ld_pairs(M + ra * CP + s);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) part[0][j] = f2_fma(c.y, xb[j].y, f2_fma(c.x, xb[j].x, part[0][j]));
+                }
+                add_pairs(y, part);
+            }
+            // on the diagonal the entries behind the row's own are left out, not multiplied by zero: a token that is not a
+            // number does not reach the tokens before it
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int row = half ? rb : ra, s = half ? f : e;
+                const float4 m = *reinterpret_cast<const float4*>(M + row * CP + s);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float4 x = *reinterpret_cast<const float4*>(X + (cg + 8 * j) * CP + s);
+                    float d = m.x * x.x;
+                    if (rg >= 1) d = fmaf(m.y, x.y, d);
+                    if (rg >= 2) d = fmaf(m.z, x.z, d);
+                    if (rg >= 3) d = fmaf(m.w, x.w, d);
+                    y[half][j] = f2_pack(f2_lo(y[half][j]) + d, f2_hi(y[half][j]));
+                }
+            }
+        };
+        uint64_t y[2][4] = {};
+        triangular(Ms, Rs, y);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            Us[(cg + 8 * i) * CP + ra] = f2_lo(y[0][i]) + f2_hi(y[0][i]);
+            Us[(cg + 8 * i) * CP + rb] = f2_lo(y[1][i]) + f2_hi(y[1][i]);
+        }
+        mma::cp_async_wait<KB>();              // P of this chunk (the groups behind it: Q and, with two buffers, K)
+        __syncthreads();
+        square(0, Ms, c + 1);
+        factors(c + 1);
+        mma::cp_async_commit();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y[0][i] = y[1][i] = 0ull;
+        triangular(Ps, Rs, y);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (t0 + ra < n) orow[(long long)(t0 + ra) * H * Dv + cg + 8 * i] = o[0][i] + (f2_lo(y[0][i]) + f2_hi(y[0][i]));
+            if (t0 + rb < n) orow[(long long)(t0 + rb) * H * Dv + cg + 8 * i] = o[1][i] + (f2_lo(y[1][i]) + f2_hi(y[1][i]));
+        }
+        // S[.][j] <- Gamma S + sum_s last_s U[s][j] K[s][.]: DT key channels x 4 value columns per thread
+        {
+            const int d0 = ((warp & 3) * 8 + cg) * DT, j0 = (warp >> 2) * 16 + rg;       // columns j0 + 4 i
+            const uint64_t gl = f2_pack(gam[CH - 1], gam[CH - 1]);
+            uint64_t st[4][DT / 2] = {};       // the chunk's own part; the decayed state joins it once
+#pragma unroll 1
+            for (int s0 = 0; s0 < CH; s0 += 16) {
+                uint64_t part[4][DT / 2] = {};
+#pragma unroll 2
+                for (int s = s0; s < s0 + 16; s += 4) {
+                    float u[4][4], lw[4];
+                    *reinterpret_cast<float4*>(lw) = *reinterpret_cast<const float4*>(last + s);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        *reinterpret_cast<float4*>(u[i]) = *reinterpret_cast<const float4*>(Us + (j0 + 4 * i) * CP + s);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        uint64_t kv[DT / 2];
+#pragma unroll
+                        for (int x = 0; x < DT / 2; ++x)
+                            kv[x] = *reinterpret_cast<const uint64_t*>(Ks + (s + q) * DP + d0 + 2 * x);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float w = u[i][q] * lw[q];
+                            const uint64_t ww = f2_pack(w, w);
+#pragma unroll
+                            for (int x = 0; x < DT / 2; ++x) part[i][x] = f2_fma(kv[x], ww, part[i][x]);
+                        }
+                    }
+                }
+                add_pairs(st, part);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int x = 0; x < DT / 2; ++x) {
+                    uint64_t* at = reinterpret_cast<uint64_t*>(Ss + (j0 + 4 * i) * DP + d0 + 2 * x);
+                    *at = f2_fma(*at, gl, st[i][x]);
+                }
+        }
+        __syncthreads();                       // K, P, U and the old state are free
+        if (KB == 1) rows(kn, Kb, c + 1);
+        mma::cp_async_commit();
+        square(CH * CH, Ps, c + 1);
+        mma::cp_async_commit();
+    }
+    for (int i = tid; i < D * CW_COLS; i += CW_THREADS) {
+        const int d = i / CW_COLS, j = i % CW_COLS;
+        Sb[(long long)d * Dv + j] = Ss[j * DP + d];
+    }
+}
+
+// The tensor-core scan reads operand tiles (147 to 344 KB) that another kernel writes per (row, head, chunk); with one or two slices of 32
+// value columns and enough (row, head) pairs to fill the chip they cost more than its short chain saves.  Tensor cores / fp32, us, 1024
+// tokens:  one slice, 64 and 128 channels, 64 pairs 181 / 207 and 235 / 279, 96 247 / 246 and 330 / 332, 256 612 / 484 and 852 / 732;
+// two slices of 64 channels, 256 pairs 683 / 692, 512 1340 / 1266, and 192 tokens, 96 pairs 64 / 69, 128 88 / 80, 384 213 / 207 (320
+// tokens 333 / 335).  Two slices of 128 channels, 512 pairs 1826 / 1959.  One slice of 256 channels crosses at 96 too (128 pairs 764 /
+// 613, 512 1515 / 1214 at 512 tokens), but up to 256 pairs a row is to come out the same alone and among others.
+bool tensor_core_scan(int B, int Tn, int H, int D, int Dv) {
+    const long long pairs = (long long)B * H;
+    if (Dv == CW_COLS) return pairs < (D == 256 ? 257 : 96);
+    if (Dv == 2 * CW_COLS && D == 64) return pairs < (Tn <= 5 * CH ? 128 : 512);
+    return true;
+}
+
 // chunks of a step that are worked on at once: the operand tiles (147 to 344 KB per row, head and chunk) take half a gigabyte at most,
 // longer steps run in several launches
 int segment_chunks(int B, int Tn, int H, int D) {
@@ -648,9 +904,22 @@ int launch_chunks(const nxd_delta::Step& p, const float* gate, long long ld_a, i
                   float* scratch, long long wait_clocks, cudaStream_t st) {
     const int NC = (p.Tn + CH - 1) / CH, seg = segment_chunks(p.B, p.Tn, p.H, D);
     const size_t smem = (size_t)3 * CH * DPITCH * sizeof(double);
+    NXD_CHECK_CUDA(nxd_allow_smem<delta_chunk_system_kernel<D>>((int)smem));
+    if (!tensor_core_scan(p.B, p.Tn, p.H, D, p.Dv)) {
+        constexpr int DP = D + 4;
+        constexpr int scan = ((D <= 128 ? 3 : 2) * CH * DP + CW_COLS * DP + 2 * CH * CP + 2 * CW_COLS * CP + 4 * CH) * (int)sizeof(float);
+        static_assert(scan <= 232448, "shared memory");
+        NXD_CHECK_CUDA(nxd_allow_smem<delta_chunk_scan_fp32_kernel<D>>(scan));
+        delta_chunk_system_kernel<D><<<dim3(NC, p.H, p.B), CW_THREADS, smem, st>>>(p.qn, p.kn, gate, ld_a, a_off, beta, ld_b, b_off,
+                                                                                  scratch, p.n_new, p.Tn, 0, p.H, p.G);
+        NXD_LAUNCH_CHECK();
+        delta_chunk_scan_fp32_kernel<D><<<dim3(p.Dv / CW_COLS, p.H, p.B), CW_THREADS, scan, st>>>(
+            p.qn, p.kn, p.vn, scratch, p.S, p.out, p.q_start, p.n_new, p.seq_ids, p.Tn, NC, p.H, p.G, p.Dv);
+        NXD_LAUNCH_CHECK();
+        return 0;
+    }
     uint8_t* tiles = reinterpret_cast<uint8_t*>(scratch);
     float* systems = scratch + (long long)p.B * p.H * seg * (nxd_delta::chunk_tiles(D) * nxd_delta::TILE_BYTES / 4);
-    NXD_CHECK_CUDA(nxd_allow_smem<delta_chunk_system_kernel<D>>((int)smem));
     for (int c0 = 0; c0 < NC; c0 += seg) {
         const int count = min(seg, NC - c0);
         delta_chunk_system_kernel<D><<<dim3(count, p.H, p.B), CW_THREADS, smem, st>>>(p.qn, p.kn, gate, ld_a, a_off, beta, ld_b, b_off,
@@ -734,6 +1003,7 @@ NXD_API int nxd_delta_conv_state(int dtype, const void* proj, long long ld, int 
 // sizes of 64 / 128 / 256, value sizes in whole slices of 32 columns, steps of at least three chunks.
 NXD_API long long nxd_delta_scan_scratch(int B, int Tn, int H, int D, int Dv, int per_channel) {
     if (per_channel || (D != 64 && D != 128 && D != 256) || Dv % CW_COLS != 0 || Tn < 3 * CH || B > 65535 || H > 65535) return 0;
+    if (!tensor_core_scan(B, Tn, H, D, Dv)) return (long long)B * H * ((Tn + CH - 1) / CH) * CHUNK_FLOATS;
     return (long long)B * H * segment_chunks(B, Tn, H, D) * (CHUNK_FLOATS + nxd_delta::chunk_tiles(D) * nxd_delta::TILE_BYTES / 4);
 }
 

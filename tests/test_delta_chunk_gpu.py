@@ -229,3 +229,31 @@ def test_a_wait_that_runs_out_is_reported(D, Dv):
         assert gave_up != (clocks == -1) or 0 < clocks   # in between it depends on the clock
         if clocks == 0:
             assert s.isnan().all() and x.isnan().all()
+
+
+# on either side of the lines between the scans: (row, head) pairs and tokens with one slice of 32 value columns and with two
+@pytest.mark.parametrize("D,Dv,B,H,T,fp32", [(64, 32, 5, 19, 200, False), (64, 32, 3, 32, 200, True), (128, 32, 3, 32, 257, True),
+                                             (256, 32, 8, 32, 192, False), (256, 32, 9, 32, 192, True), (64, 64, 4, 32, 320, True),
+                                             (64, 64, 4, 32, 321, False), (64, 64, 16, 32, 385, True), (64, 96, 16, 32, 192, False)])
+def test_both_scans_match_float64(D, Dv, B, H, T, fp32):
+    from neuronx_distributed_llama3_2_b200.ops import _lib, delta_rule as dr
+
+    gen = torch.Generator(device="cuda").manual_seed(D + Dv + B)
+
+    def normal(*s):
+        return torch.randn(*s, generator=gen, device="cuda")
+
+    floats = _lib.lib().nxd_delta_scan_scratch(B, T, H, D, Dv, 0)
+    assert (floats == B * H * -(-T // 64) * (2 * 64 * 64 + 2 * 64)) == fp32          # the fp32 scan has no operand tiles
+    q, k = (F.normalize(normal(B, T, H, D), dim=-1) for _ in range(2))
+    v, g, beta, S = normal(B, T, H, Dv), normal(B * T, H), normal(B * T, H), normal(B, H, D, Dv)
+    new = [T, 130] + [T - b for b in range(2, B)]
+    before = S.clone()
+    out = dr.delta_scan(q, k, v, g, 0, beta, 0, normal(H) - 2, normal(H), S, torch.ones(B, dtype=torch.int32, device="cuda"), False,
+                        n_new=torch.tensor(new, dtype=torch.int32, device="cuda"))
+    for b in (0, 1, B - 1):
+        n, rows = new[b], slice(b * T, b * T + new[b])
+        want, state = _oracle(q[b, :n].double(), k[b, :n].double(), v[b, :n].double(), g[rows].double(), beta[rows].double(), before[b].double())
+        # sums of fp32 roundings whose traces fade over some eight tokens: 8 ** 0.5 of the 2^-24 of one token
+        assert (out[b, :n] - want).norm() <= 2.0 ** -22.5 * want.norm() and not out[b, n:].any()
+        assert (S[b] - state).norm() <= 2.0 ** -22.5 * state.norm()
