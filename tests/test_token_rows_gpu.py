@@ -70,7 +70,8 @@ def test_norm_inside_the_projections(rows, K, n_q, n_kv, D, I):
     from neuronx_distributed_llama3_2_b200.ops import decode_fused as df, norm, rope
 
     g = torch.Generator(device="cuda").manual_seed(K + rows)
-    x = torch.randn(rows, 2 * K, generator=g, device="cuda").bfloat16()[:, :K] * 3          # a row pitch of its own
+    x = (torch.randn(rows, 2 * K, generator=g, device="cuda").bfloat16() * 3)[:, :K]        # a row pitch of its own
+    assert x.stride(0) == 2 * K
     nw = (torch.randn(K, generator=g, device="cuda") * 0.1 + 1).bfloat16()
     w_qkv = torch.randn((n_q + 2 * n_kv) * D, K, generator=g, device="cuda").bfloat16() * 0.02
     w_gu = torch.randn(2 * I, K, generator=g, device="cuda").bfloat16() * 0.02
