@@ -100,3 +100,23 @@ def test_few_tokens_over_a_long_cache_keep_fp32_weights(T, kernel):
     assert T * k.shape[2] >= wa.TC_CACHE_MIN_WORK
     auto, same = (wa.window_attention_prefill(q, k, v, start, 0.1, 300, impl=i) for i in ("auto", kernel))
     assert torch.equal(auto, same)
+
+
+# windows and kept first rows around the 64-row key tile; the oldest visible key scores highest, so that the running maximum moves in
+# every tile on the way back from the diagonal, and the first tiles of a row may hold nothing that it sees
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("window,keep", [(1, 0), (63, 1), (64, 64), (65, 63), (64, 65), (129, 130), (500, 3)])
+def test_masks_and_the_order_of_the_tiles(D, window, keep):
+    from neuronx_distributed_llama3_2_b200.ops import window_attention as wa
+
+    B, T, H, G = 2, 200, 4, 2
+    g = torch.Generator(device="cuda").manual_seed(D + window)
+    starts, S = [333, 5], 640
+    q = torch.ones(B, T, H, D, device="cuda") + 0.1 * torch.randn(B, T, H, D, generator=g, device="cuda")
+    k = torch.linspace(2, -2, S, device="cuda")[:, None] + 0.1 * torch.randn(B, G, S, D, generator=g, device="cuda")
+    q, k, v = q.bfloat16(), k.bfloat16(), torch.randn(B, G, S, D, generator=g, device="cuda").bfloat16()
+    out = wa.window_attention_prefill(q, k, v, torch.tensor(starts, dtype=torch.int32, device="cuda"), D ** -0.5, window, keep, impl="tc")
+    for b, s in enumerate(starts):
+        ref = wa.window_attention_ref(q[b], k[b, :, :s + T], v[b, :, :s + T], torch.arange(s, s + T, device="cuda"), D ** -0.5, window, keep,
+                                      None)
+        assert (out[b].float() - ref).norm() <= 2.0 ** -7 * ref.norm()          # weights and result in bf16, as above
