@@ -500,6 +500,7 @@ int nxd_moe_gather_combine(int dtype, const void* ys, const int* slot, const int
  * csrc/gemm_tcgen05.cu (mode 1 plain, 2 gate | up through the clamped gated activation, 3 max(., 0)^2) */
 int nxd_moe_sort_rows(const void* h, const int* idx, int* counts, int* slot, const float* in_scale, float* row_scale, void* x,
                       long long P, int top, int W, int E, void* stream);
+int nxd_moe_sort_counts_itself(long long P); /* whether so many pairs are sorted without zeroed counts */
 int nxd_experts_gemm_bf16(const void* a, const void* b, void* d, const int* counts, const float* row_scale, int E, int rows,
                           int pairs, int N, int K, int mode, float limit, float alpha, float up_shift, void* stream);
 /* the whole mixture after its router on sorted rows (csrc/moe_forward.cu) */
@@ -508,6 +509,11 @@ int nxd_moe_sorted_forward(const void* h, const int* idx, const float* wts, cons
                            const void* w_down, const void* s_in, const void* s_down, const float* sgate, float* y, void* work,
                            long long N, int top, int W, int F, int E, int Fs, int gated, float limit, float s_limit,
                            float alpha, float up_shift, void* stream);
+/* the same with its router in front */
+int nxd_moe_routed_forward(const void* h, const float* wr, const float* corr, const float* wsg, const float* zbias, int R,
+                           float out_scale, int mode, const void* w_in, const void* w_down, const void* s_in,
+                           const void* s_down, float* y, void* work, long long N, int top, int W, int F, int E, int Fs,
+                           int gated, float limit, float s_limit, float alpha, float up_shift, void* stream);
 
 /* Retention (csrc/retention.cu): S_t = decay_h S_(t-1) + k_t v_t^T, o_t = S_t^T q_t on the fp32 state [lines, H, D, Dv] of
  * cache line seq_ids[b] (or b; zero state where q_start[b] == 0).  proj [B * Tn, ld] holds q / k / v head-major at the

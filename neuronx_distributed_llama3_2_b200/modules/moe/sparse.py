@@ -115,10 +115,10 @@ class SparseMoE(torch.nn.Module):
             path, weights = self._device_path(h)
             if (path == "device" and not self.weight_on_input and type(self.router).select is RouterBiasedTopK.select
                     and "select" not in self.router.__dict__ and moe_sparse.router_fits(self.router, shared_gate_w)):
-                return self._forward_device_sorted(h, None, None, shared_gate_w, weights)
+                return self._forward_device_sorted(h, weights, None, shared_gate_w)
         idx, wts, sg = self.router.select(h, shared_gate_w)
         if path == "device":
-            return self._forward_device_sorted(h, idx, wts, sg, weights or self._sorted_weights())
+            return self._forward_device_sorted(h, weights or self._sorted_weights(), (idx, wts, sg))
         sorted_path = self._use_sorted(h.shape[0]) if path is None else path == "sorted"
         if sorted_path:
             return self._forward_sorted(h, idx, wts, sg)
@@ -146,18 +146,20 @@ class SparseMoE(torch.nn.Module):
             ones = self._ones = torch.ones_like(wts)
         return ones
 
-    def _forward_device_sorted(self, h, idx, wts, sg, weights):
-        """``idx`` ``None``: the router runs in the same call, ``sg`` is its weight for the shared expert's gate."""
-        if idx is None:
-            return moe_sparse.routed_forward(h, self.router, sg, weights, self.gated, self.limit, self.alpha, self.up_shift,
-                                             self.shared_limit if self.shared is not None else 0.0)
+    def _forward_device_sorted(self, h, weights, routing, shared_gate_w=None):
+        """``routing``: what the router chose ``(idx, wts, sg)``, or ``None``: it runs in the same call, the shared expert's gate with
+        ``shared_gate_w``."""
+        shared_limit = self.shared_limit if self.shared is not None else 0.0
+        if routing is None:
+            return moe_sparse.routed_forward(h, self.router, shared_gate_w, weights, self.gated, self.limit, self.alpha, self.up_shift,
+                                             shared_limit)
+        idx, wts, sg = routing
         in_scale = None
         if self.weight_on_input:
             in_scale, wts = wts, self._ones_like(wts)
         w_in, w_down, *shared = weights
         return moe_sparse.sorted_forward(h, idx, wts, w_in, w_down, self.gated, self.limit, self.alpha, self.up_shift, in_scale,
-                                         *(shared or (None, None)), shared_limit=self.shared_limit if shared else 0.0,
-                                         shared_gate=sg)
+                                         *(shared or (None, None)), shared_limit=shared_limit, shared_gate=sg)
 
     def _forward_sorted(self, h, idx, wts, sg):
         N, E, k = h.shape[0], self.num_experts, self.top_k
