@@ -4,8 +4,10 @@ residual in their epilogue (``fused_comm.skinny_gemm``) and the decode attention
 token-generation graph is six launches (reference graph: ``examples/inference/modules/model_base.py:459-518``).
 
 Batches of 1 to 128 sequences on one process take the tensor-core counterparts (``csrc/gemm_smallm.cu``: weight rows as the
-UMMA M dimension, cluster split-K) unless the weights are small (``gemm.streams_on_tensor_cores``): fused QKV GEMM + RoPE + cache write, gate/up GEMM + SwiGLU (<= 64 rows), and the plain GEMM
-with the residual in its epilogue; the two RMSNorms stay separate launches there (eight launches per layer)."""
+UMMA M dimension, cluster split-K) unless the weights are small (``gemm.streams_on_tensor_cores``): fused QKV GEMM + RoPE + cache
+write, gate/up GEMM + SwiGLU (<= 64 rows), and the plain GEMM with the residual in its epilogue.  Few sequences of a narrow model
+(``norm_fits``) have the two RMSNorms inside the projections behind them, six launches per layer; else they are launches of their own,
+eight."""
 from __future__ import annotations
 
 import ctypes as _c

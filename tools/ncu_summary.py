@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Turn an .ncu-rep (``ncu --set full``) into the per-kernel table committed under profiles/: duration, DRAM bytes read and
 written, L2 bytes, tensor-pipe and issue activity, shared-memory data-pipe wavefronts (LSU and tensor-core side),
-registers, achieved occupancy.  Usage: tools/ncu_summary.py gpurun_out/hot_kernels.ncu-rep > profiles/.../ncu_summary.md"""
+registers, achieved occupancy.  Usage: tools/ncu_summary.py REPORT.ncu-rep > profiles/.../ncu_summary.md"""
 import csv
 import io
 import subprocess
