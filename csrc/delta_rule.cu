@@ -891,18 +891,26 @@ bool tensor_core_scan(int B, int Tn, int H, int D, int Dv) {
     return true;
 }
 
-// chunks of a step that are worked on at once: the operand tiles (147 to 344 KB per row, head and chunk) take half a gigabyte at most,
-// longer steps run in several launches
-int segment_chunks(int B, int Tn, int H, int D) {
-    const long long each = (long long)B * H * nxd_delta::chunk_tiles(D) * nxd_delta::TILE_BYTES;
-    const long long fit = (512ll << 20) / each;
-    return (int)max(1ll, min((long long)(Tn + CH - 1) / CH, fit));
+// What is worked on at once: rows of the batch and chunks of them, whose operand tiles (147 to 344 KB per row, head and chunk; the systems
+// take 33 KB more) are half a gigabyte at most, or one chunk of one row.  Longer steps and larger batches run in several launches.  A
+// launch takes six chunks if it can and fewer rows for it: a block of the scan sets up and moves its state for one chunk as for many (64
+// rows of 1024 tokens, 32 heads of 256 x 256, chunk by chunk 27.1 ms, by four 20.4, by six to eight 19.5; 8 rows of 421 tokens, 32 heads
+// of 256 x 128, four rows with all chunks 898 us, all rows with six 868).
+struct Segment {
+    int rows, chunks;
+};
+
+Segment segment(int B, int Tn, int H, int D) {
+    const int NC = (Tn + CH - 1) / CH;
+    const long long fit = max(1ll, (512ll << 20) / ((long long)H * nxd_delta::chunk_tiles(D) * nxd_delta::TILE_BYTES));
+    const int parts = (int)min((long long)B, ((long long)B * min(NC, 6) + fit - 1) / fit), rows = (B + parts - 1) / parts;
+    return {rows, (int)max(1ll, min((long long)NC, fit / rows))};
 }
 
 template <int D>
 int launch_chunks(const nxd_delta::Step& p, const float* gate, long long ld_a, int a_off, const float* beta, long long ld_b, int b_off,
                   float* scratch, long long wait_clocks, cudaStream_t st) {
-    const int NC = (p.Tn + CH - 1) / CH, seg = segment_chunks(p.B, p.Tn, p.H, D);
+    const int NC = (p.Tn + CH - 1) / CH;
     const size_t smem = (size_t)3 * CH * DPITCH * sizeof(double);
     NXD_CHECK_CUDA(nxd_allow_smem<delta_chunk_system_kernel<D>>((int)smem));
     if (!tensor_core_scan(p.B, p.Tn, p.H, D, p.Dv)) {
@@ -918,14 +926,24 @@ int launch_chunks(const nxd_delta::Step& p, const float* gate, long long ld_a, i
         NXD_LAUNCH_CHECK();
         return 0;
     }
+    const Segment seg = segment(p.B, p.Tn, p.H, D);
     uint8_t* tiles = reinterpret_cast<uint8_t*>(scratch);
-    float* systems = scratch + (long long)p.B * p.H * seg * (nxd_delta::chunk_tiles(D) * nxd_delta::TILE_BYTES / 4);
-    for (int c0 = 0; c0 < NC; c0 += seg) {
-        const int count = min(seg, NC - c0);
-        delta_chunk_system_kernel<D><<<dim3(count, p.H, p.B), CW_THREADS, smem, st>>>(p.qn, p.kn, gate, ld_a, a_off, beta, ld_b, b_off,
-                                                                                     systems, p.n_new, p.Tn, c0, p.H, p.G);
-        NXD_LAUNCH_CHECK();
-        if (int rc = nxd_delta::launch_chunks_tc(p, systems, tiles, c0, count, wait_clocks, st)) return rc;
+    float* systems = scratch + (long long)seg.rows * p.H * seg.chunks * (nxd_delta::chunk_tiles(D) * nxd_delta::TILE_BYTES / 4);
+    for (int b0 = 0; b0 < p.B; b0 += seg.rows) {
+        nxd_delta::Step r = p;
+        const long long t0 = (long long)b0 * p.Tn;
+        r.B = min(seg.rows, p.B - b0);
+        r.qn += t0 * p.G * D, r.kn += t0 * p.G * D, r.vn += t0 * p.H * p.Dv, r.out += t0 * p.H * p.Dv, r.q_start += b0;
+        if (p.n_new != nullptr) r.n_new += b0;
+        if (p.seq_ids != nullptr) r.seq_ids += b0;
+        else r.S += (long long)b0 * p.H * D * p.Dv;
+        for (int c0 = 0; c0 < NC; c0 += seg.chunks) {
+            const int count = min(seg.chunks, NC - c0);
+            delta_chunk_system_kernel<D><<<dim3(count, p.H, r.B), CW_THREADS, smem, st>>>(
+                r.qn, r.kn, gate + t0 * ld_a, ld_a, a_off, beta + t0 * ld_b, ld_b, b_off, systems, r.n_new, p.Tn, c0, p.H, p.G);
+            NXD_LAUNCH_CHECK();
+            if (int rc = nxd_delta::launch_chunks_tc(r, systems, tiles, c0, count, wait_clocks, st)) return rc;
+        }
     }
     return 0;
 }
@@ -1004,7 +1022,8 @@ NXD_API int nxd_delta_conv_state(int dtype, const void* proj, long long ld, int 
 NXD_API long long nxd_delta_scan_scratch(int B, int Tn, int H, int D, int Dv, int per_channel) {
     if (per_channel || (D != 64 && D != 128 && D != 256) || Dv % CW_COLS != 0 || Tn < 3 * CH || B > 65535 || H > 65535) return 0;
     if (!tensor_core_scan(B, Tn, H, D, Dv)) return (long long)B * H * ((Tn + CH - 1) / CH) * CHUNK_FLOATS;
-    return (long long)B * H * segment_chunks(B, Tn, H, D) * (CHUNK_FLOATS + nxd_delta::chunk_tiles(D) * nxd_delta::TILE_BYTES / 4);
+    const Segment seg = segment(B, Tn, H, D);
+    return (long long)seg.rows * H * seg.chunks * (CHUNK_FLOATS + nxd_delta::chunk_tiles(D) * nxd_delta::TILE_BYTES / 4);
 }
 
 // qn, kn, vn as written by nxd_delta_prep.  apre fp32 [B * Tn, ld_a]: decay pre-activation of head h at column a_off + h

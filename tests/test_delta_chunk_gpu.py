@@ -257,3 +257,31 @@ def test_both_scans_match_float64(D, Dv, B, H, T, fp32):
         # sums of fp32 roundings whose traces fade over some eight tokens: 8 ** 0.5 of the 2^-24 of one token
         assert (out[b, :n] - want).norm() <= 2.0 ** -22.5 * want.norm() and not out[b, n:].any()
         assert (S[b] - state).norm() <= 2.0 ** -22.5 * state.norm()
+
+
+# operand tiles of more rows than half a gigabyte holds: rows in two launches, with and without lines of their own, each as it is alone
+@pytest.mark.parametrize("lines", [False, True])
+def test_rows_in_several_launches_are_the_same(lines):
+    from neuronx_distributed_llama3_2_b200.ops import _lib, delta_rule as dr
+
+    B, T, H, D, Dv = 25, 193, 64, 256, 64
+    assert 4 * _lib.lib().nxd_delta_scan_scratch(B, T, H, D, Dv, 0) <= (512 << 20) * 11 // 10        # tiles and their systems
+    gen = torch.Generator(device="cuda").manual_seed(3)
+
+    def normal(*s):
+        return torch.randn(*s, generator=gen, device="cuda")
+
+    q, k = (F.normalize(normal(B, T, H, D), dim=-1) for _ in range(2))
+    v, a_pre, b_pre, S = normal(B, T, H, Dv), normal(B * T, H), normal(B * T, H), normal(B + 1, H, D, Dv)
+    a_log, dt_bias = normal(H) - 2, normal(H)
+    start = (torch.arange(B, device="cuda") % 2).int()
+    new = torch.tensor([T, 1, 0] + [T - b for b in range(3, B)], dtype=torch.int32, device="cuda")
+    line = torch.randperm(B + 1, generator=gen, device="cuda")[:B].int() if lines else None
+    state = S.clone()
+    out = dr.delta_scan(q, k, v, a_pre.clone(), 0, b_pre.clone(), 0, a_log, dt_bias, state, start, False, n_new=new, seq_ids=line)
+    for b in (0, 1, 2, 11, 12, 13, 14, B - 1):
+        rows, at = slice(b * T, (b + 1) * T), int(line[b]) if lines else b
+        one = S[at:at + 1].clone()
+        ref = dr.delta_scan(q[b:b + 1], k[b:b + 1], v[b:b + 1], a_pre[rows].clone(), 0, b_pre[rows].clone(), 0, a_log, dt_bias, one,
+                            start[b:b + 1], False, n_new=new[b:b + 1])
+        assert torch.equal(out[b], ref[0]) and torch.equal(state[at], one[0])
