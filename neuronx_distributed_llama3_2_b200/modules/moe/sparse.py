@@ -40,14 +40,15 @@ SORTED_PATH_MIN_PAIRS_PER_EXPERT = 16.0
 
 
 def pairs_win(tokens: int, top: int, width: int, ff: int, shared_ff: int, gated: bool) -> bool:
-    """Whether the per-pair GEMVs beat the device-sorted path, whose six launches and 256-row tiles cost 20 to 25 us more at any
-    size.  A pair's products are two serial chains, over ``width`` (half as long without a gate) and over the chosen experts' ``ff``,
-    and the pairs together stream ``work`` million weights a matrix.  Fitted to captured graphs of 1 to 256 tokens, widths 256 to
-    2048, ff 64 to 1024, 4 to 64 experts, 1 to 4 chosen (1200 sizes): the form taken is 0.2 % slower than the faster one on average
-    and 13 % at most with a gate, 31 % in the worst of 300 sizes without one; with a shared expert 1.4 % and 31 %.  Sorted / pairs:
-    28 / 17 us (4 tokens, 256, 4 experts, 2, 256), 30 / 21 (512, 32, 1, 128), 39 / 48 (1, 1024, 16, 4, 512)."""
+    """Whether the per-pair GEMVs beat the device-sorted path: five launches with the router, two more with a shared expert, two
+    more above 2048 pairs, and 256-row tiles, 22 us or more at any size.  A pair's products are two serial chains, over ``width``
+    (half as long without a gate) and over the chosen experts' ``ff``, and the pairs together stream ``work`` million weights a matrix.
+    Fitted to captured graphs of 1 to 256 tokens, widths 256 to 2048, ff 64 to 1024, 4 to 64 experts, 1 to 4 chosen (500 sizes): the
+    form taken is slower than the faster one by 0.3 % on average and 16 % at most with a gate (with a shared expert 0.1 % and 8 %), by
+    0.3 % and 12 % without one (0.6 % and 12 %).  Sorted / pairs: 25 / 36 us (101 tokens, 512, 8 experts, 1, 384), 26 / 31 (4, 768, 8, 2,
+    384), 27 / 27 (2, 768, 16, 3, 128)."""
     chain, work = top * ff + shared_ff, tokens * width * (top * ff + shared_ff) / 2 ** 20
-    return width + 0.5 * chain + 40 * work <= 1500 if gated else 0.2 * chain + 50 * work <= 1500
+    return width + 0.3 * chain + 35 * work <= 1000 if gated else 0.2 * width + 0.4 * chain + 30 * work <= 1150
 
 
 class SparseMoE(torch.nn.Module):
