@@ -18,8 +18,8 @@ Three execution paths over the same parameters:
   * device-sorted  the same in bf16 on the GPU with the counts read on the device: the sort, the two products (all experts
             in one launch each, the activation inside the first) and the combination are one call, capturable.  It
             serves every number of tokens but for small mixtures (``pairs_win``): in captured graphs of 1 .. 256 tokens at
-            (width, experts, top, ff) = (2048, 8, 2, 2048) / (4096, 8, 2, 4096) / (1024, 16, 4, 512) it takes 49 .. 80 / 95 .. 202 /
-            38 .. 44 us where the pairs take 82 .. 1948 / 402 .. 7539 / 45 .. 504 us.
+            (width, experts, top, ff) = (2048, 8, 2, 2048) / (4096, 8, 2, 4096) / (1024, 16, 4, 512) it takes 46 .. 75 / 92 .. 194 /
+            33 .. 39 us where the pairs take 82 .. 1954 / 411 .. 7548 / 47 .. 505 us.
 The combination (chosen experts, identity experts, shared expert times its sigmoid gate) is summed in fp32.
 """
 from __future__ import annotations

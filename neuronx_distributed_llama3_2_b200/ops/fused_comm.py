@@ -51,7 +51,7 @@ def dump_traces(limit: int = 6):  # noqa: D401
 def _ag_block_n(tp: int, R: int, N: int, comm_ctas: int) -> int:
     """Tile width of the AG->GEMM kernel.  256 everywhere: at TP8 the 128-wide tiles were tried for the narrow
     projections (a wave-count model picked them for qkv N = 640 and gate_up N = 2048) and lost -- 123 vs 115 us and
-    171 vs 131 us (``profiles/r2/fused_comm_tp8_bn*.jsonl``): the kernel is bound by the gather, and narrower tiles only
+    171 vs 131 us (``profiles/training_and_decode/fused_comm_tp8_bn*.jsonl``): the kernel is bound by the gather, and narrower tiles only
     add B-operand traffic.  ``NXD_AG_BLOCK_N=128`` keeps the variant reachable (the tests run both)."""
     env = os.environ.get("NXD_AG_BLOCK_N")
     return int(env) if env else 256
@@ -81,7 +81,7 @@ def fused_ag_gemm(ctx, x_shard: torch.Tensor, weight: torch.Tensor, layout: str 
     mc_base = 0
     # NVLS: the copy CTAs store the local shard ONCE to the multicast address of the gathered buffer (multimem.st, the
     # switch replicates it) instead of once per peer.  Verified at 2 and 8 GPUs; TP8 step 55.8 -> 53.2 ms
-    # (profiles/r2/bench_tp8_nvls.json).  Falls back to per-peer pushes where no multicast object can be bound.
+    # (profiles/training_and_decode/bench_tp8_nvls.json).  Falls back to per-peer pushes where no multicast object can be bound.
     nvls = os.environ.get("NXD_NVLS")          # unset: on for tp > 2 (one peer gains nothing); "1": always; "0": never
     if nvls == "1" or (nvls is None and tp > 2):
         got = ctx.region_mc(cfg, 2 * total_bytes)
