@@ -909,11 +909,11 @@ Segment segment(int B, int Tn, int H, int D) {
 
 template <int D>
 int launch_chunks(const nxd_delta::Step& p, const float* gate, long long ld_a, int a_off, const float* beta, long long ld_b, int b_off,
-                  float* scratch, long long wait_clocks, cudaStream_t st) {
+                  float* scratch, bool tensor_cores, long long wait_clocks, cudaStream_t st) {
     const int NC = (p.Tn + CH - 1) / CH;
     const size_t smem = (size_t)3 * CH * DPITCH * sizeof(double);
     NXD_CHECK_CUDA(nxd_allow_smem<delta_chunk_system_kernel<D>>((int)smem));
-    if (!tensor_core_scan(p.B, p.Tn, p.H, D, p.Dv)) {
+    if (!tensor_cores) {
         constexpr int DP = D + 4;
         constexpr int scan = ((D <= 128 ? 3 : 2) * CH * DP + CW_COLS * DP + 2 * CH * CP + 2 * CW_COLS * CP + 4 * CH) * (int)sizeof(float);
         static_assert(scan <= 232448, "shared memory");
@@ -1048,12 +1048,15 @@ NXD_API int nxd_delta_scan_limited(const float* qn, const float* kn, const float
                                                                       N, H, per_head);
     NXD_LAUNCH_CHECK();
     auto al = [](const void* p) { return ((uintptr_t)p % 16) == 0; };
-    if (scratch != nullptr && nxd_delta_scan_scratch(B, Tn, H, D, Dv, per_channel) > 0 && al(qn) && al(kn) && al(vn) && al(S) &&
-        al(out) && al(scratch)) {
+    const long long floats = nxd_delta_scan_scratch(B, Tn, H, D, Dv, per_channel);
+    // values, state and outputs at any address run on the fp32 scan, where the scratch holds its systems of all chunks
+    const bool tc = tensor_core_scan(B, Tn, H, D, Dv) && al(vn) && al(S) && al(out);
+    if (scratch != nullptr && floats > 0 && al(qn) && al(kn) && al(scratch) &&
+        (tc || (long long)B * H * ((Tn + CH - 1) / CH) * CHUNK_FLOATS <= floats)) {
         const nxd_delta::Step step{qn, kn, vn, S, out, q_start, n_new, seq_ids, B, Tn, H, G, D, Dv};
-        if (D == 64) return launch_chunks<64>(step, apre, ld_a, a_off, bpre, ld_b, b_off, scratch, wait_clocks, st);
-        if (D == 128) return launch_chunks<128>(step, apre, ld_a, a_off, bpre, ld_b, b_off, scratch, wait_clocks, st);
-        return launch_chunks<256>(step, apre, ld_a, a_off, bpre, ld_b, b_off, scratch, wait_clocks, st);
+        if (D == 64) return launch_chunks<64>(step, apre, ld_a, a_off, bpre, ld_b, b_off, scratch, tc, wait_clocks, st);
+        if (D == 128) return launch_chunks<128>(step, apre, ld_a, a_off, bpre, ld_b, b_off, scratch, tc, wait_clocks, st);
+        return launch_chunks<256>(step, apre, ld_a, a_off, bpre, ld_b, b_off, scratch, tc, wait_clocks, st);
     }
     // rows of a column per thread (NPT) and lanes per column (R, a power of two): the smallest slice that keeps R <= 4,
     // wider keys spread over more lanes (measured at 8 heads of 256 x 512, 2 x 4096 tokens: slices of 32 / 16 / 8 rows take

@@ -119,7 +119,8 @@ def delta_scan(qn: torch.Tensor, kn: torch.Tensor, vn: torch.Tensor, a_pre: torc
     fp32 the beta pre-activations at ``b_offset + h``; ``a_log [H]``, ``dt_bias [H]`` or ``[H * dim]`` fp32;
     ``S [lines, H, dim, vdim]`` fp32, updated in place for line ``seq_ids[b]`` (default ``b``).  Tokens ``t >= n_new[b]``
     are padding: they leave the state alone and come out as zeros.  On the GPU ``a_pre`` and ``b_pre`` are overwritten
-    with the decay factors and beta.  Returns fp32 ``o [B, T, H, vdim]``."""
+    with the decay factors and beta.  Returns fp32 ``o [B, T, H, vdim]``.  A kernel whose waits run out (two seconds, a device that does
+    not answer) leaves NaN and says so to ``scan_gave_up``."""
     B, T, G, D = qn.shape
     H, Dv = vn.shape[2], vn.shape[3]
     if qn.is_cuda and _lib.available(GROUP):

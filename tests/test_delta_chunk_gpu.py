@@ -285,3 +285,33 @@ def test_rows_in_several_launches_are_the_same(lines):
         ref = dr.delta_scan(q[b:b + 1], k[b:b + 1], v[b:b + 1], a_pre[rows].clone(), 0, b_pre[rows].clone(), 0, a_log, dt_bias, one,
                             start[b:b + 1], False, n_new=new[b:b + 1])
         assert torch.equal(out[b], ref[0]) and torch.equal(state[at], one[0])
+
+
+# values, state and outputs that are not 16-byte aligned keep the chunks: where the fp32 scan serves anyway, bit for bit
+@pytest.mark.parametrize("Dv,H,same", [(32, 48, True), (64, 4, False)])
+def test_values_and_state_at_odd_addresses(Dv, H, same):
+    from neuronx_distributed_llama3_2_b200.ops import delta_rule as dr
+
+    B, T, D = 2, 200, 64
+    gen = torch.Generator(device="cuda").manual_seed(4)
+
+    def normal(*s):
+        return torch.randn(*s, generator=gen, device="cuda")
+
+    def odd(x):
+        y = torch.empty(x.numel() + 1, device="cuda")[1:].view(x.shape)
+        assert y.data_ptr() % 16 != 0
+        return y.copy_(x)
+
+    q, k = (F.normalize(normal(B, T, H, D), dim=-1) for _ in range(2))
+    v, a_pre, b_pre, S = normal(B, T, H, Dv), normal(B * T, H), normal(B * T, H), normal(B, H, D, Dv)
+    a_log, dt_bias, start = normal(H) - 2, normal(H), torch.ones(B, dtype=torch.int32, device="cuda")
+
+    def run(v, S):
+        return dr.delta_scan(q, k, v, a_pre.clone(), 0, b_pre.clone(), 0, a_log, dt_bias, S, start, False), S
+
+    (x, s), (y, z) = run(v, S.clone()), run(odd(v), odd(S))
+    if same:
+        assert torch.equal(x, y) and torch.equal(s, z)
+    # two scans, each within 2^-22.5 of float64
+    assert (x - y).norm() <= 2.0 ** -21.5 * x.norm() and (s - z).norm() <= 2.0 ** -21.5 * s.norm()
