@@ -361,11 +361,11 @@ ag_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a_local, const __grid_co
             int acc = 0;
             uint32_t acc_phase = 0;
             for (int tile = cluster_id; tile < num_tiles; tile += num_clusters) {
-                ptx::mbar_wait_cluster(&tmem_empty_bar[acc], acc_phase ^ 1);
+                ptx::mbar_wait(&tmem_empty_bar[acc], acc_phase ^ 1);
                 ptx::tcgen05_fence_after();
                 const uint32_t tmem_d = tmem_base + acc * BN;
                 for (int kb = 0; kb < num_k_blocks; ++kb) {
-                    ptx::mbar_wait_cluster(&full_bar[stage], phase);
+                    ptx::mbar_wait(&full_bar[stage], phase);
                     ptx::tcgen05_fence_after();
                     const uint32_t sa = ptx::smem_u32(smem + stage * L::kStageBytes);
                     const uint32_t sb = sa + L::kABytes;

@@ -85,7 +85,7 @@ retention_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     uint64_t* acc_full = empty + kStages;
     uint64_t* acc_empty = acc_full + kAcc;
     uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc_empty + kAcc);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t rank = ptx::cluster_ctarank();
     const bool leader = rank == 0;
     const int num_tiles = p.E * p.n_tiles, k_blocks = p.k_blocks1 + p.k_blocks2;
@@ -149,7 +149,7 @@ retention_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             }
         }
     } else if (warp == 1) {
-        if (leader && lane == 0) {
+        if (leader && ptx::elect_one()) {
             constexpr uint32_t idesc = ptx::make_idesc_bf16(256, kBN, A_MN ? 1 : 0, B_MN ? 1 : 0);
             constexpr uint32_t a_lbo = A_MN ? kBK * 128 : 16, b_lbo = B_MN ? kBK * 128 : 16;
             constexpr uint32_t a_step = A_MN ? 2048 : 32, b_step = B_MN ? 2048 : 32;
@@ -158,8 +158,8 @@ retention_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             for (int tile = blockIdx.x >> 1; tile < num_tiles; tile += gridDim.x >> 1) {
                 for (int kb = 0; kb < k_blocks; ++kb) {
                     const int nb = kb >= p.k_blocks1 ? 3 : NB1;
-                    ptx::mbar_wait_cluster(&acc_empty[acc], acc_ph ^ 1);
-                    ptx::mbar_wait_cluster(&full[st], ph);
+                    ptx::mbar_wait(&acc_empty[acc], acc_ph ^ 1);
+                    ptx::mbar_wait(&full[st], ph);
                     ptx::tcgen05_fence_after();
                     const uint32_t sa = ptx::smem_u32(smem + st * kStageBytes), sb = sa + 3 * kABytes;
                     uint32_t add = 0;
