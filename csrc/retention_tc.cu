@@ -14,11 +14,14 @@
 //   states   sequential over chunks, one thread per four state elements: state at every chunk's start -> pieces, line's state
 //   <kP>     P of all chunks; decay and causal mask in the epilogue, result split into pieces
 //   <kO>     both output products of a tile in one pass, [P | q] over [V ; S_c]
-// The three products run the persistent CTA-pair pipeline of gemm_tcgen05.cu with 256 x 128 tiles; one pipeline stage holds the
-// three pieces of both operands for 64 terms (72 KB), 24 MMAs.  The chunk is as long as the tile is high: a shorter one would
-// leave half the rows of the CTA pair empty, and the state traffic falls with the chunk's length.
-// 2 x 4096 tokens, 8 heads of 256 x 512, fp32: 159 us prep, 103 + 65 + 175 us the products (1.0 to 1.2 PF of piece products), 52 us
-// states, 567 us in all against 3482 us on the fp32 kernels (error against float64 1.6e-7 against 3.4e-7).  bf16: 511 us.
+// The three products run the persistent CTA-pair pipeline of gemm_tcgen05.cu with 256 x 128 tiles; 64 terms are 24 MMAs over the three
+// pieces of both operands, each piece (24 KB) in a slot of its own that is free again behind its last product: the smallest pieces are
+// used first, so their slots load again while the others are multiplied (all pieces as one stage, two stages: every stage waited for its
+// loads).  The chunk is as long as the tile is high: a shorter one would leave half the rows of the CTA pair empty, and the state traffic
+// falls with the chunk's length.
+// 2 x 4096 tokens, 8 heads of 256 x 512, fp32 (stages and rows through shared memory before): prep 158 -> 150 us, products 166 + 95 + 64 ->
+// 145 + 82 + 57, states 52; 633 -> 560 us through the entry point, 3482 us on the fp32 kernels (error against float64 1.6e-7 against
+// 3.4e-7).  2.6 GB of pieces and intermediates at 5.2 TB/s: memory bounds it now.
 #include "attn_tc_common.cuh"
 #include "common.cuh"
 #include "gemm_tcgen05.cuh"
@@ -31,18 +34,27 @@ using nxd_gemm::make_tmap_3d;
 
 constexpr int kC = 256;              // tokens of a chunk
 constexpr int kBN = 128, kBK = 64;
-constexpr int kStages = 2, kAcc = 4;
+constexpr int kSlots = 8, kAcc = 4;
 constexpr int kThreads = 256;
 constexpr int kABytes = 128 * kBK * 2, kBBytes = (kBN / 2) * kBK * 2;       // one piece: this CTA's rows of A, its half of B
-constexpr int kStageBytes = 3 * (kABytes + kBBytes);
-constexpr int kStagingOff = kStages * kStageBytes;
+constexpr int kSlotBytes = kABytes + kBBytes;                               // one piece of both
+constexpr int kStagingOff = kSlots * kSlotBytes;
 constexpr int kStagingPerWarp = 2 * 32 * 128;
 constexpr int kTableOff = kStagingOff + 4 * kStagingPerWarp;                // kP: decay^j, j < kC
 constexpr int kBarOff = kTableOff + kC * 4;
-constexpr int kSmem = kBarOff + (2 * kStages + 2 * kAcc) * 8 + 16 + 1024;
+constexpr int kSmem = kBarOff + (2 * kSlots + 2 * kAcc) * 8 + 16 + 1024;
 static_assert(kSmem <= 232448, "shared memory budget exceeded");
 
 enum { kU = 0, kP = 1, kO = 2 };
+
+// Slots of the ring: a block of 64 terms takes three, its pieces 2, 1 and 0
+struct Slot {
+    int i = 0;
+    uint32_t phase = 0;
+    __device__ __forceinline__ void next() {
+        if (++i == kSlots) i = 0, phase ^= 1;
+    }
+};
 
 __device__ __forceinline__ float ldf(const float* p) { return *p; }
 __device__ __forceinline__ float ldf(const bf16* p) { return __bfloat162float(*p); }
@@ -81,8 +93,8 @@ retention_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = ptx::align_smem_1024(smem_raw);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kBarOff);
-    uint64_t* empty = full + kStages;
-    uint64_t* acc_full = empty + kStages;
+    uint64_t* empty = full + kSlots;
+    uint64_t* acc_full = empty + kSlots;
     uint64_t* acc_empty = acc_full + kAcc;
     uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc_empty + kAcc);
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -98,7 +110,7 @@ retention_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         ptx::prefetch_tensormap(&tmap_d);
     }
     if (warp == 1 && lane == 0) {
-        for (int i = 0; i < kStages; ++i) {
+        for (int i = 0; i < kSlots; ++i) {
             ptx::mbar_init(&full[i], 1);
             ptx::mbar_init(&empty[i], 1);
         }
@@ -116,8 +128,7 @@ retention_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 
     if (warp == 0) {
         if (lane == 0) {
-            int st = 0;
-            uint32_t ph = 0;
+            Slot st;
             for (int tile = blockIdx.x >> 1; tile < num_tiles; tile += gridDim.x >> 1) {
                 const int e = tile / p.n_tiles, tn = tile % p.n_tiles;
                 const int m0 = (int)rank * 128, n0 = tn * kBN + (int)rank * (kBN / 2);
@@ -127,24 +138,24 @@ retention_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     const int nb = second ? 3 : NB1;
                     const CUtensorMap* ma = second ? &tmap_a2 : &tmap_a;
                     const CUtensorMap* mb = second ? &tmap_b2 : &tmap_b;
-                    ptx::mbar_wait(&empty[st], ph ^ 1);
-                    uint8_t* sa = smem + st * kStageBytes;
-                    uint8_t* sb = sa + 3 * kABytes;
-                    if (leader) ptx::mbar_arrive_expect_tx(&full[st], 2 * (3 * kABytes + nb * kBBytes));
 #pragma unroll
-                    for (int x = 0; x < 3; ++x) {
+                    for (int x = 2; x >= 0; --x) {
+                        uint8_t* sa = smem + st.i * kSlotBytes;
+                        uint8_t* sb = sa + kABytes;
+                        ptx::mbar_wait(&empty[st.i], st.phase ^ 1);
+                        if (leader) ptx::mbar_arrive_expect_tx(&full[st.i], 2 * (kABytes + (x < nb ? kBBytes : 0)));
                         if constexpr (A_MN) {
-                            ptx::tma_load_3d_pair(ma, &full[st], sa + x * kABytes, m0, k0, e * 3 + x);
-                            ptx::tma_load_3d_pair(ma, &full[st], sa + x * kABytes + kBK * 128, m0 + 64, k0, e * 3 + x);
+                            ptx::tma_load_3d_pair(ma, &full[st.i], sa, m0, k0, e * 3 + x);
+                            ptx::tma_load_3d_pair(ma, &full[st.i], sa + kBK * 128, m0 + 64, k0, e * 3 + x);
                         } else {
-                            ptx::tma_load_3d_pair(ma, &full[st], sa + x * kABytes, k0, m0, e * 3 + x);
+                            ptx::tma_load_3d_pair(ma, &full[st.i], sa, k0, m0, e * 3 + x);
                         }
+                        if (x < nb) {
+                            if constexpr (B_MN) ptx::tma_load_3d_pair(mb, &full[st.i], sb, n0, k0, e * nb + x);
+                            else ptx::tma_load_3d_pair(mb, &full[st.i], sb, k0, n0, e * nb + x);
+                        }
+                        st.next();
                     }
-                    for (int x = 0; x < nb; ++x) {
-                        if constexpr (B_MN) ptx::tma_load_3d_pair(mb, &full[st], sb + x * kBBytes, n0, k0, e * nb + x);
-                        else ptx::tma_load_3d_pair(mb, &full[st], sb + x * kBBytes, k0, n0, e * nb + x);
-                    }
-                    if (++st == kStages) st = 0, ph ^= 1;
                 }
             }
         }
@@ -153,36 +164,45 @@ retention_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             constexpr uint32_t idesc = ptx::make_idesc_bf16(256, kBN, A_MN ? 1 : 0, B_MN ? 1 : 0);
             constexpr uint32_t a_lbo = A_MN ? kBK * 128 : 16, b_lbo = B_MN ? kBK * 128 : 16;
             constexpr uint32_t a_step = A_MN ? 2048 : 32, b_step = B_MN ? 2048 : 32;
-            int st = 0, acc = 0;
-            uint32_t ph = 0, acc_ph = 0;
+            Slot st;
+            int acc = 0;
+            uint32_t acc_ph = 0;
             for (int tile = blockIdx.x >> 1; tile < num_tiles; tile += gridDim.x >> 1) {
                 for (int kb = 0; kb < k_blocks; ++kb) {
                     const int nb = kb >= p.k_blocks1 ? 3 : NB1;
                     ptx::mbar_wait(&acc_empty[acc], acc_ph ^ 1);
-                    ptx::mbar_wait(&full[st], ph);
+                    uint32_t sa[3];
+                    uint64_t* freed[3];
+#pragma unroll
+                    for (int x = 2; x >= 0; --x) {
+                        ptx::mbar_wait(&full[st.i], st.phase);
+                        sa[x] = ptx::smem_u32(smem + st.i * kSlotBytes);
+                        freed[x] = &empty[st.i];
+                        st.next();
+                    }
                     ptx::tcgen05_fence_after();
-                    const uint32_t sa = ptx::smem_u32(smem + st * kStageBytes), sb = sa + 3 * kABytes;
                     uint32_t add = 0;
                     auto product = [&](int x, int y) {
 #pragma unroll
                         for (int k = 0; k < kBK / 16; ++k) {
-                            const uint64_t da = ptx::make_smem_desc(sa + x * kABytes + k * a_step, a_lbo, 1024);
-                            const uint64_t db = ptx::make_smem_desc(sb + y * kBBytes + k * b_step, b_lbo, 1024);
+                            const uint64_t da = ptx::make_smem_desc(sa[x] + k * a_step, a_lbo, 1024);
+                            const uint64_t db = ptx::make_smem_desc(sa[y] + kABytes + k * b_step, b_lbo, 1024);
                             ptx::umma_bf16<2>(tmem + acc * kBN, da, db, idesc, add);
                             add = 1;
                         }
                     };
                     product(2, 0);                          // the smallest first
+                    if (nb == 3) product(0, 2);
+                    ptx::umma_commit_pair(freed[2], 0b11);
                     if (nb == 3) {
-                        product(0, 2);
                         product(1, 1);
                         product(0, 1);
                     }
                     product(1, 0);
+                    ptx::umma_commit_pair(freed[1], 0b11);
                     product(0, 0);
-                    ptx::umma_commit_pair(&empty[st], 0b11);
+                    ptx::umma_commit_pair(freed[0], 0b11);
                     ptx::umma_commit_pair(&acc_full[acc], 0b11);
-                    if (++st == kStages) st = 0, ph ^= 1;
                     if (++acc == kAcc) acc = 0, acc_ph ^= 1;
                 }
             }
@@ -304,11 +324,29 @@ retention_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     if (warp == 2) ptx::tmem_dealloc<2>(tmem, kAcc * kBN);
 }
 
-constexpr int PT = 16, PREP_THREADS = 256;
+constexpr int PT = 32, PREP_THREADS = 256;
 
-// grid (chunks * kC / PT, H, B).  q3 / k3 / kd3 [E][3][kC][D], v3 [E][NB][kC][Dv].  Bound by memory.
+// eight consecutive values of a row
+template <typename T>
+__device__ __forceinline__ void load8(const T* src, int vec, float (&f)[8]) {
+    if (!vec) {
+#pragma unroll
+        for (int x = 0; x < 8; ++x) f[x] = ldf(src + x);
+    } else if constexpr (sizeof(T) == 2) {
+        unpack8(*reinterpret_cast<const bf16x8*>(src), f);
+    } else {
+        *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(src);
+        *reinterpret_cast<float4*>(f + 4) = *reinterpret_cast<const float4*>(src + 4);
+    }
+}
+
+// grid (3 * chunks * kC / PT, H, B): the queries, the keys or the values of PT tokens of a head.  q3 / k3 / kd3 [E][3][kC][D], v3
+// [E][NB][kC][Dv].  Bound by memory: no shared memory and no barrier between a thread's loads and its stores, so that enough loads are in
+// flight (rows laid out in shared memory for the rotation, two CTAs a SM: 159 us at the sizes above).  A thread rotates eight pairs of
+// `halves`, which lie half a rotation apart, at a time.
 // A value that is not finite would reach the tokens before it through 0 * value: it goes over as zero, the first such token s
 // of a column is kept as bad[e][j] = kC - s, and the consumers put NaN where it would have arrived.
+// vec: bit 0 the rows of proj in 16-byte loads, bit 1 the rotation in whole vectors
 template <typename T, int NB>
 __global__ void __launch_bounds__(PREP_THREADS)
 retention_tc_prep_kernel(const T* __restrict__ proj, long long ld, int q_off, int k_off, int v_off,
@@ -317,92 +355,110 @@ retention_tc_prep_kernel(const T* __restrict__ proj, long long ld, int q_off, in
                          const int* __restrict__ n_new, int Tn, int NC, int H, int D, int Dv, float kscale,
                          const float* __restrict__ rope_cos, const float* __restrict__ rope_sin, int rot, int halves,
                          int max_pos, int vec) {
-    extern __shared__ __align__(16) float smem[];
-    const int DP = D + 4;
-    float* Qs = smem;                        // [PT][DP]
-    float* Ks = Qs + PT * DP;                // [PT][DP]
     __shared__ float fade[PT];               // decay^(n - 1 - s) of the chunk's tokens
-    const int hd = blockIdx.y, b = blockIdx.z, tid = threadIdx.x;
-    const int t0 = blockIdx.x * PT, c = t0 / kC, s0 = t0 % kC;
+    const int hd = blockIdx.y, role = blockIdx.x % 3, b = blockIdx.z, tid = threadIdx.x;
+    const int t0 = (int)(blockIdx.x / 3) * PT, c = t0 / kC, s0 = t0 % kC;
     const int n = n_new != nullptr ? min(n_new[b], Tn) : Tn;
     const int nt = max(0, min(PT, n - t0)), chunk_n = min(kC, n - c * kC);
     const long long e = ((long long)b * H + hd) * NC + c, row0 = (long long)b * Tn + t0;
-    if (tid < PT) fade[tid] = tid < nt ? powf(decay[hd], (float)(chunk_n - 1 - (s0 + tid))) : 0.f;
-#pragma unroll 4
-    for (int i = tid; i < PT * D; i += PREP_THREADS) {
-        const int t = i / D, d = i - t * D;
-        const T* row = proj + (row0 + t) * ld + hd * D + d;
-        Qs[t * DP + d] = t < nt ? ldf(row + q_off) : 0.f;
-        Ks[t * DP + d] = t < nt ? ldf(row + k_off) * kscale : 0.f;
-    }
-    __syncthreads();
-    if (rope_cos != nullptr && rot > 0) {
-        const int half = rot / 2, p0 = q_start[b] + t0;
-        for (int i = tid; i < nt * half; i += PREP_THREADS) {
-            const int t = i / half, x = i - t * half;
-            const int iu = halves ? x : 2 * x, iv = halves ? x + half : 2 * x + 1;
-            const int pos = min(p0 + t, max_pos - 1);
-            const float cs = rope_cos[(long long)pos * half + x], sn = rope_sin[(long long)pos * half + x];
-            float u = Qs[t * DP + iu], v = Qs[t * DP + iv];
-            Qs[t * DP + iu] = u * cs - v * sn;
-            Qs[t * DP + iv] = v * cs + u * sn;
-            u = Ks[t * DP + iu], v = Ks[t * DP + iv];
-            Ks[t * DP + iu] = u * cs - v * sn;
-            Ks[t * DP + iv] = v * cs + u * sn;
-        }
-        __syncthreads();
-    }
-    auto put = [&](bf16* base, int pieces, int width, int t, int d, const bf16x8 (&w)[3]) {
+    auto put = [&](bf16* base, int pieces, int width, int t, int d, const float (&f)[8]) {
+        bf16x8 w[3];
+        split8(f, w);
 #pragma unroll
         for (int x = 0; x < 3; ++x)
             if (x < pieces)
                 *reinterpret_cast<bf16x8*>(base + ((e * pieces + x) * kC + s0 + t) * width + d) = w[x];
     };
-    for (int i = tid; i < PT * (D / 8); i += PREP_THREADS) {
-        const int t = i / (D / 8), d = (i - t * (D / 8)) * 8;
-        float f[8];
-        bf16x8 w[3];
-        *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(Qs + t * DP + d);
-        *reinterpret_cast<float4*>(f + 4) = *reinterpret_cast<const float4*>(Qs + t * DP + d + 4);
-        split8(f, w);
-        put(q3, 3, D, t, d, w);
-        *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(Ks + t * DP + d);
-        *reinterpret_cast<float4*>(f + 4) = *reinterpret_cast<const float4*>(Ks + t * DP + d + 4);
-        split8(f, w);
-        put(k3, 3, D, t, d, w);
-        const float a = fade[t];
+    if (role == 2) {
+        const int W8 = Dv / 8;
+#pragma unroll 4
+        for (int i = tid; i < PT * W8; i += PREP_THREADS) {
+            const int t = i / W8, d = (i - t * W8) * 8;
+            float f[8] = {};
+            if (t < nt) {
+                load8(proj + (row0 + t) * ld + v_off + (long long)hd * Dv + d, vec & 1, f);
 #pragma unroll
-        for (int x = 0; x < 8; ++x) f[x] *= a;
-        split8(f, w);
-        put(kd3, 3, D, t, d, w);
+                for (int x = 0; x < 8; ++x)
+                    if (!isfinite(f[x])) {
+                        f[x] = 0.f;
+                        atomicMax(bad + e * Dv + d + x, kC - (s0 + t));
+                        atomicMax(flag + e, 1);
+                    }
+            }
+            put(v3, NB, Dv, t, d, f);
+        }
+        return;
     }
-    for (int i = tid; i < PT * (Dv / 8); i += PREP_THREADS) {
-        const int t = i / (Dv / 8), d = (i - t * (Dv / 8)) * 8;
+    if (role == 1) {
+        if (tid < PT) fade[tid] = tid < nt ? powf(decay[hd], (float)(chunk_n - 1 - (s0 + tid))) : 0.f;
+        __syncthreads();
+    }
+    bf16* out = role == 0 ? q3 : k3;
+    const T* src = proj + row0 * ld + (role == 0 ? q_off : k_off) + hd * D;
+    const float scale = role == 0 ? 1.f : kscale;
+    const int half = rope_cos != nullptr ? rot / 2 : 0, p0 = half > 0 ? q_start[b] + t0 : 0;
+    auto finish = [&](int t, int d, float (&f)[8]) {
+        put(out, 3, D, t, d, f);
+        if (role == 1) {
+            const float a = fade[t];
+#pragma unroll
+            for (int x = 0; x < 8; ++x) f[x] *= a;
+            put(kd3, 3, D, t, d, f);
+        }
+    };
+    auto load = [&](int t, int d, float (&f)[8]) {
+        load8(src + t * ld + d, vec & 1, f);
+#pragma unroll
+        for (int x = 0; x < 8; ++x) f[x] *= scale;
+    };
+    const bool pairs = half > 0 && halves && (vec & 2);           // an item is two vectors half a rotation apart, or one behind it
+    const int items = pairs ? half / 8 + (D - rot) / 8 : D / 8;
+#pragma unroll 2
+    for (int i = tid; i < PT * items; i += PREP_THREADS) {
+        const int t = i / items, x = i - t * items;
+        const long long at = half > 0 ? (long long)min(p0 + t, max_pos - 1) * half : 0;
+        if (pairs && x < half / 8) {
+            const int d = x * 8;
+            float u[8] = {}, v[8] = {};
+            if (t < nt) {
+                float cs[8], sn[8];
+                load(t, d, u);
+                load(t, d + half, v);
+                load8(rope_cos + at + d, 1, cs);
+                load8(rope_sin + at + d, 1, sn);
+#pragma unroll
+                for (int y = 0; y < 8; ++y) {
+                    const float a = u[y], g = v[y];
+                    u[y] = a * cs[y] - g * sn[y];
+                    v[y] = g * cs[y] + a * sn[y];
+                }
+            }
+            finish(t, d, u);
+            finish(t, d + half, v);
+            continue;
+        }
+        const int d = pairs ? rot + (x - half / 8) * 8 : x * 8;
         float f[8] = {};
         if (t < nt) {
-            const T* src = proj + (row0 + t) * ld + v_off + (long long)hd * Dv + d;
-            if (vec) {
-                if constexpr (NB == 1) {
-                    unpack8(*reinterpret_cast<const bf16x8*>(src), f);
-                } else {
-                    *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(src);
-                    *reinterpret_cast<float4*>(f + 4) = *reinterpret_cast<const float4*>(src + 4);
-                }
-            } else {
+            load(t, d, f);
+            if (!pairs && d < 2 * half) {
+                float g[8];
 #pragma unroll
-                for (int x = 0; x < 8; ++x) f[x] = ldf(src + x);
+                for (int y = 0; y < 8; ++y) {
+                    const int dd = d + y;
+                    g[y] = f[y];
+                    if (dd >= 2 * half) continue;
+                    const bool first = halves ? dd < half : (dd & 1) == 0;
+                    const int j = halves ? (first ? dd : dd - half) : dd / 2;
+                    const float cs = rope_cos[at + j], sn = rope_sin[at + j];
+                    const float o = halves ? ldf(src + t * ld + (first ? dd + half : dd - half)) * scale : f[y ^ 1];
+                    g[y] = first ? f[y] * cs - o * sn : f[y] * cs + o * sn;
+                }
+#pragma unroll
+                for (int y = 0; y < 8; ++y) f[y] = g[y];
             }
-#pragma unroll
-            for (int x = 0; x < 8; ++x)
-                if (!isfinite(f[x])) {
-                    f[x] = 0.f;
-                    atomicMax(bad + e * Dv + d + x, kC - (s0 + t));
-                    atomicMax(flag + e, 1);
-                }
         }
-        bf16x8 w[3];
-        split8(f, w);
-        put(v3, NB, Dv, t, d, w);
+        finish(t, d, f);
     }
 }
 
@@ -500,9 +556,10 @@ int run(const T* proj, long long ld, int q_off, int k_off, int v_off, const floa
     float* u = (float*)(work + l.u);
     int *flag = (int*)(work + l.flag), *bad = (int*)(work + l.bad);
     NXD_CHECK_CUDA(cudaMemsetAsync(flag, 0, l.bytes - l.flag, st));
-    const size_t sm = (size_t)2 * PT * (D + 4) * sizeof(float);
-    const int vec = ld % (16 / (int)sizeof(T)) == 0 && v_off % (16 / (int)sizeof(T)) == 0 && ((uintptr_t)proj % 16) == 0;
-    retention_tc_prep_kernel<T, NB><<<dim3(NC * (kC / PT), H, B), PREP_THREADS, sm, st>>>(
+    const int per = 16 / (int)sizeof(T);
+    const int vec = (ld % per == 0 && q_off % per == 0 && k_off % per == 0 && v_off % per == 0 && ((uintptr_t)proj % 16) == 0) |
+                    (rot % 16 == 0 && (((uintptr_t)rope_cos | (uintptr_t)rope_sin) % 16) == 0 ? 2 : 0);
+    retention_tc_prep_kernel<T, NB><<<dim3(3 * NC * (kC / PT), H, B), PREP_THREADS, 0, st>>>(
         proj, ld, q_off, k_off, v_off, decay, q3, k3, kd3, v3, flag, bad, q_start, n_new, Tn, NC, H, D, Dv, kscale, rope_cos,
         rope_sin, rot, halves, max_pos, vec);
     NXD_LAUNCH_CHECK();

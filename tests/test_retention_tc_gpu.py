@@ -97,3 +97,28 @@ def test_a_value_that_is_not_a_number_leaves_the_tokens_before_it_alone():
             assert out[token:].isnan().all() and S[column].isnan().all()
         else:
             assert out[token].isnan().all() and torch.equal(out[token + 1:], good[token + 1:]) and torch.equal(S, good_S)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+# rotations of whole vectors, of parts of one and of neighbours; rows, values and tables that take 16-byte loads and ones that do not
+@pytest.mark.parametrize("D,rot,layout", [(64, 48, "halves"), (64, 40, "halves"), (128, 24, "pairs"), (64, 64, "pairs"), (256, 32, "halves")])
+@pytest.mark.parametrize("first", [0, 3])
+def test_rotations_and_rows_at_odd_addresses(dtype, D, rot, layout, first, monkeypatch):
+    from neuronx_distributed_llama3_2_b200.ops import retention as ret
+
+    monkeypatch.setattr(ret, "_tc_wanted", lambda *sizes: True)
+    T, H, Dv = 67, 2, 64
+    gen = torch.Generator(device="cuda").manual_seed(D + rot)
+    proj = torch.randn(1, T, 2 * H * D + H * Dv + first, generator=gen, device="cuda").to(dtype)
+    ang = torch.outer(torch.arange(T, dtype=torch.float64), 0.7 ** torch.arange(rot // 2, dtype=torch.float64))
+    tables = torch.stack([ang.cos(), ang.sin()]).float().cuda()
+    decay, S = torch.tensor([0.98, 0.9], device="cuda"), torch.zeros(1, H, D, Dv, device="cuda")
+    out = ret.retention_chunkwise(proj, (first, first + H * D, first + 2 * H * D), decay, S,
+                                  torch.zeros(1, dtype=torch.int32, device="cuda"), H, D, Dv, D ** -0.5, tuple(tables), layout)[0]
+    q, k, v = proj[0, :, first:].double().split([H * D, H * D, H * Dv], dim=-1)
+    q, k = (_turn(x.unflatten(-1, (H, D)), torch.arange(T, device="cuda"), *tables, layout) for x in (q, k))
+    t = torch.arange(T, dtype=torch.float64, device="cuda")
+    for h in range(H):
+        scores = (q[:, h] @ k[:, h].t() * D ** -0.5 * decay[h].double() ** (t.unsqueeze(1) - t).clamp(min=0)).tril()
+        ref = scores @ v.unflatten(-1, (H, Dv))[:, h]
+        assert (out[:, h] - ref).norm() <= 3e-7 * ref.norm()             # as above
