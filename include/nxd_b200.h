@@ -109,6 +109,14 @@ int nxd_kv_cache_update(const void* new_k, const void* new_v, void* cache_k, voi
                         const int* seq_ids, const int* block_table, long long stride_b, long long stride_h,
                         int page_size, int max_pages, int B, int n_kv, int T_new, int D, void* stream);
 
+/* all decoder layers of a token step of one sequence in one launch (csrc/token_stack.cu); bytes of scratch, 0: does not apply */
+long long nxd_token_stack_scratch(int layers, int B, int H, int I, int n_q, int n_kv, int D);
+int nxd_token_stack(const void* hidden, void* out, const void* const* pointers, const float* eps, int layers, const float* cos_t,
+                    const float* sin_t, const int* positions, const int* lengths, const int* seq_ids, const int* block_table,
+                    long long stride_b, long long stride_h, int page_size, int max_pages, void* scratch, int H, int I, int n_q,
+                    int n_kv, int D, float scale, long long wait_clocks, void* stream);
+int nxd_token_stack_status(int* gave_up, void* stream);
+
 /* ---- embedding (reference: parallel_layers/layers.py:215-238) ---------------------------------- */
 int nxd_embedding_fwd(const long long* ids, const void* weight, void* out, long long T, int H, int vocab_start,
                       int vocab_local, int B, int S, int seq_first_out, void* stream);

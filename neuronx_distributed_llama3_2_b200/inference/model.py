@@ -273,6 +273,45 @@ class KVCacheInferenceMixin:
             return gemm_smallm(act, mlp.down_proj.weight, residual=x2).reshape(B, 1, -1), None
         return all_reduce(gemm_smallm(act, mlp.down_proj.weight)).reshape(B, 1, -1), x2.reshape(B, 1, -1)
 
+    def _token_stack(self, hidden, residual, positions, seq_ids, lengths):
+        """All decoder layers of a step of one sequence in one launch (``csrc/token_stack.cu``), ``None`` where that does not
+        apply: the layers that ``_layer_batched_decode`` takes on one process, all alike, of a size that is compiled, with contiguous
+        weights."""
+        from ..ops import decode_fused
+
+        layers, base, cls = list(self._decoder_layers()), KVCacheInferenceMixin, type(self)
+        if (hidden.shape[0] != 1 or residual is not None or not layers or not hidden.is_cuda
+                or hidden.dtype != torch.bfloat16 or not hidden.is_contiguous() or ps.get_tensor_model_parallel_size() > 1
+                or any(getattr(cls, n) is not getattr(base, n) for n in ("_layer", "_layer_batched_decode", "_decode_attention", "_rope"))
+                or os.environ.get("NXD_DECODE_ATTN", "")[:1] == "f"):
+            return None
+        B, H = hidden.shape[0], hidden.shape[-1]
+        if not all(self._tensor_core_decode(layer, hidden) and self._fused_decode_ok(layer, hidden, batched=True) for layer in layers):
+            return None
+        attn, kc = layers[0].self_attn, self.kv_cache
+        nq, nkv, D, I = attn.q_heads_local, attn.kv_heads_local, attn.head_dim, layers[0].mlp.down_proj.weight.shape[1]
+        scratch = decode_fused.token_stack_scratch(len(layers), B, H, I, nq, nkv, D)
+        if not scratch:
+            return None
+        shapes = [(H,), ((nq + 2 * nkv) * D, H), (H, nq * D), (H,), (2 * I, H), (H, I)]
+        stack = []
+        for i, layer in enumerate(layers):
+            n1, n2, at, mlp = layer.input_layernorm, layer.post_attention_layernorm, layer.self_attn, layer.mlp
+            ws = (n1.weight, at.qkv_proj.weight_qkv, at.o_proj.weight, n2.weight, mlp.gate_up_proj.weight, mlp.down_proj.weight)
+            caches = kc.layer(i)
+            if ((at.q_heads_local, at.kv_heads_local, at.head_dim) != (nq, nkv, D) or any(
+                    t.dtype != torch.bfloat16 or tuple(t.shape) != s or not t.is_contiguous() or t.data_ptr() % 16 for t, s in zip(ws, shapes))
+                    or any(t.dtype != torch.bfloat16 or t.stride() != kc.layer(0)[0].stride() or t.data_ptr() % 16 for t in caches)):
+                return None
+            stack.append(((*ws, *caches), n1.variance_epsilon, n2.variance_epsilon))
+        if kc.layer(0)[0].stride(0) % 8 or kc.layer(0)[0].stride(1) % 8:
+            return None
+        pos, sid = self._decode_i32(positions, seq_ids)
+        cos, sin = self._rope(hidden.device)
+        return decode_fused.token_stack(hidden.view(B, H), stack, cos, sin, pos, lengths, nq, nkv, D, scratch, seq_ids=sid,
+                                        block_table=kc.block_table if kc.paged else None,
+                                        page_size=kc.page_size if kc.paged else 0).view(B, 1, H)
+
     def _layer_fused_decode(self, i: int, layer, hidden, residual, positions, seq_ids, lengths):
         """One token per sequence: RMSNorm+QKV+RoPE+cache write | attention (split, merge) | o_proj+residual |
         RMSNorm+gate/up+SwiGLU | down_proj+residual.  The residual stream leaves every row-parallel GEMV already
@@ -416,8 +455,12 @@ class KVCacheInferenceMixin:
         identity = default_lines or not self.inference_config.is_continuous_batching
         sid = None if (identity and not prefill) else (
             seq_ids if seq_ids is not None else torch.arange(B, device=input_ids.device, dtype=torch.int32))
-        for i, layer in enumerate(self._decoder_layers()):
-            hidden, residual = self._layer(i, layer, hidden, residual, position_ids, sid, lengths, prefill)
+        stacked = None if prefill else self._token_stack(hidden, residual, position_ids, sid, lengths)
+        if stacked is not None:
+            hidden = stacked
+        else:
+            for i, layer in enumerate(self._decoder_layers()):
+                hidden, residual = self._layer(i, layer, hidden, residual, position_ids, sid, lengths, prefill)
         if logit_index is not None:
             rows, cols = logit_index[0].long(), logit_index[1].long()
             hidden, residual = hidden[rows, cols], (residual[rows, cols] if residual is not None else None)

@@ -11,7 +11,7 @@ eight."""
 from __future__ import annotations
 
 import ctypes as _c
-from typing import Optional
+from typing import Optional, Sequence, Tuple
 
 import torch
 
@@ -141,3 +141,45 @@ def gate_up_swiglu_batched(xn: torch.Tensor, w_gate_up: torch.Tensor, splits: in
         _c.c_longlong(out.stride(0)), _c.c_int(B), _c.c_int(K), _c.c_int(I), _c.c_int(splits), _lib.stream_ptr())
     _lib.check(rc, "nxd_smallm_gate_up_swiglu")
     return out
+
+
+def token_stack_scratch(layers: int, B: int, H: int, I: int, n_q: int, n_kv: int, D: int) -> int:
+    """Bytes of scratch with which ``token_stack`` takes such layers, 0 where it does not (``csrc/token_stack.cu``)."""
+    fn = _lib.lib().nxd_token_stack_scratch
+    fn.restype = _c.c_longlong
+    return int(fn(*(_c.c_int(v) for v in (layers, B, H, I, n_q, n_kv, D))))
+
+
+def token_stack(x: torch.Tensor, layers: Sequence[Tuple[Sequence[torch.Tensor], float, float]], cos: torch.Tensor, sin: torch.Tensor,
+                positions: torch.Tensor, lengths: torch.Tensor, n_q: int, n_kv: int, D: int, scratch: int,
+                seq_ids: Optional[torch.Tensor] = None, block_table: Optional[torch.Tensor] = None, page_size: int = 0,
+                wait_clocks: int = -1) -> torch.Tensor:
+    """A token-generation step ``x [1, H]`` through whole decoder layers in one launch -> ``[1, H]`` (``nxd_token_stack``).  A layer is
+    ``((input norm, q|k|v, o, norm behind the attention, gate|up, down, cache of keys, of values), eps, eps)``; the caches are written
+    at ``positions``.  ``scratch``: bytes, of ``token_stack_scratch``.  ``wait_clocks``: clocks after which a wait inside gives up, -1:
+    two seconds (``token_stack_gave_up``)."""
+    H = x.shape[1]
+    tensors = [t for layer in layers for t in layer[0]]
+    ck = layers[0][0][6]
+    assert x.shape[0] == 1 and x.is_contiguous() and cos.is_contiguous() and sin.is_contiguous() and cos.shape[1] == D // 2
+    assert all(t.dtype == torch.bfloat16 for t in tensors) and all(t.stride() == ck.stride() for s, _, _ in layers for t in s[6:])
+    assert all(t.is_contiguous() for s, _, _ in layers for t in s[:6]) and positions.dtype == lengths.dtype == torch.int32
+    out = torch.empty_like(x)
+    work = torch.empty(scratch, dtype=torch.uint8, device=x.device)
+    pointers = (_c.c_void_p * len(tensors))(*(t.data_ptr() for t in tensors))
+    eps = (_c.c_float * (2 * len(layers)))(*(e for layer in layers for e in layer[1:]))
+    rc = _lib.lib().nxd_token_stack(
+        _lib.ptr(x), _lib.ptr(out), pointers, eps, _c.c_int(len(layers)), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(positions),
+        _lib.ptr(lengths), _lib.ptr(seq_ids), _lib.ptr(block_table), _c.c_longlong(ck.stride(0)), _c.c_longlong(ck.stride(1)),
+        _c.c_int(page_size), _c.c_int(block_table.shape[1] if block_table is not None else 0), _lib.ptr(work), _c.c_int(H),
+        _c.c_int(layers[0][0][5].shape[1]), _c.c_int(n_q), _c.c_int(n_kv), _c.c_int(D), _c.c_float(D ** -0.5),
+        _c.c_longlong(wait_clocks), _lib.stream_ptr())
+    _lib.check(rc, "nxd_token_stack")
+    return out
+
+
+def token_stack_gave_up() -> bool:
+    """Whether a ``token_stack`` on this device has given up a wait since the last call (its results are NaN).  Waits for the stream."""
+    flag = _c.c_int(0)
+    _lib.check(_lib.lib().nxd_token_stack_status(_c.byref(flag), _lib.stream_ptr()), "nxd_token_stack_status")
+    return bool(flag.value)

@@ -1,0 +1,159 @@
+"""All decoder layers of a one-sequence step in one launch, against the layers kernel by kernel and against float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SIZES = {"64": (2048, 8192, 32, 8, 64), "128": (3072, 8192, 24, 8, 128)}      # hidden, feed-forward, heads, key / value heads, head size
+EPS = 1e-5
+
+
+def _draw(size, layers, lines, rows, seed):
+    H, I, nq, nkv, D = SIZES[size]
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+
+    def normal(*shape, std=0.02, mean=0.0):
+        return torch.empty(shape, dtype=torch.bfloat16, device="cuda").normal_(mean, std, generator=gen)
+
+    return [[normal(H, std=0.1, mean=1.0), normal((nq + 2 * nkv) * D, H), normal(H, nq * D), normal(H, std=0.1, mean=1.0),
+             normal(2 * I, H), normal(H, I), normal(lines, nkv, rows, D, std=1.0), normal(lines, nkv, rows, D, std=1.0)]
+            for _ in range(layers)], normal(1, H, std=1.0)
+
+
+def _tables(D, rows):
+    ang = torch.outer(torch.arange(rows, dtype=torch.float64), 500000.0 ** (-torch.arange(0, D, 2, dtype=torch.float64) / D))
+    return ang.cos().float().cuda(), ang.sin().float().cuda()
+
+
+def _chain(x, layers, size, cos, sin, pos, lens, **place):
+    from neuronx_distributed_llama3_2_b200.ops import decode_fused as df
+    from neuronx_distributed_llama3_2_b200.ops.attention import decode_attention
+    from neuronx_distributed_llama3_2_b200.ops.gemm import gemm_smallm
+    from neuronx_distributed_llama3_2_b200.ops.norm import rms_norm
+
+    H, I, nq, nkv, D = SIZES[size]
+    for n1, wqkv, wo, n2, wgu, wd, ck, cv in layers:
+        q = df.qkv_rope_cache_batched(rms_norm(x, n1, EPS), wqkv, cos, sin, pos, ck, cv, nq, nkv, D, **place)
+        o = decode_attention(q, ck, cv, lens, block_table=place.get("block_table"), page_size=place.get("page_size", 0),
+                             seq_ids=place.get("seq_ids")).reshape(1, nq * D)
+        x = gemm_smallm(o, wo, residual=x)
+        x = gemm_smallm(df.gate_up_swiglu_batched(rms_norm(x, n2, EPS), wgu), wd, residual=x)
+    return x
+
+
+def _exact(x, layers, size, cos, sin, n, rows_of):
+    H, I, nq, nkv, D = SIZES[size]
+    x = x[0].double()
+    c, s = cos[n - 1].double(), sin[n - 1].double()
+
+    def norm(v, w):
+        return v * torch.rsqrt(v.square().mean() + EPS) * w.double()
+
+    def turn(v):
+        a, b = v.chunk(2, dim=-1)
+        return torch.cat([a * c - b * s, b * c + a * s], dim=-1)
+
+    for n1, wqkv, wo, n2, wgu, wd, ck, cv in layers:
+        q, k, v = (wqkv.double() @ norm(x, n1)).reshape(-1, D).split([nq, nkv, nkv])
+        keys = torch.cat([rows_of(ck)[:, :n - 1].double(), turn(k).unsqueeze(1)], dim=1)
+        values = torch.cat([rows_of(cv)[:, :n - 1].double(), v.unsqueeze(1)], dim=1)
+        p = torch.softmax(torch.einsum("ghd,gnd->ghn", turn(q).reshape(nkv, -1, D), keys) * D ** -0.5, dim=-1)
+        x = x + wo.double() @ torch.einsum("ghn,gnd->ghd", p, values).flatten()
+        g, u = (wgu.double() @ norm(x, n2)).chunk(2)
+        x = x + wd.double() @ (torch.nn.functional.silu(g) * u)
+    return x
+
+
+def _stack(x, layers, size, cos, sin, pos, lens, **place):
+    from neuronx_distributed_llama3_2_b200.ops import decode_fused as df
+
+    H, I, nq, nkv, D = SIZES[size]
+    scratch = df.token_stack_scratch(len(layers), 1, H, I, nq, nkv, D)
+    assert scratch > 0 and df.token_stack_scratch(len(layers), 2, H, I, nq, nkv, D) == 0
+    return df.token_stack(x, [(tuple(w), EPS, EPS) for w in layers], cos, sin, pos, lens, nq, nkv, D, scratch, **place)
+
+
+@pytest.mark.parametrize("size", SIZES)
+# the first token, edges of the parts of 256 keys, of the ring's slots of 64 and 128 keys, more keys than 16 parts of 256; pages that end inside a
+# slot and hold whole ones
+@pytest.mark.parametrize("n,page", [(1, 0), (2, 16), (64, 0), (257, 128), (511, 16), (4500, 128)])
+def test_layers_in_one_launch(size, n, page):
+    H, I, nq, nkv, D = SIZES[size]
+    lines, rows = 2, (n + 127) // 128 * 128
+    layers, x = _draw(size, 2, lines, rows, n)
+    cos, sin = _tables(D, rows)
+    place = {"seq_ids": torch.tensor([1], dtype=torch.int32, device="cuda")}
+
+    def rows_of(cache):
+        return cache[1]
+
+    if page:
+        order = torch.randperm(lines * rows // page, generator=torch.Generator().manual_seed(n)).cuda()
+        place.update(block_table=order.to(torch.int32).reshape(lines, -1), page_size=page)
+        for w in layers:
+            w[6:] = [t.reshape(-1, nkv, page, D) for t in w[6:]]
+
+        def rows_of(cache):
+            return cache[order.reshape(lines, -1)[1]].transpose(0, 1).flatten(1, 2)
+
+    pos, lens = (torch.tensor([v], dtype=torch.int32, device="cuda") for v in (n - 1, n))
+    ref = _exact(x, layers, size, cos, sin, n, rows_of)
+    other = [[t.clone() for t in w] for w in layers]
+    chain = _chain(x, other, size, cos, sin, pos, lens, **place)
+    before = [[rows_of(t).clone() for t in w[6:]] for w in layers]
+    out = _stack(x, layers, size, cos, sin, pos, lens, **place)
+
+    def off(y):
+        return float((y[0].double() - ref).norm() / ref.norm())
+
+    assert off(out) <= 1.25 * off(chain)          # the same roundings of other sums: 0.97 to 1.03 times as far off
+    for w, c, b in zip(layers, other, before):
+        for mine, theirs, was in zip(w[6:], c[6:], b):
+            mine, theirs = rows_of(mine), rows_of(theirs)
+            assert torch.equal(mine[:, :n - 1], was[:, :n - 1]) and torch.equal(mine[:, n:], was[:, n:])
+            # projections of streams that differ by a few roundings to bf16
+            assert (mine[:, n - 1].float() - theirs[:, n - 1].float()).norm() <= 2e-2 * theirs[:, n - 1].float().norm()
+    assert torch.equal(out, _stack(x, layers, size, cos, sin, pos, lens, **place))
+
+
+def test_replays_follow_the_position():
+    H, I, nq, nkv, D = SIZES["64"]
+    layers, x = _draw("64", 2, 1, 640, 7)
+    cos, sin = _tables(D, 640)
+    pos, lens = (torch.tensor([v], dtype=torch.int32, device="cuda") for v in (300, 301))
+    run = [[t.clone() for t in w] for w in layers]
+    _stack(x, run, "64", cos, sin, pos, lens)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = _stack(x, run, "64", cos, sin, pos, lens)
+    for n in (301, 302, 20, 600):
+        pos.fill_(n - 1)
+        lens.fill_(n)
+        for w, given in zip(run, layers):
+            for mine, theirs in zip(w[6:], given[6:]):
+                mine.copy_(theirs)
+        graph.replay()
+        eager = [[t.clone() for t in w] for w in layers]
+        assert torch.equal(out, _stack(x, eager, "64", cos, sin, pos, lens))
+        assert all(torch.equal(a, b) for w, e in zip(run, eager) for a, b in zip(w[6:], e[6:]))
+
+
+def test_waits_give_up():
+    """Limits from none at all up to more than a step takes: what is left is the result or NaN, and the host is told."""
+    from neuronx_distributed_llama3_2_b200.ops import decode_fused as df
+
+    H, I, nq, nkv, D = SIZES["64"]
+    layers, x = _draw("64", 2, 1, 256, 9)
+    cos, sin = _tables(D, 256)
+    pos, lens = (torch.tensor([v], dtype=torch.int32, device="cuda") for v in (99, 100))
+    df.token_stack_gave_up()
+    good = _stack(x, layers, "64", cos, sin, pos, lens)
+    assert not df.token_stack_gave_up() and torch.isfinite(good).all()
+    for clocks in (0, 100, 1000, 10000, 100000, -1):
+        out = _stack(x, layers, "64", cos, sin, pos, lens, wait_clocks=clocks)
+        gave_up = df.token_stack_gave_up()
+        assert (out.isnan() | (out == good)).all() and (gave_up or not out.isnan().any())
+        if clocks == 0:
+            assert gave_up and out.isnan().all()
+        if clocks == -1:
+            assert not gave_up
