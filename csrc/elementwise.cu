@@ -128,6 +128,8 @@ __global__ void rope_cache_kernel(bf16* __restrict__ x, const float* __restrict_
                                   const int* __restrict__ positions, bf16* __restrict__ cache_k, bf16* __restrict__ cache_v,
                                   const int* __restrict__ seq_ids, const int* __restrict__ block_table, long long stride_b,
                                   long long stride_h, int page_size, int max_pages, int Tn, size_t rows, int n_q, int n_kv, int D) {
+    pdl_trigger();
+    pdl_wait();
     const int half_vec = D >> 4, heads = n_q + 2 * n_kv;
     const size_t total = rows * (size_t)heads * half_vec;
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
@@ -242,9 +244,9 @@ NXD_API int nxd_rope_cache_write(void* qkv, const float* cos_t, const float* sin
     NXD_REQUIRE(D % 16 == 0, "rope_cache: head dim %d must be a multiple of 16", D);
     const size_t rows = (size_t)B * Tn;
     if (rows == 0) return 0;
-    rope_cache_kernel<<<grid_for(rows * (n_q + 2 * n_kv) * (D / 16), 256), 256, 0, (cudaStream_t)stream>>>(
-        (bf16*)qkv, cos_t, sin_t, positions, (bf16*)cache_k, (bf16*)cache_v, seq_ids, block_table, stride_b, stride_h,
-        page_size > 0 ? page_size : 1, max_pages, Tn, rows, n_q, n_kv, D);
+    NXD_CHECK_CUDA(nxd_launch_pdl(rope_cache_kernel, dim3(grid_for(rows * (n_q + 2 * n_kv) * (D / 16), 256)), dim3(256), 0,
+                                  (cudaStream_t)stream, (bf16*)qkv, cos_t, sin_t, positions, (bf16*)cache_k, (bf16*)cache_v, seq_ids,
+                                  block_table, stride_b, stride_h, page_size > 0 ? page_size : 1, max_pages, Tn, rows, n_q, n_kv, D));
     NXD_LAUNCH_CHECK();
     return 0;
 }

@@ -106,6 +106,8 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(pv_done + 1);
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    pdl_trigger();
+    if (CACHE) pdl_wait();
     // grid = (q heads, batch, q blocks): the q block is the slowest launch dimension and counted from the end, so the
     // long causal rows of EVERY head are scheduled before any short one (longest-first list scheduling)
     const int mb = gridDim.z - 1 - blockIdx.z;
@@ -149,6 +151,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         ptx::fence_barrier_init();
     }
     if (warp == 1) ptx::tmem_alloc<1>(tmem_ptr_smem, L::kTmemCols);
+    if (!CACHE) pdl_wait();
     float* dtab = reinterpret_cast<float*>(sP);          // bias table (SCORE): the P staging area is free, P lives in TMEM
     constexpr float kL2e = score::kLog2e;                // r1 ln(.) in log2 units is r1 log2(.)
     constexpr float kSign = SCORE == 2 ? -1.f : 1.f;     // sigmoid weights are computed from the negative score
@@ -557,7 +560,7 @@ int launch_fwd_tc_one(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
     dim3 grid(p.Hq, p.B, (p.Sq + kBM - 1) / kBM);
     constexpr auto kern = fa_fwd_tc_kernel<D, CAUSAL, DROP>;
     NXD_CHECK_CUDA(nxd_allow_smem<kern>(L::kBytes));
-    kern<<<grid, kThreadsTc, L::kBytes, st>>>(tq, tk, tv, to, p);
+    NXD_CHECK_CUDA(nxd_launch_pdl(kern, grid, dim3(kThreadsTc), L::kBytes, st, tq, tk, tv, to, p));
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -579,7 +582,7 @@ int launch_fwd_tc_win(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
     dim3 grid(p.Hq, p.B, (p.Sq + kBM - 1) / kBM);
     constexpr auto kern = fa_fwd_tc_kernel<D, true, false, true, SCORE, CACHE>;
     NXD_CHECK_CUDA(nxd_allow_smem<kern>(L::kBytes));
-    kern<<<grid, kThreadsTc, L::kBytes, st>>>(tq, tk, tv, to, p);
+    NXD_CHECK_CUDA(nxd_launch_pdl(kern, grid, dim3(kThreadsTc), L::kBytes, st, tq, tk, tv, to, p));
     NXD_LAUNCH_CHECK();
     return 0;
 }

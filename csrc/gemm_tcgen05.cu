@@ -65,7 +65,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     int* seg_tile = reinterpret_cast<int*>(smem + L::kBarrierOffset + L::kBarrierBytes);   // first tile of every expert
     int* seg_row = seg_tile + kSegMaxExperts + 1;                                          // first row of every expert
     if constexpr (kSorted) {
-        if (warp == 3) segment_starts(seg.counts, batches, num_n_tiles, seg_row, seg_tile);
+        if (warp == 3) {
+            pdl_wait();
+            segment_starts(seg.counts, batches, num_n_tiles, seg_row, seg_tile);
+        }
     }
     const int num_k_blocks = (K + kBlockK - 1) / kBlockK;
     const int cluster_id = blockIdx.x >> 1;
@@ -92,6 +95,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     ptx::cluster_sync();
     ptx::tcgen05_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_smem, 0);
+    pdl_wait();                    // barriers, tensor memory and tensor maps were set up beside the end of the kernel before
     if constexpr (kSorted) num_tiles = seg_tile[batches];
     // problem index, tile coordinates and first row of a tile
     auto locate = [&](int tile, int& e, int& tm, int& tn, int& row_base) {
@@ -150,6 +154,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                     if (++stage == kStages) { stage = 0; phase ^= 1; }
                 }
             }
+            pdl_trigger();         // behind this CTA's last loads: what follows may set itself up now, not while tiles are still to come
         }
     } else if (warp == 1) {
         // ======================= MMA issuer (leader CTA) =======================
@@ -303,7 +308,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
     const int num_tiles = ((M + kTileM - 1) / kTileM) * ((N + BN - 1) / BN);
     int clusters = nxd_num_sms() / 2;
     if (clusters > num_tiles) clusters = num_tiles;
-    kern<<<dim3(clusters * 2), dim3(kThreads), L::kSmemBytes, stream>>>(ta, tb, td, M, N, K, 1, SegArgs{});
+    NXD_CHECK_CUDA(nxd_launch_pdl(kern, dim3(clusters * 2), dim3(kThreads), L::kSmemBytes, stream, ta, tb, td, M, N, K, 1, SegArgs{}));
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -377,7 +382,8 @@ static int launch_grouped(const CUtensorMap& ta, const CUtensorMap& tb, const CU
     const long num_tiles = (long)E * ((M + kTileM - 1) / kTileM) * ((N + BN - 1) / BN);
     long clusters = nxd_num_sms() / 2;
     if (clusters > num_tiles) clusters = num_tiles;
-    kern<<<dim3((unsigned)clusters * 2), dim3(kThreads), L::kSmemBytes, stream>>>(ta, tb, td, M, N, K, E, SegArgs{});
+    NXD_CHECK_CUDA(nxd_launch_pdl(kern, dim3((unsigned)clusters * 2), dim3(kThreads), L::kSmemBytes, stream, ta, tb, td, M, N, K, E,
+                                  SegArgs{}));
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -440,7 +446,7 @@ static int launch_experts(const CUtensorMap& ta, const CUtensorMap& tb, const CU
     const long most = ((long)rows / kTileM + E) * ((N + out_n - 1) / out_n);
     long clusters = nxd_num_sms() / 2;
     if (clusters > most) clusters = most;
-    kern<<<dim3((unsigned)clusters * 2), dim3(kThreads), kSmem, stream>>>(ta, tb, td, rows, N, K, E, seg);
+    NXD_CHECK_CUDA(nxd_launch_pdl(kern, dim3((unsigned)clusters * 2), dim3(kThreads), kSmem, stream, ta, tb, td, rows, N, K, E, seg));
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -508,7 +514,8 @@ static int launch_swiglu(const CUtensorMap& ta, const CUtensorMap& tb, const CUt
     const long tiles = (long)((M + kTileM - 1) / kTileM) * ((N + BN / 2 - 1) / (BN / 2));
     long clusters = nxd_num_sms() / 2;
     if (clusters > tiles) clusters = tiles;
-    kern<<<dim3((unsigned)clusters * 2), dim3(kThreads), L::kSmemBytes, stream>>>(ta, tb, td, M, N, K, 1, SegArgs{});
+    NXD_CHECK_CUDA(nxd_launch_pdl(kern, dim3((unsigned)clusters * 2), dim3(kThreads), L::kSmemBytes, stream, ta, tb, td, M, N, K, 1,
+                                  SegArgs{}));
     NXD_LAUNCH_CHECK();
     return 0;
 }

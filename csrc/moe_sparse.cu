@@ -169,6 +169,8 @@ moe_router_kernel(const T* __restrict__ h, const float* __restrict__ wr, const f
                   float* __restrict__ sgate, long long N, int W, int R, int top, float out_scale,
                   const float* __restrict__ zbias, int mode) {
     extern __shared__ float smem[];
+    pdl_trigger();
+    pdl_wait();
     constexpr int G = SHARE ? 4 : 8;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long n0 = SHARE ? blockIdx.x : ((long long)blockIdx.x * RT_WARPS + warp) * TOK;
@@ -467,6 +469,8 @@ __global__ void moe_gather_combine_kernel(const TY* __restrict__ ys, const int* 
                                           const int* __restrict__ idx, const float* __restrict__ wts,
                                           const T* __restrict__ h, const TY* __restrict__ shared_out,
                                           const float* __restrict__ sgate, float* __restrict__ y, int top, int W, int E) {
+    pdl_trigger();
+    pdl_wait();
     const long long t = blockIdx.x;
     for (int c = threadIdx.x * V; c < W; c += blockDim.x * V) {
         float a[V];
@@ -507,6 +511,8 @@ __global__ void __launch_bounds__(CNT_THREADS)
 moe_count_kernel(const int* __restrict__ idx, int* __restrict__ counts, int* __restrict__ place, long long P, int top, int E) {
     extern __shared__ int hist[];                       // [E] pairs of this block, then [E] the block's first place
     int* first = hist + E;
+    pdl_trigger();
+    pdl_wait();
     for (int e = threadIdx.x; e < E; e += CNT_THREADS) hist[e] = 0;
     __syncthreads();
     if (blockIdx.x == 0 && threadIdx.x == 0) counts[E] = (int)(P / top);      // the tokens: rows of a shared expert
@@ -538,6 +544,8 @@ moe_gather_rows_kernel(const bf16* __restrict__ h, const int* __restrict__ idx, 
                        bf16* __restrict__ x, long long P, int top, int W8, int E) {
     __shared__ int row0[nxd_gemm::kSegMaxExperts + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    pdl_trigger();
+    pdl_wait();
     if (warp == 0) nxd_gemm::segment_starts(counts, E, 0, row0, nullptr);
     __syncthreads();
     const long long p = (long long)blockIdx.x * GA_WARPS + warp;
@@ -567,8 +575,10 @@ moe_sort_few_kernel(const bf16* __restrict__ h, const int* __restrict__ idx, int
                     int E) {
     __shared__ int expert[FEW_PAIRS], cnt[nxd_gemm::kSegMaxExperts], row0[nxd_gemm::kSegMaxExperts + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    pdl_trigger();
     for (int e = threadIdx.x; e < E; e += GA_WARPS * 32) cnt[e] = 0;
     __syncthreads();
+    pdl_wait();
     for (int p = threadIdx.x; p < P; p += GA_WARPS * 32) {
         const int e = idx[p];
         expert[p] = e;
@@ -619,8 +629,8 @@ NXD_API int nxd_moe_router(int dtype, const void* h, const float* wr, const floa
     const size_t smem = (size_t)(tok == 0 ? 2 : RT_WARPS * (tok + 1)) * R * sizeof(float);
     const unsigned blocks = (unsigned)(tok == 0 ? N : (N + RT_WARPS * tok - 1) / (RT_WARPS * tok));
 #define NXD_RT(T, V, TOK, SHARE)                                                                                        \
-    moe_router_kernel<T, V, TOK, SHARE><<<blocks, RT_WARPS * 32, smem, (cudaStream_t)stream>>>(                         \
-        (const T*)h, wr, corr, wsg, idx, wts, sgate, N, W, R, top, out_scale, zbias, mode)
+    NXD_CHECK_CUDA(nxd_launch_pdl(moe_router_kernel<T, V, TOK, SHARE>, dim3(blocks), dim3(RT_WARPS * 32), smem, (cudaStream_t)stream, \
+                                  (const T*)h, wr, corr, wsg, idx, wts, sgate, N, W, R, top, out_scale, zbias, mode))
 #define NXD_RT_V(T, V)                                                                                                  \
     do {                                                                                                                \
         if (tok == 0) NXD_RT(T, V, 1, true);                                                                            \
@@ -651,16 +661,16 @@ NXD_API int nxd_moe_sort_rows(const void* h, const int* idx, int* counts, int* s
     NXD_REQUIRE(((uintptr_t)h % 16) == 0 && ((uintptr_t)x % 16) == 0, "sort rows: rows must be 16-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
     if (nxd_moe_sort_counts_itself(P)) {
-        moe_sort_few_kernel<<<(unsigned)((P + GA_WARPS - 1) / GA_WARPS), GA_WARPS * 32, 0, st>>>(
-            (const bf16*)h, idx, counts, slot, in_scale, row_scale, (bf16*)x, (int)P, top, W / 8, E);
+        NXD_CHECK_CUDA(nxd_launch_pdl(moe_sort_few_kernel, dim3((unsigned)((P + GA_WARPS - 1) / GA_WARPS)), dim3(GA_WARPS * 32), 0, st,
+                                      (const bf16*)h, idx, counts, slot, in_scale, row_scale, (bf16*)x, (int)P, top, W / 8, E));
         NXD_LAUNCH_CHECK();
         return 0;
     }
-    moe_count_kernel<<<(unsigned)((P + CNT_PAIRS - 1) / CNT_PAIRS), CNT_THREADS, 2 * E * sizeof(int), st>>>(idx, counts, slot,
-                                                                                                           P, top, E);
+    NXD_CHECK_CUDA(nxd_launch_pdl(moe_count_kernel, dim3((unsigned)((P + CNT_PAIRS - 1) / CNT_PAIRS)), dim3(CNT_THREADS),
+                                  2 * E * sizeof(int), st, idx, counts, slot, P, top, E));
     NXD_LAUNCH_CHECK();
-    moe_gather_rows_kernel<<<(unsigned)((P + GA_WARPS - 1) / GA_WARPS), GA_WARPS * 32, 0, st>>>(
-        (const bf16*)h, idx, counts, slot, in_scale, row_scale, (bf16*)x, P, top, W / 8, E);
+    NXD_CHECK_CUDA(nxd_launch_pdl(moe_gather_rows_kernel, dim3((unsigned)((P + GA_WARPS - 1) / GA_WARPS)), dim3(GA_WARPS * 32), 0, st,
+                                  (const bf16*)h, idx, (const int*)counts, slot, in_scale, row_scale, (bf16*)x, P, top, W / 8, E));
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -776,12 +786,12 @@ NXD_API int nxd_moe_gather_combine(int dtype, const void* ys, const int* slot, c
     auto al = [](const void* p) { return ((uintptr_t)p % 16) == 0; };
     const bool vec = W % 8 == 0 && al(ys) && al(h) && al(shared_out) && al(y);
 #define NXD_GC(T, V)                                                                                     \
-    moe_gather_combine_kernel<T, V><<<(unsigned)N, 128, 0, (cudaStream_t)stream>>>(                      \
-        (const T*)ys, slot, idx, wts, (const T*)h, (const T*)shared_out, sgate, y, top, W, E)
+    NXD_CHECK_CUDA(nxd_launch_pdl(moe_gather_combine_kernel<T, V>, dim3((unsigned)N), dim3(128), 0, (cudaStream_t)stream, \
+                                  (const T*)ys, slot, idx, wts, (const T*)h, (const T*)shared_out, sgate, y, top, W, E))
     if (dtype == 2) {
 #define NXD_GC_WIDE(V)                                                                                   \
-    moe_gather_combine_kernel<bf16, V, float><<<(unsigned)N, 128, 0, (cudaStream_t)stream>>>(            \
-        (const float*)ys, slot, idx, wts, (const bf16*)h, (const float*)shared_out, sgate, y, top, W, E)
+    NXD_CHECK_CUDA(nxd_launch_pdl(moe_gather_combine_kernel<bf16, V, float>, dim3((unsigned)N), dim3(128), 0, (cudaStream_t)stream, \
+                                  (const float*)ys, slot, idx, wts, (const bf16*)h, (const float*)shared_out, sgate, y, top, W, E))
         if (vec) NXD_GC_WIDE(8); else NXD_GC_WIDE(1);
 #undef NXD_GC_WIDE
     } else if (dtype == 0) {
