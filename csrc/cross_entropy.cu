@@ -12,6 +12,8 @@ namespace {
 
 __global__ void ce_stats_kernel(const bf16* __restrict__ logits, const long long* __restrict__ target,
                                 float4* __restrict__ stats, int V, int vocab_start) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ float red[32];
     const size_t row = blockIdx.x;
     const bf16* z = logits + row * (size_t)V;
@@ -57,6 +59,8 @@ __global__ void ce_bwd_kernel(const bf16* __restrict__ logits, const long long* 
                               const float* __restrict__ lse, const float* __restrict__ gout,
                               bf16* __restrict__ grad, int V, int vocab_start, float smoothing,
                               float inv_vocab_global) {
+    pdl_trigger();
+    pdl_wait();
     const size_t row = blockIdx.x;
     const bf16* z = logits + row * (size_t)V;
     bf16* g = grad + row * (size_t)V;
@@ -94,8 +98,8 @@ NXD_API int nxd_ce_stats(const void* logits, const long long* target, float* sta
     NXD_REQUIRE(V % 8 == 0, "ce_stats: V/tp=%d must be a multiple of 8 (pad the vocab)", V);
     if (T == 0) return 0;
     const int threads = V >= 8192 ? 1024 : 256;
-    ce_stats_kernel<<<(unsigned)T, threads, 0, (cudaStream_t)stream>>>((const bf16*)logits, target,
-                                                                       (float4*)stats, V, vocab_start);
+    NXD_CHECK_CUDA((nxd_launch_pdl(ce_stats_kernel, dim3((unsigned)T), dim3(threads), 0, (cudaStream_t)stream, (const bf16*)logits,
+        target, (float4*)stats, V, vocab_start)));
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -106,9 +110,8 @@ NXD_API int nxd_ce_bwd(const void* logits, const long long* target, const float*
     NXD_REQUIRE(V % 8 == 0, "ce_bwd: V/tp=%d must be a multiple of 8 (pad the vocab)", V);
     if (T == 0) return 0;
     const int threads = V >= 8192 ? 1024 : 256;
-    ce_bwd_kernel<<<(unsigned)T, threads, 0, (cudaStream_t)stream>>>(
-        (const bf16*)logits, target, lse, grad_out, (bf16*)grad_logits, V, vocab_start, smoothing,
-        1.f / (float)vocab_global);
+    NXD_CHECK_CUDA((nxd_launch_pdl(ce_bwd_kernel, dim3((unsigned)T), dim3(threads), 0, (cudaStream_t)stream, (const bf16*)logits,
+        target, lse, grad_out, (bf16*)grad_logits, V, vocab_start, smoothing, 1.f / (float)vocab_global)));
     NXD_LAUNCH_CHECK();
     return 0;
 }

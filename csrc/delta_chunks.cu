@@ -97,6 +97,8 @@ template <int D>
 __global__ void __launch_bounds__(FT, D == 256 ? 1 : 2)
 delta_chunk_factors_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ systems,
                            uint8_t* __restrict__ tiles, const int* __restrict__ n_new, int Tn, int c0, int H, int G) {
+    pdl_trigger();
+    pdl_wait();
     constexpr int V = D / 32, A1 = D / 64;
     extern __shared__ __align__(16) float smem[];
     float* Ks = smem;                                    // [CH][D]
@@ -337,6 +339,7 @@ delta_chunk_scan_kernel(const Step p, const float* __restrict__ systems, const u
     // one by the elected thread of such a warp 35
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int col0 = blockIdx.x * CW_COLS, h = blockIdx.y, b = blockIdx.z;
+    pdl_wait();                                          // and no tensor memory before
     const int n = p.n_new != nullptr ? min(p.n_new[b], p.Tn) : p.Tn;
     const long long row0 = (long long)b * p.Tn;
     float* orow = p.out + (row0 * p.H + h) * p.Dv + col0;                        // + t * H * Dv
@@ -584,10 +587,11 @@ int launch(const Step& s, const float* systems, uint8_t* tiles, int c0, int coun
     constexpr int factors = (CH * D + CH * MTP) * 4;
     NXD_CHECK_CUDA(nxd_allow_smem<delta_chunk_factors_kernel<D>>(factors));
     NXD_CHECK_CUDA(nxd_allow_smem<delta_chunk_scan_kernel<D>>(Cfg<D>::kSmem));
-    delta_chunk_factors_kernel<D><<<dim3(count, s.H, s.B), FT, factors, st>>>(s.qn, s.kn, systems, tiles, s.n_new, s.Tn, c0, s.H, s.G);
+    NXD_CHECK_CUDA((nxd_launch_pdl(delta_chunk_factors_kernel<D>, dim3(count, s.H, s.B), dim3(FT), factors, st, s.qn, s.kn,
+        systems, tiles, s.n_new, s.Tn, c0, s.H, s.G)));
     NXD_LAUNCH_CHECK();
-    delta_chunk_scan_kernel<D><<<dim3(s.Dv / CW_COLS, s.H, s.B), kThreads, Cfg<D>::kSmem, st>>>(s, systems, tiles, c0, count,
-                                                                                                   limit);
+    NXD_CHECK_CUDA((nxd_launch_pdl(delta_chunk_scan_kernel<D>, dim3(s.Dv / CW_COLS, s.H, s.B), dim3(kThreads), Cfg<D>::kSmem, st,
+        s, systems, tiles, c0, count, limit)));
     NXD_LAUNCH_CHECK();
     return 0;
 }

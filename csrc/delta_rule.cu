@@ -140,6 +140,8 @@ delta_prep_strip_kernel(const T* __restrict__ proj, long long ld, int off_q, int
                         float* __restrict__ kn, float* __restrict__ vn, const int* __restrict__ q_start,
                         const int* __restrict__ n_new, const int* __restrict__ seq_ids, int units, int Tn, int H, int G, int Dv,
                         float qscale, float unit_eps, int strip) {
+    pdl_trigger();
+    pdl_wait();
     constexpr int D = 32 * V, TAPS = 4, K = TAPS - 1;
     const int lane = threadIdx.x & 31, u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (u >= units) return;
@@ -216,8 +218,8 @@ int launch_prep_strip(const void* proj, long long ld, int off_q, int off_k, int 
     // 256: 13.1 us in strips of 16, 7.6 in strips of 4 (13.8 in the general kernel); 8 x 128 tokens, 3 x 16 heads of 128: 19.2 / 20.2
     const int strip = (long long)units * ((Tn + PREP_STRIP - 1) / PREP_STRIP) * B < 1536 ? PREP_SHORT : PREP_STRIP;
     dim3 grid((units + 7) / 8, (Tn + strip - 1) / strip, B);
-    delta_prep_strip_kernel<T, V><<<grid, 256, 0, st>>>((const T*)proj, ld, off_q, off_k, off_v, conv_w, conv_state, qn, kn, vn,
-                                                        q_start, n_new, seq_ids, units, Tn, H, G, Dv, qscale, unit_eps, strip);
+    NXD_CHECK_CUDA((nxd_launch_pdl(delta_prep_strip_kernel<T, V>, grid, dim3(256), 0, st, (const T*)proj, ld, off_q, off_k, off_v,
+        conv_w, conv_state, qn, kn, vn, q_start, n_new, seq_ids, units, Tn, H, G, Dv, qscale, unit_eps, strip)));
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -227,6 +229,8 @@ __global__ void delta_conv_state_kernel(const T* __restrict__ proj, long long ld
                                         float* __restrict__ conv_state, const int* __restrict__ q_start,
                                         const int* __restrict__ n_new, const int* __restrict__ seq_ids, int B, int Tn,
                                         int GD, int C, int taps) {
+    pdl_trigger();
+    pdl_wait();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)B * C) return;
     const int b = (int)(idx / C), c = (int)(idx % C);
@@ -250,6 +254,8 @@ constexpr int SCAN_THREADS = 128, SCAN_TS = 16;
 __global__ void delta_gates_kernel(float* __restrict__ apre, long long ld_a, int a_off, float* __restrict__ bpre,
                                    long long ld_b, int b_off, const float* __restrict__ a_log,
                                    const float* __restrict__ dt_bias, long long N, int H, int per_head) {
+    pdl_trigger();
+    pdl_wait();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int cols = H * per_head + H;                 // decay columns, then beta columns
     if (idx >= N * cols) return;
@@ -506,6 +512,8 @@ __global__ void __launch_bounds__(CW_THREADS, 2)
 delta_chunk_system_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ gate,
                           long long ld_a, int a_off, const float* __restrict__ beta, long long ld_b, int b_off,
                           float* __restrict__ scratch, const int* __restrict__ n_new, int Tn, int chunk0, int H, int G) {
+    pdl_trigger();
+    pdl_wait();
     extern __shared__ __align__(16) float smem[];
     double* Kd = reinterpret_cast<double*>(smem);      // [CH][DPITCH] 64 key channels at a time; then X = (I + A)^-1
     double* Qd = Kd + CH * DPITCH;                     // [CH][DPITCH] the same of the queries; then P
@@ -918,8 +926,8 @@ int launch_chunks(const nxd_delta::Step& p, const float* gate, long long ld_a, i
         constexpr int scan = ((D <= 128 ? 3 : 2) * CH * DP + CW_COLS * DP + 2 * CH * CP + 2 * CW_COLS * CP + 4 * CH) * (int)sizeof(float);
         static_assert(scan <= 232448, "shared memory");
         NXD_CHECK_CUDA(nxd_allow_smem<delta_chunk_scan_fp32_kernel<D>>(scan));
-        delta_chunk_system_kernel<D><<<dim3(NC, p.H, p.B), CW_THREADS, smem, st>>>(p.qn, p.kn, gate, ld_a, a_off, beta, ld_b, b_off,
-                                                                                  scratch, p.n_new, p.Tn, 0, p.H, p.G);
+        NXD_CHECK_CUDA((nxd_launch_pdl(delta_chunk_system_kernel<D>, dim3(NC, p.H, p.B), dim3(CW_THREADS), smem, st, p.qn, p.kn,
+            gate, ld_a, a_off, beta, ld_b, b_off, scratch, p.n_new, p.Tn, 0, p.H, p.G)));
         NXD_LAUNCH_CHECK();
         delta_chunk_scan_fp32_kernel<D><<<dim3(p.Dv / CW_COLS, p.H, p.B), CW_THREADS, scan, st>>>(
             p.qn, p.kn, p.vn, scratch, p.S, p.out, p.q_start, p.n_new, p.seq_ids, p.Tn, NC, p.H, p.G, p.Dv);
@@ -939,8 +947,8 @@ int launch_chunks(const nxd_delta::Step& p, const float* gate, long long ld_a, i
         else r.S += (long long)b0 * p.H * D * p.Dv;
         for (int c0 = 0; c0 < NC; c0 += seg.chunks) {
             const int count = min(seg.chunks, NC - c0);
-            delta_chunk_system_kernel<D><<<dim3(count, p.H, r.B), CW_THREADS, smem, st>>>(
-                r.qn, r.kn, gate + t0 * ld_a, ld_a, a_off, beta + t0 * ld_b, ld_b, b_off, systems, r.n_new, p.Tn, c0, p.H, p.G);
+            NXD_CHECK_CUDA((nxd_launch_pdl(delta_chunk_system_kernel<D>, dim3(count, p.H, r.B), dim3(CW_THREADS), smem, st, r.qn,
+                r.kn, gate + t0 * ld_a, ld_a, a_off, beta + t0 * ld_b, ld_b, b_off, systems, r.n_new, p.Tn, c0, p.H, p.G)));
             NXD_LAUNCH_CHECK();
             if (int rc = nxd_delta::launch_chunks_tc(r, systems, tiles, c0, count, wait_clocks, st)) return rc;
         }
@@ -1008,11 +1016,11 @@ NXD_API int nxd_delta_conv_state(int dtype, const void* proj, long long ld, int 
     const unsigned blocks = (unsigned)(((long long)B * C + 255) / 256);
     cudaStream_t st = (cudaStream_t)stream;
     if (dtype == 0)
-        delta_conv_state_kernel<bf16><<<blocks, 256, 0, st>>>((const bf16*)proj, ld, off_q, off_k, off_v, conv_state, q_start,
-                                                             n_new, seq_ids, B, Tn, G * D, C, taps);
+        NXD_CHECK_CUDA((nxd_launch_pdl(delta_conv_state_kernel<bf16>, dim3(blocks), dim3(256), 0, st, (const bf16*)proj, ld, off_q,
+            off_k, off_v, conv_state, q_start, n_new, seq_ids, B, Tn, G * D, C, taps)));
     else
-        delta_conv_state_kernel<float><<<blocks, 256, 0, st>>>((const float*)proj, ld, off_q, off_k, off_v, conv_state,
-                                                              q_start, n_new, seq_ids, B, Tn, G * D, C, taps);
+        NXD_CHECK_CUDA((nxd_launch_pdl(delta_conv_state_kernel<float>, dim3(blocks), dim3(256), 0, st, (const float*)proj, ld,
+            off_q, off_k, off_v, conv_state, q_start, n_new, seq_ids, B, Tn, G * D, C, taps)));
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -1044,8 +1052,8 @@ NXD_API int nxd_delta_scan_limited(const float* qn, const float* kn, const float
     const long long N = (long long)B * Tn;
     const int per_head = per_channel ? D : 1;
     const long long vals = N * ((long long)H * per_head + H);
-    delta_gates_kernel<<<(unsigned)((vals + 255) / 256), 256, 0, st>>>(apre, ld_a, a_off, bpre, ld_b, b_off, a_log, dt_bias,
-                                                                      N, H, per_head);
+    NXD_CHECK_CUDA((nxd_launch_pdl(delta_gates_kernel, dim3((unsigned)((vals + 255) / 256)), dim3(256), 0, st, apre, ld_a, a_off,
+        bpre, ld_b, b_off, a_log, dt_bias, N, H, per_head)));
     NXD_LAUNCH_CHECK();
     auto al = [](const void* p) { return ((uintptr_t)p % 16) == 0; };
     const long long floats = nxd_delta_scan_scratch(B, Tn, H, D, Dv, per_channel);

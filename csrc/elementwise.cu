@@ -14,6 +14,8 @@
 namespace {
 
 __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, size_t rows, int I) {
+    pdl_trigger();
+    pdl_wait();
     const int nvec = I >> 3;
     const size_t total = rows * (size_t)nvec;
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -37,6 +39,8 @@ __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict_
 
 __global__ void swiglu_bwd_kernel(const bf16* __restrict__ gu, const bf16* __restrict__ dy,
                                   bf16* __restrict__ dgu, size_t rows, int I) {
+    pdl_trigger();
+    pdl_wait();
     const int nvec = I >> 3;
     const size_t total = rows * (size_t)nvec;
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -72,6 +76,8 @@ template <int kHeads>
 __global__ void rope_kernel(const bf16* x, bf16* y, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                             const int* __restrict__ positions, size_t T, int heads_total, int n_heads, int n_rot, int D,
                             int pos_div, int pos_mod, float sin_sign) {
+    pdl_trigger();
+    pdl_wait();
     const int half_vec = D >> 4;  // 16-byte vectors in half a head
     const int groups = (n_heads + kHeads - 1) / kHeads;
     const size_t total = T * (size_t)groups * half_vec;
@@ -190,8 +196,8 @@ NXD_API int nxd_swiglu_fwd(const void* gate_up, void* out, long long rows, int I
     NXD_REQUIRE(I % 8 == 0, "swiglu: I=%d must be a multiple of 8", I);
     if (rows == 0) return 0;
     const size_t work = (size_t)rows * (I / 8);
-    swiglu_fwd_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)gate_up, (bf16*)out,
-                                                                             (size_t)rows, I);
+    NXD_CHECK_CUDA((nxd_launch_pdl(swiglu_fwd_kernel, dim3(grid_for(work, 256)), dim3(256), 0, (cudaStream_t)stream,
+        (const bf16*)gate_up, (bf16*)out, (size_t)rows, I)));
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -201,8 +207,8 @@ NXD_API int nxd_swiglu_bwd(const void* gate_up, const void* dy, void* dgate_up, 
     NXD_REQUIRE(I % 8 == 0, "swiglu_bwd: I=%d must be a multiple of 8", I);
     if (rows == 0) return 0;
     const size_t work = (size_t)rows * (I / 8);
-    swiglu_bwd_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
-        (const bf16*)gate_up, (const bf16*)dy, (bf16*)dgate_up, (size_t)rows, I);
+    NXD_CHECK_CUDA((nxd_launch_pdl(swiglu_bwd_kernel, dim3(grid_for(work, 256)), dim3(256), 0, (cudaStream_t)stream,
+        (const bf16*)gate_up, (const bf16*)dy, (bf16*)dgate_up, (size_t)rows, I)));
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -223,9 +229,9 @@ NXD_API int nxd_rope(const void* x, void* y, const float* cos_t, const float* si
     const bool four = D >= 128 && quads >= 1 << 16;
     const size_t work = four ? quads : (size_t)T * n_heads * (D / 16);
     auto kern = four ? rope_kernel<4> : rope_kernel<1>;
-    kern<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
-        (const bf16*)x, (bf16*)y, cos_t, sin_t, positions, (size_t)T, heads_total, n_heads, n_rot_heads, D,
-        pos_div < 1 ? 1 : pos_div, pos_mod < 1 ? 1 : pos_mod, inverse ? -1.f : 1.f);
+    NXD_CHECK_CUDA((nxd_launch_pdl(kern, dim3(grid_for(work, 256)), dim3(256), 0, (cudaStream_t)stream, (const bf16*)x, (bf16*)y,
+        cos_t, sin_t, positions, (size_t)T, heads_total, n_heads, n_rot_heads, D, pos_div < 1 ? 1 : pos_div, pos_mod < 1 ? 1 :
+        pos_mod, inverse ? -1.f : 1.f)));
     NXD_LAUNCH_CHECK();
     return 0;
 }

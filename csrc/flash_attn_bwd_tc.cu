@@ -144,6 +144,7 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         ptx::mbar_init(dq_empty, kDrainThreads);
         ptx::fence_barrier_init();
     }
+    pdl_wait();         // ahead of the allocation: nothing that this grid waits for may be short of tensor memory
     if (warp == 1) ptx::tmem_alloc<1>(tmem_ptr_smem, 512);
     ptx::tcgen05_fence_before();
     __syncthreads();
@@ -496,6 +497,8 @@ __global__ void __launch_bounds__(256) fa_bwd_tc_prep_kernel(const bf16* __restr
                                                              long long o_sh, long long o_ss, long long do_sb,
                                                              long long do_sh, long long do_ss, int B, int Hq, int Sq,
                                                              int Sq_pad) {
+    pdl_trigger();
+    pdl_wait();
     constexpr int L = kD / 8, R = 32 / L, U = 4;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = lane / L, l = lane % L;
@@ -539,6 +542,8 @@ __global__ void __launch_bounds__(256) fa_bwd_tc_prep_kernel(const bf16* __restr
 // fp32 [B, Hq, Sq, D] accumulator -> strided bf16 dq
 __global__ void fa_bwd_tc_dq_convert_kernel(const float* __restrict__ acc, bf16* __restrict__ dq, long long sb,
                                             long long sh, long long ss, int B, int Hq, int Sq, int kD) {
+    pdl_trigger();
+    pdl_wait();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;  // one thread = 8 elements
     const long long total = (long long)B * Hq * Sq * (kD / 8);
     if (idx >= total) return;
@@ -561,6 +566,8 @@ template <int kD>
 __global__ void __launch_bounds__(256)
 fa_bwd_tc_dq_transpose_kernel(const float* __restrict__ acc, bf16* __restrict__ dq, long long sb, long long sh,
                               long long ss, int Hq, int Sq, int Sq_pad) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ float tile[kD][65];
     const int q0 = blockIdx.x * 64, h = blockIdx.y, b = blockIdx.z;
     const float* src = acc + ((long long)b * Hq + h) * kD * Sq_pad + q0;
@@ -593,7 +600,8 @@ int launch_bwd_tc(dim3 grid, cudaStream_t st, const CUtensorMap& tq, const CUten
                   const CUtensorMap& tdka, const CUtensorMap& tdva, const BwdParams& p) {
     constexpr auto kern = fa_bwd_tc_kernel<kD, CAUSAL, DROP>;
     NXD_CHECK_CUDA(nxd_allow_smem<kern>(BwdSmem<kD>::kBytes));
-    kern<<<grid, kThreadsBwd, BwdSmem<kD>::kBytes, st>>>(tq, tdo, tk, tv, tdk, tdv, tdq, tdka, tdva, p);
+    NXD_CHECK_CUDA((nxd_launch_pdl(kern, grid, dim3(kThreadsBwd), BwdSmem<kD>::kBytes, st, tq, tdo, tk, tv, tdk, tdv, tdq, tdka,
+        tdva, p)));
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -643,13 +651,13 @@ static int bwd_tc_impl(const void* q, const void* k, const void* v, const void* 
     {
         const long long rows = (long long)B * Hq * p.Sq_pad;
         if (D == 128) {
-            fa_bwd_tc_prep_kernel<128><<<(unsigned)((rows + 63) / 64), 256, 0, st>>>(
-                (const bf16*)o, (const bf16*)dout, lse, lse_pad, delta_pad, strides[9], strides[10], strides[11],
-                strides[12], strides[13], strides[14], B, Hq, Sq, p.Sq_pad);
+            NXD_CHECK_CUDA((nxd_launch_pdl(fa_bwd_tc_prep_kernel<128>, dim3((unsigned)((rows + 63) / 64)), dim3(256), 0, st,
+                (const bf16*)o, (const bf16*)dout, lse, lse_pad, delta_pad, strides[9], strides[10], strides[11], strides[12],
+                strides[13], strides[14], B, Hq, Sq, p.Sq_pad)));
         } else {
-            fa_bwd_tc_prep_kernel<64><<<(unsigned)((rows + 127) / 128), 256, 0, st>>>(
-                (const bf16*)o, (const bf16*)dout, lse, lse_pad, delta_pad, strides[9], strides[10], strides[11],
-                strides[12], strides[13], strides[14], B, Hq, Sq, p.Sq_pad);
+            NXD_CHECK_CUDA((nxd_launch_pdl(fa_bwd_tc_prep_kernel<64>, dim3((unsigned)((rows + 127) / 128)), dim3(256), 0, st,
+                (const bf16*)o, (const bf16*)dout, lse, lse_pad, delta_pad, strides[9], strides[10], strides[11], strides[12],
+                strides[13], strides[14], B, Hq, Sq, p.Sq_pad)));
         }
         NXD_LAUNCH_CHECK();
     }
@@ -692,20 +700,20 @@ static int bwd_tc_impl(const void* q, const void* k, const void* v, const void* 
     if (rc) return rc;
     if (p.nsplit > 1) {
         const long long n = kv_elems / 8;
-        fa_bwd_tc_dq_convert_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(dk_acc, (bf16*)dk, strides[18], strides[19],
-                                                                                strides[20], B, Hkv, Sk, D);
-        fa_bwd_tc_dq_convert_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(dv_acc, (bf16*)dv, strides[21], strides[22],
-                                                                                strides[23], B, Hkv, Sk, D);
+        NXD_CHECK_CUDA((nxd_launch_pdl(fa_bwd_tc_dq_convert_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, dk_acc,
+            (bf16*)dk, strides[18], strides[19], strides[20], B, Hkv, Sk, D)));
+        NXD_CHECK_CUDA((nxd_launch_pdl(fa_bwd_tc_dq_convert_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, dv_acc,
+            (bf16*)dv, strides[21], strides[22], strides[23], B, Hkv, Sk, D)));
         NXD_LAUNCH_CHECK_N(2);
     }
     {
         dim3 g((unsigned)((Sq + 63) / 64), (unsigned)Hq, (unsigned)B);
         if (D == 128)
-            fa_bwd_tc_dq_transpose_kernel<128><<<g, 256, 0, st>>>(dq_accum, (bf16*)dq, strides[15], strides[16],
-                                                                  strides[17], Hq, Sq, p.Sq_pad);
+            NXD_CHECK_CUDA((nxd_launch_pdl(fa_bwd_tc_dq_transpose_kernel<128>, g, dim3(256), 0, st, dq_accum, (bf16*)dq,
+                strides[15], strides[16], strides[17], Hq, Sq, p.Sq_pad)));
         else
-            fa_bwd_tc_dq_transpose_kernel<64><<<g, 256, 0, st>>>(dq_accum, (bf16*)dq, strides[15], strides[16],
-                                                                 strides[17], Hq, Sq, p.Sq_pad);
+            NXD_CHECK_CUDA((nxd_launch_pdl(fa_bwd_tc_dq_transpose_kernel<64>, g, dim3(256), 0, st, dq_accum, (bf16*)dq,
+                strides[15], strides[16], strides[17], Hq, Sq, p.Sq_pad)));
         NXD_LAUNCH_CHECK();
     }
     return 0;

@@ -106,7 +106,6 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(pv_done + 1);
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    pdl_trigger();
     if (CACHE) pdl_wait();
     // grid = (q heads, batch, q blocks): the q block is the slowest launch dimension and counted from the end, so the
     // long causal rows of EVERY head are scheduled before any short one (longest-first list scheduling)
@@ -168,6 +167,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     ptx::tcgen05_fence_before();
     __syncthreads();
     ptx::tcgen05_fence_after();
+    pdl_trigger();      // not before this CTA has its tensor memory: a successor that waits for this grid may hold the rest of it
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_smem, 0);
     const uint32_t tmem_o = tmem_base;
     const uint32_t tmem_s = tmem_base + D;

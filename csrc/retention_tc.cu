@@ -125,6 +125,7 @@ retention_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     ptx::cluster_sync();
     ptx::tcgen05_fence_after();
     const uint32_t tmem = *tmem_ptr;
+    pdl_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -355,6 +356,8 @@ retention_tc_prep_kernel(const T* __restrict__ proj, long long ld, int q_off, in
                          const int* __restrict__ n_new, int Tn, int NC, int H, int D, int Dv, float kscale,
                          const float* __restrict__ rope_cos, const float* __restrict__ rope_sin, int rot, int halves,
                          int max_pos, int vec) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ float fade[PT];               // decay^(n - 1 - s) of the chunk's tokens
     const int hd = blockIdx.y, role = blockIdx.x % 3, b = blockIdx.z, tid = threadIdx.x;
     const int t0 = (int)(blockIdx.x / 3) * PT, c = t0 / kC, s0 = t0 % kC;
@@ -469,6 +472,8 @@ retention_tc_states_kernel(const float* __restrict__ U, bf16* __restrict__ s3, f
                            const float* __restrict__ decay, const int* __restrict__ flag, const int* __restrict__ bad,
                            const int* __restrict__ q_start, const int* __restrict__ n_new, const int* __restrict__ seq_ids, int Tn,
                            int NC, int H, int Dv, long long E4) {
+    pdl_trigger();
+    pdl_wait();
     const long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (at >= E4) return;
     const int hd = blockIdx.y, b = blockIdx.z, j = (int)(at * 4 % Dv);
@@ -540,7 +545,7 @@ int launch(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& a2, co
     auto kern = retention_tc_kernel<MODE, NB>;
     NXD_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     const int clusters = min(nxd_num_sms() / 2, p.E * p.n_tiles);
-    kern<<<dim3(clusters * 2), dim3(kThreads), kSmem, st>>>(a, b, a2, b2, d, p);
+    NXD_CHECK_CUDA((nxd_launch_pdl(kern, dim3(clusters * 2), dim3(kThreads), kSmem, st, a, b, a2, b2, d, p)));
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -559,9 +564,9 @@ int run(const T* proj, long long ld, int q_off, int k_off, int v_off, const floa
     const int per = 16 / (int)sizeof(T);
     const int vec = (ld % per == 0 && q_off % per == 0 && k_off % per == 0 && v_off % per == 0 && ((uintptr_t)proj % 16) == 0) |
                     (rot % 16 == 0 && (((uintptr_t)rope_cos | (uintptr_t)rope_sin) % 16) == 0 ? 2 : 0);
-    retention_tc_prep_kernel<T, NB><<<dim3(3 * NC * (kC / PT), H, B), PREP_THREADS, 0, st>>>(
+    NXD_CHECK_CUDA((nxd_launch_pdl(retention_tc_prep_kernel<T, NB>, dim3(3 * NC * (kC / PT), H, B), dim3(PREP_THREADS), 0, st,
         proj, ld, q_off, k_off, v_off, decay, q3, k3, kd3, v3, flag, bad, q_start, n_new, Tn, NC, H, D, Dv, kscale, rope_cos,
-        rope_sin, rot, halves, max_pos, vec);
+        rope_sin, rot, halves, max_pos, vec)));
     NXD_LAUNCH_CHECK();
     Args p{};
     p.decay = decay; p.n_new = n_new; p.flag = flag; p.bad = bad;
@@ -582,8 +587,8 @@ int run(const T* proj, long long ld, int q_off, int k_off, int v_off, const floa
     p.k_blocks1 = kC / kBK, p.k_blocks2 = 0;
     if ((rc = launch<kU, NB>(mkd, mv, mkd, mv, mu, p, st))) return rc;
     const long long E4 = dv / 4;
-    retention_tc_states_kernel<<<dim3((unsigned)((E4 + 255) / 256), H, B), 256, 0, st>>>(u, s3, state, decay, flag, bad, q_start,
-                                                                                       n_new, seq_ids, Tn, NC, H, Dv, E4);
+    NXD_CHECK_CUDA((nxd_launch_pdl(retention_tc_states_kernel, dim3((unsigned)((E4 + 255) / 256), H, B), dim3(256), 0, st, u, s3,
+        state, decay, flag, bad, q_start, n_new, seq_ids, Tn, NC, H, Dv, E4)));
     NXD_LAUNCH_CHECK();
     p.n_tiles = kC / kBN;
     p.k_blocks1 = D / kBK;

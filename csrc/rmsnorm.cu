@@ -97,6 +97,8 @@ __global__ void __launch_bounds__(VPT == 1 ? 256 : 512)
 rmsnorm_bwd_ring_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w,
                         const float* __restrict__ rstd, const bf16* __restrict__ dres, bf16* __restrict__ dx,
                         float* __restrict__ dw_partial, int rows, int H) {
+    pdl_trigger();
+    pdl_wait();
     constexpr int kRing = RingCfg<VPT>::kRows;
     extern __shared__ __align__(16) bf16x8 ring[];       // [kRing][dy | x | dres][nvec]
     __shared__ float red[2][32];
@@ -202,6 +204,8 @@ constexpr int kSumWarps = 16;
 __global__ void __launch_bounds__(32 * kSumWarps)
 colsum_partials_kernel(const float* __restrict__ partial, int P, int H, bf16* __restrict__ dw_bf16,
                        float* __restrict__ dw_f32, int accumulate) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ float part[kSumWarps][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, h = blockIdx.x * 32 + lane;
     float s = 0.f;
@@ -284,8 +288,8 @@ static int rmsnorm_bwd_ring(const void* dy, const void* x, const void* w, const 
     int per_sm = 232448 / (smem + 1024 + 256);
     if (per_sm > C::kCtas) per_sm = C::kCtas;
     if (P > per_sm * nxd_num_sms()) P = per_sm * nxd_num_sms();
-    rmsnorm_bwd_ring_kernel<VPT><<<P, threads, smem, s>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd,
-                                                          (const bf16*)dresidual, (bf16*)dx, scratch, rows, H);
+    NXD_CHECK_CUDA((nxd_launch_pdl(rmsnorm_bwd_ring_kernel<VPT>, dim3(P), dim3(threads), smem, s, (const bf16*)dy, (const bf16*)x,
+        (const bf16*)w, rstd, (const bf16*)dresidual, (bf16*)dx, scratch, rows, H)));
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -298,7 +302,8 @@ static int rmsnorm_bwd_impl(const void* dy, const void* x, const void* w, const 
                    : H <= RingCfg<2>::kMaxH ? rmsnorm_bwd_ring<2>(dy, x, w, rstd, dresidual, dx, scratch, P, rows, H, s)
                                             : rmsnorm_bwd_ring<4>(dy, x, w, rstd, dresidual, dx, scratch, P, rows, H, s);
     if (rc) return rc;
-    colsum_partials_kernel<<<(H + 31) / 32, 32 * kSumWarps, 0, s>>>(scratch, P, H, (bf16*)dw_bf16, dw_f32, accumulate);
+    NXD_CHECK_CUDA((nxd_launch_pdl(colsum_partials_kernel, dim3((H + 31) / 32), dim3(32 * kSumWarps), 0, s, scratch, P, H,
+        (bf16*)dw_bf16, dw_f32, accumulate)));
     NXD_LAUNCH_CHECK();
     return 0;
 }
@@ -307,7 +312,8 @@ static int rmsnorm_bwd_impl(const void* dy, const void* x, const void* w, const 
 // (the column-sum kernel with no partial rows reads nothing and stores 0).
 static int rmsnorm_bwd_empty(void* dw_bf16, float* dw_f32, int accumulate, int H, cudaStream_t s) {
     if (accumulate || (dw_bf16 == nullptr && dw_f32 == nullptr)) return 0;
-    colsum_partials_kernel<<<(H + 31) / 32, 32 * kSumWarps, 0, s>>>(nullptr, 0, H, (bf16*)dw_bf16, dw_f32, 0);
+    NXD_CHECK_CUDA((nxd_launch_pdl(colsum_partials_kernel, dim3((H + 31) / 32), dim3(32 * kSumWarps), 0, s, nullptr, 0, H,
+        (bf16*)dw_bf16, dw_f32, 0)));
     NXD_LAUNCH_CHECK();
     return 0;
 }
