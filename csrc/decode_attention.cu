@@ -56,6 +56,7 @@ __global__ void __launch_bounds__(128) decode_attn_split_kernel(
     const bf16* __restrict__ q,  // [B, n_q, D]
     CacheView cache, const int* __restrict__ lengths, int len_step, float* __restrict__ part_o,  // [B, n_q, splits, D]
     float* __restrict__ part_ml,                                                   // [B, n_q, splits, 2]
+    bf16* __restrict__ out,      // [B, n_q, D]: what one split alone finishes itself
     int n_q, int n_kv, int n_splits, float scale_log2) {
     constexpr int kLanes = 8;            // lanes per cache row
     constexpr int kE = D / kLanes;       // channels per lane: 8 (D = 64) or 16 (D = 128)
@@ -201,6 +202,10 @@ __global__ void __launch_bounds__(128) decode_attn_split_kernel(
             l += s_l[t][g] * w;
             acc += s_o[t][g][d] * w;
         }
+        if (n_splits == 1) {
+            out[((size_t)b * n_q + h0 + g) * D + d] = __float2bfloat16(l > 0.f ? acc / l : 0.f);
+            continue;
+        }
         const size_t base = (((size_t)b * n_q + h0 + g) * n_splits + split);
         part_o[base * D + d] = acc;
         if (d == 0) {
@@ -238,6 +243,7 @@ __global__ void __launch_bounds__(128) decode_attn_mma_kernel(
     const bf16* __restrict__ q,  // [B, n_q, D]
     CacheView cache, const int* __restrict__ lengths, int len_step, float* __restrict__ part_o,  // [B, n_q, splits, D]
     float* __restrict__ part_ml,                                                   // [B, n_q, splits, 2]
+    bf16* __restrict__ out,      // [B, n_q, D]: as above
     int n_q, int n_kv, int n_splits, float scale_log2) {
     using C = MmaDecodeCfg<D>;
     extern __shared__ __align__(128) uint8_t dsmem[];
@@ -417,6 +423,10 @@ __global__ void __launch_bounds__(128) decode_attn_mma_kernel(
             l += s_ml[(w * 16 + g) * 2 + 1] * wgt;
             acc += s_o[(w * 16 + g) * (D + 4) + d] * wgt;
         }
+        if (n_splits == 1) {
+            out[((size_t)b * n_q + h0 + g) * D + d] = __float2bfloat16(l > 0.f ? acc / l : 0.f);
+            continue;
+        }
         const size_t base = (((size_t)b * n_q + h0 + g) * n_splits + split);
         part_o[base * D + d] = acc;
         if (d == 0) {
@@ -426,9 +436,10 @@ __global__ void __launch_bounds__(128) decode_attn_mma_kernel(
     }
 }
 
-// D threads per (sequence, query head).  A chain of loads: the weights of all splits come from one load per lane and a warp
-// reduction, the partial rows are read eight at a time (split by split, a merge of 16 splits took longer than the attention
-// of 128 keys).
+// D threads per (sequence, query head), for two splits and more; one split writes the result itself (64 sequences through four 1B layers
+// and the head: 451.8 us with a merge of one part each, 446.5).  A chain of loads: the weights of all splits come from one load per
+// lane and a warp reduction, the partial rows are read eight at a time (split by split, a merge of 16 splits took longer than the
+// attention of 128 keys).
 constexpr int kMaxSplits = 64, kFewSplits = 4;
 
 template <int D>
@@ -571,7 +582,7 @@ static int decode_attn_impl(const void* q, const void* cache_k, const void* cach
     const float scale_log2 = scale * 1.4426950408889634f;
 #define NXD_DECODE_LAUNCH(DD, GG)                                                                                  \
     NXD_CHECK_CUDA(nxd_launch_pdl(decode_attn_split_kernel<DD, GG>, grid, dim3(128), 0, s, (const bf16*)q, cv, lengths, len_step, \
-                                  part_o, part_ml, n_q, n_kv, n_splits, scale_log2))
+                                  part_o, part_ml, (bf16*)out, n_q, n_kv, n_splits, scale_log2))
 #define NXD_DECODE_DISPATCH(DD)                 \
     switch (G) {                                \
         case 1: NXD_DECODE_LAUNCH(DD, 1); break; \
@@ -584,13 +595,14 @@ static int decode_attn_impl(const void* q, const void* cache_k, const void* cach
         if (D == 64) {
             NXD_CHECK_CUDA(nxd_allow_smem<decode_attn_mma_kernel<64>>(MmaDecodeCfg<64>::kSmemBytes));
             NXD_CHECK_CUDA(nxd_launch_pdl(decode_attn_mma_kernel<64>, mgrid, dim3(128), MmaDecodeCfg<64>::kSmemBytes, s,
-                                          (const bf16*)q, cv, lengths, len_step, part_o, part_ml, n_q, n_kv, n_splits, scale_log2));
+                                          (const bf16*)q, cv, lengths, len_step, part_o, part_ml, (bf16*)out, n_q, n_kv, n_splits, scale_log2));
         } else {
             NXD_CHECK_CUDA(nxd_allow_smem<decode_attn_mma_kernel<128>>(MmaDecodeCfg<128>::kSmemBytes));
             NXD_CHECK_CUDA(nxd_launch_pdl(decode_attn_mma_kernel<128>, mgrid, dim3(128), MmaDecodeCfg<128>::kSmemBytes, s,
-                                          (const bf16*)q, cv, lengths, len_step, part_o, part_ml, n_q, n_kv, n_splits, scale_log2));
+                                          (const bf16*)q, cv, lengths, len_step, part_o, part_ml, (bf16*)out, n_q, n_kv, n_splits, scale_log2));
         }
         NXD_LAUNCH_CHECK();
+        if (n_splits == 1) return 0;
         if (D == 64) {
             NXD_CHECK_CUDA(nxd_launch_pdl(decode_attn_merge_kernel<64>, dim3(B * n_q), dim3(64), 0, s, (const float*)part_o,
                                           (const float*)part_ml, (bf16*)out, n_splits));
@@ -604,11 +616,13 @@ static int decode_attn_impl(const void* q, const void* cache_k, const void* cach
     if (D == 64) {
         NXD_DECODE_DISPATCH(64)
         NXD_LAUNCH_CHECK();
+        if (n_splits == 1) return 0;
         NXD_CHECK_CUDA(nxd_launch_pdl(decode_attn_merge_kernel<64>, dim3(B * n_q), dim3(64), 0, s, (const float*)part_o,
                                       (const float*)part_ml, (bf16*)out, n_splits));
     } else {
         NXD_DECODE_DISPATCH(128)
         NXD_LAUNCH_CHECK();
+        if (n_splits == 1) return 0;
         NXD_CHECK_CUDA(nxd_launch_pdl(decode_attn_merge_kernel<128>, dim3(B * n_q), dim3(128), 0, s, (const float*)part_o,
                                       (const float*)part_ml, (bf16*)out, n_splits));
     }

@@ -77,3 +77,23 @@ def test_lengths_of_64_bits_are_read_as_they_are(n_q):
     ref = decode_attention(q, k, v, lens.int())
     assert torch.equal(decode_attention(q, k, v, lens), ref)
     assert torch.equal(decode_attention(q, k, v, lens.repeat_interleave(2)[::2]), ref)      # not contiguous: converted
+
+
+# as many pairs of a sequence and a key head as make one split (its kernel finishes alone) and one fewer than make two, empty sequences among
+# them; multiply-add kernel and tensor cores
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("group", [1, 4])
+@pytest.mark.parametrize("pairs", [148, 149, 296, 297])
+def test_one_split_finishes_alone(D, group, pairs):
+    from neuronx_distributed_llama3_2_b200.ops.attention import decode_attention
+
+    g = torch.Generator(device="cuda").manual_seed(pairs + D)
+    q = torch.randn(pairs, group, D, generator=g, device="cuda").bfloat16()
+    k, v = (torch.randn(pairs, 1, 160, D, generator=g, device="cuda").bfloat16() for _ in range(2))
+    lens = torch.randint(1, 161, (pairs,), generator=g, device="cuda")
+    lens[:3] = torch.tensor([160, 0, 129])
+    out = decode_attention(q, k, v, lens)
+    assert not out[1].any()
+    real = lens > 0
+    ref = _reference(q[real], k[real], v[real], lens[real].tolist())
+    assert (out[real].double() - ref).norm() <= 2 * 2.0 ** -8 * ref.norm()          # as above
