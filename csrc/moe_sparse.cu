@@ -169,7 +169,6 @@ moe_router_kernel(const T* __restrict__ h, const float* __restrict__ wr, const f
                   float* __restrict__ sgate, long long N, int W, int R, int top, float out_scale,
                   const float* __restrict__ zbias, int mode) {
     extern __shared__ float smem[];
-    pdl_trigger();
     pdl_wait();
     constexpr int G = SHARE ? 4 : 8;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -198,6 +197,7 @@ moe_router_kernel(const T* __restrict__ h, const float* __restrict__ wr, const f
             if (lane == 0 && t < nt) sgate[n0 + t] = 1.f / (1.f + expf(-z));
         }
     }
+    pdl_trigger();
     if constexpr (SHARE) {
         __syncthreads();
         if (warp == 0) router_select(ps, ps + R, corr, idx, wts, n0, R, top, out_scale, mode);
@@ -460,6 +460,18 @@ __global__ void glu_bias_vec_kernel(const bf16* __restrict__ src, long long ld, 
     }
 }
 
+// Programmatic dependents beside the end of the kernel before go to the few SMs that have room by then and stay there.  For the sorting
+// kernel and the combination that is worth it while they have few blocks themselves and the router, a block per token, leaves SMs free:
+// 2048 x 8 experts, the step as a graph, dependents or not, 64 tokens 66.5 / 66.7 us, 400 84.3 / 71.2, 800 87.3 / 75.5; 1024 x 16 64 tokens
+// 31.9 / 32.1, 300 41.3 / 35.3, 6000 156.3 / 153.1.  (The line lies above 100 and below 150 tokens.)  For the same reason every kernel
+// of the step triggers behind its work: beside the router, the products' shared memory took its L1 away (24 -> 35 us at width 4096).
+template <typename... KArgs, typename... Args>
+cudaError_t launch_beside(long long tokens, void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t stream, Args... args) {
+    if (tokens <= 128) return nxd_launch_pdl(kernel, grid, block, 0, stream, args...);
+    kernel<<<grid, block, 0, stream>>>(args...);
+    return cudaGetLastError();
+}
+
 // Bound by memory.  V = 8: a thread takes 8 consecutive columns (16-byte loads of bf16 rows, W a multiple of 8, aligned
 // rows); V = 1: any W.  8190 tokens x 2048, top 2: 61 us with one column per thread, 24 us on bf16 outputs (134 MB), 35 us on fp32
 // outputs (201 MB, 5.8 TB/s).
@@ -469,7 +481,6 @@ __global__ void moe_gather_combine_kernel(const TY* __restrict__ ys, const int* 
                                           const int* __restrict__ idx, const float* __restrict__ wts,
                                           const T* __restrict__ h, const TY* __restrict__ shared_out,
                                           const float* __restrict__ sgate, float* __restrict__ y, int top, int W, int E) {
-    pdl_trigger();
     pdl_wait();
     const long long t = blockIdx.x;
     for (int c = threadIdx.x * V; c < W; c += blockDim.x * V) {
@@ -498,6 +509,7 @@ __global__ void moe_gather_combine_kernel(const TY* __restrict__ ys, const int* 
             y[t * W + c] = a[0];
         }
     }
+    pdl_trigger();
 }
 
 // ---- rows sorted by expert, without a host read ---------------------------------------------------------------------------
@@ -511,7 +523,6 @@ __global__ void __launch_bounds__(CNT_THREADS)
 moe_count_kernel(const int* __restrict__ idx, int* __restrict__ counts, int* __restrict__ place, long long P, int top, int E) {
     extern __shared__ int hist[];                       // [E] pairs of this block, then [E] the block's first place
     int* first = hist + E;
-    pdl_trigger();
     pdl_wait();
     for (int e = threadIdx.x; e < E; e += CNT_THREADS) hist[e] = 0;
     __syncthreads();
@@ -527,6 +538,7 @@ moe_count_kernel(const int* __restrict__ idx, int* __restrict__ counts, int* __r
     __syncthreads();
     for (int e = threadIdx.x; e < E; e += CNT_THREADS) first[e] = hist[e] > 0 ? atomicAdd(counts + e, hist[e]) : 0;
     __syncthreads();
+    pdl_trigger();
 #pragma unroll
     for (int i = 0; i < CNT_PAIRS / CNT_THREADS; ++i) {
         const long long p = p0 + i * CNT_THREADS + threadIdx.x;
@@ -544,7 +556,6 @@ moe_gather_rows_kernel(const bf16* __restrict__ h, const int* __restrict__ idx, 
                        bf16* __restrict__ x, long long P, int top, int W8, int E) {
     __shared__ int row0[nxd_gemm::kSegMaxExperts + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    pdl_trigger();
     pdl_wait();
     if (warp == 0) nxd_gemm::segment_starts(counts, E, 0, row0, nullptr);
     __syncthreads();
@@ -562,6 +573,7 @@ moe_gather_rows_kernel(const bf16* __restrict__ h, const int* __restrict__ idx, 
     bf16x8* dst = reinterpret_cast<bf16x8*>(x) + (long long)row * W8;
 #pragma unroll 4
     for (int c = lane; c < W8; c += 32) dst[c] = src[c];
+    pdl_trigger();
 }
 
 // Both of the above for few pairs, in one launch and without zeroed counts: every block counts all pairs itself, a warp finds its
@@ -575,7 +587,6 @@ moe_sort_few_kernel(const bf16* __restrict__ h, const int* __restrict__ idx, int
                     int E) {
     __shared__ int expert[FEW_PAIRS], cnt[nxd_gemm::kSegMaxExperts], row0[nxd_gemm::kSegMaxExperts + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    pdl_trigger();
     for (int e = threadIdx.x; e < E; e += GA_WARPS * 32) cnt[e] = 0;
     __syncthreads();
     pdl_wait();
@@ -606,6 +617,7 @@ moe_sort_few_kernel(const bf16* __restrict__ h, const int* __restrict__ idx, int
     bf16x8* dst = reinterpret_cast<bf16x8*>(x) + (long long)row * W8;
 #pragma unroll 4
     for (int c = lane; c < W8; c += 32) dst[c] = src[c];
+    pdl_trigger();
 }
 
 }  // namespace
@@ -661,8 +673,8 @@ NXD_API int nxd_moe_sort_rows(const void* h, const int* idx, int* counts, int* s
     NXD_REQUIRE(((uintptr_t)h % 16) == 0 && ((uintptr_t)x % 16) == 0, "sort rows: rows must be 16-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
     if (nxd_moe_sort_counts_itself(P)) {
-        NXD_CHECK_CUDA(nxd_launch_pdl(moe_sort_few_kernel, dim3((unsigned)((P + GA_WARPS - 1) / GA_WARPS)), dim3(GA_WARPS * 32), 0, st,
-                                      (const bf16*)h, idx, counts, slot, in_scale, row_scale, (bf16*)x, (int)P, top, W / 8, E));
+        NXD_CHECK_CUDA(launch_beside(P / top, moe_sort_few_kernel, dim3((unsigned)((P + GA_WARPS - 1) / GA_WARPS)), dim3(GA_WARPS * 32), st,
+                                     (const bf16*)h, idx, counts, slot, in_scale, row_scale, (bf16*)x, (int)P, top, W / 8, E));
         NXD_LAUNCH_CHECK();
         return 0;
     }
@@ -786,12 +798,12 @@ NXD_API int nxd_moe_gather_combine(int dtype, const void* ys, const int* slot, c
     auto al = [](const void* p) { return ((uintptr_t)p % 16) == 0; };
     const bool vec = W % 8 == 0 && al(ys) && al(h) && al(shared_out) && al(y);
 #define NXD_GC(T, V)                                                                                     \
-    NXD_CHECK_CUDA(nxd_launch_pdl(moe_gather_combine_kernel<T, V>, dim3((unsigned)N), dim3(128), 0, (cudaStream_t)stream, \
-                                  (const T*)ys, slot, idx, wts, (const T*)h, (const T*)shared_out, sgate, y, top, W, E))
+    NXD_CHECK_CUDA(launch_beside(N, moe_gather_combine_kernel<T, V>, dim3((unsigned)N), dim3(128), (cudaStream_t)stream, \
+                                 (const T*)ys, slot, idx, wts, (const T*)h, (const T*)shared_out, sgate, y, top, W, E))
     if (dtype == 2) {
 #define NXD_GC_WIDE(V)                                                                                   \
-    NXD_CHECK_CUDA(nxd_launch_pdl(moe_gather_combine_kernel<bf16, V, float>, dim3((unsigned)N), dim3(128), 0, (cudaStream_t)stream, \
-                                  (const float*)ys, slot, idx, wts, (const bf16*)h, (const float*)shared_out, sgate, y, top, W, E))
+    NXD_CHECK_CUDA(launch_beside(N, moe_gather_combine_kernel<bf16, V, float>, dim3((unsigned)N), dim3(128), (cudaStream_t)stream, \
+                                 (const float*)ys, slot, idx, wts, (const bf16*)h, (const float*)shared_out, sgate, y, top, W, E))
         if (vec) NXD_GC_WIDE(8); else NXD_GC_WIDE(1);
 #undef NXD_GC_WIDE
     } else if (dtype == 0) {

@@ -222,7 +222,7 @@ class KVCacheInferenceMixin:
         """One token per sequence for up to 128 sequences on the small-M tensor-core kernels (``csrc/gemm_smallm.cu``); a few
         sequences of a narrow model have both RMSNorms inside the projections behind them, six launches.  Else:
         RMSNorm | QKV GEMM+RoPE+cache write | attention (split, merge) | o_proj+residual | RMSNorm | gate/up+SwiGLU |
-        down_proj+residual -- eight launches, no copies between them.  Tensor parallel: the two row-parallel GEMMs are
+        down_proj+residual -- eight launches, no copies between them, and seven where attention has one split.  Tensor parallel: the two row-parallel GEMMs are
         followed by the one-shot all-reduce and the residual moves into the fused add+RMSNorm (ten launches)."""
         from ..ops import activation, decode_fused
         from ..ops.fused_comm import oneshot_all_reduce

@@ -1,7 +1,8 @@
 """Bindings of the fused token-generation projections (``csrc/decode_fused.cu``): RMSNorm + fused QKV GEMV + RoPE + KV-cache
 write in one launch, RMSNorm + gate/up GEMV + SwiGLU in one launch.  With the two row-parallel GEMVs that take the
 residual in their epilogue (``fused_comm.skinny_gemm``) and the decode attention (split + merge) a decoder layer of the
-token-generation graph is six launches (reference graph: ``examples/inference/modules/model_base.py:459-518``).
+token-generation graph is six launches (reference graph: ``examples/inference/modules/model_base.py:459-518``).  One sequence of the
+compiled layer sizes takes all layers in one launch instead (``token_stack``).
 
 Batches of 1 to 128 sequences on one process take the tensor-core counterparts (``csrc/gemm_smallm.cu``: weight rows as the
 UMMA M dimension, cluster split-K) unless the weights are small (``gemm.streams_on_tensor_cores``): fused QKV GEMM + RoPE + cache
