@@ -97,7 +97,6 @@ template <int D>
 __global__ void __launch_bounds__(FT, D == 256 ? 1 : 2)
 delta_chunk_factors_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ systems,
                            uint8_t* __restrict__ tiles, const int* __restrict__ n_new, int Tn, int c0, int H, int G) {
-    pdl_trigger();
     pdl_wait();
     constexpr int V = D / 32, A1 = D / 64;
     extern __shared__ __align__(16) float smem[];
@@ -237,6 +236,7 @@ delta_chunk_factors_kernel(const float* __restrict__ qn, const float* __restrict
             shift[x] = f2_pack(grid_shift(__uint_as_float(channel_max[d + 2 * x])), grid_shift(__uint_as_float(channel_max[d + 2 * x + 1])));
         split_store<8>(k, shift, img + (1 + A1 + d / 128) * TILE_BYTES + ((d >> 6) & 1) * 8192 + t * 128 + ((((d & 63) >> 3) ^ (t & 7)) << 4));
     }
+    pdl_trigger();
 }
 
 template <int D>

@@ -140,7 +140,6 @@ delta_prep_strip_kernel(const T* __restrict__ proj, long long ld, int off_q, int
                         float* __restrict__ kn, float* __restrict__ vn, const int* __restrict__ q_start,
                         const int* __restrict__ n_new, const int* __restrict__ seq_ids, int units, int Tn, int H, int G, int Dv,
                         float qscale, float unit_eps, int strip) {
-    pdl_trigger();
     pdl_wait();
     constexpr int D = 32 * V, TAPS = 4, K = TAPS - 1;
     const int lane = threadIdx.x & 31, u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -207,6 +206,8 @@ delta_prep_strip_kernel(const T* __restrict__ proj, long long ld, int off_q, int
 #pragma unroll
             for (int e = 0; e < V; ++e) x[i][e] = x[PREP_AHEAD + i][e];
     }
+    pdl_trigger();      // behind the work, as in all kernels of a prompt: at their start, 4 x 1500 tokens of 8 heads of 256 x 512 took 839 us,
+                        // 826 so, 831 without programmatic dependents (blocks that start early crowd the SMs that have room)
 }
 
 template <typename T, int V>
@@ -229,7 +230,6 @@ __global__ void delta_conv_state_kernel(const T* __restrict__ proj, long long ld
                                         float* __restrict__ conv_state, const int* __restrict__ q_start,
                                         const int* __restrict__ n_new, const int* __restrict__ seq_ids, int B, int Tn,
                                         int GD, int C, int taps) {
-    pdl_trigger();
     pdl_wait();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)B * C) return;
@@ -245,6 +245,7 @@ __global__ void delta_conv_state_kernel(const T* __restrict__ proj, long long ld
     for (int s = 0; s < K; ++s)                                  // slot s <- position (p0 + n) - K + s
         vals[s] = conv_input(proj, ld, st, (long long)b * Tn, n - K + s, p0, K, C, c, col);
     for (int s = 0; s < K; ++s) st[(long long)s * C + c] = vals[s];
+    pdl_trigger();
 }
 
 constexpr int SCAN_THREADS = 128, SCAN_TS = 16;
@@ -254,7 +255,6 @@ constexpr int SCAN_THREADS = 128, SCAN_TS = 16;
 __global__ void delta_gates_kernel(float* __restrict__ apre, long long ld_a, int a_off, float* __restrict__ bpre,
                                    long long ld_b, int b_off, const float* __restrict__ a_log,
                                    const float* __restrict__ dt_bias, long long N, int H, int per_head) {
-    pdl_trigger();
     pdl_wait();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int cols = H * per_head + H;                 // decay columns, then beta columns
@@ -268,6 +268,7 @@ __global__ void delta_gates_kernel(float* __restrict__ apre, long long ld_a, int
         float* p = bpre + n * ld_b + b_off + (c - H * per_head);
         *p = 1.f / (1.f + expf(-*p));
     }
+    pdl_trigger();
 }
 
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
@@ -512,7 +513,6 @@ __global__ void __launch_bounds__(CW_THREADS, 2)
 delta_chunk_system_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ gate,
                           long long ld_a, int a_off, const float* __restrict__ beta, long long ld_b, int b_off,
                           float* __restrict__ scratch, const int* __restrict__ n_new, int Tn, int chunk0, int H, int G) {
-    pdl_trigger();
     pdl_wait();
     extern __shared__ __align__(16) float smem[];
     double* Kd = reinterpret_cast<double*>(smem);      // [CH][DPITCH] 64 key channels at a time; then X = (I + A)^-1
@@ -642,6 +642,7 @@ delta_chunk_system_kernel(const float* __restrict__ qn, const float* __restrict_
         put(out, i, v[0], v[1]);
         put(out + CH * CH, i, y[0], y[1]);
     }
+    pdl_trigger();
 }
 
 // The rest in fp32, per (32 value columns, head, row), sequential over chunks with the state slice in shared memory: four products per
