@@ -43,7 +43,13 @@ __device__ __forceinline__ float glu_act(float g, float u, float limit, float al
 }
 
 // ---- router ---------------------------------------------------------------------------------------------------------
-constexpr int RT_WARPS = 4;
+constexpr int RT_WARPS = 4, RT_SHARE_WARPS = 8;
+
+// parts of the width that the warps of one token's CTA take: all warps busy also with few outputs
+__host__ __device__ inline int router_parts(int R, int warps) {
+    const int groups = (R + 3) / 4;
+    return groups < warps ? warps / groups : 1;
+}
 
 // 8 consecutive values of a row
 __device__ __forceinline__ void ld8(const float* p, float* f) {
@@ -52,17 +58,18 @@ __device__ __forceinline__ void ld8(const float* p, float* f) {
 }
 __device__ __forceinline__ void ld8(const bf16* p, float* f) { unpack8(*reinterpret_cast<const bf16x8*>(p), f); }
 
-// acc[t][i] += <h row t, wr row i> over the columns of this lane.  V = 8: 16- / 32-byte loads (W a multiple of 8, aligned
+// acc[t][i] += <h row t, wr row i> over the columns of this lane in every `parts`-th piece of 32 V from piece `part` on.  V = 8: 16- / 32-byte loads (W a multiple of 8, aligned
 // rows); V = 1: any W.  Rows past nt / nr repeat the last one (their sums are not used).
 template <typename T, int V, int TOK, int G>
-__device__ __forceinline__ void router_dots(const T* h, const float* wr, int W, int nt, int nr, float (&acc)[TOK][G]) {
+__device__ __forceinline__ void router_dots(const T* h, const float* wr, int W, int nt, int nr, float (&acc)[TOK][G], int part = 0,
+                                            int parts = 1) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int t = 0; t < TOK; ++t)
 #pragma unroll
         for (int i = 0; i < G; ++i) acc[t][i] = 0.f;
 #pragma unroll (TOK == 1 ? 2 : 1)
-    for (int c = lane * V; c < W; c += 32 * V) {
+    for (int c = (part * 32 + lane) * V; c < W; c += parts * 32 * V) {
         float hv[TOK][V];
 #pragma unroll
         for (int t = 0; t < TOK; ++t) {
@@ -159,11 +166,13 @@ __device__ __forceinline__ void router_select(float* ps, float* cs, const float*
     }
 }
 
-// A CTA of RT_WARPS warps.  SHARE: one token, the warps share its experts (few tokens: the latency of one token counts).  Else
+// A CTA of RT_WARPS warps.  SHARE: one token and up to RT_SHARE_WARPS warps, they share its experts and the width (few tokens: the latency of
+// one token counts, a chain of loads along the width: 64 tokens of 1024 x
+// 16 5.6 -> 4.9 us against four warps that share the outputs only, 1024 x 64 14.1 -> 9.1, 2048 x 8 6.9 -> 4.3, 4096 x 8 11.3 -> 5.2).  Else
 // every warp takes TOK tokens and all experts, so a row of wr that is loaded serves TOK tokens (many tokens: the fp32 rows of wr
 // come from L1 / L2 and are the larger operand).
 template <typename T, int V, int TOK, bool SHARE>
-__global__ void __launch_bounds__(RT_WARPS * 32)
+__global__ void __launch_bounds__((SHARE ? RT_SHARE_WARPS : RT_WARPS) * 32)
 moe_router_kernel(const T* __restrict__ h, const float* __restrict__ wr, const float* __restrict__ corr,
                   const float* __restrict__ wsg, int* __restrict__ idx, float* __restrict__ wts,
                   float* __restrict__ sgate, long long N, int W, int R, int top, float out_scale,
@@ -175,33 +184,65 @@ moe_router_kernel(const T* __restrict__ h, const float* __restrict__ wr, const f
     const long long n0 = SHARE ? blockIdx.x : ((long long)blockIdx.x * RT_WARPS + warp) * TOK;
     if (n0 >= N) return;                            // SHARE: never; else whole warps, which share nothing
     const int nt = (int)min((long long)TOK, N - n0);
-    float* ps = smem + (SHARE ? 0 : warp * (TOK + 1) * R);          // logits [TOK][R], then scratch [R]
     const T* hr = h + n0 * W;
-    for (int r0 = SHARE ? warp * G : 0; r0 < R; r0 += SHARE ? RT_WARPS * G : G) {
-        float acc[TOK][G];
-        router_dots<T, V, TOK, G>(hr, wr + (long long)r0 * W, W, nt, R - r0, acc);
-#pragma unroll
-        for (int t = 0; t < TOK; ++t)
+    if constexpr (SHARE) {
+        const int warps = blockDim.x >> 5, groups = (R + G - 1) / G, parts = router_parts(R, warps), part = parts > 1 ? warp / groups : 0;
+        float* ps = smem + R;                                       // scratch [R], sums [parts][R], the gate's [warps]
+        float* gate = ps + parts * R;
+        for (int r0 = (parts > 1 ? warp % groups : warp) * G; r0 < R && part < parts; r0 += warps * G) {
+            float acc[1][G];
+            router_dots<T, V, 1, G>(hr, wr + (long long)r0 * W, W, 1, R - r0, acc, part, parts);
 #pragma unroll
             for (int i = 0; i < G; ++i) {
-                const float z = warp_sum(acc[t][i]);
-                if (lane == 0 && r0 + i < R) ps[t * R + r0 + i] = z + (zbias != nullptr ? zbias[r0 + i] : 0.f);
+                const float z = warp_sum(acc[0][i]);
+                if (lane == 0 && r0 + i < R) ps[part * R + r0 + i] = z;
             }
-    }
-    if (wsg != nullptr && sgate != nullptr && (!SHARE || warp == RT_WARPS - 1)) {
-        float acc[TOK][1];
-        router_dots<T, V, TOK, 1>(hr, wsg, W, nt, 1, acc);
-#pragma unroll
-        for (int t = 0; t < TOK; ++t) {
-            const float z = warp_sum(acc[t][0]);
-            if (lane == 0 && t < nt) sgate[n0 + t] = 1.f / (1.f + expf(-z));
         }
-    }
-    pdl_trigger();
-    if constexpr (SHARE) {
+        const bool gated = wsg != nullptr && sgate != nullptr;
+        if (gated) {
+            float acc[1][1];
+            router_dots<T, V, 1, 1>(hr, wsg, W, 1, 1, acc, warp, warps);
+            const float z = warp_sum(acc[0][0]);
+            if (lane == 0) gate[warp] = z;
+        }
+        pdl_trigger();
         __syncthreads();
-        if (warp == 0) router_select(ps, ps + R, corr, idx, wts, n0, R, top, out_scale, mode);
+        if (warp != 0) return;
+        for (int r = lane; r < R; r += 32) {
+            float z = ps[r];
+            for (int i = 1; i < parts; ++i) z += ps[i * R + r];
+            ps[r] = z + (zbias != nullptr ? zbias[r] : 0.f);
+        }
+        if (gated && lane == 0) {
+            float z = gate[0];
+            for (int i = 1; i < warps; ++i) z += gate[i];
+            sgate[n0] = 1.f / (1.f + expf(-z));
+        }
+        __syncwarp();
+        router_select(ps, smem, corr, idx, wts, n0, R, top, out_scale, mode);
     } else {
+        float* ps = smem + warp * (TOK + 1) * R;                    // logits [TOK][R], then scratch [R]
+        for (int r0 = 0; r0 < R; r0 += G) {
+            float acc[TOK][G];
+            router_dots<T, V, TOK, G>(hr, wr + (long long)r0 * W, W, nt, R - r0, acc);
+#pragma unroll
+            for (int t = 0; t < TOK; ++t)
+#pragma unroll
+                for (int i = 0; i < G; ++i) {
+                    const float z = warp_sum(acc[t][i]);
+                    if (lane == 0 && r0 + i < R) ps[t * R + r0 + i] = z + (zbias != nullptr ? zbias[r0 + i] : 0.f);
+                }
+        }
+        if (wsg != nullptr && sgate != nullptr) {
+            float acc[TOK][1];
+            router_dots<T, V, TOK, 1>(hr, wsg, W, nt, 1, acc);
+#pragma unroll
+            for (int t = 0; t < TOK; ++t) {
+                const float z = warp_sum(acc[t][0]);
+                if (lane == 0 && t < nt) sgate[n0 + t] = 1.f / (1.f + expf(-z));
+            }
+        }
+        pdl_trigger();
         __syncwarp();
         for (int t = 0; t < nt; ++t) {
             router_select(ps + t * R, ps + TOK * R, corr, idx, wts, n0 + t, R, top, out_scale, mode);
@@ -638,10 +679,14 @@ NXD_API int nxd_moe_router(int dtype, const void* h, const float* wr, const floa
     const long long sms = nxd_num_sms(), load = (long long)W * R;
     const bool quad = (N >= (vec ? 24 : 64) * sms && N * load >= 1ll << 25) || (vec && N >= 16 * sms && load >= 1 << 16);
     const int tok = N < 8 * sms ? 0 : quad && (size_t)RT_WARPS * 5 * R * sizeof(float) <= 48 * 1024 ? 4 : 1;
-    const size_t smem = (size_t)(tok == 0 ? 2 : RT_WARPS * (tok + 1)) * R * sizeof(float);
+    // a token's CTA has eight warps while all tokens together leave room for them (with eight / four, 1000 tokens of 1024 x 16 11.9 / 9.6 us,
+    // 400 6.3 / 6.4) and each has a piece to work on (256 x 16: 3.4 / 3.1)
+    const int pieces = (R + 3) / 4 * ((W + (vec ? 255 : 31)) / (vec ? 256 : 32));
+    const int warps = tok == 0 && N <= 3 * sms && pieces > RT_WARPS ? RT_SHARE_WARPS : RT_WARPS;
+    const size_t smem = ((size_t)(tok == 0 ? 1 + router_parts(R, warps) : RT_WARPS * (tok + 1)) * R + (tok == 0 ? warps : 0)) * sizeof(float);
     const unsigned blocks = (unsigned)(tok == 0 ? N : (N + RT_WARPS * tok - 1) / (RT_WARPS * tok));
 #define NXD_RT(T, V, TOK, SHARE)                                                                                        \
-    NXD_CHECK_CUDA(nxd_launch_pdl(moe_router_kernel<T, V, TOK, SHARE>, dim3(blocks), dim3(RT_WARPS * 32), smem, (cudaStream_t)stream, \
+    NXD_CHECK_CUDA(nxd_launch_pdl(moe_router_kernel<T, V, TOK, SHARE>, dim3(blocks), dim3(warps * 32), smem, (cudaStream_t)stream, \
                                   (const T*)h, wr, corr, wsg, idx, wts, sgate, N, W, R, top, out_scale, zbias, mode))
 #define NXD_RT_V(T, V)                                                                                                  \
     do {                                                                                                                \

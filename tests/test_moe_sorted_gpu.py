@@ -82,6 +82,26 @@ def test_router_forms_match_float64(N, W, R, dtype):
     assert (sg.double() - torch.sigmoid(h.double() @ gate.double()[0])).abs().max() <= 1e-5
 
 
+# a token's CTA splits the width between its warps: four and eight of them (3 tokens per SM), parts that do not divide the warps, widths of
+# fewer pieces than parts, outputs of one to nine groups of four
+@pytest.mark.parametrize("N,W,R", [(1, 4096, 8), (7, 2048, 12), (9, 2056, 1), (3, 264, 5), (2, 33, 9), (444, 520, 33), (445, 520, 8), (1183, 1000, 8)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_warps_that_share_a_token_match_float64(N, W, R, dtype):
+    from neuronx_distributed_llama3_2_b200.ops import moe_sparse as ms
+
+    g = torch.Generator(device="cuda").manual_seed(N + W)
+    h = torch.randn(N, W, generator=g, device="cuda").to(dtype)
+    w = torch.randn(R, W, generator=g, device="cuda") * W ** -0.5
+    gate = torch.randn(1, W, generator=g, device="cuda") * W ** -0.5
+    bias = torch.randn(R, generator=g, device="cuda")
+    idx, wts, sg = ms.route(h, w, None, 1, 1.5, gate, logit_bias=bias)
+    p = torch.softmax(h.double() @ w.double().t() + bias.double(), dim=-1)
+    chosen = p.gather(1, idx.long())
+    # fp32 sums of W terms of size 1: a choice may differ only between scores that are closer than their rounding
+    assert (chosen[:, 0] - p.amax(-1)).abs().max() <= 1e-5
+    assert (wts.double() - 1.5 * chosen).abs().max() <= 1e-5
+    assert (sg.double() - torch.sigmoid(h.double() @ gate.double()[0])).abs().max() <= 1e-5
+
 # below and above 16 pairs per expert (32 tokens), one and several row tiles; with and without a shared expert
 @pytest.mark.parametrize("N", [1, 31, 32, 200, 1000])
 @pytest.mark.parametrize("shared", [0, 72])
