@@ -415,7 +415,9 @@ __global__ void __launch_bounds__(kThreads, 1) token_stack_kernel(const __grid_c
                     }
                     for (int kb = 0; kb < keys; kb += kKeys) {
                         const bool ours = kb / 128 % 2 == warp / 4;
-                        if (ours && !__all_sync(0xffffffffu, wait(&full[st], ph, p.limit, &dead))) break;
+                        // the warps that skip a slot wait for it as well: `empty` counts arrivals, not warps, and one that is ahead by a round of
+                        // the ring would arrive a second time in the place of one that still reads
+                        if (!__all_sync(0xffffffffu, wait(&full[st], ph, p.limit, &dead))) break;
                         const uint8_t* slot = smem + st * kSlotBytes;
                         // keys first, then values: both in registers at once would not fit beside the states
                         auto fetch = [&](int u, int half, const uint4 (&own_row)[kV], float (&f)[kE]) {
