@@ -555,11 +555,13 @@ __global__ void __launch_bounds__(kThreads, 1) token_stack_kernel(const __grid_c
             if (step == 0) {
                 if (has_rot && !dead) {
                     const float y = rounded(sum_of(2 * tid)), z = rounded(sum_of(2 * tid + 1));
-                    const float lo = y * rot_cos - z * rot_sin, hi = z * rot_cos + y * rot_sin;          // values: turned by nothing
+                    // values go over as they are: turned by nothing, one that is not finite would reach its partner as inf * 0
+                    const bool turned = rot_head < p.n_q + p.n_kv;
+                    const float lo = turned ? y * rot_cos - z * rot_sin : y, hi = turned ? z * rot_cos + y * rot_sin : z;
                     if (rot_head < p.n_q) {
                         send(p.q + rot_head * (D / 2) + rot_d, two(lo, hi), number);
                     } else {
-                        const bool value = rot_head >= p.n_q + p.n_kv;
+                        const bool value = !turned;
                         const int kvh = rot_head - p.n_q - (value ? p.n_kv : 0);
                         send(p.kv + (kvh * 2 + value) * (D / 2) + rot_d, two(lo, hi), number);
                         bf16* dst = (value ? cache.v : cache.k) + cache_row(cache, 0, kvh, position, D);

@@ -118,6 +118,23 @@ def test_layers_in_one_launch(size, n, page):
         assert torch.equal(out, _stack(x, layers, size, cos, sin, pos, lens, **place))
 
 
+@pytest.mark.parametrize("size", SIZES)
+def test_a_value_that_is_not_finite_stays_in_its_channel(size):
+    H, I, nq, nkv, D = SIZES[size]
+    layers, x = _draw(size, 1, 1, 128, 3)
+    for i, row in ((5, float("inf")), (D + D // 2 + 2, float("nan"))):                 # of the value heads: a lower and an upper half
+        layers[0][1][(nq + nkv) * D + i] = row
+    cos, sin = _tables(D, 128)
+    pos, lens = (torch.tensor([v], dtype=torch.int32, device="cuda") for v in (99, 100))
+    other = [[t.clone() for t in w] for w in layers]
+    _chain(x, other, size, cos, sin, pos, lens)
+    _stack(x, layers, size, cos, sin, pos, lens)
+    (ck, cv), (k, v) = layers[0][6:], other[0][6:]
+    finite = torch.isfinite(cv[0, :, 99])
+    assert torch.equal(finite, torch.isfinite(v[0, :, 99])) and (~finite).sum() == 2 and torch.isfinite(ck).all()
+    assert (cv[0, :, 99][finite].float() - v[0, :, 99][finite].float()).norm() <= 2e-2 * v[0, :, 99][finite].float().norm()     # as above
+
+
 def test_replays_follow_the_position():
     H, I, nq, nkv, D = SIZES["64"]
     layers, x = _draw("64", 2, 1, 640, 7)
