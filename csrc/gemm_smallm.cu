@@ -161,7 +161,6 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
     const int tpr = (B + splits - 1) / splits;          // token columns per owner CTA
 
     TRACE_STAMP(0, threadIdx.x == 0);
-    pdl_trigger();
     // warp 0 lane 0 owns the barriers and the TMA queue: it starts the weight stream right after initialising them,
     // before the CTA (or, with split-K, the cluster) has met -- the weights do not depend on the previous kernel either
     auto load_w = [&](int kb, int stage) {
@@ -193,6 +192,7 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
     if (warp == 1) ptx::tmem_alloc<1>(tmem_ptr_smem, C::kTmemCols);
     ptx::tcgen05_fence_before();
     __syncthreads();
+    pdl_trigger();      // not before this CTA has its tensor memory: prompt attention allocates before it waits, and two of its CTAs take all columns
     // split-K: a peer may only send once this CTA's receive barrier exists.  Every thread arrives at the cluster barrier
     // now and waits for it after its main loop (measured: a full cluster barrier here costs ~1 us of start-up)
     if (splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");

@@ -3,6 +3,7 @@ shared memory belongs to one device, so every device that a process launches fro
 import ctypes as c
 import glob
 import os
+import re
 import shutil
 import subprocess
 
@@ -118,3 +119,25 @@ def test_every_device_is_given_its_shared_memory(library, name):
                                                        (1, 8, 8, 100000, 37), (64, 8, 1, 200, 2), (1, 32, 1, 100000, 64)])
 def test_splits_of_a_token_step(library, B, n_q, n_kv, max_len, splits):
     assert library.nxd_decode_attn_splits(B, n_q, n_kv, max_len) == splits
+
+
+def test_kernels_trigger_behind_their_tensor_memory():
+    """A programmatic dependent that allocates tensor memory and then waits for the grid before it must not find CTAs of that grid
+    that have none yet: in the source of every kernel that allocates, the allocation comes before the trigger."""
+    root = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "csrc")
+    seen = set()
+    for path in glob.glob(os.path.join(root, "*.cu")):
+        with open(path) as f:
+            text = re.sub(r"//[^\n]*", "", f.read())
+        for start in re.finditer(r"__global__", text):
+            first = text.index("{", start.end())
+            depth, end = 1, first + 1
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[end], 0)
+                end += 1
+            body = text[first:end]
+            trigger, alloc = body.find("pdl_trigger()"), body.find("tmem_alloc")
+            if trigger >= 0 and alloc >= 0:
+                seen.add(os.path.basename(path))
+                assert alloc < trigger, f"{os.path.basename(path)}: {text[start.start():first][:120]}"
+    assert {"gemm_smallm.cu", "gemm_tcgen05.cu", "flash_attn_tc.cu"} <= seen
