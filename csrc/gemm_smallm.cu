@@ -63,6 +63,7 @@ struct EpiArgs {
     CacheDst cache;
     int n_q, n_kv, D;
     int up_row0;               // SwiGLU: first "up" row of w (= I)
+    bool w_ready;              // no kernel in flight writes w: its first tiles are loaded before the kernel in front has ended
     // NORM: the activations before their RMSNorm, its weight and epsilon
     const bf16* raw;
     long long ld_raw;
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
 
     TRACE_STAMP(0, threadIdx.x == 0);
     // warp 0 lane 0 owns the barriers and the TMA queue: it starts the weight stream right after initialising them,
-    // before the CTA (or, with split-K, the cluster) has met -- the weights do not depend on the previous kernel either
+    // before the CTA (or, with split-K, the cluster) has met -- and, of weights that are ready, before the previous kernel has ended
     auto load_w = [&](int kb, int stage) {
         uint8_t* sw = smem + stage * C::kStageBytes;
         ptx::mbar_arrive_expect_tx(&full_bar[stage], C::kStageBytes);
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
         ptx::fence_barrier_init();
         // every CTA of the cluster sends this one a [tpr][128] fp32 block per accumulator
         if (splits > 1 && split * tpr < B) ptx::mbar_arrive_expect_tx(recv_bar, (uint32_t)(splits * C::kAcc * tpr * kWRows * 4));
-        for (int i = 0; i < pre; ++i) load_w(kb_begin + i, i);
+        for (int i = 0; ep.w_ready && i < pre; ++i) load_w(kb_begin + i, i);
     }
     if (warp == 1) ptx::tmem_alloc<1>(tmem_ptr_smem, C::kTmemCols);
     ptx::tcgen05_fence_before();
@@ -204,7 +205,10 @@ __global__ void __launch_bounds__(kThreads) gemm_smallm_kernel(const __grid_cons
         if (lane == 0) {
             if (!NORM) pdl_wait();      // the activations come from the previous kernel (programmatic dependent launch)
             TRACE_STAMP(2, true);
-            for (int i = 0; i < pre; ++i) load_x(kb_begin + i, i);
+            for (int i = 0; i < pre; ++i) {
+                if (!ep.w_ready) load_w(kb_begin + i, i);
+                load_x(kb_begin + i, i);
+            }
             int stage = pre == C::kStages ? 0 : pre;
             uint32_t phase = pre == C::kStages ? 1 : 0;
             for (int kb = kb_begin + pre; kb < kb_end; ++kb) {
@@ -629,14 +633,23 @@ int run_norm(const void* x, long long ldx, const void* norm_w, float eps, const 
 
 // x [B, K] (pitch ldx), w [N, K] (pitch ldw), residual [B, N] (pitch ldr) or NULL, out [B, N] (pitch ldo); bf16.
 // 1 <= B <= 128; K, ldx, ldw multiples of 8; x and w 16-byte aligned.  splits: 0 = choose, else 1 / 2 / 4 / 8.
-NXD_API int nxd_gemm_smallm_bf16(const void* x, const void* w, const void* residual, void* out, int B, int N, int K,
-                                 long long ldx, long long ldw, long long ldo, long long ldr, int splits, void* stream) {
+// w_ready: no kernel before this one on the stream that may still run writes w (the kernels of this library let the next one start before
+// they end).  The entries with the neighbouring work of a decoder layer inside take that for granted of their weights.
+NXD_API int nxd_gemm_smallm_ready_bf16(const void* x, const void* w, const void* residual, void* out, int B, int N, int K,
+                                       long long ldx, long long ldw, long long ldo, long long ldr, int splits, int w_ready,
+                                       void* stream) {
     EpiArgs ep = {};
+    ep.w_ready = w_ready != 0;
     ep.out = (bf16*)out;
     ep.ldo = ldo;
     ep.residual = (const bf16*)residual;
     ep.ldr = ldr;
     return run<kEpiPlain>(x, w, ep, B, N, N, K, ldx, ldw, splits, (cudaStream_t)stream);
+}
+
+NXD_API int nxd_gemm_smallm_bf16(const void* x, const void* w, const void* residual, void* out, int B, int N, int K,
+                                 long long ldx, long long ldw, long long ldo, long long ldr, int splits, void* stream) {
+    return nxd_gemm_smallm_ready_bf16(x, w, residual, out, B, N, K, ldx, ldw, ldo, ldr, splits, 0, stream);
 }
 
 // Batched form of nxd_decode_qkv_rope_cache WITHOUT the norm (x is the normalised activation): w fused projection
@@ -648,6 +661,7 @@ NXD_API int nxd_smallm_qkv_rope_cache(const void* x, long long ldx, const void* 
                                       long long stride_h, int page_size, int max_pages, int B, int K, int n_q, int n_kv,
                                       int D, int splits, void* stream) {
     EpiArgs ep = {};
+    ep.w_ready = true;
     if (int rc = qkv_args(ep, cos_t, sin_t, positions, q_out, cache_k, cache_v, seq_ids, block_table, stride_b, stride_h, page_size,
                           max_pages, n_q, n_kv, D))
         return rc;
@@ -667,6 +681,7 @@ NXD_API int nxd_smallm_norm_qkv_rope_cache(const void* x, long long ldx, const v
                                            const int* block_table, long long stride_b, long long stride_h, int page_size,
                                            int max_pages, int B, int K, int n_q, int n_kv, int D, void* stream) {
     EpiArgs ep = {};
+    ep.w_ready = true;
     if (int rc = qkv_args(ep, cos_t, sin_t, positions, q_out, cache_k, cache_v, seq_ids, block_table, stride_b, stride_h, page_size,
                           max_pages, n_q, n_kv, D))
         return rc;
@@ -679,6 +694,7 @@ NXD_API int nxd_smallm_norm_gate_up_swiglu(const void* x, long long ldx, const v
     NXD_REQUIRE(I % 8 == 0 && ldo % 8 == 0 && ((uintptr_t)out & 15) == 0,
                 "smallm_gate_up: I=%d and ldo must be multiples of 8, out 16-byte aligned", I);
     EpiArgs ep = {};
+    ep.w_ready = true;
     ep.out = (bf16*)out;
     ep.ldo = ldo;
     ep.up_row0 = I;
@@ -691,6 +707,7 @@ NXD_API int nxd_smallm_gate_up_swiglu(const void* x, long long ldx, const void* 
     NXD_REQUIRE(I % 8 == 0 && ldo % 8 == 0 && ((uintptr_t)out & 15) == 0,
                 "smallm_gate_up: I=%d and ldo must be multiples of 8, out 16-byte aligned", I);
     EpiArgs ep = {};
+    ep.w_ready = true;
     ep.out = (bf16*)out;
     ep.ldo = ldo;
     ep.up_row0 = I;

@@ -223,12 +223,16 @@ int nxd_skinny_gemm_ar_bf16(const void* x, const void* w, const void* residual, 
 /* Weight-streaming tcgen05 GEMM for 1..128 activation rows (batched token generation): out[B, N] = x[B, K] @ w[N, K]^T
  * (+ residual[B, N]); the weight rows are the UMMA M dimension, the padded row count (16/32/64/128) the UMMA N dimension;
  * split-K over a thread-block cluster with a distributed-shared-memory reduction.  K, ldx, ldw % 8 == 0;
- * splits: 0 = choose, else 1 / 2 / 4 / 8. */
+ * splits: 0 = choose, else 1 / 2 / 4 / 8.  w_ready: no kernel on the stream that may still run writes w (kernels of this library
+ * start before the one in front has ended), so its first tiles are fetched at once; without it, and in the first form, behind that. */
 int nxd_gemm_smallm_bf16(const void* x, const void* w, const void* residual, void* out, int B, int N, int K,
                          long long ldx, long long ldw, long long ldo, long long ldr, int splits, void* stream);
+int nxd_gemm_smallm_ready_bf16(const void* x, const void* w, const void* residual, void* out, int B, int N, int K,
+                               long long ldx, long long ldw, long long ldo, long long ldr, int splits, int w_ready, void* stream);
 /* The same kernel with the decoder layer's element-wise neighbours in its epilogue (batched counterparts of
  * nxd_decode_qkv_rope_cache / nxd_decode_gate_up_swiglu, without the norm: x is the normalised activation).
- * qkv: B <= 128, D in {64, 128}; gate_up: B <= 64, I % 8 == 0 (a CTA streams gate slab t and up slab t). */
+ * qkv: B <= 128, D in {64, 128}; gate_up: B <= 64, I % 8 == 0 (a CTA streams gate slab t and up slab t).  Their weights are taken
+ * as ready (above). */
 int nxd_smallm_qkv_rope_cache(const void* x, long long ldx, const void* w, long long ldw, const float* cos_t,
                               const float* sin_t, const int* positions, void* q_out, void* cache_k, void* cache_v,
                               const int* seq_ids, const int* block_table, long long stride_b, long long stride_h,

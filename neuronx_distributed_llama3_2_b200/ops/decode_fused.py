@@ -8,7 +8,7 @@ Batches of 1 to 128 sequences on one process take the tensor-core counterparts (
 UMMA M dimension, cluster split-K) unless the weights are small (``gemm.streams_on_tensor_cores``): fused QKV GEMM + RoPE + cache
 write, gate/up GEMM + SwiGLU (<= 64 rows), and the plain GEMM with the residual in its epilogue.  Few sequences of a narrow model
 (``norm_fits``) have the two RMSNorms inside the projections behind them, six launches per layer; else they are launches of their own,
-eight."""
+eight.  Their weights are fetched before the kernel in front has ended, so no kernel that may still run may write them."""
 from __future__ import annotations
 
 import ctypes as _c

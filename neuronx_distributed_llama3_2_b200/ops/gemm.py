@@ -117,12 +117,15 @@ def streams_on_tensor_cores(rows: int, n: int, k: int) -> bool:
     return rows > 8 or n * k >= 1 << 21 or (rows > 4 and k >= 1024)
 
 
-def gemm_smallm(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor] = None, splits: int = 0
-                ) -> Optional[torch.Tensor]:
+def gemm_smallm(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor] = None, splits: int = 0,
+                w_ready: Optional[bool] = None) -> Optional[torch.Tensor]:
     """``x[B, K] @ w[N, K]^T (+ residual)`` for ``B <= 128`` rows on the tensor cores with the WEIGHT rows as the UMMA M
     dimension (``csrc/gemm_smallm.cu``): a pure stream of the weight matrix, split-K over a thread-block cluster for
     narrow layers.  The batched token-generation GEMM (reference: the parallel linear layers of
-    ``parallel_layers/layers.py`` at ``[batch, 1, hidden]``).  ``None`` when the shape does not qualify."""
+    ``parallel_layers/layers.py`` at ``[batch, 1, hidden]``).  ``None`` when the shape does not qualify.
+
+    ``w_ready``: no kernel that may still run writes ``w``, so that it is fetched before the kernel in front has ended (``None``: a
+    ``Parameter`` is ready, any other tensor may come from the kernel right before)."""
     B, K = x.shape
     N = w.shape[0]
     if (not (x.is_cuda and w.is_cuda) or B == 0 or B > SMALLM_MAX_ROWS or x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or K % 8
@@ -136,9 +139,11 @@ def gemm_smallm(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tenso
         if residual.stride(1) != 1:
             residual = residual.contiguous()
         ldr = residual.stride(0)
-    rc = _lib.lib().nxd_gemm_smallm_bf16(
+    if w_ready is None:
+        w_ready = isinstance(w, torch.nn.Parameter)
+    rc = _lib.lib().nxd_gemm_smallm_ready_bf16(
         _lib.ptr(x), _lib.ptr(w), _lib.ptr(residual), _lib.ptr(out), _c.c_int(B), _c.c_int(N), _c.c_int(K),
         _c.c_longlong(x.stride(0)), _c.c_longlong(w.stride(0)), _c.c_longlong(out.stride(0)), _c.c_longlong(ldr),
-        _c.c_int(splits), _lib.stream_ptr())
-    _lib.check(rc, "nxd_gemm_smallm_bf16")
+        _c.c_int(splits), _c.c_int(w_ready), _lib.stream_ptr())
+    _lib.check(rc, "nxd_gemm_smallm_ready_bf16")
     return out

@@ -47,7 +47,8 @@ def _use_kernel(a: torch.Tensor, b: torch.Tensor, m: int, n: int, k: int, layout
 
 def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None,
             out_dtype: Optional[torch.dtype] = None, accumulate: bool = False) -> torch.Tensor:
-    """``a[M,K] @ b[N,K]^T``.  ``accumulate`` adds into ``out`` (fp32 grad accumulation)."""
+    """``a[M,K] @ b[N,K]^T``.  ``accumulate`` adds into ``out`` (fp32 grad accumulation).  ``b`` may come from the kernel right before,
+    unless it is a ``Parameter``: up to 128 rows of ``a``, those are fetched while that kernel may still run (``gemm.gemm_smallm``)."""
     m, k = a.shape
     n = b.shape[0]
     if (m <= 128 and out is None and not accumulate and out_dtype in (None, torch.bfloat16) and a.is_cuda

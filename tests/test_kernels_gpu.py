@@ -545,6 +545,36 @@ def test_gemm_smallm(B, K, N, splits):
     assert torch.equal(out, gemm_smallm(x, w, residual=res, splits=splits))
 
 
+def test_an_operand_of_the_kernel_right_before(monkeypatch):
+    """The kernels let the next one start before they end: only parameters are read that early, any other right operand behind the wait."""
+    import neuronx_distributed_llama3_2_b200.ops.gemm as gemm_ops
+    from neuronx_distributed_llama3_2_b200.ops.linear import gemm_nt
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    a, left, right = (torch.randn(*shape, generator=g, device="cuda").bfloat16() * 0.1 for shape in ((16, 2048), (4096, 2048), (2048, 2048)))
+    b = gemm_ops.gemm(left, right, "nt")
+    torch.cuda.synchronize()
+    ref = gemm_nt(a, b)
+    asked, library = [], gemm_ops._lib.lib()
+
+    class Spy:
+        def __getattr__(self, name):
+            fn = getattr(library, name)
+            if name != "nxd_gemm_smallm_ready_bf16":
+                return fn
+            return lambda *args: asked.append(args[-2].value) or fn(*args)
+
+    with monkeypatch.context() as m:
+        m.setattr(gemm_ops._lib, "lib", lambda *_: Spy())
+        assert torch.equal(gemm_nt(a, b), ref) and torch.equal(gemm_nt(a, torch.nn.Parameter(b, requires_grad=False)), ref)
+    assert asked == [0, 1]
+    for _ in range(50):
+        made = torch.full_like(b, float("nan"))
+        torch.cuda.synchronize()
+        gemm_ops.gemm(left, right, "nt", out=made)
+        assert torch.equal(gemm_nt(a, made), ref)
+
+
 @pytest.mark.parametrize("C", [384, 200, 37])
 @pytest.mark.parametrize("layout", ["nn", "nt", "tn"])
 def test_grouped_expert_gemm(layout, C):
