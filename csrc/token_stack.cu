@@ -22,7 +22,7 @@
 // with 192 everything else waits behind them (743 against 702).
 //
 // Waits end: one that has taken `limit` clocks gives up, the CTA sends nothing more and leaves NaN in its part of the result, so all
-// others give up too; nxd_token_stack_status says so.
+// others give up too; the caller's word, which may be pinned host memory, and nxd_token_stack_status say so.
 #include <type_traits>
 
 #include "attn_tc_common.cuh"
@@ -67,6 +67,7 @@ struct Args {
     CacheDst cache;                      // k, v: per layer
     float scale_log2;
     long long limit;
+    int* gave_up;                        // the caller's, or null
 };
 
 __device__ int stack_gave_up;
@@ -612,7 +613,10 @@ __global__ void __launch_bounds__(kThreads, 1) token_stack_kernel(const __grid_c
         if (verdict != 0) break;
     }
     if (verdict != 0) {
-        if (tid == 0) stack_gave_up = 1;
+        if (tid == 0) {
+            stack_gave_up = 1;
+            if (p.gave_up != nullptr) *reinterpret_cast<volatile int*>(p.gave_up) = 1;
+        }
         if (has_pair) *reinterpret_cast<uint32_t*>(p.out + h0 + pair_r) = 0x7fff7fffu;
     }
 }
@@ -683,11 +687,13 @@ NXD_API long long nxd_token_stack_scratch(int layers, int B, int H, int I, int n
 // hidden, out [H] bf16; pointers: per layer the weights input norm [H], q | k | v [(n_q + 2 n_kv) D, H], o [H, H], norm behind the
 // attention [H], gate | up [2 I, H], down [H, I], all contiguous and 16-byte aligned, and the caches of keys and values; eps: the two
 // norms' per layer.  positions, lengths: the sequence's, int32, the step's token the last of its length; cache as for
-// nxd_smallm_qkv_rope_cache.  wait_clocks: -1, or the limit of a wait.
-NXD_API int nxd_token_stack(const void* hidden, void* out, const void* const* pointers, const float* eps, int layers, const float* cos_t,
-                            const float* sin_t, const int* positions, const int* lengths, const int* seq_ids, const int* block_table,
-                            long long stride_b, long long stride_h, int page_size, int max_pages, void* scratch, int H, int I,
-                            int n_q, int n_kv, int D, float scale, long long wait_clocks, void* stream) {
+// nxd_smallm_qkv_rope_cache.  wait_clocks: -1, or the limit of a wait.  gave_up: a word of device or pinned host memory that a step which
+// gave up a wait sets to 1, or NULL.
+NXD_API int nxd_token_stack_telling(const void* hidden, void* out, const void* const* pointers, const float* eps, int layers,
+                                    const float* cos_t, const float* sin_t, const int* positions, const int* lengths, const int* seq_ids,
+                                    const int* block_table, long long stride_b, long long stride_h, int page_size, int max_pages,
+                                    void* scratch, int H, int I, int n_q, int n_kv, int D, float scale, long long wait_clocks,
+                                    int* gave_up, void* stream) {
     NXD_REQUIRE(nxd_token_stack_scratch(layers, 1, H, I, n_q, n_kv, D) > 0, "token_stack: no kernel for %d layers of %d", layers, H);
     Args a = {};
     for (int l = 0; l < layers; ++l) {
@@ -708,7 +714,16 @@ NXD_API int nxd_token_stack(const void* hidden, void* out, const void* const* po
     a.cache = CacheDst{nullptr, nullptr, block_table, seq_ids, stride_b, stride_h, page_size > 0 ? page_size : 1, max_pages};
     a.scale_log2 = scale * 1.4426950408889634f;
     a.limit = wait_clocks < 0 ? kWaitClocks : wait_clocks;
+    a.gave_up = gave_up;
     return dispatch(a, D, s.words, (cudaStream_t)stream);
+}
+
+NXD_API int nxd_token_stack(const void* hidden, void* out, const void* const* pointers, const float* eps, int layers, const float* cos_t,
+                            const float* sin_t, const int* positions, const int* lengths, const int* seq_ids, const int* block_table,
+                            long long stride_b, long long stride_h, int page_size, int max_pages, void* scratch, int H, int I,
+                            int n_q, int n_kv, int D, float scale, long long wait_clocks, void* stream) {
+    return nxd_token_stack_telling(hidden, out, pointers, eps, layers, cos_t, sin_t, positions, lengths, seq_ids, block_table, stride_b,
+                                   stride_h, page_size, max_pages, scratch, H, I, n_q, n_kv, D, scale, wait_clocks, nullptr, stream);
 }
 
 // *gave_up <- whether a step on this device gave up a wait since the last call (its results are NaN).  Waits for the stream.

@@ -115,6 +115,11 @@ int nxd_token_stack(const void* hidden, void* out, const void* const* pointers, 
                     const float* sin_t, const int* positions, const int* lengths, const int* seq_ids, const int* block_table,
                     long long stride_b, long long stride_h, int page_size, int max_pages, void* scratch, int H, int I, int n_q,
                     int n_kv, int D, float scale, long long wait_clocks, void* stream);
+/* the same; gave_up: a word of device or pinned host memory that a step whose waits gave up sets to 1 (its results are NaN), or NULL */
+int nxd_token_stack_telling(const void* hidden, void* out, const void* const* pointers, const float* eps, int layers, const float* cos_t,
+                            const float* sin_t, const int* positions, const int* lengths, const int* seq_ids, const int* block_table,
+                            long long stride_b, long long stride_h, int page_size, int max_pages, void* scratch, int H, int I, int n_q,
+                            int n_kv, int D, float scale, long long wait_clocks, int* gave_up, void* stream);
 int nxd_token_stack_status(int* gave_up, void* stream);
 
 /* ---- embedding (reference: parallel_layers/layers.py:215-238) ---------------------------------- */

@@ -92,7 +92,10 @@ class ContinuousBatcher:
         out = self.model.forward_infer(toks, pos, seq_ids=lines)
         self.stats["decode_calls"] += 1
         self.stats["decode_rows"] += n
-        return [int(t) for t in out[:n]]
+        tokens = [int(t) for t in out[:n]]
+        if hasattr(self.model, "check_steps"):
+            self.model.check_steps()
+        return tokens
 
     # -- the loop ------------------------------------------------------------------------------------------------------
     def step(self) -> List[int]:

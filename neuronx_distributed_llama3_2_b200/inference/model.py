@@ -80,7 +80,25 @@ class KVCacheInferenceMixin:
         self.kv_cache = KVCache(cfg.num_hidden_layers, ic.max_batch_size, attn0.kv_heads_local, ic.seq_len, cfg.head_dim,
                                 dtype=dtype or cfg.torch_dtype, device=device, paged=ic.paged_kv, page_size=ic.page_size,
                                 num_pages=ic.num_kv_pages if ic.paged_kv else None)
+        self._steps_gave_up()                # host memory cannot be pinned while a graph is captured
         return self.kv_cache
+
+    _gave_up = None
+
+    def _steps_gave_up(self):
+        if self._gave_up is None and torch.cuda.is_available() and not torch.cuda.is_current_stream_capturing():
+            from ..ops.decode_fused import GaveUp
+
+            self._gave_up = GaveUp()
+        return self._gave_up
+
+    def check_steps(self) -> None:
+        """Raises if a token step that has ended gave up one of its waits (``csrc/token_stack.cu``: two seconds): its logits are NaN and its
+        keys and values incomplete, so the sequence has to start over.  Costs a read of host memory; every step asks for the ones before it,
+        the generation loops behind their last one as well."""
+        if self._gave_up is not None and self._gave_up.take():
+            raise RuntimeError("a token-generation step gave up waiting inside its kernel: its tokens are not valid and the cache of its "
+                               "sequence is incomplete")
 
     def _rope(self, device) -> Tuple[torch.Tensor, torch.Tensor]:
         if self._rope_tables is None or self._rope_tables[0].device != device:
@@ -273,6 +291,8 @@ class KVCacheInferenceMixin:
             return gemm_smallm(act, mlp.down_proj.weight, residual=x2).reshape(B, 1, -1), None
         return all_reduce(gemm_smallm(act, mlp.down_proj.weight)).reshape(B, 1, -1), x2.reshape(B, 1, -1)
 
+    _token_stack_clocks = -1                  # of a wait inside, -1: two seconds
+
     def _token_stack(self, hidden, residual, positions, seq_ids, lengths):
         """All decoder layers of a step of one sequence in one launch (``csrc/token_stack.cu``), ``None`` where that does not
         apply: the layers that ``_layer_batched_decode`` takes on one process, all alike, of a size that is compiled, with contiguous
@@ -306,11 +326,15 @@ class KVCacheInferenceMixin:
             stack.append(((*ws, *caches), n1.variance_epsilon, n2.variance_epsilon))
         if kc.layer(0)[0].stride(0) % 8 or kc.layer(0)[0].stride(1) % 8:
             return None
+        gave_up = self._steps_gave_up()
+        if gave_up is None:
+            return None
         pos, sid = self._decode_i32(positions, seq_ids)
         cos, sin = self._rope(hidden.device)
         return decode_fused.token_stack(hidden.view(B, H), stack, cos, sin, pos, lengths, nq, nkv, D, scratch, seq_ids=sid,
                                         block_table=kc.block_table if kc.paged else None,
-                                        page_size=kc.page_size if kc.paged else 0).view(B, 1, H)
+                                        page_size=kc.page_size if kc.paged else 0, wait_clocks=self._token_stack_clocks,
+                                        gave_up=gave_up).view(B, 1, H)
 
     def _layer_fused_decode(self, i: int, layer, hidden, residual, positions, seq_ids, lengths):
         """One token per sequence: RMSNorm+QKV+RoPE+cache write | attention (split, merge) | o_proj+residual |
@@ -434,6 +458,7 @@ class KVCacheInferenceMixin:
         already have tokens in the cache (``position_ids`` do not start at 0); only families whose prefill reads the
         cache accept it."""
         assert self.kv_cache is not None, "call init_kv_cache() first"
+        self.check_steps()
         B, T = input_ids.shape
         prefill = T > 1
         # the int32 position / cache-line copies are shared by the layers of ONE forward only: a captured graph is
@@ -567,6 +592,7 @@ class KVCacheInferenceMixin:
             L = int(lens[b])
             res[b, :L] = input_ids[b, :L]
             res[b, L:L + gen.shape[1]] = gen[b]
+        self.check_steps()                   # reading the lengths has waited for all of them
         return res
 
 

@@ -179,6 +179,9 @@ class NxDModel(torch.nn.Module):
 
     def forward(self, *args: torch.Tensor):
         _, bucket = self.router(args)
+        for m in self.models.values():      # a replay asks nobody whether the steps before it went well
+            if hasattr(m, "check_steps"):
+                m.check_steps()
         return bucket(*args)
 
     def initialize_spmd_models(self, states=None, weights: Optional[Dict[str, torch.Tensor]] = None) -> None:

@@ -153,6 +153,14 @@ class InferenceRunner:
         for line in range(n_lines):
             cache.reserve(line, min(n_tokens, self.config.seq_len))
 
+    def _check_steps(self, wait: bool = True) -> None:
+        """Raises if a step gave up (``KVCacheInferenceMixin.check_steps``); ``wait``: also one that has not ended yet."""
+        check = getattr(self.model, "check_steps", None)
+        if check is not None:
+            if wait and self.device.type == "cuda":
+                torch.cuda.current_stream(self.device).synchronize()
+            check()
+
     def _bucket_len(self, n: int) -> int:
         if self.nxd_model is not None:
             hit = self.nxd_model.route_padded(CONTEXT_ENCODING_MODEL, self.config.ctx_batch_size, n)
@@ -211,12 +219,14 @@ class InferenceRunner:
                 tkg.hook()
             cur = cur + 1
             outs.append(tok[:B])
+            self._check_steps(wait=False)
         gen = torch.stack(outs, dim=1)
         res = torch.full((B, T + gen.shape[1]), ic.pad_token_id, dtype=torch.long, device=dev)
         for b in range(B):
             L = int(lens[b])
             res[b, :L] = input_ids[b, :L]
             res[b, L:L + gen.shape[1]] = gen[b]
+        self._check_steps()
         return res
 
     @torch.no_grad()
@@ -253,6 +263,8 @@ class InferenceRunner:
 
         spec = NeuronSpeculation(draft_step, target_verify, ic.speculation_length)
         new = spec.generate(first[:1], torch.tensor([T], device=dev), max_new - 1, eos_token_id=ic.eos_token_id)
+        for r in (draft, self):
+            r._check_steps()
         self.last_acceptance = list(spec.accepted_hist)
         return torch.cat([input_ids.to(dev)[0], first[:1], new]).unsqueeze(0)
 

@@ -154,11 +154,11 @@ def token_stack_scratch(layers: int, B: int, H: int, I: int, n_q: int, n_kv: int
 def token_stack(x: torch.Tensor, layers: Sequence[Tuple[Sequence[torch.Tensor], float, float]], cos: torch.Tensor, sin: torch.Tensor,
                 positions: torch.Tensor, lengths: torch.Tensor, n_q: int, n_kv: int, D: int, scratch: int,
                 seq_ids: Optional[torch.Tensor] = None, block_table: Optional[torch.Tensor] = None, page_size: int = 0,
-                wait_clocks: int = -1) -> torch.Tensor:
+                wait_clocks: int = -1, gave_up: Optional["GaveUp"] = None) -> torch.Tensor:
     """A token-generation step ``x [1, H]`` through whole decoder layers in one launch -> ``[1, H]`` (``nxd_token_stack``).  A layer is
     ``((input norm, q|k|v, o, norm behind the attention, gate|up, down, cache of keys, of values), eps, eps)``; the caches are written
     at ``positions``.  ``scratch``: bytes, of ``token_stack_scratch``.  ``wait_clocks``: clocks after which a wait inside gives up, -1:
-    two seconds (``token_stack_gave_up``)."""
+    two seconds (``gave_up`` and ``token_stack_gave_up`` say so then)."""
     H = x.shape[1]
     tensors = [t for layer in layers for t in layer[0]]
     ck = layers[0][0][6]
@@ -169,14 +169,35 @@ def token_stack(x: torch.Tensor, layers: Sequence[Tuple[Sequence[torch.Tensor], 
     work = torch.empty(scratch, dtype=torch.uint8, device=x.device)
     pointers = (_c.c_void_p * len(tensors))(*(t.data_ptr() for t in tensors))
     eps = (_c.c_float * (2 * len(layers)))(*(e for layer in layers for e in layer[1:]))
-    rc = _lib.lib().nxd_token_stack(
+    rc = _lib.lib().nxd_token_stack_telling(
         _lib.ptr(x), _lib.ptr(out), pointers, eps, _c.c_int(len(layers)), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(positions),
         _lib.ptr(lengths), _lib.ptr(seq_ids), _lib.ptr(block_table), _c.c_longlong(ck.stride(0)), _c.c_longlong(ck.stride(1)),
         _c.c_int(page_size), _c.c_int(block_table.shape[1] if block_table is not None else 0), _lib.ptr(work), _c.c_int(H),
         _c.c_int(layers[0][0][5].shape[1]), _c.c_int(n_q), _c.c_int(n_kv), _c.c_int(D), _c.c_float(D ** -0.5),
-        _c.c_longlong(wait_clocks), _lib.stream_ptr())
-    _lib.check(rc, "nxd_token_stack")
+        _c.c_longlong(wait_clocks), _lib.ptr(gave_up.word) if gave_up is not None else None, _lib.stream_ptr())
+    _lib.check(rc, "nxd_token_stack_telling")
     return out
+
+
+class GaveUp:
+    """A word of pinned host memory that a ``token_stack`` whose waits gave up sets: read without a copy, of use once the step has ended."""
+
+    def __init__(self):
+        self.word = torch.zeros(1, dtype=torch.int32, pin_memory=torch.cuda.is_available())
+        self._view = self.word.numpy()
+
+    def take(self) -> bool:
+        """Whether it was set since the last call."""
+        told = bool(self._view[0])
+        if told:
+            self._view[0] = 0
+        return told
+
+    def __deepcopy__(self, memo):
+        return GaveUp()
+
+    def __reduce__(self):
+        return GaveUp, ()
 
 
 def token_stack_gave_up() -> bool:

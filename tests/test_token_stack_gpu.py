@@ -1,4 +1,6 @@
 """All decoder layers of a one-sequence step in one launch, against the layers kernel by kernel and against float64."""
+import copy
+
 import pytest
 import torch
 
@@ -176,3 +178,56 @@ def test_waits_give_up():
             assert gave_up and out.isnan().all()
         if clocks == -1:
             assert not gave_up
+
+
+def _model(cls=None, lines=1, **cache):
+    """Two layers of the 2048-wide model with a small vocabulary."""
+    from neuronx_distributed_llama3_2_b200.inference import InferenceConfig, LlamaInferenceModel
+    from neuronx_distributed_llama3_2_b200.models import LlamaConfig
+
+    H, I, nq, nkv, D = SIZES["64"]
+    torch.manual_seed(11)
+    cfg = LlamaConfig(vocab_size=512, hidden_size=H, intermediate_size=I, num_hidden_layers=2, num_attention_heads=nq, num_key_value_heads=nkv)
+    model = (cls or LlamaInferenceModel)(cfg, InferenceConfig(batch_size=lines, max_context_length=64, seq_len=256, **cache),
+                                         device=torch.device("cuda"))
+    model.init_kv_cache(device=torch.device("cuda"))
+    return model
+
+
+def test_a_step_that_gave_up_reaches_the_program():
+    from neuronx_distributed_llama3_2_b200.inference.model_builder import BaseModelInstance, ModelBuilder
+
+    model = _model()
+    ids = torch.randint(1, 512, (1, 20), device="cuda")
+    good = model.generate(ids, max_new_tokens=6)
+    tok, pos = ids[:, :1], torch.full((1, 1), 20, device="cuda")
+    model._token_stack_clocks = 0                        # every wait gives up at once
+    model.forward_infer(tok, pos)
+    torch.cuda.synchronize()
+    model._token_stack_clocks = -1
+    with pytest.raises(RuntimeError, match="gave up"):
+        model.forward_infer(tok, pos)
+    model.forward_infer(tok, pos)                        # told once
+    model._token_stack_clocks = 0
+    with pytest.raises(RuntimeError, match="gave up"):
+        model.generate(ids, max_new_tokens=2)
+    model._token_stack_clocks = -1
+    assert torch.equal(model.generate(ids, max_new_tokens=6), good)
+    model.check_steps()
+    copy.deepcopy(model).check_steps()
+    graph = torch.cuda.CUDAGraph()                       # a replay asks nobody: the word is there behind it
+    model._token_stack_clocks = 0
+    with torch.cuda.graph(graph):
+        model.forward_infer(tok, pos)
+    model.check_steps()
+    graph.replay()
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="gave up"):
+        model.check_steps()
+    model._token_stack_clocks = -1
+    traced = ModelBuilder().add("token", BaseModelInstance(lambda: model), [(tok, pos)]).trace(initialize_model_weights=False)
+    traced(tok, pos)
+    model._gave_up.word.fill_(1)
+    with pytest.raises(RuntimeError, match="gave up"):
+        traced(tok, pos)
+    traced(tok, pos)
