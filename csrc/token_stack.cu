@@ -23,6 +23,8 @@
 //
 // Waits end: one that has taken `limit` clocks gives up, the CTA sends nothing more and leaves NaN in its part of the result, so all
 // others give up too; the caller's word, which may be pinned host memory, and nxd_token_stack_status say so.
+#include <cudaTypedefs.h>
+
 #include <type_traits>
 
 #include "attn_tc_common.cuh"
@@ -682,6 +684,30 @@ NXD_API long long nxd_token_stack_scratch(int layers, int B, int H, int I, int n
         kWarps * (n_q / n_kv) * (D + 4) * 4 > kPartBytes)
         return 0;
     return scratch_of(H, I, n_q, n_kv, D).words * (long long)sizeof(word);
+}
+
+// Whether a CTA on every SM of the device can be resident on that stream: not if it belongs to a green context of fewer SMs, where such a
+// cooperative launch fails (and a chain of kernels runs).
+NXD_API int nxd_token_stack_runs_on(void* stream) {
+    static PFN_cuStreamGetCtx_v12050 get_ctx = nullptr;
+    static PFN_cuGreenCtxGetDevResource_v12040 get_resource = nullptr;
+    if (get_ctx == nullptr || get_resource == nullptr) {
+        void *a = nullptr, *b = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuStreamGetCtx", &a, 12050, cudaEnableDefault, &q) != cudaSuccess || a == nullptr ||
+            cudaGetDriverEntryPointByVersion("cuGreenCtxGetDevResource", &b, 12040, cudaEnableDefault, &q) != cudaSuccess || b == nullptr) {
+            cudaGetLastError();
+            return 1;                    // a driver without green contexts
+        }
+        get_ctx = reinterpret_cast<PFN_cuStreamGetCtx_v12050>(a);
+        get_resource = reinterpret_cast<PFN_cuGreenCtxGetDevResource_v12040>(b);
+    }
+    const int sms = nxd_num_sms();       // a runtime call: the driver's need a context
+    CUcontext ctx = nullptr;
+    CUgreenCtx green = nullptr;
+    CUdevResource r;
+    if (get_ctx((CUstream)stream, &ctx, &green) != CUDA_SUCCESS || green == nullptr) return 1;
+    return get_resource(green, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS && (int)r.sm.smCount >= sms;
 }
 
 // hidden, out [H] bf16; pointers: per layer the weights input norm [H], q | k | v [(n_q + 2 n_kv) D, H], o [H, H], norm behind the

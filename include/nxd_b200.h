@@ -110,6 +110,7 @@ int nxd_kv_cache_update(const void* new_k, const void* new_v, void* cache_k, voi
                         int page_size, int max_pages, int B, int n_kv, int T_new, int D, void* stream);
 
 /* all decoder layers of a token step of one sequence in one launch (csrc/token_stack.cu); bytes of scratch, 0: does not apply */
+int nxd_token_stack_runs_on(void* stream);        /* 0: the stream has not all SMs of the device, as the launch needs */
 long long nxd_token_stack_scratch(int layers, int B, int H, int I, int n_q, int n_kv, int D);
 int nxd_token_stack(const void* hidden, void* out, const void* const* pointers, const float* eps, int layers, const float* cos_t,
                     const float* sin_t, const int* positions, const int* lengths, const int* seq_ids, const int* block_table,

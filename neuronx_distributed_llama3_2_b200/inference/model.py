@@ -327,7 +327,7 @@ class KVCacheInferenceMixin:
         if kc.layer(0)[0].stride(0) % 8 or kc.layer(0)[0].stride(1) % 8:
             return None
         gave_up = self._steps_gave_up()
-        if gave_up is None:
+        if gave_up is None or not decode_fused.token_stack_runs_here():
             return None
         pos, sid = self._decode_i32(positions, seq_ids)
         cos, sin = self._rope(hidden.device)

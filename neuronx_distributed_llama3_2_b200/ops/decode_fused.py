@@ -151,6 +151,11 @@ def token_stack_scratch(layers: int, B: int, H: int, I: int, n_q: int, n_kv: int
     return int(fn(*(_c.c_int(v) for v in (layers, B, H, I, n_q, n_kv, D))))
 
 
+def token_stack_runs_here() -> bool:
+    """Whether the current stream has all SMs of the device, as ``token_stack`` needs (one of a green context has not)."""
+    return bool(_lib.lib().nxd_token_stack_runs_on(_lib.stream_ptr()))
+
+
 def token_stack(x: torch.Tensor, layers: Sequence[Tuple[Sequence[torch.Tensor], float, float]], cos: torch.Tensor, sin: torch.Tensor,
                 positions: torch.Tensor, lengths: torch.Tensor, n_q: int, n_kv: int, D: int, scratch: int,
                 seq_ids: Optional[torch.Tensor] = None, block_table: Optional[torch.Tensor] = None, page_size: int = 0,

@@ -231,3 +231,28 @@ def test_a_step_that_gave_up_reaches_the_program():
     with pytest.raises(RuntimeError, match="gave up"):
         traced(tok, pos)
     traced(tok, pos)
+
+
+def test_a_stream_of_fewer_multiprocessors_takes_the_layers_one_by_one():
+    """One launch needs every SM of the device at once; in a green context of half of them the chain of kernels runs, as it always did."""
+    from torch.cuda.green_contexts import SUPPORTED, GreenContext
+
+    if not SUPPORTED:
+        pytest.skip("this torch has no green contexts")
+    from neuronx_distributed_llama3_2_b200.ops import decode_fused as df
+
+    model = _model()
+    tok, pos = torch.full((1, 1), 5, device="cuda"), torch.zeros((1, 1), dtype=torch.long, device="cuda")
+    assert df.token_stack_runs_here()
+    stacked = model.forward_infer(tok, pos, return_logits=True)[1]
+    torch.cuda.synchronize()
+    some = GreenContext.create(64, 0)
+    some.set_context()
+    try:
+        here = df.token_stack_runs_here()
+        chain = model.forward_infer(tok, pos, return_logits=True)[1]
+        torch.cuda.synchronize()
+    finally:
+        some.pop_context()
+    assert not here
+    assert (stacked - chain).float().norm() <= 4e-2 * chain.float().norm()       # two layers, rounded to bf16 at the same places
