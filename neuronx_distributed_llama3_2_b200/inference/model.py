@@ -299,10 +299,11 @@ class KVCacheInferenceMixin:
         weights."""
         from ..ops import decode_fused
 
-        layers, base, cls = list(self._decoder_layers()), KVCacheInferenceMixin, type(self)
+        layers, base = list(self._decoder_layers()), KVCacheInferenceMixin
         if (hidden.shape[0] != 1 or residual is not None or not layers or not hidden.is_cuda
                 or hidden.dtype != torch.bfloat16 or not hidden.is_contiguous() or ps.get_tensor_model_parallel_size() > 1
-                or any(getattr(cls, n) is not getattr(base, n) for n in ("_layer", "_layer_batched_decode", "_decode_attention", "_rope"))
+                or any(getattr(getattr(self, n), "__func__", None) is not getattr(base, n)           # a subclass's or the object's own
+                       for n in ("_layer", "_layer_batched_decode", "_decode_attention", "_rope"))
                 or os.environ.get("NXD_DECODE_ATTN", "")[:1] == "f"):
             return None
         B, H = hidden.shape[0], hidden.shape[-1]

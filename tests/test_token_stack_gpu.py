@@ -256,3 +256,29 @@ def test_a_stream_of_fewer_multiprocessors_takes_the_layers_one_by_one():
         some.pop_context()
     assert not here
     assert (stacked - chain).float().norm() <= 4e-2 * chain.float().norm()       # two layers, rounded to bf16 at the same places
+
+
+def _counted(model, monkeypatch):
+    """How often the model's layers ran in one launch."""
+    from neuronx_distributed_llama3_2_b200.ops import decode_fused as df
+
+    calls, real = [], df.token_stack
+    monkeypatch.setattr(df, "token_stack", lambda *a, **k: calls.append(1) or real(*a, **k))
+    return calls
+
+
+def test_what_a_program_puts_in_the_place_of_a_step_is_called(monkeypatch):
+    from neuronx_distributed_llama3_2_b200.inference import LlamaInferenceModel
+
+    class Own(LlamaInferenceModel):
+        def _decode_attention(self, q, ck, cv, seq_ids, lengths):
+            return torch.zeros_like(q)
+
+    tok, pos = torch.full((1, 1), 5, device="cuda"), torch.zeros((1, 1), dtype=torch.long, device="cuda")
+    own = _model(Own).forward_infer(tok, pos, return_logits=True)[1]
+    model = _model()
+    calls = _counted(model, monkeypatch)
+    model._decode_attention = lambda q, ck, cv, seq_ids, lengths: torch.zeros_like(q)
+    assert torch.equal(model.forward_infer(tok, pos, return_logits=True)[1], own) and not calls
+    del model._decode_attention
+    assert not torch.equal(model.forward_infer(tok, pos, return_logits=True)[1], own) and len(calls) == 1
