@@ -282,3 +282,51 @@ def test_what_a_program_puts_in_the_place_of_a_step_is_called(monkeypatch):
     assert torch.equal(model.forward_infer(tok, pos, return_logits=True)[1], own) and not calls
     del model._decode_attention
     assert not torch.equal(model.forward_infer(tok, pos, return_logits=True)[1], own) and len(calls) == 1
+
+
+@pytest.mark.parametrize("kind", ["contiguous", "paged", "lines", "paged lines"])
+def test_the_model_takes_it(kind, monkeypatch):
+    """Order and shape of the weights, cache lines and pages: against the same model's layers kernel by kernel."""
+    model = _model(lines=3, paged_kv="paged" in kind, page_size=16, is_continuous_batching="lines" in kind)
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    ids = torch.randint(1, 512, (3, 40), generator=gen, device="cuda")
+    pos = torch.arange(40, device="cuda").unsqueeze(0).expand(3, 40)
+    lines = torch.arange(3, dtype=torch.int32, device="cuda")
+    model.forward_infer(ids, pos, seq_ids=lines)
+    saved = [t.clone() for t in model.kv_cache.k + model.kv_cache.v]
+    line = lines[2:] if "lines" in kind else None
+    step = (ids[:1, :1], torch.full((1, 1), 40, device="cuda"), line)
+    calls = _counted(model, monkeypatch)
+    stacked = model.forward_infer(*step, return_logits=True)[1]
+    assert len(calls) == 1
+    mine = [t.clone() for t in model.kv_cache.k + model.kv_cache.v]
+    for t, was in zip(model.kv_cache.k + model.kv_cache.v, saved):
+        t.copy_(was)
+    with monkeypatch.context() as m:
+        m.setattr(model, "_token_stack", lambda *_: None)
+        chain = model.forward_infer(*step, return_logits=True)[1]
+    assert len(calls) == 1
+    # two layers, every value rounded to bf16 at the same places: 2^-8 of a vector each, some ten of them on the way
+    assert (stacked - chain).float().norm() <= 4e-2 * chain.float().norm()
+    for a, b, was in zip(mine, model.kv_cache.k + model.kv_cache.v, saved):
+        changed = (b != was).any(-1)                     # one row per key head, of that line
+        assert torch.equal((a != was).any(-1), changed) and changed.sum() == 8
+        assert (a[changed].float() - b[changed].float()).norm() <= 2e-2 * b[changed].float().norm()
+    other = lines[:1] if "lines" in kind else None
+    if other is not None:                                # another line, another context
+        assert not torch.equal(model.forward_infer(step[0], step[1], other, return_logits=True)[1], stacked)
+
+
+def test_the_model_leaves_other_steps_alone(monkeypatch):
+    model = _model(lines=2)
+    calls = _counted(model, monkeypatch)
+    two = torch.full((2, 1), 5, device="cuda"), torch.zeros((2, 1), dtype=torch.long, device="cuda")
+    one = two[0][:1], two[1][:1]
+    model.forward_infer(*two)                                                  # two sequences
+    model.forward_infer(torch.full((1, 4), 5, device="cuda"), torch.arange(4, device="cuda").unsqueeze(0))      # a prompt
+    assert not calls
+    model.forward_infer(*one)
+    assert len(calls) == 1
+    norm = model.model.layers[1].post_attention_layernorm
+    norm.weight.data = norm.weight.data.float()                                # a norm that is kept in fp32
+    assert torch.isfinite(model.forward_infer(*one, return_logits=True)[1]).all() and len(calls) == 1
