@@ -15,10 +15,11 @@
 // step (fp32 multiply-adds keep up with the stream; tensor cores would want 16 sequences) and no warp waits for another before the
 // step's sums.
 //
-// A token through 16 layers of 2048, 2048 tokens in the cache, and the head: 675 us as a chain of kernels, 600 here; 4 layers of 3072: 347,
-// 325.  A layer takes 59 thousand clocks, its weights 36 of them.  What is left are the six times that every CTA waits for the slowest one
-// (4000 clocks each under load), and instructions: every step's code is fetched once a layer, so it is kept short (loops unrolled further
-// and a copy of the products per step: 623).  Copies in flight: 64 KB a CTA; with 32 the stream is slower (649 against 584 at that time),
+// A token through 16 layers of 2048, 2048 tokens in the cache, and the head: 675 us as a chain of kernels, 578 here.  Four layers and no head,
+// 200 / 2048 / 16384 / 131072 tokens: 2048 wide 160 / 164 / 194 / 336 as a chain, 133 / 139 / 164 / 316 here; 3072 wide 223 / 229 / 273 /
+// 553 and 196 / 200 / 239 / 521.  A layer takes some 56 thousand clocks, its weights 36 of them.  What is left are the six times that every
+// CTA waits for the slowest one (4000 clocks each under load), and instructions: every step's code is fetched once a layer, so it is kept
+// short (loops unrolled further and a copy of the products per step: 623 us against 600 at that time).  Copies in flight: 64 KB a CTA; with 32 the stream is slower (649 against 584 at that time),
 // with 192 everything else waits behind them (743 against 702).
 //
 // Waits end: one that has taken `limit` clocks gives up, the CTA sends nothing more and leaves NaN in its part of the result, so all
@@ -29,6 +30,7 @@
 
 #include "attn_tc_common.cuh"
 #include "decode_common.cuh"
+#include "mma_sync.cuh"
 #include "ptx.cuh"
 
 namespace {
@@ -40,7 +42,11 @@ constexpr int kWarps = 8, kThreads = (kWarps + 1) * 32;
 constexpr int kRingBytes = 196608, kPartBytes = 28672;   // the weights; the phase's sums or the warps' attention states
 constexpr int kSmem = kRingBytes + kPartBytes;
 constexpr int kFlightBytes = 65536;                      // of a CTA's copies in flight
-constexpr int kMaxLayers = 64, kMaxParts = 16, kPartKeys = 256;
+constexpr int kMaxLayers = 64, kPartKeys = 256;
+// Parts of a head's keys.  With 18 nearly all CTAs attend, with 16 the others' weights keep the stream going: 4 layers of 2048 / 3072, 8000
+// tokens 154 us with 16 and 161 with 18 / 219 and 226, 32768 190 and 192 / 281 and 285, 65536 235 and 233 / 364 and 366, 131072 330 and 316 /
+// 526 and 521.
+constexpr int kFewParts = 16, kMaxParts = 18, kManyKeys = 65536;
 constexpr long long kWaitClocks = 4000000000ll;          // two seconds
 
 struct Layer {
@@ -132,6 +138,12 @@ __device__ __forceinline__ void widen(uint2 w, uint64_t (&f)[2]) {
 }
 __device__ __forceinline__ float rounded(float v) { return __bfloat162float(__float2bfloat16(v)); }
 
+__device__ __forceinline__ float largest(float v) {      // of a warp; sm_100a
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 // R sums over the lanes at once: the lanes with the same lane / (32 / R) end with that sum
 template <int R>
 __device__ __forceinline__ float sum_rows(float (&a)[R]) {
@@ -209,7 +221,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_stack_kernel(const __grid_c
 
     // attention: parts of kPartKeys keys, one for a CTA at most
     const int length = p.lengths[0], position = p.positions[0];
-    const int parts = max(1, min(min((length + kPartKeys - 1) / kPartKeys, kMaxParts), ctas / p.n_kv));
+    const int parts = max(1, min(min((length + kPartKeys - 1) / kPartKeys, length > kManyKeys ? kMaxParts : kFewParts), ctas / p.n_kv));
     const bool attends = cta < p.n_kv * parts;
     const int kv_head = cta / parts, my_part = cta % parts;
     const int keys_per = ((length + parts - 1) / parts + 127) / 128 * 128, key0 = my_part * keys_per;
@@ -372,110 +384,141 @@ __global__ void __launch_bounds__(kThreads, 1) token_stack_kernel(const __grid_c
         for (int step = 0; step < 3; ++step) {
             uint64_t x[NVH][2];
             if (step == 1) {
-                // attention: eight lanes a key row, four keys a warp and load.  Keys and values come through the ring, ahead of the activations; only
-                // the step's own row had not been written then.  Four warps take 128 keys and the other four the next 128, a warp a quarter of a
-                // slot at a time: the tiles, and so the weights that are rounded to bf16 beside their tiles' largest ones, are those of
-                // decode_attn_mma_kernel.
+                // attention.  Keys and values come through the ring, ahead of the activations; only the step's own row had not been written
+                // then, and goes into its slot here.  Four warps take 128 keys and the other four the next 128, a warp a quarter of a slot at
+                // a time: the tiles, and so the weights that are rounded to bf16 beside their tiles' largest ones, are those of
+                // decode_attn_mma_kernel.  Scores on mma.sync, keys as its 16 rows and the group's query heads as its 8 columns; its 16 terms
+                // are taken from the row in an order in which every lane loads 16 bytes at once.  Values by multiply-adds of pairs, eight
+                // lanes a row (as mma.sync operands they would have to be transposed, eight rows of one bank at a time).  A slot then takes
+                // less than the memory does: with the scores by multiply-adds and shuffles too, 2600 clocks against 1200, and beyond 20000
+                // tokens the chain of kernels was faster (figures above; 131072 tokens 498 and 731 us).
                 if (attends) {
-                    constexpr int kE = D / 8, kV = kE / 8, kTile = kKeys / 4, kUnroll = kTile / 4;
-                    const int sub = lane >> 3, l8 = lane & 7, own = position - key0;
-                    float qf[G][kE], m[G], sum[G], o[G][kE];
+                    constexpr int kE = D / 8, kV = kE / 8, kTile = kKeys / 4, kHalf = D / 2, kWords = 4 * kV;
+                    static_assert(G <= 4 && kTile % 16 == 0 && kTile <= 32, "a lane for every key of a tile, columns for its heads");
+                    const int sub = lane >> 3, l8 = lane & 7, row = lane >> 2, t4 = lane & 3, own = position - key0;
+                    float m[G], sum[G];
+                    uint64_t o[G][kE / 2];
+                    uint4 qb[D / 32];                            // of query head lane / 4: values 32 i + 8 (lane % 4) and the next seven
                     uint4 own_k[kV], own_v[kV];
                     {
-                        // a word holds the values d and d + D / 2: a lane has the first or the second ones of eight words (D = 64), or both
-                        constexpr int kHalf = D / 2;
-                        const int d0 = D == 64 ? (l8 & 3) * 8 : l8 * 8;
-                        uint2 raw[(G + 2) * 4];
+                        // a word holds the values d and d + D / 2
+                        const int head = kv_head * G + min(row, G - 1), d0 = D == 64 ? (l8 & 3) * 8 : l8 * 8;
+                        uint2 raw[kWords + 8];
                         receive(
                             [&](int j) {
-                                return (j / 4 < G ? p.q + (kv_head * G + j / 4) * kHalf
-                                                    : p.kv + (kv_head * 2 + j / 4 - G) * kHalf) + d0 + j % 4 * 2;
+                                return j < kWords ? p.q + head * kHalf + t4 * 8 + j / 4 * 32 + j % 4 * 2
+                                                  : p.kv + (kv_head * 2 + (j - kWords) / 4) * kHalf + d0 + j % 4 * 2;
                             },
-                            l + 1, raw, p.limit, &dead);
-                        auto half = [&](int row, bool upper) {
+                            number, raw, p.limit, &dead);
+                        auto eight = [&](int first, bool upper) {
                             uint32_t r[4];
-        #pragma unroll
-                            for (int i = 0; i < 4; ++i) r[i] = __byte_perm(raw[row * 4 + i].x, raw[row * 4 + i].y, upper ? 0x7632 : 0x5410);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) r[i] = __byte_perm(raw[first + i].x, raw[first + i].y, upper ? 0x7632 : 0x5410);
                             return make_uint4(r[0], r[1], r[2], r[3]);
                         };
-        #pragma unroll
+#pragma unroll
+                        for (int i = 0; i < D / 32; ++i) {
+                            qb[i] = eight(i % kV * 4, i >= kV);
+                            if (row >= G) qb[i] = make_uint4(0, 0, 0, 0);
+                        }
+#pragma unroll
                         for (int v = 0; v < kV; ++v) {
                             const bool upper = D == 64 ? l8 >= 4 : v == 1;
-                            own_k[v] = half(G, upper);
-                            own_v[v] = half(G + 1, upper);
-        #pragma unroll
-                            for (int g = 0; g < G; ++g) {
-                                const uint4 t = half(g, upper);
-                                unpack8(*reinterpret_cast<const bf16x8*>(&t), qf[g] + v * 8);
-                            }
+                            own_k[v] = eight(kWords, upper);
+                            own_v[v] = eight(kWords + 4, upper);
                         }
                     }
-        #pragma unroll
+#pragma unroll
                     for (int g = 0; g < G; ++g) {
                         m[g] = -INFINITY, sum[g] = 0.f;
-        #pragma unroll
-                        for (int e = 0; e < kE; ++e) qf[g][e] *= p.scale_log2, o[g][e] = 0.f;
+#pragma unroll
+                        for (int e = 0; e < kE / 2; ++e) o[g][e] = 0;
                     }
+                    // the tile's scores, then its weights, each twice: what a multiply-add of a pair takes
+                    float* const scores = part + 4096 + warp * 256;
+                    ulonglong2* const weights = reinterpret_cast<ulonglong2*>(scores);
                     for (int kb = 0; kb < keys; kb += kKeys) {
                         const bool ours = kb / 128 % 2 == warp / 4;
                         // the warps that skip a slot wait for it as well: `empty` counts arrivals, not warps, and one that is ahead by a round of
                         // the ring would arrive a second time in the place of one that still reads
                         if (!__all_sync(0xffffffffu, wait(&full[st], ph, p.limit, &dead))) break;
-                        const uint8_t* slot = smem + st * kSlotBytes;
-                        // keys first, then values: both in registers at once would not fit beside the states
-                        auto fetch = [&](int u, int half, const uint4 (&own_row)[kV], float (&f)[kE]) {
-                            const int i = warp % 4 * kTile + u * 4 + sub;
-        #pragma unroll
-                            for (int v = 0; v < kV; ++v) {
-                                const uint4 raw = kb + i == own ? own_row[v]
-                                                                : *reinterpret_cast<const uint4*>(slot + (half * kKeys + i) * D * 2 + (l8 + v * 8) * 16);
-                                unpack8(*reinterpret_cast<const bf16x8*>(&raw), f + v * 8);
-                            }
-                        };
+                        const int first = warp % 4 * kTile;                  // of the slot's keys
+                        uint8_t* const kt = smem + st * kSlotBytes + first * D * 2;
+                        const uint8_t* const vt = kt + kKeys * D * 2;
                         if (ours) {
-                            float sc[G];                         // the lane's score: key u of its group of lanes belongs to lane u
+                            if (own >= kb + first && own < kb + first + kTile) {
+                                if (sub == 0) {
 #pragma unroll
-                            for (int g = 0; g < G; ++g) sc[g] = -INFINITY;
-#pragma unroll 2
-                            for (int u = 0; u < kUnroll; ++u) {
-                                float kf[kE];
-                                fetch(u, 0, own_k, kf);
-                                const bool mine = u == l8 && kb + warp % 4 * kTile + u * 4 + sub < keys;
+                                    for (int v = 0; v < kV; ++v) {
+                                        const int at = (own - kb - first) * D * 2 + (l8 + v * 8) * 16;
+                                        *reinterpret_cast<uint4*>(kt + at) = own_k[v];
+                                        *reinterpret_cast<uint4*>(kt + kKeys * D * 2 + at) = own_v[v];
+                                    }
+                                }
+                                ptx::fence_proxy_async();                    // the slot's next copy comes behind these stores
+                                __syncwarp();
+                            }
 #pragma unroll
-                                for (int g = 0; g < G; ++g) {
-                                    float t = 0.f;
+                            for (int r0 = 0; r0 < kTile; r0 += 16) {
+                                float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                                    for (int e = 0; e < kE; ++e) t = fmaf(kf[e], qf[g][e], t);
-                                    t += __shfl_xor_sync(0xffffffffu, t, 1);
-                                    t += __shfl_xor_sync(0xffffffffu, t, 2);
-                                    t += __shfl_xor_sync(0xffffffffu, t, 4);
-                                    if (mine) sc[g] = t;
+                                for (int i = 0; i < D / 32; ++i) {
+                                    const uint4 a = *reinterpret_cast<const uint4*>(kt + (r0 + row) * D * 2 + (t4 + 4 * i) * 16);
+                                    const uint4 b = *reinterpret_cast<const uint4*>(kt + (r0 + row + 8) * D * 2 + (t4 + 4 * i) * 16);
+                                    const uint32_t lo[4] = {a.x, b.x, a.y, b.y}, hi[4] = {a.z, b.z, a.w, b.w};
+                                    mma::mma16816(c, lo, qb[i].x, qb[i].y);
+                                    mma::mma16816(c, hi, qb[i].z, qb[i].w);
+                                }
+                                if (t4 < 2) {
+                                    *reinterpret_cast<float2*>(scores + (r0 + row) * 4 + 2 * t4) = make_float2(c[0], c[1]);
+                                    *reinterpret_cast<float2*>(scores + (r0 + row + 8) * 4 + 2 * t4) = make_float2(c[2], c[3]);
                                 }
                             }
+                            __syncwarp();
+                            float sc[4];                                     // the scores of the lane's key
+                            *reinterpret_cast<float4*>(sc) = *reinterpret_cast<const float4*>(scores + lane % kTile * 4);
+                            __syncwarp();
+                            const bool mine = lane < kTile && kb + first + lane < keys;
 #pragma unroll
                             for (int g = 0; g < G; ++g) {
-                                const float top = fmaxf(m[g], warp_max(sc[g])), use = top == -INFINITY ? 0.f : top, fade = exp2f(m[g] - use);
+                                const float t = mine ? sc[g] * p.scale_log2 : -INFINITY;
+                                const float top = fmaxf(m[g], largest(t)), use = top == -INFINITY ? 0.f : top, fade = exp2f(m[g] - use);
                                 m[g] = top;
-                                const float exact = exp2f(sc[g] - use);
+                                const float exact = exp2f(t - use);
                                 sum[g] = fmaf(sum[g], fade, exact);
                                 sc[g] = rounded(exact);
+                                const uint64_t fades = f2_pack(fade, fade);
 #pragma unroll
-                                for (int e = 0; e < kE; ++e) o[g][e] *= fade;
+                                for (int e = 0; e < kE / 2; ++e) o[g][e] = f2_mul(o[g][e], fades);
                             }
-#pragma unroll 2
-                            for (int u = 0; u < kUnroll; ++u) {
-                                float vf[kE];
-                                fetch(u, 1, own_v, vf);
-                                const bool real = kb + warp % 4 * kTile + u * 4 + sub < keys;       // what lies behind the last key may be anything
+                            if (lane < kTile) {
+                                weights[lane * 2] = make_ulonglong2(f2_pack(sc[0], sc[0]), f2_pack(sc[1], sc[1]));
+                                weights[lane * 2 + 1] = make_ulonglong2(f2_pack(sc[2], sc[2]), f2_pack(sc[3], sc[3]));
+                            }
+                            __syncwarp();
+                            const bool whole = kb + first + kTile <= keys;
+#pragma unroll(D == 64 ? 4 : 1)
+                            for (int u = 0; u < kTile; u += 4) {
+                                uint64_t v[kE / 2];
 #pragma unroll
-                                for (int e = 0; e < kE; ++e)
-                                    if (!real) vf[e] = 0.f;
-#pragma unroll
-                                for (int g = 0; g < G; ++g) {
-                                    const float pw = __shfl_sync(0xffffffffu, sc[g], (lane & 24) + u);
-#pragma unroll
-                                    for (int e = 0; e < kE; ++e) o[g][e] = fmaf(pw, vf[e], o[g][e]);
+                                for (int i = 0; i < kV; ++i) {
+                                    const uint4 raw = *reinterpret_cast<const uint4*>(vt + (u + sub) * D * 2 + (l8 + i * 8) * 16);
+                                    uint64_t f[2];
+                                    widen(make_uint2(raw.x, raw.y), f);
+                                    v[i * 4] = f[0], v[i * 4 + 1] = f[1];
+                                    widen(make_uint2(raw.z, raw.w), f);
+                                    v[i * 4 + 2] = f[0], v[i * 4 + 3] = f[1];
                                 }
+                                if (!whole && kb + first + u + sub >= keys) {                // what lies behind the last key may be anything
+#pragma unroll
+                                    for (int e = 0; e < kE / 2; ++e) v[e] = 0;
+                                }
+                                const ulonglong2 w01 = weights[(u + sub) * 2], w23 = weights[(u + sub) * 2 + 1];
+                                const uint64_t w[4] = {w01.x, w01.y, w23.x, w23.y};
+#pragma unroll
+                                for (int g = 0; g < G; ++g)
+#pragma unroll
+                                    for (int e = 0; e < kE / 2; ++e) o[g][e] = f2_fma(w[g], v[e], o[g][e]);
                             }
                         }
                         __syncwarp();
@@ -489,7 +532,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_stack_kernel(const __grid_c
                         float* dst = part + (warp * G + g) * kRow;
         #pragma unroll
                         for (int e = 0; e < kE; ++e) {
-                            float y = o[g][e];
+                            float y = e % 2 == 0 ? f2_lo(o[g][e / 2]) : f2_hi(o[g][e / 2]);
                             y += __shfl_xor_sync(0xffffffffu, y, 8);
                             y += __shfl_xor_sync(0xffffffffu, y, 16);
                             if (sub == 0) dst[(e / 8) * 64 + l8 * 8 + e % 8] = y;

@@ -77,9 +77,10 @@ def _stack(x, layers, size, cos, sin, pos, lens, **place):
 
 @pytest.mark.parametrize("size", SIZES)
 # the first token, edges of the parts of 256 keys, of the ring's slots of 64 and 128 keys, more keys than 16 parts of 256; pages that end inside a
-# slot and hold whole ones; as many keys that a CTA's share goes through the ring of six slots once (12.5 and 6.5 thousand), three and ten times
+# slot and hold whole ones; as many keys that a CTA's share goes through the ring of six slots once (12.5 and 6.5 thousand), three and ten
+# times, in 16 and 18 parts
 @pytest.mark.parametrize("n,page", [(1, 0), (2, 16), (64, 0), (257, 128), (511, 16), (4500, 128), (6500, 0), (12500, 16), (20000, 128), (40000, 0),
-                                    (65000, 128), (131072, 0)])
+                                    (65536, 128), (65537, 0), (131072, 0)])
 def test_layers_in_one_launch(size, n, page):
     H, I, nq, nkv, D = SIZES[size]
     lines, rows = 2, (n + 127) // 128 * 128
