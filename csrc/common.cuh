@@ -66,7 +66,9 @@ inline cudaError_t nxd_allow_smem(int bytes) {
 // nxd_launch_pdl may START while their predecessor in the stream is still running (as soon as all its CTAs have executed
 // pdl_trigger() or exited); they must call pdl_wait() before they read anything the predecessor wrote and before ANY
 // global write (the predecessor may still be reading a buffer the allocator has handed to this kernel).  Constant data
-// (weights) may be fetched before pdl_wait().  Both instructions are no-ops in a launch without the attribute.
+// (weights) may be fetched before pdl_wait(), if the caller says that no kernel in flight writes them.  A kernel that allocates
+// tensor memory triggers behind its allocation: a dependent may hold columns while it waits.  Both instructions are no-ops in a
+// launch without the attribute.
 // NXD_PDL=0 turns the attribute off.
 int nxd_pdl_enabled();
 

@@ -90,6 +90,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
         ptx::fence_barrier_init();
     }
+    // ahead of the wait: kernels trigger behind their own allocation, so nothing that this grid waits for is short of tensor memory
     if (warp == 2) ptx::tmem_alloc<2>(tmem_ptr_smem, L::kTmemCols);
     ptx::tcgen05_fence_before();
     ptx::cluster_sync();

@@ -58,8 +58,8 @@ __device__ __forceinline__ void ld8(const float* p, float* f) {
 }
 __device__ __forceinline__ void ld8(const bf16* p, float* f) { unpack8(*reinterpret_cast<const bf16x8*>(p), f); }
 
-// acc[t][i] += <h row t, wr row i> over the columns of this lane in every `parts`-th piece of 32 V from piece `part` on.  V = 8: 16- / 32-byte loads (W a multiple of 8, aligned
-// rows); V = 1: any W.  Rows past nt / nr repeat the last one (their sums are not used).
+// acc[t][i] += <h row t, wr row i> over the columns of this lane in every `parts`-th piece of 32 V from piece `part` on.  V = 8: 16- /
+// 32-byte loads (W a multiple of 8, aligned rows); V = 1: any W.  Rows past nt / nr repeat the last one (their sums are not used).
 template <typename T, int V, int TOK, int G>
 __device__ __forceinline__ void router_dots(const T* h, const float* wr, int W, int nt, int nr, float (&acc)[TOK][G], int part = 0,
                                             int parts = 1) {
@@ -167,10 +167,9 @@ __device__ __forceinline__ void router_select(float* ps, float* cs, const float*
 }
 
 // A CTA of RT_WARPS warps.  SHARE: one token and up to RT_SHARE_WARPS warps, they share its experts and the width (few tokens: the latency of
-// one token counts, a chain of loads along the width: 64 tokens of 1024 x
-// 16 5.6 -> 4.9 us against four warps that share the outputs only, 1024 x 64 14.1 -> 9.1, 2048 x 8 6.9 -> 4.3, 4096 x 8 11.3 -> 5.2).  Else
-// every warp takes TOK tokens and all experts, so a row of wr that is loaded serves TOK tokens (many tokens: the fp32 rows of wr
-// come from L1 / L2 and are the larger operand).
+// one token counts, a chain of loads along the width; 64 tokens against four warps that share the outputs only, 1024 x 16 5.6 -> 4.9 us,
+// 1024 x 64 14.1 -> 9.1, 2048 x 8 6.9 -> 4.3, 4096 x 8 11.3 -> 5.2).  Else every warp takes TOK tokens and all experts, so a row of wr that is
+// loaded serves TOK tokens (many tokens: the fp32 rows of wr come from L1 / L2 and are the larger operand).
 template <typename T, int V, int TOK, bool SHARE>
 __global__ void __launch_bounds__((SHARE ? RT_SHARE_WARPS : RT_WARPS) * 32)
 moe_router_kernel(const T* __restrict__ h, const float* __restrict__ wr, const float* __restrict__ corr,

@@ -120,7 +120,7 @@ retention_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
         ptx::fence_barrier_init();
     }
-    if (warp == 2) ptx::tmem_alloc<2>(tmem_ptr, kAcc * kBN);
+    if (warp == 2) ptx::tmem_alloc<2>(tmem_ptr, kAcc * kBN);        // ahead of the wait, as in gemm_tcgen05.cu
     ptx::tcgen05_fence_before();
     ptx::cluster_sync();
     ptx::tcgen05_fence_after();

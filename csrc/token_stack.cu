@@ -526,11 +526,11 @@ __global__ void __launch_bounds__(kThreads, 1) token_stack_kernel(const __grid_c
                         if (++st == kSlots) st = 0, ph ^= 1;
                     }
                     constexpr int kRow = D + 4;                  // values, maximum, sum
-        #pragma unroll
+#pragma unroll
                     for (int g = 0; g < G; ++g) {
                         const float t = warp_sum(sum[g]);
                         float* dst = part + (warp * G + g) * kRow;
-        #pragma unroll
+#pragma unroll
                         for (int e = 0; e < kE; ++e) {
                             float y = e % 2 == 0 ? f2_lo(o[g][e / 2]) : f2_hi(o[g][e / 2]);
                             y += __shfl_xor_sync(0xffffffffu, y, 8);
@@ -544,9 +544,9 @@ __global__ void __launch_bounds__(kThreads, 1) token_stack_kernel(const __grid_c
                     for (int i = tid; i < G * D && !dead; i += kWarps * 32) {
                         const int g = i / D, d = i - g * D;
                         float top = -INFINITY, t = 0.f, y = 0.f;
-        #pragma unroll
+#pragma unroll
                         for (int x = 0; x < kWarps; ++x) top = fmaxf(top, part[(x * G + g) * kRow + D]);
-        #pragma unroll
+#pragma unroll
                         for (int x = 0; x < kWarps; ++x) {
                             const float* src = part + (x * G + g) * kRow;
                             const float f = src[D] == -INFINITY ? 0.f : exp2f(src[D] - top);
@@ -573,11 +573,11 @@ __global__ void __launch_bounds__(kThreads, 1) token_stack_kernel(const __grid_c
                                 },
                                 number, raw, p.limit, &dead);
                             float now = top;
-        #pragma unroll
+#pragma unroll
                             for (int j = 0; j < 4; ++j) now = fmaxf(now, __uint_as_float(raw[2 * j + 1].x));
                             const float use = now == -INFINITY ? 0.f : now, fade = exp2f(top - use);
                             top = now, t *= fade, y0 *= fade, y1 *= fade;
-        #pragma unroll
+#pragma unroll
                             for (int j = 0; j < 4; ++j) {
                                 const float f = s0 + j < parts ? exp2f(__uint_as_float(raw[2 * j + 1].x) - use) : 0.f;
                                 t = fmaf(__uint_as_float(raw[2 * j + 1].y), f, t);
@@ -626,7 +626,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_stack_kernel(const __grid_c
             } else {
                 if (2 * tid < is && !dead) {
                     float y[2];
-        #pragma unroll
+#pragma unroll
                     for (int j = 0; j < 2; ++j) {
                         const float g = rounded(sum_of(4 * tid + 2 * j)), up = rounded(sum_of(4 * tid + 2 * j + 1));
                         y[j] = g / (1.f + __expf(-g)) * up;
