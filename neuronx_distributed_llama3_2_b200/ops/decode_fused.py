@@ -188,7 +188,7 @@ class GaveUp:
     """A word of pinned host memory that a ``token_stack`` whose waits gave up sets: read without a copy, of use once the step has ended."""
 
     def __init__(self):
-        self.word = torch.zeros(1, dtype=torch.int32, pin_memory=torch.cuda.is_available())
+        self.word = torch.zeros(1, dtype=torch.int32, device="cpu", pin_memory=torch.cuda.is_available())
         self._view = self.word.numpy()
 
     def take(self) -> bool:

@@ -216,6 +216,8 @@ def test_a_step_that_gave_up_reaches_the_program():
     assert torch.equal(model.generate(ids, max_new_tokens=6), good)
     model.check_steps()
     copy.deepcopy(model).check_steps()
+    with torch.device("cuda"):                           # the word is host memory whatever the default device is
+        copy.deepcopy(model).init_kv_cache()
     graph = torch.cuda.CUDAGraph()                       # a replay asks nobody: the word is there behind it
     model._token_stack_clocks = 0
     with torch.cuda.graph(graph):
